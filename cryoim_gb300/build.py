@@ -12,8 +12,8 @@ include/cryoim.h carries no torch types).  Translation units:
 * local.cu -- -fmad=false: local_refine's sub-particle refinement;
 * learn.cu -- the learned orientation proposer (features, CNN forward / backward, Adam);
 * conv_tc.cu -- the proposer's convolutions on the tcgen05 tensor cores (TF32);
-* io.cpp, local_host.cpp -- host only (g++): MRC / orientation / tnf files, local_box
-  geometry and local_refine parameters.
+* io.cpp, local_host.cpp, origin_basis.cpp -- host only (g++): MRC / orientation / tnf
+  files, local_box geometry and local_refine parameters, the origin grid's basis.
 """
 from __future__ import annotations
 
@@ -87,7 +87,7 @@ def build_library(verbose: bool = False, extra: list[str] | None = None) -> str:
     return lib
 
 
-HOST_UNITS = ["io.cpp", "local_host.cpp"]
+HOST_UNITS = ["io.cpp", "local_host.cpp", "origin_basis.cpp"]
 TOOLS = {"icosprocess": "icosprocess.cpp", "proc_icos": "proc_icos.cpp",
          "merge_icosprocess_subrec": "merge_subrec.cpp", "local_box": "local_box.cpp",
          "local_refine": "local_refine.cpp"}

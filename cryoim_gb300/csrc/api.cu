@@ -14,6 +14,7 @@
 #include <cstdio>
 #include <cstring>
 #include <iterator>
+#include <functional>
 #include <map>
 #include <random>
 #include <string>
@@ -23,6 +24,7 @@
 #include "../../include/cryoim.h"
 #include "geom.cuh"
 #include "kernels.h"
+#include "origin_basis.h"
 
 using namespace cryoim;
 
@@ -257,6 +259,16 @@ struct LearnModel {
     }
 };
 
+// An origin grid's basis on the device, rebuilt when the grid, the band or the type changes.
+struct OriginPlan {
+    OriginDev dev{};
+    DBuf<float> q, f;
+    DBuf<int> row;
+    DBuf<int2> slot;
+    int nx = 0, min_r = -1, R = -1, n1 = 0;
+    float omax = -1.0f, step = -1.0f;
+};
+
 struct Ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -304,17 +316,25 @@ struct Ctx {
     DBuf<float2> mapcube;
     bool map_ready = false;
     DBuf<int2> csamples;
-    int cS = 0, cKpad = 0;
+    int cS = 0, cKpad = 0;  // cKpad: a local grid's row (interleaved pairs)
+    // section bank: n_orient / nom x nomr rows of 2 cKH elements (nomr: all omegas, or the
+    // first half turn where the other half are their complex conjugates)
     DBuf<uint16_t> bmat;
     long n_orient = 0;
+    int nomr = 0, cKH = 0;
     bool bmat_ready = false;
     double bmat_ms = 0.0;
     DBuf<uint16_t> amat;
-    // FP8-e4m3 operands: B8 (n_orient x cKpad8 bytes), per-sample band scales, A8
+    // FP8-e4m3 operands: B8 (rows of 2 cKH8 bytes), per-sample band scales, A8
     DBuf<uint8_t> bmat8, amat8;
     bool bmat8_ready = false;
     double bmat8_ms = 0.0;
-    int cKpad8 = 0, last_kpad = 0;
+    int cKH8 = 0, last_kpad = 0;
+    // bases of the origin grids (BF16, FP8, coarse) and the products of a sub-batch or pass
+    OriginPlan op, op8, op_c;
+    DBuf<float> cprod, ccmax;
+    DBuf<int> lmap;
+    DBuf<UpGroup> upg;
     double last_slice_ms = 0.0;
     int last_fallbacks = 0;   // particles of the last contraction call re-searched exhaustively
     float interp_sigma = 0.0f;  // sections: 0 trilinear, > 0 Gaussian kernel of this width (voxels)
@@ -332,13 +352,12 @@ struct Ctx {
     // form's cut sections (bgather)
     ViewGrid cgrid;
     DBuf<int2> csamples_c;
-    int cS_c = 0, cKpad_c = 0, n_origin_c = 0;
-    float orig_max_c = -1.0f, orig_step_c = -1.0f;
+    int cS_c = 0, cKH_c = 0, nomr_c = 0;
     DBuf<uint16_t> bmat_c, amat_c;
     bool bmat_c_ready = false;
     long n_orient_c = 0;
-    DBuf<float> corigins_c, topv_c, tilev_c, kcc_c;
-    DBuf<int> topi_c, tileo_c, tileorig_c, kor_c, korig_c, gidx;
+    DBuf<float> tilev_c, kcc_c;
+    DBuf<int> tileo_c, kor_c, korig_c, gidx;
     DBuf<double> pnorm_c;
     DBuf<uint8_t> bgather;
     DBuf<float> corigins, topv, kcc, kcand;
@@ -352,7 +371,7 @@ struct Ctx {
     int n_origin = 0;
     float orig_max = -1.0f, orig_step = -1.0f;
     DBuf<float> tilev, xcand, xpr;
-    DBuf<int> tileo, tileorig;
+    DBuf<int> tileo;
     DBuf<float2> xalpha;
     DBuf<float4> sband;
     DBuf<int> xcount;
@@ -365,7 +384,7 @@ struct Ctx {
     LearnModel lm;
     // view <-> grid slot (itheta * (2 Nphi + 1) + iphi + Nphi) maps for neighbours
     std::vector<int> view_slot, slot_view;
-    std::vector<uint8_t> list_mark;  // one byte per fine-grid orientation (expand_seeds)
+    std::vector<int> row_held;  // one word per bank row (expand_seeds)
     int num_sms = 0;
     // CUDA-event timing of the contraction launches (with prof)
     double prof_gemm_ms = 0.0;
@@ -395,11 +414,12 @@ struct Ctx {
         topv.release(); kcc.release(); kcand.release(); topi.release(); gerr.release();
         kor.release(); korig.release(); pnorm.release(); kcc64.release(); pnorm0.release(); pctf.release();
         xorient.release();
-        tilev.release(); xcand.release(); xpr.release(); tileo.release(); tileorig.release();
+        tilev.release(); xcand.release(); xpr.release(); tileo.release();
         xalpha.release(); bmat8.release(); amat8.release(); mulA.release(); mulB.release();
         bandmax.release(); fexp.release();
-        csamples_c.release(); bmat_c.release(); amat_c.release(); corigins_c.release(); topv_c.release();
-        tilev_c.release(); kcc_c.release(); topi_c.release(); tileo_c.release(); tileorig_c.release();
+        csamples_c.release(); bmat_c.release(); amat_c.release();
+        tilev_c.release(); kcc_c.release(); tileo_c.release();
+        cprod.release(); ccmax.release(); lmap.release(); upg.release();
         kor_c.release(); korig_c.release(); gidx.release(); pnorm_c.release(); bgather.release();
         sband.release(); xcount.release(); kpart.release(); ggroups.release(); gseg.release(); tbandc.release(); xgroups.release(); lcentre.release();
         lm.release();
@@ -847,7 +867,39 @@ int ensure_samples(Ctx* c) {
     CK(cudaMemcpyAsync(c->csamples.p, s.data(), sizeof(int2) * s.size(), cudaMemcpyHostToDevice, c->stream));
     c->cS = (int)s.size();
     c->cKpad = (2 * c->cS + 63) / 64 * 64;
-    c->cKpad8 = (2 * c->cS + 127) / 128 * 128;
+    c->cKH = (c->cS + 63) / 64 * 64;
+    c->cKH8 = (c->cS + 127) / 128 * 128;
+    return CRYOIM_OK;
+}
+
+// omega + 180 degrees is a grid point for every omega of the grid: the bank keeps the first
+// half turn (a section half a turn on is the complex conjugate)
+int bank_omegas(int nom, float step) {
+    return nom % 2 == 0 && std::fabs(step * (float)(nom / 2) - 180.0f) < 1e-3f ? nom / 2 : nom;
+}
+
+int ensure_origin_plan(Ctx* c, OriginPlan& o, int R, float omax, float step, bool f8) {
+    const int n1 = (int)(2.0f * omax / step + 0.5f) + 1;
+    if (o.nx == c->p.fftsize && o.min_r == c->p.min_r && o.R == R && o.omax == omax && o.step == step)
+        return CRYOIM_OK;
+    o.nx = 0;
+    const OriginBasis b = make_origin_basis(c->p.fftsize, c->p.min_r, R, omax, step, n1, f8);
+    if (b.nb > 512) return fail(CRYOIM_ERR_SIZE, "origin grid of %d x %d", n1, n1);
+    std::vector<int> row(b.slots);
+    std::vector<int2> slot((size_t)b.nb * b.nb);
+    for (int i = 0; i < b.slots; ++i) row[i] = b.mx[i] < 0 ? -1 : b.mx[i] | b.my[i] << 12 | b.part[i] << 24;
+    for (size_t i = 0; i < slot.size(); ++i) slot[i] = make_int2(b.slot[2 * i], b.slot[2 * i + 1]);
+    int r;
+    if ((r = o.q.ensure(b.q.size())) || (r = o.f.ensure(b.f.size())) || (r = o.row.ensure(b.slots)) || (r = o.slot.ensure(slot.size())))
+        return r;
+    CK(cudaMemcpyAsync(o.q.p, b.q.data(), sizeof(float) * b.q.size(), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(o.f.p, b.f.data(), sizeof(float) * b.f.size(), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(o.row.p, row.data(), sizeof(int) * b.slots, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(o.slot.p, slot.data(), sizeof(int2) * slot.size(), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    o.dev = OriginDev{o.q.p, o.f.p, o.row.p, o.slot.p, b.n1, b.nb, b.slots, b.units, b.R, b.layout, b.mid,
+                      f8 ? 0.0625f : 1.0f};
+    o.nx = c->p.fftsize; o.min_r = c->p.min_r; o.R = R; o.n1 = n1; o.omax = omax; o.step = step;
     return CRYOIM_OK;
 }
 
@@ -857,7 +909,10 @@ int ensure_bmat(Ctx* c) {
     if ((r = ensure_samples(c))) return r;
     const long n = (long)c->V * c->nom;
     if (c->bmat_ready && c->n_orient == n) return CRYOIM_OK;
-    if ((r = c->bmat.ensure((size_t)n * c->cKpad))) return r;
+    c->nomr = bank_omegas(c->nom, c->p.searchstep);
+    const long rows = (long)c->V * c->nomr;
+    if (n < 1) return fail(CRYOIM_ERR_SIZE, "search grid is empty");
+    if ((r = c->bmat.ensure((size_t)rows * 2 * c->cKH))) return r;
     std::vector<float> v2(2 * (size_t)c->V);
     for (int v = 0; v < c->V; ++v) { v2[2 * v] = c->views[4 * v]; v2[2 * v + 1] = c->views[4 * v + 1]; }
     DBuf<float> dv;
@@ -871,8 +926,8 @@ int ensure_bmat(Ctx* c) {
     cudaError_t te = make_cube_texture(c->mapcube.p, c->cube_r, c->stream, &arr, &tex);
     if (te == cudaSuccess) te = cudaEventRecord(e0, c->stream);
     if (te == cudaSuccess)
-        te = launch_slice_bf16(tex, c->cube_r, c->csamples.p, c->cS, c->cKpad, dv.p, c->nom, c->p.searchstep, 0,
-                               n, c->bmat.p, c->stream, c->mapcube.p, c->interp_sigma, (float)c->ovs);
+        te = launch_slice_bf16(tex, c->cube_r, c->csamples.p, c->cS, c->cKH, dv.p, c->nomr, c->p.searchstep, 0,
+                               rows, c->bmat.p, c->stream, c->mapcube.p, c->interp_sigma, (float)c->ovs);
     if (te == cudaSuccess) te = cudaEventRecord(e1, c->stream);
     if (te == cudaSuccess) te = cudaEventSynchronize(e1);
     free_cube_texture(arr, tex);
@@ -908,9 +963,10 @@ int ensure_coarse(Ctx* c, float omax, float ostep) {
         if ((r = c->csamples_c.ensure(s.size()))) return r;
         CK(cudaMemcpyAsync(c->csamples_c.p, s.data(), sizeof(int2) * s.size(), cudaMemcpyHostToDevice, c->stream));
         c->cS_c = (int)s.size();
-        c->cKpad_c = (2 * c->cS_c + 63) / 64 * 64;
-        const long n = (long)g.V * g.nom;
-        if ((r = c->bmat_c.ensure((size_t)n * c->cKpad_c))) return r;
+        c->cKH_c = (c->cS_c + 63) / 64 * 64;
+        c->nomr_c = bank_omegas(g.nom, g.step);
+        const long n = (long)g.V * g.nom, rows = (long)g.V * c->nomr_c;
+        if ((r = c->bmat_c.ensure((size_t)rows * 2 * c->cKH_c))) return r;
         std::vector<float> v2(2 * (size_t)g.V);
         for (int v = 0; v < g.V; ++v) { v2[2 * v] = g.views[4 * v]; v2[2 * v + 1] = g.views[4 * v + 1]; }
         DBuf<float> dv;
@@ -920,94 +976,133 @@ int ensure_coarse(Ctx* c, float omax, float ostep) {
         cudaTextureObject_t tex = 0;
         cudaError_t te = make_cube_texture(c->mapcube.p, c->cube_r, c->stream, &arr, &tex);
         if (te == cudaSuccess)
-            te = launch_slice_bf16(tex, c->cube_r, c->csamples_c.p, c->cS_c, c->cKpad_c, dv.p, g.nom, g.step, 0, n,
-                                   c->bmat_c.p, c->stream, c->mapcube.p, c->interp_sigma, (float)c->ovs);
+            te = launch_slice_bf16(tex, c->cube_r, c->csamples_c.p, c->cS_c, c->cKH_c, dv.p, c->nomr_c, g.step, 0,
+                                   rows, c->bmat_c.p, c->stream, c->mapcube.p, c->interp_sigma, (float)c->ovs);
         if (te == cudaSuccess) te = cudaStreamSynchronize(c->stream);
         free_cube_texture(arr, tex);
         if (te != cudaSuccess) return fail(CRYOIM_ERR_CUDA, "coarse sections: %s", cudaGetErrorString(te));
         c->n_orient_c = n;
         c->bmat_c_ready = true;
     }
-    if (omax != c->orig_max_c || 2.0f * ostep != c->orig_step_c) {
-        const float st = 2.0f * ostep;
-        const int n1 = (int)(2.0f * omax / st + 0.5f) + 1;
-        std::vector<float> og;
-        for (int iy = 0; iy < n1; ++iy)
-            for (int ix = 0; ix < n1; ++ix) {
-                og.push_back(-omax + st * (float)ix);
-                og.push_back(-omax + st * (float)iy);
-            }
-        if ((r = c->corigins_c.ensure(og.size()))) return r;
-        CK(cudaMemcpyAsync(c->corigins_c.p, og.data(), sizeof(float) * og.size(), cudaMemcpyHostToDevice,
-                           c->stream));
-        c->n_origin_c = n1 * n1;
-        c->orig_max_c = omax;
-        c->orig_step_c = st;
-    }
-    return CRYOIM_OK;
+    return ensure_origin_plan(c, c->op_c, std::max(c->p.min_r + 1, c->p.max_r / 2), omax, 2.0f * ostep, false);
 }
 
+// A particle's proposed orientations: fine-grid indices, each once, in the order first
+// reached; the bank rows they are, each once; and per orientation its row's position in rows,
+// x 2, + 1 where it is the row's complex conjugate.
+struct Proposals {
+    std::vector<int> n, rows, map;
+};
+
 // The fine-grid orientations within nbf steps (theta, phi, omega) of each seed (fine
-// grid theta index, signed phi index, omega index), each once, in the order first
-// reached: lists[i] for seeds[i].  One byte per grid orientation marks what a list
-// already holds (cleared after each list), so the cost is linear in the seeds.
-void expand_seeds(Ctx* c, const std::vector<std::vector<int3>>& seeds, int nbf,
-                  std::vector<std::vector<int>>& lists) {
-    const int span = 2 * c->nph + 1;
-    std::vector<uint8_t>& mark = c->list_mark;
-    if (mark.size() < (size_t)c->n_orient) mark.assign((size_t)c->n_orient, 0);
-    lists.assign(seeds.size(), std::vector<int>());
+// grid theta index, signed phi index, omega index) -> lists[i] for seeds[i].  One word per
+// bank row says what a list already holds of it (cleared after each list), so the cost is
+// linear in the seeds.
+void expand_seeds(Ctx* c, const std::vector<std::vector<int3>>& seeds, int nbf, std::vector<Proposals>& lists) {
+    const int span = 2 * c->nph + 1, nom = c->nom, nomr = c->nomr;
+    std::vector<int>& held = c->row_held;  // -1, or position << 2 | conjugate listed << 1 | itself listed
+    const size_t bank_rows = (size_t)c->V * nomr;
+    if (held.size() < bank_rows) held.assign(bank_rows, -1);
+    lists.assign(seeds.size(), Proposals());
     for (size_t i = 0; i < seeds.size(); ++i) {
-        std::vector<int>& lst = lists[i];
-        lst.reserve(seeds[i].size() * (2 * nbf + 1) * (2 * nbf + 1) * (2 * nbf + 1));
-        for (const int3& sd : seeds[i])
+        Proposals& L = lists[i];
+        const size_t most = seeds[i].size() * (2 * nbf + 1) * (2 * nbf + 1) * (2 * nbf + 1);
+        L.n.reserve(most);
+        L.map.reserve(most);
+        L.rows.reserve(most);
+        auto add = [&](int v, int io) {
+            const int half = io >= nomr ? 1 : 0, q = v * nomr + io - (half ? nomr : 0);
+            int& h = held[q];
+            if (h < 0) {
+                h = (int)L.rows.size() << 2;
+                L.rows.push_back(q);
+            }
+            if (h >> half & 1) return;
+            h |= 1 << half;
+            L.n.push_back(v * nom + io);
+            L.map.push_back(h >> 2 << 1 | half);
+        };
+        for (const int3& sd : seeds[i]) {
+            const int io0 = ((sd.z - nbf) % nom + nom) % nom;
             for (int dt = -nbf; dt <= nbf; ++dt)
                 for (int dp = -nbf; dp <= nbf; ++dp) {
                     const int it2 = sd.x + dt, ips2 = sd.y + dp;
                     if (it2 < 0 || it2 > c->nth || ips2 < -c->nph || ips2 > c->nph) continue;
                     const int v2 = c->slot_view[(size_t)it2 * span + ips2 + c->nph];
                     if (v2 < 0) continue;
-                    for (int dw = -nbf; dw <= nbf; ++dw) {
-                        const int n = v2 * c->nom + ((sd.z + dw) % c->nom + c->nom) % c->nom;
-                        if (!mark[n]) {
-                            mark[n] = 1;
-                            lst.push_back(n);
-                        }
+                    for (int dw = 0, io = io0; dw <= 2 * nbf; ++dw) {
+                        add(v2, io);
+                        if (++io == nom) io = 0;
                     }
                 }
-        for (int n : lst) mark[n] = 0;
-        if (lst.empty()) lst.push_back(0);
+        }
+        if (L.n.empty()) add(0, 0);
+        for (int q : L.rows) held[q] = -1;
     }
+}
+
+// Particles per exhaustive product: its FP32 products (122 MB a particle at 119,520 rows)
+// within 1.25 GB, equal sub-batches
+int product_batch(int nb, int parts, int slots, long pitch) {
+    const long each = (long)parts * slots * pitch * 4;
+    const int most = (int)std::max(1L, std::min(64L, (5L << 28) / std::max(1L, each)));
+    const int cuts = (nb + most - 1) / most;
+    return (nb + cuts - 1) / cuts;
+}
+
+// The k best orientations (one per block of 256) of np particles against every row of a
+// bank: A of np x ob.slots rows, products and their expansion in sub-batches, queued back to
+// back on c's stream.  mark (profiling) is called before and after every contraction launch.
+int exhaustive_topk(Ctx* c, const OriginDev& ob, const void* A, const void* bank, long rows, int nom, int nomr, int K,
+                    bool f8, int np, int k, int ntiles, float* tilev, int* tileo, int* kor, int* korig, float* kcc,
+                    bool want_origin, const std::function<int()>& mark = nullptr) {
+    const int parts = nom / nomr, tn = gemm_tile_n();
+    const long n_orient = rows / nomr * nom, pitch = (rows + tn - 1) / tn * tn;
+    const int pb = product_batch(np, parts, ob.slots, pitch);
+    int r;
+    if ((r = c->cprod.ensure((size_t)pb * parts * ob.slots * pitch)) || (r = c->ccmax.ensure((size_t)pb * n_orient)))
+        return r;
+    for (int s0 = 0; s0 < np; s0 += pb) {
+        const int ns = std::min(pb, np - s0);
+        GemmArgmaxArgs g{};
+        g.b_mode = 1;  // the banks' rows are pre-swizzled
+        g.err = c->gerr.p;
+        g.cstore = c->cprod.p;
+        g.k_parts = parts;
+        g.c_units = ob.units;
+        g.c_rows = ob.slots / ob.units;
+        if (mark && (r = mark())) return r;
+        CK(launch_gemm_argmax((const char*)A + (size_t)s0 * ob.slots * K * (f8 ? 1 : 2), bank, ns * ob.slots, (int)rows,
+                              K, f8, g, c->num_sms, c->stream));
+        if (mark && (r = mark())) return r;
+        CK(launch_up_topk(ob, c->cprod.p, pitch, rows, nom, nomr, ns, k, c->ccmax.p, ntiles, tilev, tileo,
+                          kor + (size_t)s0 * k, korig + (size_t)s0 * k, kcc + (size_t)s0 * k, want_origin, c->num_sms,
+                          c->stream));
+    }
+    return CRYOIM_OK;
 }
 
 // Coarse level for nb prepared particles (c->band, ctfp): the best kc distinct coarse
 // orientations of each, mapped onto the fine grid (twice the coarse indices) with their
 // fine neighbours within nbf steps in theta, phi and omega -> lists[i].
-int coarse_lists(Ctx* c, int nb, const float* ctfp, int kc, int nbf, std::vector<std::vector<int>>& lists) {
+int coarse_lists(Ctx* c, int nb, const float* ctfp, const float* poff, const OriginDev& ob, int kc, int nbf,
+                 std::vector<Proposals>& lists) {
     const ViewGrid& g = c->cgrid;
-    const int Oc = c->n_origin_c;
     const int ntc = (int)((c->n_orient_c + gemm_tile_n() - 1) / gemm_tile_n());
     int r;
-    if ((r = c->amat_c.ensure((size_t)nb * Oc * c->cKpad_c)) || (r = c->topv_c.ensure((size_t)nb * Oc * ntc)) ||
-        (r = c->topi_c.ensure((size_t)nb * Oc * ntc)) || (r = c->tilev_c.ensure((size_t)nb * ntc)) ||
-        (r = c->tileo_c.ensure((size_t)nb * ntc)) || (r = c->tileorig_c.ensure((size_t)nb * ntc)) ||
-        (r = c->kor_c.ensure((size_t)nb * kc)) || (r = c->korig_c.ensure((size_t)nb * kc)) ||
-        (r = c->kcc_c.ensure((size_t)nb * kc)) || (r = c->pnorm_c.ensure(nb)))
+    if ((r = c->amat_c.ensure((size_t)nb * ob.slots * 2 * c->cKH_c)) || (r = c->tilev_c.ensure((size_t)nb * ntc)) ||
+        (r = c->tileo_c.ensure((size_t)nb * ntc)) || (r = c->kor_c.ensure((size_t)nb * kc)) ||
+        (r = c->korig_c.ensure((size_t)nb * kc)) || (r = c->kcc_c.ensure((size_t)nb * kc)) ||
+        (r = c->pnorm_c.ensure(nb)))
         return r;
     launch_particle_norm(c->band.p, ctfp, c->bd, c->csamples_c.p, c->cS_c, nb, c->pnorm_c.p, c->stream);
-    launch_build_a(c->band.p, ctfp, c->bd, c->csamples_c.p, c->cS_c, c->cKpad_c, c->corigins_c.p, Oc, c->pnorm_c.p,
-                   nb, c->amat_c.p, c->stream);
-    GemmArgmaxArgs ga{};
-    ga.b_mode = 1;  // the coarse bank's rows are pre-swizzled
-    ga.topv = c->topv_c.p;
-    ga.topi = c->topi_c.p;
-    ga.err = c->gerr.p;
+    CK(launch_build_basis(c->band.p, ctfp, c->bd, c->csamples_c.p, c->cS_c, c->cKH_c, ob, c->pnorm_c.p, nb, c->amat_c.p,
+                          false, nullptr, nullptr, c->stream, poff));
     CK(cudaMemsetAsync(c->gerr.p, 0, sizeof(int), c->stream));
-    CK(launch_gemm_argmax(c->amat_c.p, c->bmat_c.p, nb * Oc, (int)c->n_orient_c, c->cKpad_c, false, ga, c->num_sms,
-                          c->stream));
-    launch_select_topk(c->topv_c.p, c->topi_c.p, Oc, ntc, kc, nb, c->tilev_c.p, c->tileo_c.p, c->tileorig_c.p,
-                       c->kor_c.p, c->korig_c.p, c->kcc_c.p, c->stream);
-    CK(cudaGetLastError());
+    if ((r = exhaustive_topk(c, ob, c->amat_c.p, c->bmat_c.p, c->n_orient_c / g.nom * c->nomr_c, g.nom, c->nomr_c,
+                             2 * c->cKH_c, false, nb, kc, ntc, c->tilev_c.p, c->tileo_c.p, c->kor_c.p, c->korig_c.p,
+                             c->kcc_c.p, false)))
+        return r;
     std::vector<int> kor((size_t)nb * kc);
     int gerr = 0;
     CK(cudaMemcpyAsync(&gerr, c->gerr.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -1444,7 +1539,7 @@ int learn_train_impl(Ctx* c, const float* map3d, const cryoim_learn_opts* o, flo
 // Proposals of the trained model for the nb particles whose band is in c->band: the
 // top kl cells, each as two fine-grid seeds (angle, angle + 180 degrees), expanded to
 // their fine neighbourhoods within nbf steps -> lists[i].
-int learned_lists(Ctx* c, int nb, int kl, int nbf, std::vector<std::vector<int>>& lists) {
+int learned_lists(Ctx* c, int nb, int kl, int nbf, std::vector<Proposals>& lists) {
     LearnModel& L = c->lm;
     int r;
     if ((r = learn_activations(c, nb))) return r;
@@ -1478,15 +1573,15 @@ int learned_lists(Ctx* c, int nb, int kl, int nbf, std::vector<std::vector<int>>
 }
 
 // FP8-e4m3 copy of operand B with per-band power-of-two scales (contract.cu explains the
-// scaling): band maxima of the BF16 rows (every 4th orientation), e_b = floor(log2(224 /
+// scaling): band maxima of the BF16 rows (every 4th row), e_b = floor(log2(224 /
 // max_b)), mulB = 2^e_b and mulA = 2^-e_b per sample, then the conversion.
 int ensure_bmat8(Ctx* c) {
     int r;
     if ((r = ensure_bmat(c))) return r;
     if (c->bmat8_ready) return CRYOIM_OK;
     const int S = c->cS, nband = c->p.max_r + 2;
-    const long n = c->n_orient;
-    if ((r = c->bmat8.ensure((size_t)n * c->cKpad8)) || (r = c->bandmax.ensure(nband)) ||
+    const long n = (long)c->V * c->nomr;
+    if ((r = c->bmat8.ensure((size_t)n * 2 * c->cKH8)) || (r = c->bandmax.ensure(nband)) ||
         (r = c->mulA.ensure(S)) || (r = c->mulB.ensure(S)))
         return r;
     if (c->num_sms == 0) CK(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, c->device));
@@ -1494,7 +1589,7 @@ int ensure_bmat8(Ctx* c) {
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
     CK(cudaEventRecord(e0, c->stream));
-    CK(launch_band_absmax(c->bmat.p, n, c->cKpad, c->csamples.p, S, nband, 4, c->bandmax.p, c->num_sms,
+    CK(launch_band_absmax(c->bmat.p, n, c->cKH, c->csamples.p, S, nband, 4, c->bandmax.p, c->num_sms,
                           c->stream));
     std::vector<unsigned> hm(nband);
     std::vector<int2> hs(S);
@@ -1515,7 +1610,7 @@ int ensure_bmat8(Ctx* c) {
     }
     CK(cudaMemcpyAsync(c->mulA.p, ma.data(), sizeof(float) * S, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(c->mulB.p, mb.data(), sizeof(float) * S, cudaMemcpyHostToDevice, c->stream));
-    CK(launch_b_to_e4m3(c->bmat.p, n, c->cKpad, S, c->mulB.p, c->cKpad8, c->bmat8.p, c->stream));
+    CK(launch_b_to_e4m3(c->bmat.p, n, c->cKH, S, c->mulB.p, c->cKH8, c->bmat8.p, c->stream));
     CK(cudaEventRecord(e1, c->stream));
     CK(cudaEventSynchronize(e1));
     float ms = 0.f;
@@ -1561,21 +1656,19 @@ int refresh_lane(Ctx* c, int i) {
     h->ovs = c->ovs;
     h->cube_r = c->cube_r;
     h->csamples.borrow(c->csamples);
-    h->cS = c->cS; h->cKpad = c->cKpad;
+    h->cS = c->cS; h->cKpad = c->cKpad; h->cKH = c->cKH; h->nomr = c->nomr;
     h->bmat.borrow(c->bmat);
     h->n_orient = c->n_orient;
     h->bmat_ready = c->bmat_ready; h->bmat_ms = c->bmat_ms;
     h->bmat8.borrow(c->bmat8);
-    h->bmat8_ready = c->bmat8_ready; h->bmat8_ms = c->bmat8_ms; h->cKpad8 = c->cKpad8;
+    h->bmat8_ready = c->bmat8_ready; h->bmat8_ms = c->bmat8_ms; h->cKH8 = c->cKH8;
     h->mulA.borrow(c->mulA);
     h->mulB.borrow(c->mulB);
     h->cgrid = c->cgrid;
     h->csamples_c.borrow(c->csamples_c);
-    h->cS_c = c->cS_c; h->cKpad_c = c->cKpad_c; h->n_origin_c = c->n_origin_c;
-    h->orig_max_c = c->orig_max_c; h->orig_step_c = c->orig_step_c;
+    h->cS_c = c->cS_c; h->cKH_c = c->cKH_c; h->nomr_c = c->nomr_c;
     h->bmat_c.borrow(c->bmat_c);
     h->bmat_c_ready = c->bmat_c_ready; h->n_orient_c = c->n_orient_c;
-    h->corigins_c.borrow(c->corigins_c);
     h->corigins.borrow(c->corigins);
     h->n_origin = c->n_origin; h->orig_max = c->orig_max; h->orig_step = c->orig_step;
     h->view_slot = c->view_slot;
@@ -1639,7 +1732,7 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
     if (P == 0) return CRYOIM_OK;
     if ((r = local ? ensure_samples(c) : (f8 ? ensure_bmat8(c) : ensure_bmat(c)))) return r;
     if (kc > 0 && (r = ensure_coarse(c, opts->origin_max, opts->origin_step))) return r;
-    const int kpad = f8 ? c->cKpad8 : c->cKpad;
+    const int kpad = local ? c->cKpad : 2 * (f8 ? c->cKH8 : c->cKH);
     c->last_kpad = kpad;
     c->last_slice_ms = c->bmat_ms + (f8 ? c->bmat8_ms : 0.0);
     if (c->n_orient > 0x7fffffffL) return fail(CRYOIM_ERR_SIZE, "too many orientations");
@@ -1661,14 +1754,27 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
     }
     const int O = c->n_origin, T = c->T, nx = c->p.fftsize;
     const long nn = (long)nx * nx, w2 = (long)c->bd.W * c->bd.W;
-    // Particles per pass (transform, rescoring: large grids, two host waits per pass) and
-    // per exhaustive contraction launch (operand A of about 2400 rows stays L2-resident
-    // while the sections stream).  The proposal form builds A for the whole pass: its
-    // grouped launch reads each particle's A against that particle's own few tiles.
+    // the global forms correlate the origin grid's basis, the local form its origins: its
+    // rows are the particle's own (no half turn to share), the BF16 score of every origin
+    // decides which one the FP64 rescoring sees, and 289 origins of a 128 box are 3 row tiles
+    // against 1: 8 % of its time, the sections' cut 83 %
+    OriginPlan& plan = f8 ? c->op8 : c->op;
+    if (!local && (r = ensure_origin_plan(c, plan, c->p.max_r, opts->origin_max, opts->origin_step, f8))) return r;
+    const OriginDev ob = plan.dev, ob_c = c->op_c.dev;
+    const int parts_k = local ? 1 : c->nom / c->nomr;
+    // Particles per pass (transform, rescoring: large grids, two host waits per pass);
+    // operand A is built for the whole pass.
     const int PB = std::max(1, c->batch);
-    const int pb = std::max(1, std::min(PB, 2400 / std::max(O, 1)));
-    const int arows = (kc > 0 || kl > 0 || local) ? PB : pb;
+    const int arows = local ? O : ob.slots;  // rows of A per particle
     const int ntiles = (int)(((local ? nloc : c->n_orient) + gemm_tile_n() - 1) / gemm_tile_n());
+    // list positions of a particle in the proposal forms, at most: seeds x neighbourhood
+    const long nlist = std::min((long)c->n_orient,
+                                (long)std::max(kc, 2 * kl) * (2 * nbf + 1) * (2 * nbf + 1) * (2 * nbf + 1));
+    const bool listed = kc > 0 || kl > 0;
+    const long toptiles = local ? ntiles : (listed ? (nlist + gemm_tile_n() - 1) / gemm_tile_n() : 0);
+    // the FP64 correlations decide the pick (pick = 1) or are returned with the
+    // candidates; a phase-residual pick without candidate output does not read them
+    const bool need_cc64 = opts->pick != 0 || cands != nullptr;
     // the band cube as a filtering texture for the local form's sections (shared by the lanes)
     struct LocalTexture {
         cudaArray_t arr = nullptr;
@@ -1689,7 +1795,7 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
     }
     std::vector<float> ohost(2 * (size_t)O);
     CK(cudaMemcpyAsync(ohost.data(), c->corigins.p, sizeof(float) * 2 * O, cudaMemcpyDeviceToHost, c->stream));
-    const long row_bytes = f8 ? (long)c->cKpad8 : 2L * c->cKpad;
+    const long row_bytes = f8 ? (long)kpad : 2L * kpad;
     // Passes are dealt round-robin to lanes (this context and c->xlanes, each with its own
     // stream, per-pass buffers and host thread), so that one lane's host work between
     // its waits overlaps the other lanes' kernels.
@@ -1697,10 +1803,11 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
     auto alloc = [&](Ctx* L) -> int {
         int r;
         if ((r = ensure_batch(L, PB))) return r;
-        if (f8 ? ((r = L->amat8.ensure((size_t)arows * O * L->cKpad8)) || (r = L->fexp.ensure(PB)))
-               : (r = L->amat.ensure((size_t)arows * O * L->cKpad)))
+        const int ps = std::min(PB, P);  // particles of the largest pass
+        if (f8 ? ((r = L->amat8.ensure((size_t)ps * arows * kpad)) || (r = L->fexp.ensure(PB)))
+               : (r = L->amat.ensure((size_t)ps * arows * kpad)))
             return r;
-        if ((r = L->topv.ensure((size_t)arows * O * ntiles)) || (r = L->topi.ensure((size_t)arows * O * ntiles)))
+        if ((r = L->topv.ensure((size_t)ps * O * toptiles)) || (r = L->topi.ensure((size_t)ps * O * toptiles)))
             return r;
         if ((r = L->gerr.ensure(1)) || (r = L->pnorm.ensure(PB)) || (r = L->pcband.ensure((size_t)PB * L->cS)) ||
             (r = L->kor.ensure((size_t)PB * k)) ||
@@ -1709,8 +1816,8 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
             (r = L->kpart.ensure((size_t)cc_fp64_scratch(k, PB))))
             return r;
         if (local && ((r = L->pnorm0.ensure(PB)) || (r = L->pctf.ensure((size_t)PB * L->cS)))) return r;
-        if ((r = L->tilev.ensure((size_t)pb * ntiles)) || (r = L->tileo.ensure((size_t)pb * ntiles)) ||
-            (r = L->tileorig.ensure((size_t)pb * ntiles)) || (r = L->xcand.ensure((size_t)PB * maxx * 5)) ||
+        if ((r = L->tilev.ensure((size_t)PB * ntiles)) || (r = L->tileo.ensure((size_t)PB * ntiles)) ||
+            (r = L->xcand.ensure((size_t)PB * maxx * 5)) ||
             (r = L->xpr.ensure((size_t)PB * maxx)))
             return r;
         if (local && (r = L->lcentre.ensure(3 * (size_t)PB))) return r;
@@ -1777,20 +1884,17 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
                 for (int i = 0; i < nb; ++i) { po[2 * i] = parts[b0 + i].x; po[2 * i + 1] = parts[b0 + i].y; }
                 CK(cudaMemcpyAsync(L->poff.p, po.data(), sizeof(float) * po.size(), cudaMemcpyHostToDevice, L->stream));
             }
-            // operand A rows (particle, origin) of particles [s0, s0 + ns) at row (s0 - a0) O
-            auto build_rows = [&](int s0, int ns, int a0) {
-                const float2* bb = L->band.p + (long)s0 * w2;
-                const float* cc = ctfp ? ctfp + (long)s0 * w2 : nullptr;
-                const float* po = centred ? L->poff.p + 2 * (size_t)s0 : nullptr;
-                if (f8)
-                    launch_build_a8(bb, cc, L->bd, L->csamples.p, L->cS, L->cKpad8, L->corigins.p, O, L->pnorm.p + s0,
-                                    L->mulA.p, L->fexp.p + s0, ns, L->amat8.p + (size_t)(s0 - a0) * O * L->cKpad8,
-                                    L->stream, po);
-                else  // the local form's rows are normalised by |P| (its sections by |CTF S|)
-                    launch_build_a(bb, cc, L->bd, L->csamples.p, L->cS, L->cKpad, L->corigins.p, O,
-                                   (local ? L->pnorm0.p : L->pnorm.p) + s0, ns,
-                                   L->amat.p + (size_t)(s0 - a0) * O * L->cKpad, L->stream, po);
-            };
+            const float* po = centred ? L->poff.p : nullptr;
+            // operand A of the pass: the basis rows of every particle, or (local) its origins,
+            // normalised by |P| there (the sections by |CTF S|)
+            if (local)
+                launch_build_a(L->band.p, ctfp, L->bd, L->csamples.p, L->cS, L->cKpad, L->corigins.p, O, L->pnorm0.p,
+                               nb, L->amat.p, L->stream, po);
+            else
+                CK(launch_build_basis(L->band.p, ctfp, L->bd, L->csamples.p, L->cS, kpad / 2, ob, L->pnorm.p, nb,
+                                      f8 ? (void*)L->amat8.p : (void*)L->amat.p, f8, L->mulA.p, L->fexp.p, L->stream,
+                                      po));
+            CK(cudaGetLastError());
             GemmArgmaxArgs g{};
             g.b_mode = 1;  // section rows are stored pre-swizzled (exhaustive and local tiles)
             g.topv = L->topv.p;
@@ -1798,37 +1902,46 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
             g.cfull = nullptr;
             g.err = L->gerr.p;
             CK(cudaMemsetAsync(L->gerr.p, 0, sizeof(int), L->stream));
-            std::vector<std::vector<int>> lists, slots;
+            std::vector<Proposals> lists;
             ngev = 0;
             if (kc > 0 || kl > 0 || local) {
                 // proposal forms: the coarse contraction or the learned proposer names each
                 // particle's candidate orientations, the fine contraction runs on their
                 // sections only; the local form cuts each particle's local grid
-                if (!local &&
-                    (r = kc > 0 ? coarse_lists(L, nb, ctfp, kc, nbf, lists) : learned_lists(L, nb, kl, nbf, lists)))
+                if (!local && (r = kc > 0 ? coarse_lists(L, nb, ctfp, nullptr, ob_c, kc, nbf, lists)
+                                          : learned_lists(L, nb, kl, nbf, lists)))
                     return r;
                 CK(cudaMemsetAsync(L->gerr.p, 0, sizeof(int), L->stream));
                 const void* bsrc = f8 ? (const void*)L->bmat8.p : (const void*)L->bmat.p;
                 const char* abase = f8 ? (const char*)L->amat8.p : (const char*)L->amat.p;
-                build_rows(0, nb, 0);
-                CK(cudaGetLastError());
                 // the proposal forms read their sections from the bank by index: the
-                // contraction's producer copies each listed row into its tile (the rows are
+                // contraction's loaders copy each listed row into its tile (the rows are
                 // stored pre-swizzled; the copy re-swizzles a row for its tile row).  The
                 // local form cuts each particle's grid into the pass buffer at a start that
                 // is a multiple of 8.
                 const long lpitch = (nloc + 7) / 8 * 8;
-                if (!local) slots = lists;
-                auto rows_of = [&](int i) -> long { return local ? lpitch : (long)slots[i].size(); };
-                // particles in groups (the local form's cut sections under 8 GB per group): one
-                // grouped contraction per group (each particle's origin rows against its own
-                // sections), then the k distinct best orientations of each particle
+                const int tn = gemm_tile_n();
+                // floats of a particle's products
+                auto prod_of = [&](int i) -> long {
+                    return (long)parts_k * ob.slots * (((long)lists[i].rows.size() + tn - 1) / tn * tn);
+                };
+                // particles in groups (the local form's cut sections under 8 GB per group, the
+                // products of the proposal forms under 1 GB): one grouped contraction per group
+                // (each particle's rows of A against its own sections), then the k distinct best
+                // orientations of each particle
                 for (int i0 = 0; i0 < nb;) {
                     int i1 = i0;
-                    long rows = 0;
-                    while (i1 < nb && (i1 == i0 || !local || (rows + rows_of(i1)) * row_bytes <= (8L << 30)))
-                        rows += rows_of(i1++);
+                    long rows = 0, coff = 0;
+                    while (i1 < nb &&
+                           (i1 == i0 || (local ? (rows + lpitch) * row_bytes <= (8L << 30) : coff + prod_of(i1) <= (1L << 28)))) {
+                        if (!local) coff += prod_of(i1);
+                        rows += local ? lpitch : (long)lists[i1].rows.size();
+                        ++i1;
+                    }
                     GemmArgmaxArgs gg = g;
+                    std::vector<int> idx, lmap;
+                    std::vector<UpGroup> ug(local ? 0 : i1 - i0);
+                    int up_tiles = 1;
                     if (local) {
                         if ((r = L->bgather.ensure((size_t)rows * row_bytes))) return r;
                         std::vector<float> cen(3 * (size_t)(i1 - i0));
@@ -1844,74 +1957,85 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
                                                    c->mapcube.p, c->interp_sigma, lpitch,
                                                    L->pctf.p + (size_t)i0 * L->cS, (float)c->ovs));
                     } else {
-                        std::vector<int> idx;
                         idx.reserve(rows);
-                        for (int i = i0; i < i1; ++i) idx.insert(idx.end(), slots[i].begin(), slots[i].end());
-                        for (int n : idx)
-                            if (n < 0 || n >= L->n_orient) return fail(CRYOIM_ERR_STATE, "proposal row %d", n);
-                        if ((r = L->gidx.ensure(rows))) return r;
+                        for (int i = i0; i < i1; ++i) {
+                            idx.insert(idx.end(), lists[i].rows.begin(), lists[i].rows.end());
+                            lmap.insert(lmap.end(), lists[i].map.begin(), lists[i].map.end());
+                        }
+                        if ((r = L->gidx.ensure(rows)) || (r = L->lmap.ensure(lmap.size())) ||
+                            (r = L->upg.ensure(i1 - i0)) || (r = L->cprod.ensure((size_t)coff)))
+                            return r;
                         CK(cudaMemcpyAsync(L->gidx.p, idx.data(), sizeof(int) * rows, cudaMemcpyHostToDevice,
+                                           L->stream));
+                        CK(cudaMemcpyAsync(L->lmap.p, lmap.data(), sizeof(int) * lmap.size(), cudaMemcpyHostToDevice,
                                            L->stream));
                         gg.b_mode = 2;
                         gg.b_index = L->gidx.p;
                         gg.b_rows = (const unsigned char*)bsrc;
                         gg.b_row_bytes = row_bytes;
+                        gg.cstore = L->cprod.p;
+                        gg.k_parts = parts_k;
+                        gg.c_units = ob.units;
+                        gg.c_rows = ob.slots / ob.units;
                     }
                     std::vector<GemmGroup> hg(i1 - i0);
                     std::vector<int2> seg(i1 - i0);
-                    long roff = 0, toff = 0;
+                    long roff = 0, toff = 0, moff = 0, poffs = 0;
                     for (int i = i0; i < i1; ++i) {
-                        const int nl = (int)(local ? nloc : (long)slots[i].size());
-                        const int ntp = (nl + gemm_tile_n() - 1) / gemm_tile_n();
+                        const int nl = (int)(local ? nloc : (long)lists[i].rows.size());
+                        const int np = (int)(local ? nloc : (long)lists[i].n.size());
+                        const int ntp = (np + tn - 1) / tn;
                         GemmGroup& q = hg[i - i0];
-                        q.a_row0 = i * O;
-                        q.m_valid = O;
+                        q.a_row0 = i * arows;
+                        q.m_valid = arows;
                         q.b_row0 = (int)roff;
                         q.n_valid = nl;
                         q.topv_off = (int)toff;
+                        q.c_off = poffs;
                         seg[i - i0] = make_int2((int)toff, ntp);
+                        if (!local) {
+                            ug[i - i0] = UpGroup{poffs, (nl + tn - 1) / tn, (int)moff, np, (int)toff, ntp};
+                            up_tiles = std::max(up_tiles, ntp);
+                            poffs += prod_of(i);
+                            moff += np;
+                        }
                         roff += local ? lpitch : nl;
                         toff += (long)O * ntp;
-                        // the useful work: the particle's listed orientations (not padding slots)
-                        if (L->prof)
-                            L->prof_gemm_flops += 2.0 * (double)O * (double)(local ? nloc : (long)lists[i].size()) *
-                                                  (double)kpad;
+                        // the useful work: the rows that are correlated (not padding slots)
+                        if (L->prof) L->prof_gemm_flops += 2.0 * (double)arows * (double)nl * (double)kpad;
                     }
                     if ((r = L->ggroups.ensure(i1 - i0)) || (r = L->gseg.ensure(i1 - i0))) return r;
                     if (L->prof && (r = gmark(ngev++))) return r;
-                    CK(launch_gemm_argmax_grouped(abase, (long)nb * O, local ? (const void*)L->bgather.p : bsrc, rows,
-                                                  kpad, f8, hg.data(), i1 - i0, L->ggroups.p, gg, L->num_sms,
+                    CK(launch_gemm_argmax_grouped(abase, (long)nb * arows, local ? (const void*)L->bgather.p : bsrc,
+                                                  rows, kpad, f8, hg.data(), i1 - i0, L->ggroups.p, gg, L->num_sms,
                                                   L->stream));
                     if (L->prof && (r = gmark(ngev++))) return r;
+                    if (!local) {
+                        CK(cudaMemcpyAsync(L->upg.p, ug.data(), sizeof(UpGroup) * ug.size(), cudaMemcpyHostToDevice,
+                                           L->stream));
+                        CK(launch_up_list(ob, L->cprod.p, parts_k, L->upg.p, i1 - i0, up_tiles, L->lmap.p, L->topv.p,
+                                          L->topi.p, L->stream));
+                    }
                     CK(cudaMemcpyAsync(L->gseg.p, seg.data(), sizeof(int2) * seg.size(), cudaMemcpyHostToDevice,
                                        L->stream));
                     launch_select_distinct(L->topv.p, L->topi.p, O, L->gseg.p, i1 - i0, k, L->kor.p + (size_t)i0 * k,
                                            L->korig.p + (size_t)i0 * k, L->kcc.p + (size_t)i0 * k, L->stream);
                     CK(cudaGetLastError());
-                    // the cut-section buffer and the row lists are reused by the next group
+                    // the cut-section buffer, the products and the row lists are reused by the next group
                     if (i1 < nb) CK(cudaStreamSynchronize(L->stream));
                     i0 = i1;
                 }
             } else {
-                // exhaustive: sub-batches of pb particles against every section, queued back to back
-                for (int s0 = 0; s0 < nb; s0 += pb) {
-                    const int ns = std::min(pb, nb - s0);
-                    build_rows(s0, ns, s0);
-                    CK(cudaGetLastError());
-                    if (L->prof && (r = gmark(ngev++))) return r;
-                    if (f8)
-                        CK(launch_gemm_argmax(L->amat8.p, L->bmat8.p, ns * O, (int)L->n_orient, kpad, true, g,
-                                              L->num_sms, L->stream));
-                    else
-                        CK(launch_gemm_argmax(L->amat.p, L->bmat.p, ns * O, (int)L->n_orient, kpad, false, g,
-                                              L->num_sms, L->stream));
-                    if (L->prof && (r = gmark(ngev++))) return r;
-                    launch_select_topk(L->topv.p, L->topi.p, O, ntiles, k, ns, L->tilev.p, L->tileo.p, L->tileorig.p,
-                                       L->kor.p + (size_t)s0 * k, L->korig.p + (size_t)s0 * k,
-                                       L->kcc.p + (size_t)s0 * k, L->stream);
-                    CK(cudaGetLastError());
-                    if (L->prof) L->prof_gemm_flops += 2.0 * (double)ns * O * (double)L->n_orient * (double)kpad;
-                }
+                // exhaustive: every particle of the pass against every row of the bank
+                if ((r = exhaustive_topk(L, ob, f8 ? (const void*)L->amat8.p : (const void*)L->amat.p,
+                                         f8 ? (const void*)L->bmat8.p : (const void*)L->bmat.p,
+                                         L->n_orient / L->nom * L->nomr, L->nom, L->nomr, kpad, f8, nb, k, ntiles,
+                                         L->tilev.p, L->tileo.p, L->kor.p, L->korig.p, L->kcc.p, need_cc64,
+                                         [&]() -> int { return L->prof ? gmark(ngev++) : CRYOIM_OK; })))
+                    return r;
+                if (L->prof)
+                    L->prof_gemm_flops +=
+                        2.0 * (double)nb * ob.slots * (double)(L->n_orient / L->nom * L->nomr) * (double)kpad;
             }
             int gerr = 0;
             CK(cudaMemcpyAsync(&gerr, L->gerr.p, sizeof(int), cudaMemcpyDeviceToHost, L->stream));
@@ -1926,7 +2050,7 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
                 for (int i = 0; i < nb * k; ++i) hcc[i] = std::ldexp(hcc[i], -hfe[i / k]);
             if (kc > 0 || kl > 0)  // list position -> fine orientation index
                 for (int i = 0; i < nb * k; ++i)
-                    if (hor[i] >= 0) hor[i] = slots[i / k][hor[i]];
+                    if (hor[i] >= 0) hor[i] = lists[i / k].n[hor[i]];
             if (L->prof)
                 for (size_t e = 0; e + 1 < ngev; e += 2) {
                     float ms = 0.f;
@@ -1955,9 +2079,6 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
             }
             CK(cudaMemcpyAsync(L->kcand.p, hcand.data(), sizeof(float) * nb * k * 5, cudaMemcpyHostToDevice,
                                L->stream));
-            // the FP64 correlations decide the pick (pick = 1) or are returned with the
-            // candidates; a phase-residual pick without candidate output does not read them
-            const bool need_cc64 = opts->pick != 0 || cands != nullptr;
             if (need_cc64)
                 launch_cc_fp64(L->mapcube.p, L->pcband.p, L->bd, L->csamples.p, L->cS, L->kcand.p, k, nb,
                                local ? L->pnorm0.p : L->pnorm.p, L->kpart.p, L->kcc64.p, L->stream, c->interp_sigma,

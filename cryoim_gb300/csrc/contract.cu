@@ -17,8 +17,12 @@
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <type_traits>
+
 #include "geom.cuh"
 #include "kernels.h"
+#include "origin_basis.h"
 
 namespace cryoim {
 namespace {
@@ -103,31 +107,40 @@ __device__ __forceinline__ float2 gauss_sample(const float2* __restrict__ cube, 
 // row of the same residue mod 8 (a TMA box without swizzle) is then already in the
 // layout the tensor cores read; a row copied by index into any tile row has its chunks
 // re-ordered by the XOR of the two residues (gemm_tc.cu, B rows by index).  Index of
-// (Re, Im) pair i of row r: BF16 rows hold 32 pairs per block (4 per chunk), FP8 rows 64
-// (8 per chunk).
+// (Re, Im) pair i of a local grid's row r (interleaved pairs, 32 per block, 4 per chunk):
 __device__ __forceinline__ long bf16_pair_at(long i, long r) {
     return (i & ~31L) | ((((i >> 2) & 7) ^ (r & 7)) << 2) | (i & 3);
 }
-__device__ __forceinline__ long fp8_pair_at(long i, long r) {
-    return (i & ~63L) | ((((i >> 3) & 7) ^ (r & 7)) << 3) | (i & 7);
+
+
+// The section banks keep the parts of a row apart: elements [0, KH) are the real parts of
+// the samples, [KH, 2 KH) the imaginary parts (KH = S rounded up to a 128-byte block), so
+// that the products over each half of K come out separately (k_up_* below).  Index of
+// element e (of 2 KH) of row r, pre-swizzled as above: BF16 64 elements per block, FP8 128.
+__device__ __forceinline__ long bf16_at(long e, long r) {
+    return (e & ~63L) | ((((e >> 3) & 7) ^ (r & 7)) << 3) | (e & 7);
+}
+__device__ __forceinline__ long fp8_at(long e, long r) {
+    return (e & ~127L) | ((((e >> 4) & 7) ^ (r & 7)) << 4) | (e & 15);
 }
 
-// One CTA per orientation n = view * nomega + iomega: section samples in shared
+// One CTA per bank row r = view * nomr + iomega (nomr omegas of each view: all of them, or
+// the first half turn, the others being complex conjugates): section samples in shared
 // memory, norm (FP32 per thread, FP64 across the block), then the unit-norm row in BF16
-// (Re, Im interleaved, zero pad).  The trilinear interpolation runs on the texture
+// (split, zero pad).  The trilinear interpolation runs on the texture
 // units: the band cube is a float2 3D array with linear filtering (hardware weights in
 // 1/256 steps, well inside the BF16 rounding of the row), texel centres at +0.5, zero
 // outside the cube.
 __global__ void __launch_bounds__(512) k_slice_bf16(cudaTextureObject_t cube, int R,
-                                                    const int2* __restrict__ samples, int S, int Kpad,
-                                                    const float* __restrict__ views, int nom, float step,
-                                                    float d2r, long n0, __nv_bfloat162* __restrict__ B,
+                                                    const int2* __restrict__ samples, int S, int KH,
+                                                    const float* __restrict__ views, int nomr, float step,
+                                                    float d2r, long n0, __nv_bfloat16* __restrict__ B,
                                                     const float2* __restrict__ lin, float gk, float sc) {
     extern __shared__ float2 ssec[];
     __shared__ double sh[32];
     __shared__ float rot[9];
     const long n = n0 + blockIdx.x;
-    const int v = (int)(n / nom), io = (int)(n % nom);
+    const int v = (int)(n / nomr), io = (int)(n % nomr);
     if (threadIdx.x == 0) {
         euler_mat(views[2 * v], views[2 * v + 1], step * (float)io, d2r, rot);
         for (int i = 0; i < 9; ++i) rot[i] *= sc;  // cube voxels per frequency unit
@@ -148,17 +161,19 @@ __global__ void __launch_bounds__(512) k_slice_bf16(cudaTextureObject_t cube, in
     }
     const double nrm = block_sum_double((double)part, sh);
     const float inv = nrm > 0.0 ? (float)(1.0 / sqrt(nrm)) : 0.0f;
-    __nv_bfloat162* row = B + (long)blockIdx.x * (Kpad / 2);
-    for (int i = threadIdx.x; i < Kpad / 2; i += blockDim.x) {
-        float2 val = i < S ? ssec[i] : make_float2(0.f, 0.f);
-        row[bf16_pair_at(i, n)] = __floats2bfloat162_rn(val.x * inv, val.y * inv);
+    __nv_bfloat16* row = B + (long)blockIdx.x * (2 * KH);
+    for (int i = 2 * threadIdx.x; i < KH; i += 2 * blockDim.x) {
+        const float2 a = i < S ? ssec[i] : make_float2(0.f, 0.f);
+        const float2 c = i + 1 < S ? ssec[i + 1] : make_float2(0.f, 0.f);
+        *reinterpret_cast<__nv_bfloat162*>(row + bf16_at(i, n)) = __floats2bfloat162_rn(a.x * inv, c.x * inv);
+        *reinterpret_cast<__nv_bfloat162*>(row + bf16_at(KH + i, n)) = __floats2bfloat162_rn(a.y * inv, c.y * inv);
     }
 }
 
 // Local grids: one CTA per (particle p, grid point l) with l = (i * n + j) * n + k,
 // n = 2 m + 1, orientation (theta_p + (i - m) s, phi_p + (j - m) s, omega_p + (k - m) s)
 // from centre[3 p ..]; particle p's rows start at row p * lpitch (lpitch >= n^3); the
-// row is built exactly as k_slice_bf16 builds it.
+// row is interpolated and normalised as k_slice_bf16 does it, in (Re, Im) pairs.
 // With pctf (the CTF of each particle at each sample), a row is normalised by |CTF S|
 // instead of |S|: the particle's own grid, so the contraction's score is the unbiased
 // projection-matching correlation sum Re(P conj(CTF S)) / (|P| |CTF S|) (with A rows
@@ -312,18 +327,9 @@ __global__ void k_particle_norm(const float2* __restrict__ band, const float* __
     }
 }
 
-// The origin phase exp(i 2pi/n (sx hx + sy ky)) of a row of A is separable: the block
+// The origin phase exp(i 2pi/n (sx hx + sy ky)) of a row of A is separable: a block
 // tabulates (cos, sin) of 2pi/n sx hx for hx in [0, R] and of 2pi/n sy ky for ky in
 // [-R, R] (3R + 2 entries in shared memory) and multiplies the two per sample.
-__device__ __forceinline__ void origin_phasors(float sx, float sy, int R, float two_pi_over_n, float2* tab) {
-    for (int i = threadIdx.x; i < 3 * R + 2; i += blockDim.x) {
-        const float a = i <= R ? two_pi_over_n * (sx * (float)i) : two_pi_over_n * (sy * (float)(i - 2 * R - 1));
-        float sn, cs;
-        sincosf(a, &sn, &cs);
-        tab[i] = make_float2(cs, sn);
-    }
-    __syncthreads();
-}
 __device__ __forceinline__ void phasor_at(const float2* tab, int R, int2 hk, float* sn, float* cs) {
     const float2 ex = tab[hk.x], ey = tab[R + 1 + R + hk.y];
     *cs = ex.x * ey.x - ex.y * ey.y;
@@ -380,44 +386,499 @@ __global__ void __launch_bounds__(256) k_build_a(const float2* __restrict__ band
     }
 }
 
-// Per (particle, column tile): the best of its O origin rows -> (cc, orientation,
-// origin).  Distinct tiles hold distinct orientations.
-__global__ void k_tile_best(const float* __restrict__ topv, const int* __restrict__ topi, int O,
-                            int ntiles, float* __restrict__ bv_out, int* __restrict__ bo_out,
-                            int* __restrict__ borig_out) {
-    __shared__ float sv[32];
-    __shared__ int si[32];
-    const int t = blockIdx.x, p = blockIdx.y;
-    float bv = -3.0e38f;
-    int bi = -1;
-    for (int o = threadIdx.x; o < O; o += blockDim.x) {
-        const float v = topv[((long)p * O + o) * ntiles + t];
-        if (v > bv) { bv = v; bi = o; }
+// ---- the origin grid's basis ---------------------------------------------------
+// The global forms correlate ob.slots basis rows per particle instead of its origin grid
+// (origin_basis.h has the argument), and a half turn of omega instead of the whole: the
+// section at omega + 180 degrees is the complex conjugate of the section at omega (the map
+// is real), so with u = A_re B_re^T and v = A_im B_im^T, the two halves of K apart, the
+// scores are u + v at omega and u - v at omega + 180.  Where omega + 180 is not a grid point
+// (an odd number of omegas) the bank holds every omega and K is one piece.
+//
+// Row b = (m of x, k of y, part) of a particle: P exp(i 2 pi h.(mid + n/2 + off) / n) f_m(hx)
+// f_k(ky) i^(m odd + k odd) (the transform of q_m(x) q_k(y), f real by parity), times CTF and
+// 1/|CTF P|.  Part 1 holds what rounding part 0 to the operand type left.
+// HBM-write-bound: 160 rows x 25.6 KB a particle at box 256 (the origin grid is 625 rows:
+// 247 us a 64-particle pass against 82).
+constexpr int BO = 8;  // rows per block: a sample's transform, CTF and phase once for eight rows
+template <bool F8>
+__global__ void __launch_bounds__(256) k_build_basis(const float2* __restrict__ band, const float* __restrict__ ctf,
+                                                     Band bd, const int2* __restrict__ samples, int S, int KH,
+                                                     OriginDev ob, const float* __restrict__ poff,
+                                                     const double* __restrict__ norm, const float* __restrict__ mulA,
+                                                     const int* __restrict__ fexp, float two_pi_over_n,
+                                                     void* __restrict__ Aout) {
+    extern __shared__ float2 ptab[];  // [3 R + 2] origin phasors, then per row f_m [R + 1], f_k [2 R + 1]
+    const int b0 = blockIdx.x * BO, p = blockIdx.y, W = bd.W, R = bd.max_r, nt = 3 * R + 2, R1 = ob.R;
+    float* ft = reinterpret_cast<float*>(ptab + nt);
+    const float2* b = band + (long)p * W * W;
+    const float* c = ctf ? ctf + (long)p * W * W : nullptr;
+    const float sx = (float)(bd.nx / 2) + ob.mid + (poff ? poff[2 * p] : 0.0f);
+    const float sy = (float)(bd.nx / 2) + ob.mid + (poff ? poff[2 * p + 1] : 0.0f);
+    const float inv = norm[p] > 0.0 ? (float)(1.0 / sqrt(norm[p])) : 0.0f;
+    const float pscale = F8 ? ldexpf(1.0f, fexp[p]) : 1.0f;
+    int rot[BO], part[BO];  // rot: quarter turns of i^(...), part: -1 for an empty row
+#pragma unroll
+    for (int j = 0; j < BO; ++j) {
+        const int rw = ob.row[b0 + j];
+        const int m = rw & 0xfff, k = (rw >> 12) & 0xfff;
+        part[j] = rw < 0 ? -1 : (rw >> 24) & 1;
+        rot[j] = rw < 0 ? 0 : (m & 1) + (k & 1);
+        if (rw >= 0) {  // (the table covers |h| <= ob.R, the samples' band; zero beyond)
+            for (int i = threadIdx.x; i <= R; i += blockDim.x)
+                ft[j * nt + i] = i <= R1 ? ob.f[(long)m * (2 * R1 + 1) + R1 + i] : 0.0f;
+            for (int i = threadIdx.x; i < 2 * R + 1; i += blockDim.x)
+                ft[j * nt + R + 1 + i] = abs(i - R) <= R1 ? ob.f[(long)k * (2 * R1 + 1) + R1 + i - R] : 0.0f;
+        }
     }
-    for (int off = 16; off > 0; off >>= 1) {
-        float ov = __shfl_xor_sync(0xffffffffu, bv, off);
-        int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-        if (ov > bv || (ov == bv && oi >= 0 && oi < bi)) { bv = ov; bi = oi; }
+    for (int i = threadIdx.x; i < nt; i += blockDim.x) {
+        const float a = i <= R ? two_pi_over_n * (sx * (float)i) : two_pi_over_n * (sy * (float)(i - 2 * R - 1));
+        float sn, cs;
+        sincosf(a, &sn, &cs);
+        ptab[i] = make_float2(cs, sn);
     }
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-    if (l == 0) { sv[w] = bv; si[w] = bi; }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int q = 1; q < nw; ++q)
-            if (sv[q] > sv[0] || (sv[q] == sv[0] && si[q] >= 0 && si[q] < si[0])) { sv[0] = sv[q]; si[0] = si[q]; }
-        const long o = (long)p * ntiles + t;
-        bv_out[o] = sv[0];
-        borig_out[o] = si[0] < 0 ? 0 : si[0];
-        bo_out[o] = si[0] < 0 ? -1 : topi[((long)p * O + si[0]) * ntiles + t];
+    for (int i = 2 * threadIdx.x; i < KH; i += 2 * blockDim.x) {  // two samples a thread
+        float2 z[2];
+        int2 hk[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            z[u] = make_float2(0.f, 0.f);
+            hk[u] = make_int2(0, 0);
+            if (i + u < S) {
+                hk[u] = samples[i + u];
+                const int q = (hk[u].y + R) * W + (hk[u].x + R);
+                const float2 ab = b[q];  // (a, b) = (Re F, -Im F) referenced to pixel 0
+                const float cv = (c ? c[q] : 1.0f) * inv * (F8 ? mulA[i + u] * pscale : 1.0f);
+                float sn, cs;
+                phasor_at(ptab, R, hk[u], &sn, &cs);
+                // centshift: (a', b') = (a cos + b sin, -a sin + b cos); P = a' - i b'
+                z[u] = make_float2((ab.x * cs + ab.y * sn) * cv, (ab.x * sn - ab.y * cs) * cv);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < BO; ++j) {
+            float re[2], im[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float fv = part[j] < 0 ? 0.0f : ft[j * nt + hk[u].x] * ft[j * nt + 2 * R + 1 + hk[u].y];
+                const float x = z[u].x * fv, y = z[u].y * fv;
+                re[u] = rot[j] == 0 ? x : (rot[j] == 1 ? -y : -x);
+                im[u] = rot[j] == 0 ? y : (rot[j] == 1 ? x : -y);
+            }
+            const long row = (long)p * ob.slots + b0 + j;
+            if constexpr (F8) {
+                unsigned char* A = (unsigned char*)Aout + row * (2 * KH);
+                float2 vr = make_float2(re[0], re[1]), vi = make_float2(im[0], im[1]);
+                if (part[j] == 1) {
+                    const __half2 hr = __half2(__nv_cvt_fp8x2_to_halfraw2(__nv_cvt_float2_to_fp8x2(vr, __NV_SATFINITE, __NV_E4M3), __NV_E4M3));
+                    const __half2 hi = __half2(__nv_cvt_fp8x2_to_halfraw2(__nv_cvt_float2_to_fp8x2(vi, __NV_SATFINITE, __NV_E4M3), __NV_E4M3));
+                    vr = make_float2((vr.x - __low2float(hr)) * 16.0f, (vr.y - __high2float(hr)) * 16.0f);
+                    vi = make_float2((vi.x - __low2float(hi)) * 16.0f, (vi.y - __high2float(hi)) * 16.0f);
+                }
+                *reinterpret_cast<unsigned short*>(A + i) = __nv_cvt_float2_to_fp8x2(vr, __NV_SATFINITE, __NV_E4M3);
+                *reinterpret_cast<unsigned short*>(A + KH + i) = __nv_cvt_float2_to_fp8x2(vi, __NV_SATFINITE, __NV_E4M3);
+            } else {
+                __nv_bfloat16* A = (__nv_bfloat16*)Aout + row * (2 * KH);
+                __nv_bfloat162 vr = __floats2bfloat162_rn(re[0], re[1]), vi = __floats2bfloat162_rn(im[0], im[1]);
+                if (part[j] == 1) {
+                    vr = __floats2bfloat162_rn(re[0] - __low2float(vr), re[1] - __high2float(vr));
+                    vi = __floats2bfloat162_rn(im[0] - __low2float(vi), im[1] - __high2float(vi));
+                }
+                *reinterpret_cast<__nv_bfloat162*>(A + i) = vr;
+                *reinterpret_cast<__nv_bfloat162*>(A + KH + i) = vi;
+            }
+        }
     }
 }
 
-// Per particle: the k best entries of cnt (value, orientation, origin) triples, by
+// Expansion of the basis, one orientation per thread: C[o] = sum_mk c_mk q_m(x_o) q_k(y_o)
+// in FP32, c_mk the products of the function's rows (u or u +- v).  The functions are even
+// (m even) or odd, so a pair of mirror origins costs one pass: per pair of y the sums over
+// even and odd k apart give T_m at both, per pair of x the same over m; (even, odd) sums ride
+// in packed FP32x2 operations.  In one of origin_basis.h's fixed layouts the c_mk sit in
+// registers; more functions (origin ranges beyond ~7 px at maxR n/4) are read from C again for
+// every y (up_eval_gen).
+// emit(N, jy, jx, h[N], l[N]): (even, odd) sums over x at y hi and y lo for the pairs of x
+// jx .. jx + N - 1; the value at x hi is their sum, at x lo their difference, where hi =
+// n1/2 + j, lo = (n1-1)/2 - j.
+constexpr int UP_THREADS = 256, UP_GEN = 512, UP_N1 = 1024;
+// q at the upper half of the origins, [(n1 + 1) / 2][nb rounded up to even], zero beyond nb
+template <int LY> __host__ __device__ inline int up_table_floats(int n1) {
+    constexpr int NP = LY < 0 ? 0 : (OB_LAYOUT[LY < 0 ? 0 : LY].nb + 1) / 2 * 2;
+    return (n1 + 1) / 2 * NP;
+}
+template <int LY> __device__ __forceinline__ void up_table(const OriginDev& ob, float* sm) {
+    constexpr int NP = (OB_LAYOUT[LY].nb + 1) / 2 * 2;
+    for (int i = threadIdx.x; i < up_table_floats<LY>(ob.n1); i += blockDim.x) {
+        const int j = i / NP, m = i % NP;
+        sm[i] = m < ob.nb ? ob.q[(long)m * ob.n1 + ob.n1 / 2 + j] : 0.0f;
+    }
+}
+template <int LY> struct UpCoef {
+    static constexpr int NB = OB_LAYOUT[LY].nb, CUT = OB_LAYOUT[LY].cut, L2 = OB_LAYOUT[LY].second,
+                         ROWS = OB_LAYOUT[LY].rows, H = (NB + 1) / 2;
+    static __host__ __device__ constexpr bool in(int m, int k) { return m < NB && k < NB && m + k <= CUT; }
+    static __host__ __device__ constexpr bool pair(int m, int k) { return in(m, 2 * k) || in(m, 2 * k + 1); }
+    float2 c[2 * H][H];  // (k even, k odd) pairs; zero outside the layout
+    // get(i): product of row i; lo: scale of the second rows
+    template <class Get> __device__ __forceinline__ void load(float lo, Get get) {
+        int b = 0;
+#pragma unroll
+        for (int m = 0; m < 2 * H; ++m)
+#pragma unroll
+            for (int k = 0; k < H; ++k) {
+                c[m][k] = make_float2(0.f, 0.f);
+                if (in(m, 2 * k)) c[m][k].x = get(b++);
+                if (in(m, 2 * k + 1)) c[m][k].y = get(b++);
+            }
+#pragma unroll
+        for (int m = 0; m < L2; ++m)
+#pragma unroll
+            for (int k = 0; k < L2; ++k)
+                if (m + k < L2) {
+                    const float v = get(b++);
+                    if (k & 1) c[m][k / 2].y = fmaf(v, lo, c[m][k / 2].y);
+                    else c[m][k / 2].x = fmaf(v, lo, c[m][k / 2].x);
+                }
+    }
+};
+template <int LY, class Emit>
+__device__ __forceinline__ void up_eval(const OriginDev& ob, const UpCoef<LY>& cf, const float* sm, Emit emit) {
+    constexpr int H = UpCoef<LY>::H;
+    const int hn = (ob.n1 + 1) / 2;
+    const float2* q2 = reinterpret_cast<const float2*>(sm);
+    for (int jy = 0; jy < hn; ++jy) {
+        float2 qy[H];
+#pragma unroll
+        for (int k = 0; k < H; ++k) qy[k] = q2[jy * H + k];
+        float2 th[H], tl[H];  // (T_2k, T_2k+1) at y hi, y lo
+#pragma unroll
+        for (int m = 0; m < H; ++m) {
+            float2 e = make_float2(0.f, 0.f), o = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int k = 0; k < H; ++k) {
+                if (UpCoef<LY>::pair(2 * m, k)) e = __ffma2_rn(cf.c[2 * m][k], qy[k], e);
+                if (UpCoef<LY>::pair(2 * m + 1, k)) o = __ffma2_rn(cf.c[2 * m + 1][k], qy[k], o);
+            }
+            th[m] = make_float2(e.x + e.y, o.x + o.y);
+            tl[m] = make_float2(e.x - e.y, o.x - o.y);
+        }
+        // pairs of x four (two where the coefficients leave no registers), two, one at a time
+        auto pairs = [&](auto nc, int jx) {
+            constexpr int N = decltype(nc)::value;
+            float2 h[N], l[N];
+#pragma unroll
+            for (int u = 0; u < N; ++u) { h[u] = make_float2(0.f, 0.f); l[u] = make_float2(0.f, 0.f); }
+#pragma unroll
+            for (int k = 0; k < H; ++k)
+#pragma unroll
+                for (int u = 0; u < N; ++u) {
+                    const float2 qx = q2[(jx + u) * H + k];
+                    h[u] = __ffma2_rn(th[k], qx, h[u]);
+                    l[u] = __ffma2_rn(tl[k], qx, l[u]);
+                }
+            emit(nc, jy, jx, h, l);
+        };
+        int jx = 0;
+        constexpr int N = UpCoef<LY>::ROWS > 128 ? 2 : 4;
+        for (; jx + N <= hn; jx += N) pairs(std::integral_constant<int, N>(), jx);
+        if (N > 2 && jx + 2 <= hn) { pairs(std::integral_constant<int, 2>(), jx); jx += 2; }
+        if (jx < hn) pairs(std::integral_constant<int, 1>(), jx);
+    }
+}
+// product of function (m, k) at the column whose rows start at U, V (the two K shares; V null:
+// one share), sgn V's sign
+__device__ __forceinline__ float up_coef(const OriginDev& ob, const float* U, const float* V, float sgn, long pitch,
+                                         int m, int k) {
+    const int2 b = __ldg(ob.slot + (long)m * ob.nb + k);
+    float s = 0.0f;
+    if (b.x >= 0) {
+        s = U[b.x * pitch];
+        if (V) s = fmaf(sgn, V[b.x * pitch], s);
+    }
+    if (b.y >= 0) {
+        float c = U[b.y * pitch];
+        if (V) c = fmaf(sgn, V[b.y * pitch], c);
+        s = fmaf(c, ob.lo, s);
+    }
+    return s;
+}
+template <class Emit>
+__device__ __forceinline__ void up_eval_gen(const OriginDev& ob, const float* U, const float* V, float sgn, long pitch,
+                                            Emit emit) {
+    const int hn = (ob.n1 + 1) / 2;
+    float2 t[UP_GEN];  // (T_m at y hi, at y lo)
+    for (int jy = 0; jy < hn; ++jy) {
+        const int iy = ob.n1 / 2 + jy;
+        for (int m = 0; m < ob.nb; ++m) {
+            float e = 0.0f, o = 0.0f;
+            for (int k = 0; k < ob.nb; ++k) {
+                const float cq = up_coef(ob, U, V, sgn, pitch, m, k) * __ldg(ob.q + (long)k * ob.n1 + iy);
+                if (k & 1) o += cq;
+                else e += cq;
+            }
+            t[m] = make_float2(e + o, e - o);
+        }
+        for (int jx = 0; jx < hn; ++jx) {
+            float2 h = make_float2(0.f, 0.f), l = make_float2(0.f, 0.f);
+            for (int m = 0; m < ob.nb; ++m) {
+                const float q = __ldg(ob.q + (long)m * ob.n1 + ob.n1 / 2 + jx);
+                if (m & 1) { h.y = fmaf(t[m].x, q, h.y); l.y = fmaf(t[m].y, q, l.y); }
+                else { h.x = fmaf(t[m].x, q, h.x); l.x = fmaf(t[m].y, q, l.x); }
+            }
+            emit(std::integral_constant<int, 1>(), jy, jx, &h, &l);
+        }
+    }
+}
+
+// Best origin's value of every orientation of every particle.  Persistent blocks of 256
+// threads, one per SM; a tile is 128 bank rows, whose products (up to 160 rows of A x two K
+// shares = 160 KB) the block copies into shared memory with 16-byte cp.async, threads 0-127
+// taking the bank rows' omegas and threads 128-255 the ones half a turn on (one K share: 256
+// bank rows, a thread each).  Once the products are in registers the next tile's copies are
+// issued and land under the expansion.  FP32-issue-bound.  Measured at 625 origins and 2 x
+// 119,520 orientations: 87 us a particle; 480 us with each function's row looked up and
+// fetched by its thread (the loads' latency exposed), 118 us without the prefetch.
+template <int LY>
+__global__ void __launch_bounds__(UP_THREADS, 1) k_up_max(OriginDev ob, const float* __restrict__ C, long pitch,
+                                                          long rows, int nom, int nomr, int B,
+                                                          float* __restrict__ ccmax) {
+    constexpr int ROWS = OB_LAYOUT[LY].rows;
+    extern __shared__ __align__(16) float smem[];  // [share][row of A][columns], then the table of q
+    float* sq = smem + UP_THREADS * ROWS;
+    up_table<LY>(ob, sq);
+    const bool two = nom != nomr;
+    const int cols = two ? UP_THREADS / 2 : UP_THREADS;  // bank rows of a tile
+    const int ch = cols / 4;                             // 16-byte chunks of a row of a tile
+    const long ntile = (rows + cols - 1) / cols, total = ntile * B;
+    auto fetch = [&](long t) {
+        const long p = t / ntile, r0 = (t - p * ntile) * cols;
+        const float* src = C + p * (two ? 2 : 1) * ROWS * pitch + r0;  // (the shares' rows follow one another)
+        const int n = UP_THREADS * ROWS / 4;
+        for (int i = threadIdx.x; i < n; i += UP_THREADS) {
+            const int row = i / ch, c = i - row * ch;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem + 4 * i);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src + row * pitch + 4 * c) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    long t = blockIdx.x;
+    if (t < total) fetch(t);
+    const int cl = two ? threadIdx.x & (UP_THREADS / 2 - 1) : threadIdx.x, half = two ? threadIdx.x / (UP_THREADS / 2) : 0;
+    const float sgn = half ? -1.0f : 1.0f;
+    for (; t < total; t += gridDim.x) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        UpCoef<LY> c;
+        if (two)
+            c.load(ob.lo, [&](int i) { return fmaf(sgn, smem[(ROWS + i) * (UP_THREADS / 2) + cl], smem[i * (UP_THREADS / 2) + cl]); });
+        else
+            c.load(ob.lo, [&](int i) { return smem[i * UP_THREADS + cl]; });
+        __syncthreads();
+        if (t + gridDim.x < total) fetch(t + gridDim.x);
+        float best = -3.0e38f;
+        // the larger of e + o and e - o is e + |o|
+        up_eval<LY>(ob, c, sq, [&](auto nc, int, int, const float2* h, const float2* l) {
+#pragma unroll
+            for (int u = 0; u < decltype(nc)::value; ++u)
+                best = fmaxf(best, fmaxf(h[u].x + fabsf(h[u].y), l[u].x + fabsf(l[u].y)));
+        });
+        const long p = t / ntile, r = (t - p * ntile) * cols + cl;
+        if (r < rows) ccmax[p * (rows / nomr * nom) + r / nomr * nom + r % nomr + (long)half * nomr] = best;
+    }
+}
+// Any number of rows and functions: one thread per (bank row, particle, half turn).
+__global__ void __launch_bounds__(128) k_up_max_gen(OriginDev ob, const float* __restrict__ C, long pitch, long rows,
+                                                    int nom, int nomr, float* __restrict__ ccmax) {
+    const long r = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= rows) return;
+    const int p = blockIdx.y, parts = nom / nomr;
+    const float* U = C + (long)p * parts * ob.slots * pitch + r;
+    const float* V = parts > 1 ? U + ob.slots * pitch : nullptr;
+    float best = -3.0e38f;
+    up_eval_gen(ob, U, V, blockIdx.z ? -1.0f : 1.0f, pitch, [&](auto, int, int, const float2* h, const float2* l) {
+        best = fmaxf(best, fmaxf(h->x + fabsf(h->y), l->x + fabsf(l->y)));
+    });
+    ccmax[(long)p * (rows / nomr * nom) + r / nomr * nom + r % nomr + (long)blockIdx.z * nomr] = best;
+}
+
+// Per (particle, block of 256 orientations): the best value and its orientation.
+__global__ void __launch_bounds__(256) k_tile_best(const float* __restrict__ ccmax, long n_orient, int ntiles,
+                                                   float* __restrict__ bv_out, int* __restrict__ bo_out) {
+    __shared__ float sv[8];
+    __shared__ int si[8];
+    const int t = blockIdx.x, p = blockIdx.y;
+    const long n = (long)t * 256 + threadIdx.x;
+    float bv = n < n_orient ? ccmax[(long)p * n_orient + n] : -3.0e38f;
+    int bi = bv > -3.0e38f ? (int)n : -1;
+    for (int off = 16; off > 0; off >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
+        if (ov > bv || (ov == bv && oi >= 0 && oi < bi)) { bv = ov; bi = oi; }
+    }
+    if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = bv; si[threadIdx.x >> 5] = bi; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int q = 1; q < 8; ++q)
+            if (sv[q] > sv[0]) { sv[0] = sv[q]; si[0] = si[q]; }
+        bv_out[(long)p * ntiles + t] = sv[0];
+        bo_out[(long)p * ntiles + t] = si[0];
+    }
+}
+
+// Best origin (index iy n1 + ix) of the selected orientations: one block per (candidate,
+// particle), a thread per row of origins in turn.
+__global__ void __launch_bounds__(128) k_up_origin(OriginDev ob, const float* __restrict__ C, long pitch, int nom,
+                                                   int nomr, const int* __restrict__ orient, int k,
+                                                   int* __restrict__ origin) {
+    __shared__ float sv[4];
+    __shared__ int si[4];
+    const int p = blockIdx.y, parts = nom / nomr, n = orient[p * k + blockIdx.x];
+    float bv = -3.0e38f;
+    int bi = 0x7fffffff;
+    if (n >= 0) {
+        const int io = n % nom;
+        const long r = (long)(n / nom) * nomr + io % nomr;
+        const float* U = C + (long)p * parts * ob.slots * pitch + r;
+        const float* V = parts > 1 ? U + ob.slots * pitch : nullptr;
+        float t[UP_GEN];
+        for (int iy = threadIdx.x; iy < ob.n1; iy += blockDim.x) {
+            for (int m = 0; m < ob.nb; ++m) {
+                float s = 0.0f;
+                for (int q = 0; q < ob.nb; ++q)
+                    s = fmaf(up_coef(ob, U, V, io >= nomr ? -1.0f : 1.0f, pitch, m, q), ob.q[(long)q * ob.n1 + iy], s);
+                t[m] = s;
+            }
+            for (int ix = 0; ix < ob.n1; ++ix) {
+                float s = 0.0f;
+                for (int m = 0; m < ob.nb; ++m) s = fmaf(t[m], ob.q[(long)m * ob.n1 + ix], s);
+                if (s > bv) { bv = s; bi = iy * ob.n1 + ix; }
+            }
+        }
+    }
+    for (int off = 16; off > 0; off >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
+        if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+    }
+    if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = bv; si[threadIdx.x >> 5] = bi; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int q = 1; q < 4; ++q)
+            if (sv[q] > sv[0] || (sv[q] == sv[0] && si[q] < si[0])) { sv[0] = sv[q]; si[0] = si[q]; }
+        origin[p * k + blockIdx.x] = bi == 0x7fffffff && si[0] == 0x7fffffff ? 0 : si[0];
+    }
+}
+
+// Listed orientations (the proposal forms): one block per (block of 256 list positions,
+// particle) gives, per origin, the best of its positions and which it is (the first of
+// equal ones), as the argmax contraction does for a local grid's columns.  A warp takes 32
+// positions at a time and keeps its running maxima over the origins in shared memory (shm;
+// else one warp works on the output itself); the maximum of 32 lanes by redux on the
+// order-preserving integer image of the value, up to 16 origins at a time so that their
+// latencies overlap (one origin at a time, with its update in between: 185 us a 64-particle
+// pass of the box-256 search; so: 137 us).
+template <int LY>
+__global__ void __launch_bounds__(256, 1) k_up_list(OriginDev ob, const float* __restrict__ C, int parts,
+                                                    const UpGroup* __restrict__ groups, const int* __restrict__ map,
+                                                    float* __restrict__ topv, int* __restrict__ topi, int shm) {
+    extern __shared__ __align__(16) float smem[];
+    const UpGroup g = groups[blockIdx.y];
+    const int tile = blockIdx.x;
+    if (tile >= g.ntiles) return;
+    const int O = ob.n1 * ob.n1, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    float* sv = smem + up_table_floats<LY>(ob.n1);
+    int* si = reinterpret_cast<int*>(sv + nw * O);
+    float* ov = topv + g.topv_off + tile;  // stride ntiles
+    int* oi = topi + g.topv_off + tile;
+    long stride = 1;
+    if (shm) {
+        sv += warp * O;
+        si += warp * O;
+    } else {
+        sv = ov;
+        si = oi;
+        stride = g.ntiles;
+    }
+    if constexpr (LY >= 0) up_table<LY>(ob, smem);
+    for (int o = lane; o < O; o += 32) { sv[o * stride] = -3.0e38f; si[o * stride] = -1; }
+    __syncthreads();
+    const long pitch = 256L * g.n_tiles;
+    for (int c = warp; c < 8; c += nw) {
+        const int j0 = tile * 256 + c * 32;
+        if (j0 >= g.n_list) break;
+        const int j = j0 + lane;
+        const bool valid = j < g.n_list;
+        const int mp = map[g.map_off + (valid ? j : 0)];
+        const float* U = C + g.c_off + (mp >> 1);
+        const float* V = parts > 1 ? U + ob.slots * pitch : nullptr;
+        const float sgn = (mp & 1) ? -1.0f : 1.0f;
+        // 4 N origins at a time: their warp maxima are independent, lane i keeps the i-th and
+        // updates its running maximum
+        auto emit = [&](auto nc, int jy, int jx, const float2* h, const float2* l) {
+            constexpr int N = decltype(nc)::value;
+            float mine = 0.0f;
+            int who = -1;
+#pragma unroll
+            for (int u = 0; u < N; ++u) {
+                const float v[4] = {h[u].x + h[u].y, h[u].x - h[u].y, l[u].x + l[u].y, l[u].x - l[u].y};
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const unsigned x = __float_as_uint(v[q]);
+                    const unsigned key = valid ? ((x & 0x80000000u) ? ~x : (x | 0x80000000u)) : 0u;
+                    const unsigned mx = __reduce_max_sync(0xffffffffu, key);
+                    const unsigned eq = __ballot_sync(0xffffffffu, key == mx);
+                    if (lane == 4 * u + q) {
+                        mine = __uint_as_float((mx & 0x80000000u) ? (mx & 0x7fffffffu) : ~mx);
+                        who = __ffs(eq) - 1;
+                    }
+                }
+            }
+            if (who >= 0) {
+                const int jj = jx + (lane >> 2);
+                const int y = (lane & 2) ? (ob.n1 - 1) / 2 - jy : ob.n1 / 2 + jy;
+                const int x = (lane & 1) ? (ob.n1 - 1) / 2 - jj : ob.n1 / 2 + jj;
+                const long o = (long)(y * ob.n1 + x) * stride;
+                if (mine > sv[o]) {
+                    sv[o] = mine;
+                    si[o] = j0 + who;
+                }
+            }
+        };
+        if constexpr (LY >= 0) {
+            // (neighbouring list positions mostly stand for neighbouring columns)
+            UpCoef<LY> c;
+            c.load(ob.lo, [&](int i) {
+                const float u = __ldg(U + i * pitch);
+                return V ? fmaf(sgn, __ldg(V + i * pitch), u) : u;
+            });
+            up_eval<LY>(ob, c, smem, emit);
+        } else {
+            up_eval_gen(ob, U, V, sgn, pitch, emit);
+        }
+        __syncwarp();  // the next 32 positions update these maxima from other lanes
+    }
+    if (!shm) return;
+    __syncthreads();
+    sv = smem + up_table_floats<LY>(ob.n1);
+    si = reinterpret_cast<int*>(sv + nw * O);
+    for (int o = threadIdx.x; o < O; o += blockDim.x) {
+        float bv = -3.0e38f;
+        int bi = -1;
+        for (int w = 0; w < nw; ++w) {
+            const float x = sv[w * O + o];
+            const int i = si[w * O + o];
+            if (i >= 0 && (x > bv || (x == bv && i < bi))) { bv = x; bi = i; }
+        }
+        ov[(long)o * g.ntiles] = bv;
+        oi[(long)o * g.ntiles] = bi;
+    }
+}
+
+// Per particle: the k best entries of cnt (value, orientation) pairs, by
 // repeated block argmax (selected values are set to -inf in v, a scratch array).
-__global__ void k_select_topk(float* __restrict__ v, const int* __restrict__ orient,
-                              const int* __restrict__ origin, int cnt_per_particle, int k,
-                              int* __restrict__ out_orient, int* __restrict__ out_origin,
-                              float* __restrict__ out_cc) {
+__global__ void k_select_topk(float* __restrict__ v, const int* __restrict__ orient, int cnt_per_particle, int k,
+                              int* __restrict__ out_orient, float* __restrict__ out_cc) {
     __shared__ float sv[32];
     __shared__ long si[32];
     const int p = blockIdx.x;
@@ -445,12 +906,10 @@ __global__ void k_select_topk(float* __restrict__ v, const int* __restrict__ ori
                 if (sv[q] > v0 || (sv[q] == v0 && si[q] < i0 && si[q] >= 0)) { v0 = sv[q]; i0 = si[q]; }
             if (i0 >= 0 && v0 > -3.0e38f) {
                 out_orient[p * k + r] = orient[base + i0];
-                out_origin[p * k + r] = origin[base + i0];
                 out_cc[p * k + r] = v0;
                 topv[base + i0] = -3.0e38f;
             } else {
                 out_orient[p * k + r] = -1;
-                out_origin[p * k + r] = 0;
                 out_cc[p * k + r] = -3.0e38f;
             }
         }
@@ -662,16 +1121,16 @@ __device__ __forceinline__ int sample_band(int2 hk) {
 
 // Largest |Re| or |Im| of B per band over every stride-th row (float bits, non-negative,
 // so unsigned order is float order).
-__global__ void k_band_absmax(const __nv_bfloat162* __restrict__ B, long n, int Kpad, const int2* __restrict__ samples,
+__global__ void k_band_absmax(const __nv_bfloat16* __restrict__ B, long n, int KH, const int2* __restrict__ samples,
                               int S, int nband, int stride, unsigned* __restrict__ out) {
     extern __shared__ unsigned smax[];
     for (int b = threadIdx.x; b < nband; b += blockDim.x) smax[b] = 0u;
     __syncthreads();
     for (long r = (long)blockIdx.x * stride; r < n; r += (long)gridDim.x * stride) {
-        const __nv_bfloat162* row = B + r * (Kpad / 2);
+        const __nv_bfloat16* row = B + r * (2 * KH);
         for (int i = threadIdx.x; i < S; i += blockDim.x) {
-            const float2 v = __bfloat1622float2(row[bf16_pair_at(i, r)]);
-            const float m = fmaxf(fabsf(v.x), fabsf(v.y));
+            const float m = fmaxf(fabsf(__bfloat162float(row[bf16_at(i, r)])),
+                                  fabsf(__bfloat162float(row[bf16_at(KH + i, r)])));
             atomicMax(&smax[sample_band(samples[i])], __float_as_uint(m));
         }
     }
@@ -680,21 +1139,21 @@ __global__ void k_band_absmax(const __nv_bfloat162* __restrict__ B, long n, int 
         if (smax[b]) atomicMax(&out[b], smax[b]);
 }
 
-// One CTA per row: B8[r] = e4m3(B[r] * mulB[sample]), zero padded to Kpad8 bytes.
-__global__ void k_b_to_e4m3(const __nv_bfloat162* __restrict__ B, int Kpad, int S, const float* __restrict__ mulB,
-                            int Kpad8, unsigned short* __restrict__ B8) {
+// One CTA per row: B8[r] = e4m3(B[r] * mulB[sample]), both parts zero padded to KH8 bytes.
+__global__ void k_b_to_e4m3(const __nv_bfloat16* __restrict__ B, int KH, int S, const float* __restrict__ mulB,
+                            int KH8, unsigned char* __restrict__ B8) {
     const long r = blockIdx.x;
-    const __nv_bfloat162* row = B + r * (Kpad / 2);
-    unsigned short* out = B8 + r * (Kpad8 / 2);
-    for (int i = threadIdx.x; i < Kpad8 / 2; i += blockDim.x) {
-        float2 v = make_float2(0.f, 0.f);
-        if (i < S) {
-            v = __bfloat1622float2(row[bf16_pair_at(i, r)]);
-            v.x *= mulB[i];
-            v.y *= mulB[i];
+    const __nv_bfloat16* row = B + r * (2 * KH);
+    unsigned char* out = B8 + r * (2 * KH8);
+    for (int i = 2 * threadIdx.x; i < KH8; i += 2 * blockDim.x)
+#pragma unroll
+        for (int im = 0; im < 2; ++im) {
+            float2 v = make_float2(0.f, 0.f);
+            if (i < S) v.x = __bfloat162float(row[bf16_at(im * KH + i, r)]) * mulB[i];
+            if (i + 1 < S) v.y = __bfloat162float(row[bf16_at(im * KH + i + 1, r)]) * mulB[i + 1];
+            *reinterpret_cast<unsigned short*>(out + fp8_at(im * KH8 + i, r)) =
+                __nv_cvt_float2_to_fp8x2(v, __NV_SATFINITE, __NV_E4M3);
         }
-        out[fp8_pair_at(i, r)] = __nv_cvt_float2_to_fp8x2(v, __NV_SATFINITE, __NV_E4M3);
-    }
 }
 
 // Per particle: f_p = floor(log2(224 / max_i |A_i| mulA_i)) with |A_i| = |CTF P| / |A|.
@@ -723,76 +1182,105 @@ __global__ void k_particle_exp8(const float2* __restrict__ band, const float* __
     }
 }
 
-// Row (p, o) of A in e4m3: k_build_a's value x mulA[sample] x 2^f_p.
-__global__ void __launch_bounds__(256) k_build_a8(const float2* __restrict__ band, const float* __restrict__ ctf,
-                                                  Band bd, const int2* __restrict__ samples, int S, int Kpad8,
-                                                  const float* __restrict__ origins, int O,
-                                                  const float* __restrict__ poff,
-                                                  const double* __restrict__ norm, const float* __restrict__ mulA,
-                                                  const int* __restrict__ fexp, float two_pi_over_n,
-                                                  unsigned short* __restrict__ A8) {
-    extern __shared__ float2 ptab[];
-    const int o = blockIdx.x, p = blockIdx.y, W = bd.W, R = bd.max_r;
-    const float2* b = band + (long)p * W * W;
-    const float* c = ctf ? ctf + (long)p * W * W : nullptr;
-    const float h = (float)(bd.nx / 2);
-    const float sx = origins[2 * o] + h + (poff ? poff[2 * p] : 0.0f);
-    const float sy = origins[2 * o + 1] + h + (poff ? poff[2 * p + 1] : 0.0f);
-    const float inv = norm[p] > 0.0 ? (float)(1.0 / sqrt(norm[p])) : 0.0f;
-    const float pscale = ldexpf(1.0f, fexp[p]);
-    unsigned short* row = A8 + ((long)p * O + o) * (Kpad8 / 2);
-    origin_phasors(sx, sy, R, two_pi_over_n, ptab);
-    for (int i = threadIdx.x; i < Kpad8 / 2; i += blockDim.x) {
-        float re = 0.f, im = 0.f;
-        if (i < S) {
-            const int2 hk = samples[i];
-            const int q = (hk.y + R) * W + (hk.x + R);
-            const float2 ab = b[q];
-            float sn, cs;
-            phasor_at(ptab, R, hk, &sn, &cs);
-            const float a2 = ab.x * cs + ab.y * sn, b2 = -ab.x * sn + ab.y * cs;
-            const float cv = (c ? c[q] : 1.0f) * inv * mulA[i] * pscale;
-            re = a2 * cv;
-            im = -b2 * cv;
-        }
-        row[i] = __nv_cvt_float2_to_fp8x2(make_float2(re, im), __NV_SATFINITE, __NV_E4M3);
-    }
-}
-
 inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace
 
-cudaError_t launch_band_absmax(const void* B, long n, int Kpad, const int2* samples, int S, int nband, int stride,
+cudaError_t launch_band_absmax(const void* B, long n, int KH, const int2* samples, int S, int nband, int stride,
                                unsigned* out, int sms, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(out, 0, sizeof(unsigned) * nband, st);
     if (e != cudaSuccess) return e;
     long rows = (n + stride - 1) / stride;
     int grid = (int)(rows < 4L * sms ? rows : 4L * sms);
-    k_band_absmax<<<grid, 256, sizeof(unsigned) * nband, st>>>((const __nv_bfloat162*)B, n, Kpad, samples, S, nband,
+    k_band_absmax<<<grid, 256, sizeof(unsigned) * nband, st>>>((const __nv_bfloat16*)B, n, KH, samples, S, nband,
                                                                stride, out);
     return cudaGetLastError();
 }
 
-cudaError_t launch_b_to_e4m3(const void* B, long n, int Kpad, int S, const float* mulB, int Kpad8, void* B8,
+cudaError_t launch_b_to_e4m3(const void* B, long n, int KH, int S, const float* mulB, int KH8, void* B8,
                              cudaStream_t st) {
+    // (chunks of a multiple of 8 rows: a row's swizzle residue is its index in the bank)
     for (long r0 = 0; r0 < n; r0 += 1L << 30) {
         long nb = n - r0 < (1L << 30) ? n - r0 : (1L << 30);
-        k_b_to_e4m3<<<(unsigned)nb, 256, 0, st>>>((const __nv_bfloat162*)B + r0 * (Kpad / 2), Kpad, S, mulB, Kpad8,
-                                                  (unsigned short*)B8 + r0 * (Kpad8 / 2));
+        k_b_to_e4m3<<<(unsigned)nb, 256, 0, st>>>((const __nv_bfloat16*)B + r0 * (2 * KH), KH, S, mulB, KH8,
+                                                  (unsigned char*)B8 + r0 * (2 * KH8));
     }
     return cudaGetLastError();
 }
 
-void launch_build_a8(const float2* band, const float* ctf, Band bd, const int2* samples, int S, int Kpad8,
-                     const float* origins, int O, const double* norm, const float* mulA, int* fexp, int B, void* A8,
-                     cudaStream_t st, const float* poff) {
-    k_particle_exp8<<<B, 256, 0, st>>>(band, ctf, bd, samples, S, norm, mulA, fexp);
-    dim3 g(O, B);
+cudaError_t launch_build_basis(const float2* band, const float* ctf, Band bd, const int2* samples, int S, int KH,
+                               const OriginDev& ob, const double* norm, int B, void* A, bool f8, const float* mulA,
+                               int* fexp, cudaStream_t st, const float* poff) {
     const float tpn = 2.0f * host_angles().pi / (float)bd.nx;
-    k_build_a8<<<g, 256, sizeof(float2) * (3 * bd.max_r + 2), st>>>(band, ctf, bd, samples, S, Kpad8, origins, O,
-                                                                     poff, norm, mulA, fexp, tpn,
-                                  (unsigned short*)A8);
+    const dim3 g((ob.slots + BO - 1) / BO, B);
+    const size_t sm = (sizeof(float2) + sizeof(float) * BO) * (3 * (size_t)bd.max_r + 2);
+    if (f8) k_particle_exp8<<<B, 256, 0, st>>>(band, ctf, bd, samples, S, norm, mulA, fexp);
+    auto kern = f8 ? k_build_basis<true> : k_build_basis<false>;
+    if (sm > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if (e != cudaSuccess) return e;
+    }
+    kern<<<g, 256, sm, st>>>(band, ctf, bd, samples, S, KH, ob, poff, norm, mulA, fexp, tpn, A);
+    return cudaGetLastError();
+}
+
+// the register kernels: a fixed layout, and origins whose table leaves room for the products
+static int up_layout(const OriginDev& ob) { return ob.n1 <= UP_N1 ? ob.layout : -1; }
+
+cudaError_t launch_up_topk(const OriginDev& ob, const float* C, long pitch, long rows, int nom, int nomr, int B, int k,
+                           float* ccmax, int ntiles, float* tile_v, int* tile_o, int* orient, int* origin, float* cc,
+                           bool want_origin, int num_sms, cudaStream_t st) {
+    const long n_orient = rows / nomr * nom;
+    cudaError_t e = cudaSuccess;
+    const int ly = up_layout(ob);
+    if (ly >= 0) {
+        auto run = [&](auto lyc) {
+            constexpr int LY = decltype(lyc)::value;
+            const int cols = nom == nomr ? UP_THREADS : UP_THREADS / 2;
+            const long tiles = (rows + cols - 1) / cols * B;
+            const size_t sm = sizeof(float) * (up_table_floats<LY>(ob.n1) + (size_t)UP_THREADS * OB_LAYOUT[LY].rows);
+            e = cudaFuncSetAttribute(k_up_max<LY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            if (e != cudaSuccess) return;
+            k_up_max<LY><<<(unsigned)std::min<long>(tiles, num_sms), UP_THREADS, sm, st>>>(ob, C, pitch, rows, nom, nomr, B,
+                                                                                          ccmax);
+        };
+        switch (ly) {
+            case 0: run(std::integral_constant<int, 0>()); break;
+            case 1: run(std::integral_constant<int, 1>()); break;
+            case 2: run(std::integral_constant<int, 2>()); break;
+            case 3: run(std::integral_constant<int, 3>()); break;
+            default: run(std::integral_constant<int, 4>()); break;
+        }
+        if (e != cudaSuccess) return e;
+    } else {
+        const dim3 g((unsigned)((rows + 127) / 128), B, nom / nomr);
+        k_up_max_gen<<<g, 128, 0, st>>>(ob, C, pitch, rows, nom, nomr, ccmax);
+    }
+    k_tile_best<<<dim3(ntiles, B), 256, 0, st>>>(ccmax, n_orient, ntiles, tile_v, tile_o);
+    k_select_topk<<<B, 512, 0, st>>>(tile_v, tile_o, ntiles, k, orient, cc);
+    if (want_origin)
+        k_up_origin<<<dim3(k, B), 128, 0, st>>>(ob, C, pitch, nom, nomr, orient, k, origin);
+    else
+        return cudaMemsetAsync(origin, 0, sizeof(int) * (size_t)B * k, st);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_up_list(const OriginDev& ob, const float* C, int parts, const UpGroup* groups, int ngroups,
+                           int max_tiles, const int* map, float* topv, int* topi, cudaStream_t st) {
+    const int O = ob.n1 * ob.n1, ly = up_layout(ob);
+    // warps per block: the running maxima of each over the origins in shared memory; one warp
+    // on the output itself where a single one does not fit
+    const size_t tab = sizeof(float) * (ly >= 0 ? (ob.n1 + 1) / 2 * ((ob.nb + 1) / 2 * 2) : 0);
+    int nw = 8;
+    while (nw > 1 && tab + (size_t)nw * O * 8 > 220 * 1024) nw /= 2;
+    const bool shm = tab + (size_t)nw * O * 8 <= 220 * 1024;
+    const size_t sm = tab + (shm ? (size_t)nw * O * 8 : 0);
+    auto kern = ly < 0 ? k_up_list<-1> : ly == 0 ? k_up_list<0> : ly == 1 ? k_up_list<1> : ly == 2 ? k_up_list<2>
+                : ly == 3 ? k_up_list<3> : k_up_list<4>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    kern<<<dim3(max_tiles, ngroups), 32 * nw, sm, st>>>(ob, C, parts, groups, map, topv, topi, shm ? 1 : 0);
+    return cudaGetLastError();
 }
 
 void launch_map_checker(const float* map, int nx, float2* work, cudaStream_t st) {
@@ -836,19 +1324,16 @@ void free_cube_texture(cudaArray_t arr, cudaTextureObject_t tex) {
 }
 
 constexpr int SLICE_THREADS = 256;  // threads per section row
-cudaError_t launch_slice_bf16(cudaTextureObject_t cube, int R, const int2* samples, int S, int Kpad,
-                              const float* views, int nom, float step, long n0, long count, void* B,
+cudaError_t launch_slice_bf16(cudaTextureObject_t cube, int R, const int2* samples, int S, int KH,
+                              const float* views, int nomr, float step, long n0, long count, void* B,
                               cudaStream_t st, const float2* lin, float sigma, float sc) {
     const float gk = (lin && sigma > 0.0f) ? 1.0f / (2.0f * sigma * sigma) : 0.0f;
     size_t sm = (size_t)S * sizeof(float2);
     cudaError_t e = cudaFuncSetAttribute(k_slice_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    for (long c0 = 0; c0 < count; c0 += 65535) {
-        long nb = count - c0 < 65535 ? count - c0 : 65535;
-        k_slice_bf16<<<(unsigned)nb, SLICE_THREADS, sm, st>>>(cube, R, samples, S, Kpad, views, nom, step,
-                                                   host_angles().deg2rad, n0 + c0,
-                                                   (__nv_bfloat162*)B + c0 * (Kpad / 2), lin, gk, sc);
-    }
+    k_slice_bf16<<<(unsigned)count, SLICE_THREADS, sm, st>>>(cube, R, samples, S, KH, views, nomr, step,
+                                                             host_angles().deg2rad, n0, (__nv_bfloat16*)B, lin, gk,
+                                                             sc);
     return cudaGetLastError();
 }
 
@@ -897,14 +1382,6 @@ void launch_build_a(const float2* band, const float* ctf, Band bd, const int2* s
     if (sm > 48 * 1024) cudaFuncSetAttribute(k_build_a, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     k_build_a<<<ga, 256, sm, st>>>(band, ctf, bd, samples, S, Kpad, origins, O, poff, norm, tpn,
                                    (__nv_bfloat162*)A);
-}
-
-void launch_select_topk(const float* topv, const int* topi, int O, int ntiles, int k, int B,
-                        float* tile_v, int* tile_o, int* tile_orig, int* orient, int* origin, float* cc,
-                        cudaStream_t st) {
-    dim3 g(ntiles, B);
-    k_tile_best<<<g, 256, 0, st>>>(topv, topi, O, ntiles, tile_v, tile_o, tile_orig);
-    k_select_topk<<<B, 512, 0, st>>>(tile_v, tile_o, tile_orig, ntiles, k, orient, origin, cc);
 }
 
 void launch_select_distinct(float* topv, const int* topi, int O, const int2* seg, int B, int k, int* col,

@@ -3,8 +3,9 @@
 // TMA), with a fused per-tile argmax epilogue.  This is the dense cross-correlation of the
 // projection-matching form: C[m, n] = sum_k A[m, k] B[n, k] with both operands K-major,
 // where a row of A is one (particle, origin) and a row of B one orientation's central
-// section.  The full C is never stored: each (row, 256-column tile) reduces to
-// (max, argmax).
+// section.  The local form never stores C: each (row, 256-column tile) reduces to
+// (max, argmax).  The global forms, whose rows of A are the origin grid's basis, keep their few
+// rows of products (STORE below).
 //
 // Persistent kernel, one CTA per SM, 704 threads:
 //   warp 0    : TMA producer (one lane) filling a 4-stage ring of 128-row A and 256-row
@@ -39,7 +40,7 @@ namespace {
 constexpr int GM = 128, GN = 256, GKB = 128, NSTAGE = 4;  // GKB: bytes of K per stage
 constexpr int A_BYTES = GM * GKB, B_BYTES = GN * GKB;
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int TMEM_COLS = 512;
+constexpr int TMEM_COLS = 512, MAX_ACC = 5;
 constexpr int NWARP_CORE = 6, NWARP_B = 16;  // producer, issuer, 4 epilogue; B loaders (b_mode 2)
 // B loaders: cp.async groups (stages) in flight before the oldest is waited for and
 // signalled.  The signal of stage s follows the issue of stage s + B_LAG, which waits for
@@ -90,33 +91,42 @@ __device__ __forceinline__ void tc_fence_before() { tc::fence_before(); }
 __device__ __forceinline__ void tc_fence_after() { tc::fence_after(); }
 __device__ __forceinline__ void tc_commit(uint64_t* b) { tc::commit(b); }
 template <bool F8>
-__device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t bdesc, uint32_t acc) {
+__device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t bdesc, uint32_t acc, uint32_t idesc) {
     if constexpr (F8) {
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
             "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}" ::"r"(d),
-            "l"(a), "l"(bdesc), "r"(IDESC_E4M3), "r"(acc)
+            "l"(a), "l"(bdesc), "r"(idesc), "r"(acc)
             : "memory");
     } else {
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d),
-            "l"(a), "l"(bdesc), "r"(IDESC_BF16), "r"(acc)
+            "l"(a), "l"(bdesc), "r"(idesc), "r"(acc)
             : "memory");
     }
 }
 // Tile t of the launch -> its product, tile coordinates and operand rows.
 struct TileAt {
-    int mt, nt, a_row, b_row, m_valid, n_valid, n_tiles, topv_off;
+    int mt, nt, part, a_row, b_row, m_valid, n_valid, n_tiles, topv_off;
+    long c_off;
 };
+// k_parts > 1 (stored products): a tile is k_parts units of work, each over its own share of
+// K; the units of one tile column that read the same B rows are adjacent.
 __device__ __forceinline__ TileAt tile_at(const GemmArgmaxArgs& g, int t) {
     TileAt r;
+    r.part = 0;
+    r.c_off = 0;
     if (!g.groups) {
         r.mt = t % g.m_tiles;
         r.nt = t / g.m_tiles;
-        r.a_row = r.mt * GM;
+        if (g.k_parts > 1) {
+            r.part = r.nt % g.k_parts;
+            r.nt /= g.k_parts;
+        }
+        r.a_row = r.mt * (g.cstore ? g.c_rows : GM);
         r.b_row = r.nt * GN;
         r.m_valid = g.m_valid;
         r.n_valid = g.n_valid;
@@ -130,7 +140,12 @@ __device__ __forceinline__ TileAt tile_at(const GemmArgmaxArgs& g, int t) {
     const int local = t - __ldg(&G->tile_start), mtiles = __ldg(&G->m_tiles);
     r.mt = local % mtiles;
     r.nt = local / mtiles;
-    r.a_row = __ldg(&G->a_row0) + r.mt * GM;
+    if (g.k_parts > 1) {
+        r.part = r.nt % g.k_parts;
+        r.nt /= g.k_parts;
+    }
+    r.c_off = __ldg(&G->c_off);
+    r.a_row = __ldg(&G->a_row0) + r.mt * (g.cstore ? g.c_rows : GM);
     r.b_row = __ldg(&G->b_row0) + r.nt * GN;
     r.m_valid = __ldg(&G->m_valid);
     r.n_valid = __ldg(&G->n_valid);
@@ -140,7 +155,15 @@ __device__ __forceinline__ TileAt tile_at(const GemmArgmaxArgs& g, int t) {
 }
 
 // F8 = false: BF16 operands, 64 elements of K per stage; true: FP8-e4m3, 128 elements.
-template <bool F8>
+// STORE = false: each (row, tile) reduces to its maximum and column.  STORE = true: the
+// products are kept, for the kernels that expand the origin basis (contract.cu), and the
+// operands change places in the MMA: a stage's 256 section rows are the M side (two MMAs of
+// M128), the c_rows rows of A (a multiple of 32, up to 160) the N side, so a particle takes
+// exactly its rows (154 functions in two 128-row M tiles would do 1.6 times the work).  The 256
+// columns x c_rows of a unit (mt, nt, K share) are two accumulators in a ring of 512 / c_rows;
+// a thread owns a TMEM lane = one section, so a warp's store of one basis row is one 128-byte
+// line of GemmArgmaxArgs::cstore, under the next unit's MMAs.
+template <bool F8, bool STORE>
 __global__ void __launch_bounds__(NTHREADS, 1)
     k_gemm_argmax(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                   GemmArgmaxArgs g) {
@@ -148,13 +171,16 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     extern __shared__ unsigned char smem_raw[];
     unsigned char* sm = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* sA = sm;
-    unsigned char* sB = sm + NSTAGE * A_BYTES;
+    const int a_bytes = STORE ? g.c_rows * GKB : A_BYTES;
+    unsigned char* sB = sm + NSTAGE * a_bytes;
     uint64_t* bars = (uint64_t*)(sB + NSTAGE * B_BYTES);
     uint64_t* full = bars;
     uint64_t* empty = bars + NSTAGE;
+    // accumulators: two of 256 columns, or (STORE) a ring of 512 / c_rows of c_rows columns
+    const int nacc = STORE ? min(MAX_ACC, TMEM_COLS / g.c_rows) : 2, acc_cols = STORE ? g.c_rows : GN;
     uint64_t* accf = bars + 2 * NSTAGE;
-    uint64_t* acce = accf + 2;
-    uint64_t* drain = acce + 2;
+    uint64_t* acce = accf + MAX_ACC;
+    uint64_t* drain = acce + MAX_ACC;
     uint32_t* tmem_slot = (uint32_t*)(drain + 1);
     // b_mode 2: per tile row, the byte offset of its bank row | the bank row's residue
     unsigned long long* srow = (unsigned long long*)((unsigned char*)bars + 256);
@@ -164,7 +190,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         // b_mode 2: a stage is full after the A copy's arrival (with its bytes) and each B
         // loader warp's arrival once its copies have landed
         for (int s = 0; s < NSTAGE; ++s) { mbar_init(full + s, g.b_mode == 2 ? 1 + NWARP_B : 1); mbar_init(empty + s, 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(accf + b, 1); mbar_init(acce + b, 128); }
+        for (int b = 0; b < nacc; ++b) { mbar_init(accf + b, 1); mbar_init(acce + b, 128); }
         mbar_init(drain, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&tmA) : "memory");
@@ -181,7 +207,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    const int total = g.groups ? g.total_tiles : g.m_tiles * g.n_tiles;
+    const int total = g.groups ? g.total_tiles : g.m_tiles * g.n_tiles * g.k_parts;
 
     if (warp >= NWARP_CORE) {
         // B rows by index (b_mode 2; idle otherwise): warp w of the NWARP_B loaders copies
@@ -215,11 +241,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     soff[j] = (unsigned long long)(n * g.b_row_bytes) | (unsigned long long)(n & 7);
                 }
                 __syncwarp();
+                const int kb0 = ta.part * g.kblocks;
                 for (int kb = 0; kb < g.kblocks; ++kb) {
                     const bool okl = mbar_wait(empty + s, ph ^ 1u, g.err, true, g.wait_ns);
                     if (!__all_sync(0xffffffffu, okl)) { ok = false; break; }
                     const uint32_t sb = su32(sB + s * B_BYTES) + (uint32_t)(wb * (GN / NWARP_B) * 128);
-                    const unsigned char* src0 = g.b_rows + (long)kb * GKB + p * 16;
+                    const unsigned char* src0 = g.b_rows + (long)(kb0 + kb) * GKB + p * 16;
 #pragma unroll
                     for (int i = 0; i < GN / NWARP_B / 4; ++i) {
                         const int r = 4 * i + rq;  // row within this warp's 64 (same residue as in the tile)
@@ -255,9 +282,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                         if (++s == NSTAGE) { s = 0; ph ^= 1u; }
                         continue;
                     }
-                    mbar_expect_tx(full + s, g.b_mode == 2 ? A_BYTES : STAGE_BYTES);
-                    tma_load_2d(sA + s * A_BYTES, &tmA, kb * GK, ta.a_row, full + s);
-                    if (g.b_mode != 2) tma_load_2d(sB + s * B_BYTES, &tmB, kb * GK, ta.b_row, full + s);
+                    mbar_expect_tx(full + s, g.b_mode == 2 ? a_bytes : a_bytes + B_BYTES);
+                    tma_load_2d(sA + s * a_bytes, &tmA, (ta.part * g.kblocks + kb) * GK, ta.a_row, full + s);
+                    if (g.b_mode != 2)
+                        tma_load_2d(sB + s * B_BYTES, &tmB, (ta.part * g.kblocks + kb) * GK, ta.b_row, full + s);
                     used[s] = true;
                     last_par[s] = ph;
                     if (++s == NSTAGE) { s = 0; ph ^= 1u; }
@@ -272,6 +300,41 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             int s = 0, lt = 0;
             uint32_t ph = 0;
             bool ok = true;
+            if constexpr (STORE) {
+                const uint32_t idesc = (F8 ? 0u : (1u << 7) | (1u << 10)) | (1u << 4) | ((uint32_t)(g.c_rows >> 3) << 17) |
+                                       ((uint32_t)(GM >> 4) << 24);
+                int a0 = 0;         // ring slot of the unit's first accumulator
+                uint32_t aph = 0;   // its phase
+                for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+                    const int a1 = a0 + 1 == nacc ? 0 : a0 + 1;
+                    const uint32_t aph1 = a0 + 1 == nacc ? aph ^ 1u : aph;
+                    if (!mbar_wait(acce + a0, aph ^ 1u, g.err, true, g.wait_ns)) break;
+                    const uint32_t d0 = tmem + (uint32_t)(a0 * acc_cols), d1 = tmem + (uint32_t)(a1 * acc_cols);
+                    for (int kb = 0; kb < g.kblocks; ++kb) {
+                        if (!mbar_wait(full + s, ph, g.err, true, g.wait_ns)) { ok = false; break; }
+                        tc_fence_after();
+                        const uint32_t sa = su32(sA + s * a_bytes), sb = su32(sB + s * B_BYTES);
+#pragma unroll
+                        for (int kk = 0; kk < GKB / 32; ++kk)
+                            tc_mma<F8>(d0, sdesc(sb + kk * 32), sdesc(sa + kk * 32), (kb | kk) != 0, idesc);
+                        if (kb == 0) {
+                            if (!mbar_wait(acce + a1, aph1 ^ 1u, g.err, true, g.wait_ns)) { ok = false; break; }
+                            tc_fence_after();
+                        }
+#pragma unroll
+                        for (int kk = 0; kk < GKB / 32; ++kk)
+                            tc_mma<F8>(d1, sdesc(sb + GM * GKB + kk * 32), sdesc(sa + kk * 32), (kb | kk) != 0, idesc);
+                        tc_commit(empty + s);
+                        if (++s == NSTAGE) { s = 0; ph ^= 1u; }
+                    }
+                    if (ok) {
+                        tc_commit(accf + a0);
+                        tc_commit(accf + a1);
+                    }
+                    a0 = a1 + 1 == nacc ? 0 : a1 + 1;
+                    aph = a1 + 1 == nacc ? aph1 ^ 1u : aph1;
+                }
+            } else {
             for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++lt) {
                 const int b = lt & 1;
                 const uint32_t aph = (uint32_t)(lt >> 1) & 1u;
@@ -284,11 +347,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     const uint32_t a0 = su32(sA + s * A_BYTES), b0 = su32(sB + s * B_BYTES);
 #pragma unroll
                     for (int kk = 0; kk < GKB / 32; ++kk)
-                        tc_mma<F8>(d, sdesc(a0 + kk * 32), sdesc(b0 + kk * 32), (kb | kk) != 0);
+                        tc_mma<F8>(d, sdesc(a0 + kk * 32), sdesc(b0 + kk * 32), (kb | kk) != 0,
+                                   F8 ? IDESC_E4M3 : IDESC_BF16);
                     tc_commit(empty + s);
                     if (++s == NSTAGE) { s = 0; ph ^= 1u; }
                 }
                 if (ok) tc_commit(accf + b);
+            }
             }
             // all issued MMAs complete before TMEM is released
             tc_commit(drain);
@@ -297,6 +362,33 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     } else if (warp >= 2) {
         const int q = warp & 3;
         const int row_in_tile = 32 * q + lane;
+        if constexpr (STORE) {
+            int ai = 0;
+            uint32_t aph = 0;
+            bool ok = true;
+            for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+                const TileAt ta = tile_at(g, t);
+                // (block, its unit of c_rows rows): ta.mt counts the units of all blocks of the launch
+                const int blk = ta.mt / g.c_units, unit = ta.mt % g.c_units;
+                const long pitch = (long)ta.n_tiles * GN;
+                float* out0 = g.cstore + ta.c_off +
+                              (((long)blk * g.k_parts + ta.part) * g.c_units + unit) * g.c_rows * pitch + (long)ta.nt * GN;
+                for (int sub = 0; sub < 2; ++sub) {
+                    if (!mbar_wait(accf + ai, aph, g.err, true, g.wait_ns)) { ok = false; break; }
+                    tc_fence_after();
+                    float* out = out0 + sub * GM + row_in_tile;
+                    for (int c = 0; c < g.c_rows; c += 32) {
+                        float v[32];
+                        tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(ai * acc_cols + c), v);
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) out[(long)(c + j) * pitch] = v[j];
+                    }
+                    tc_fence_before();
+                    mbar_arrive(acce + ai);
+                    if (++ai == nacc) { ai = 0; aph ^= 1u; }
+                }
+            }
+        } else {
         int lt = 0;
         for (int t = blockIdx.x; t < total; t += gridDim.x, ++lt) {
             const int b = lt & 1;
@@ -327,6 +419,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 g.topv[ta.topv_off + row * ta.n_tiles + ta.nt] = best;
                 g.topi[ta.topv_off + row * ta.n_tiles + ta.nt] = bi;
             }
+        }
         }
     }
     tc_fence_before();
@@ -374,26 +467,48 @@ bool make_map(CUtensorMap* m, const void* base, long rows, int k, int box_rows, 
 int gemm_tile_n() { return GN; }
 int gemm_tile_m() { return GM; }
 
+// the kernel of an operand type and output form, its shared memory allowed
+static cudaError_t gemm_kernel(bool f8, bool store, int smem,
+                               void (**kern)(const CUtensorMap, const CUtensorMap, GemmArgmaxArgs)) {
+    *kern = f8 ? (store ? k_gemm_argmax<true, true> : k_gemm_argmax<true, false>)
+               : (store ? k_gemm_argmax<false, true> : k_gemm_argmax<false, false>);
+    return cudaFuncSetAttribute(*kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+}
+// stored products: units of c_rows rows (whole 32-column reads of TMEM, two accumulators and a
+// stage's tiles within TMEM and shared memory), K in k_parts equal shares of whole stages
+static bool store_ok(const GemmArgmaxArgs& g, int K, int gk) {
+    if (!g.cstore) return g.k_parts == 1;
+    return g.c_rows >= 32 && g.c_rows <= 160 && g.c_rows % 32 == 0 && g.c_units >= 1 && g.k_parts >= 1 &&
+           K % (gk * g.k_parts) == 0 && !g.cfull;
+}
+static int store_rows(const GemmArgmaxArgs& g) { return g.cstore ? g.c_rows : GM; }
+static int gemm_smem(const GemmArgmaxArgs& g) {
+    return g.cstore ? SMEM_BYTES + NSTAGE * (g.c_rows * GKB - A_BYTES) : SMEM_BYTES;
+}
+
 cudaError_t launch_gemm_argmax(const void* a, const void* b, int M, int N, int K, bool f8,
                                const GemmArgmaxArgs& in, int num_sms, cudaStream_t st) {
     const int gk = f8 ? GKB : GKB / 2;
-    if (K % gk != 0 || M < 1 || N < 1) return cudaErrorInvalidValue;
+    if (K % gk != 0 || M < 1 || N < 1 || !store_ok(in, K, gk)) return cudaErrorInvalidValue;
+    if (in.cstore && M % (in.c_units * in.c_rows)) return cudaErrorInvalidValue;
     if (((uintptr_t)a & 15) || ((uintptr_t)b & 15)) return cudaErrorInvalidValue;
     CUtensorMap ta, tb;
-    if (!make_map(&ta, a, M, K, GM, f8) || !make_map(&tb, b, N, K, GN, f8, in.b_mode == 0))
+    if (!make_map(&ta, a, M, K, store_rows(in), f8) || !make_map(&tb, b, N, K, GN, f8, in.b_mode == 0))
         return cudaErrorInvalidValue;
     GemmArgmaxArgs g = in;
-    g.m_tiles = (M + GM - 1) / GM;
+    g.m_tiles = (M + store_rows(in) - 1) / store_rows(in);
     g.n_tiles = (N + GN - 1) / GN;
-    g.kblocks = K / gk;
+    g.kblocks = K / gk / g.k_parts;
     g.m_valid = M;
     g.n_valid = N;
-    auto kern = f8 ? k_gemm_argmax<true> : k_gemm_argmax<false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    void (*kern)(const CUtensorMap, const CUtensorMap, GemmArgmaxArgs) = nullptr;
+    const int smem = gemm_smem(in);
+    cudaError_t e = gemm_kernel(f8, in.cstore != nullptr, smem, &kern);
     if (e != cudaSuccess) return e;
-    int total = g.m_tiles * g.n_tiles;
+    if ((long)g.m_tiles * g.n_tiles * g.k_parts > (1L << 30)) return cudaErrorInvalidValue;
+    int total = g.m_tiles * g.n_tiles * g.k_parts;
     int grid = total < num_sms ? total : num_sms;
-    kern<<<grid, NTHREADS, SMEM_BYTES, st>>>(ta, tb, g);
+    kern<<<grid, NTHREADS, smem, st>>>(ta, tb, g);
     return cudaGetLastError();
 }
 
@@ -401,7 +516,8 @@ cudaError_t launch_gemm_argmax_grouped(const void* a, long Mtot, const void* b, 
                                        GemmGroup* hg, int ngroups, GemmGroup* dg, const GemmArgmaxArgs& in,
                                        int num_sms, cudaStream_t st) {
     const int gk = f8 ? GKB : GKB / 2;
-    if (K % gk != 0 || Mtot < 1 || Ntot < 1 || ngroups < 1 || in.cfull) return cudaErrorInvalidValue;
+    if (K % gk != 0 || Mtot < 1 || Ntot < 1 || ngroups < 1 || in.cfull || !store_ok(in, K, gk))
+        return cudaErrorInvalidValue;
     if (((uintptr_t)a & 15) || ((uintptr_t)b & 15)) return cudaErrorInvalidValue;
     long total = 0;
     for (int i = 0; i < ngroups; ++i) {
@@ -409,10 +525,11 @@ cudaError_t launch_gemm_argmax_grouped(const void* a, long Mtot, const void* b, 
         if (q.m_valid < 1 || q.n_valid < 1 || q.a_row0 < 0 || q.b_row0 < 0 ||
             (long)q.a_row0 + q.m_valid > Mtot || (long)q.b_row0 + q.n_valid > Ntot)
             return cudaErrorInvalidValue;
-        q.m_tiles = (q.m_valid + GM - 1) / GM;
+        q.m_tiles = (q.m_valid + store_rows(in) - 1) / store_rows(in);
         q.n_tiles = (q.n_valid + GN - 1) / GN;
+        if (in.cstore && q.m_valid != in.c_units * in.c_rows) return cudaErrorInvalidValue;
         q.tile_start = (int)total;
-        total += (long)q.m_tiles * q.n_tiles;
+        total += (long)q.m_tiles * q.n_tiles * in.k_parts;
     }
     if (total > (1L << 30)) return cudaErrorInvalidValue;
     if (in.b_mode == 1)  // pre-swizzled rows: every group's tiles start at a multiple of 8 rows
@@ -423,7 +540,7 @@ cudaError_t launch_gemm_argmax_grouped(const void* a, long Mtot, const void* b, 
                            in.b_row_bytes % 16 || in.b_row_bytes < (long)K * (f8 ? 1 : 2)))
         return cudaErrorInvalidValue;
     CUtensorMap ta, tb;
-    if (!make_map(&ta, a, Mtot, K, GM, f8)) return cudaErrorInvalidValue;
+    if (!make_map(&ta, a, Mtot, K, store_rows(in), f8)) return cudaErrorInvalidValue;
     if (in.b_mode == 2)
         tb = ta;  // not read
     else if (!make_map(&tb, b, Ntot, K, GN, f8, in.b_mode == 0))
@@ -434,12 +551,13 @@ cudaError_t launch_gemm_argmax_grouped(const void* a, long Mtot, const void* b, 
     g.groups = dg;
     g.ngroups = ngroups;
     g.total_tiles = (int)total;
-    g.kblocks = K / gk;
-    auto kern = f8 ? k_gemm_argmax<true> : k_gemm_argmax<false>;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    g.kblocks = K / gk / g.k_parts;
+    void (*kern)(const CUtensorMap, const CUtensorMap, GemmArgmaxArgs) = nullptr;
+    const int smem = gemm_smem(in);
+    e = gemm_kernel(f8, in.cstore != nullptr, smem, &kern);
     if (e != cudaSuccess) return e;
     const int grid = total < num_sms ? (int)total : num_sms;
-    kern<<<grid, NTHREADS, SMEM_BYTES, st>>>(ta, tb, g);
+    kern<<<grid, NTHREADS, smem, st>>>(ta, tb, g);
     return cudaGetLastError();
 }
 

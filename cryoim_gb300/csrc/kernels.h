@@ -156,6 +156,7 @@ cudaError_t launch_insert(const InsertArgs& a, int B, cudaStream_t st);
 // topv/topi + topv_off as [m_valid][n_tiles], columns counted from b_row0.
 struct GemmGroup {
     int tile_start, m_tiles, a_row0, m_valid, b_row0, n_valid, n_tiles, topv_off;
+    long c_off;  // stored products: offset of the group's block in cstore, floats
 };
 struct GemmArgmaxArgs {
     int m_tiles, n_tiles, kblocks, m_valid, n_valid;  // set by the launcher
@@ -178,6 +179,12 @@ struct GemmArgmaxArgs {
     // b_index[b_row0 + j] of b_rows (b_row_bytes apart), copied into the tile by the
     // producer warp's 16-byte cp.async with the chunks re-swizzled for the tile row
     int b_mode = 0;
+    // stored products instead of maxima: block b of the launch or of its group (c_units x
+    // c_rows rows of A: one particle's), K share s of k_parts, row m of the block, column n (of
+    // n_tiles x 256) at cstore[c_off + ((b k_parts + s) c_units c_rows + m) n_tiles 256 + n];
+    // columns past the last valid one hold products of padding rows
+    float* cstore = nullptr;
+    int k_parts = 1, c_units = 1, c_rows = 128;
     const int* b_index = nullptr;
     const unsigned char* b_rows = nullptr;
     long b_row_bytes = 0;
@@ -205,12 +212,13 @@ void launch_map_band(const float2* ft, int nx, int R, float2* cube, cudaStream_t
 cudaError_t make_cube_texture(const float2* cube, int R, cudaStream_t st, cudaArray_t* arr,
                               cudaTextureObject_t* tex);
 void free_cube_texture(cudaArray_t arr, cudaTextureObject_t tex);
-// Rows n0 .. n0+count-1 of B (orientation n = view * nom + iomega), unit norm, BF16.
+// Rows n0 .. n0+count-1 of a section bank (row n = view * nomr + iomega), unit norm, BF16,
+// the real parts of the S samples in elements [0, KH) of a row, the imaginary in [KH, 2 KH).
 // sigma > 0 (with lin = the band cube in memory): Gaussian-kernel interpolation of
 // width sigma voxels over the 27 voxels around the nearest one instead of the texture's
 // trilinear filtering
-cudaError_t launch_slice_bf16(cudaTextureObject_t cube, int R, const int2* samples, int S, int Kpad,
-                              const float* views, int nom, float step, long n0, long count, void* B,
+cudaError_t launch_slice_bf16(cudaTextureObject_t cube, int R, const int2* samples, int S, int KH,
+                              const float* views, int nomr, float step, long n0, long count, void* B,
                               cudaStream_t st, const float2* lin = nullptr, float sigma = 0.0f, float sc = 1.0f);
 // (R: the band cube's radius, its side 2 R + 3; sc: cube voxels per frequency unit, 2 for
 // the cube of the map zero-padded to twice its side)
@@ -231,11 +239,42 @@ void launch_particle_norm(const float2* band, const float* ctf, Band bd, const i
 void launch_build_a(const float2* band, const float* ctf, Band bd, const int2* samples, int S, int Kpad,
                     const float* origins, int O, const double* norm, int B, void* A, cudaStream_t st,
                     const float* poff = nullptr);
-// Best origin per (particle, tile) (tile_*: B x ntiles scratch), then the k best tiles
-// per particle: distinct orientations with their best origin and CC.
-void launch_select_topk(const float* topv, const int* topi, int O, int ntiles, int k, int B,
-                        float* tile_v, int* tile_o, int* tile_orig, int* orient, int* origin, float* cc,
-                        cudaStream_t st);
+// The origin grid's basis (origin_basis.h) on the device.
+struct OriginDev {
+    const float* q;     // [nb][n1]
+    const float* f;     // [nb][2 R + 1]
+    const int* row;     // [slots]: mx | my << 12 | part << 24, -1 empty
+    const int2* slot;   // [nb nb]: row of part 0, of part 1, -1 none
+    int n1, nb, slots, units, R;
+    int layout;         // fixed places of the rows (OB_LAYOUT), -1: by slot alone
+    float mid;
+    float lo;           // scale of a second row's products (1, FP8 1/16)
+};
+// Operand A of the global forms: ob.slots rows per particle (the basis instead of the origin
+// grid), split as the banks are: BF16 with KH elements per part, or (f8) e4m3 with KH bytes,
+// sample scales mulA and a power of two 2^fexp[p] per particle.  poff as in launch_build_a.
+cudaError_t launch_build_basis(const float2* band, const float* ctf, Band bd, const int2* samples, int S, int KH,
+                               const OriginDev& ob, const double* norm, int B, void* A, bool f8, const float* mulA,
+                               int* fexp, cudaStream_t st, const float* poff = nullptr);
+// Exhaustive product C of B particles (GemmArgmaxArgs::cstore, pitch columns, nom / nomr K
+// shares; rows of the bank: nomr of the nom omegas per view): the best origin's value of every
+// orientation (ccmax: B x orientations), the best orientation of each of the ntiles blocks of
+// 256 (tile_v, tile_o: B x ntiles), the k best of those with their value and, if wanted,
+// origin (else 0).
+cudaError_t launch_up_topk(const OriginDev& ob, const float* C, long pitch, long rows, int nom, int nomr, int B, int k,
+                           float* ccmax, int ntiles, float* tile_v, int* tile_o, int* orient, int* origin, float* cc,
+                           bool want_origin, int num_sms, cudaStream_t st);
+// Listed products, one group per particle: list position j of group g stands for column
+// map[map_off + j] >> 1 of its block of C (parts K shares), conjugated if map & 1.  topv / topi
+// + topv_off <- [origins][ntiles] the best value of each block of 256 list positions, its
+// position.
+struct UpGroup {
+    long c_off;
+    int n_tiles;   // of C: pitch = 256 n_tiles
+    int map_off, n_list, topv_off, ntiles;
+};
+cudaError_t launch_up_list(const OriginDev& ob, const float* C, int parts, const UpGroup* groups, int ngroups,
+                           int max_tiles, const int* map, float* topv, int* topi, cudaStream_t st);
 // cand: B x k x (theta, phi, omega, x, y); out: B x k FP64 cross-correlations
 // scratch: cc_fp64_scratch(k, B) doubles
 long cc_fp64_scratch(int k, int B);
@@ -300,15 +339,11 @@ void launch_lp_topk(float* sc, int B, int V, int k, int* cell, float* val, cudaS
 void launch_select_distinct(float* topv, const int* topi, int O, const int2* seg, int B, int k, int* col,
                             int* origin, float* cc, cudaStream_t st);
 // FP8-e4m3 operands (contract.cu): per-band max |B| (R+1 bands, float bits) over every
-// stride-th row; B8 = e4m3(B x mulB) with rows of Kpad8 bytes; A8 rows with mulA and the
-// per-particle exponent fexp (written by launch_build_a8).
-cudaError_t launch_band_absmax(const void* B, long n, int Kpad, const int2* samples, int S, int nband, int stride,
+// stride-th row; B8 = e4m3(B x mulB) with KH8 bytes per part of a row.
+cudaError_t launch_band_absmax(const void* B, long n, int KH, const int2* samples, int S, int nband, int stride,
                                unsigned* out, int sms, cudaStream_t st);
-cudaError_t launch_b_to_e4m3(const void* B, long n, int Kpad, int S, const float* mulB, int Kpad8, void* B8,
+cudaError_t launch_b_to_e4m3(const void* B, long n, int KH, int S, const float* mulB, int KH8, void* B8,
                              cudaStream_t st);
-void launch_build_a8(const float2* band, const float* ctf, Band bd, const int2* samples, int S, int Kpad8,
-                     const float* origins, int O, const double* norm, const float* mulA, int* fexp, int B, void* A8,
-                     cudaStream_t st, const float* poff = nullptr);
 
 // ---- fsc.cu: half-map FSC and the FSC-weighted map ---------------------------
 struct FscArgs {

@@ -1,0 +1,190 @@
+// origin_basis.cpp — the origin grid's basis (origin_basis.h), on the host in FP64.
+#include "origin_basis.h"
+
+#include <algorithm>
+#include <cmath>
+#include <numeric>
+
+namespace cryoim {
+namespace {
+
+// Eigenvectors of the symmetric m x m matrix a (destroyed), by cyclic Jacobi rotations;
+// columns of v in descending order of eigenvalue.
+void eigenvectors(std::vector<double>& a, int m, std::vector<double>& v) {
+    v.assign((size_t)m * m, 0.0);
+    for (int i = 0; i < m; ++i) v[(size_t)i * m + i] = 1.0;
+    for (int sweep = 0; sweep < 60; ++sweep) {
+        double off = 0.0, dia = 0.0;
+        for (int i = 0; i < m; ++i)
+            for (int j = 0; j < m; ++j) (i == j ? dia : off) += a[(size_t)i * m + j] * a[(size_t)i * m + j];
+        if (off <= 1e-28 * (dia + off)) break;
+        for (int p = 0; p < m; ++p)
+            for (int q = p + 1; q < m; ++q) {
+                const double apq = a[(size_t)p * m + q];
+                if (apq == 0.0) continue;
+                const double th = 0.5 * (a[(size_t)q * m + q] - a[(size_t)p * m + p]) / apq;
+                const double t = (th >= 0 ? 1.0 : -1.0) / (std::fabs(th) + std::sqrt(th * th + 1.0));
+                const double c = 1.0 / std::sqrt(t * t + 1.0), s = t * c;
+                for (int k = 0; k < m; ++k) {
+                    const double x = a[(size_t)k * m + p], y = a[(size_t)k * m + q];
+                    a[(size_t)k * m + p] = c * x - s * y;
+                    a[(size_t)k * m + q] = s * x + c * y;
+                }
+                for (int k = 0; k < m; ++k) {
+                    const double x = a[(size_t)p * m + k], y = a[(size_t)q * m + k];
+                    a[(size_t)p * m + k] = c * x - s * y;
+                    a[(size_t)q * m + k] = s * x + c * y;
+                }
+                for (int k = 0; k < m; ++k) {
+                    const double x = v[(size_t)k * m + p], y = v[(size_t)k * m + q];
+                    v[(size_t)k * m + p] = c * x - s * y;
+                    v[(size_t)k * m + q] = s * x + c * y;
+                }
+            }
+    }
+    std::vector<int> ord(m);
+    std::iota(ord.begin(), ord.end(), 0);
+    std::sort(ord.begin(), ord.end(), [&](int x, int y) { return a[(size_t)x * m + x] > a[(size_t)y * m + y]; });
+    std::vector<double> w((size_t)m * m);
+    for (int j = 0; j < m; ++j)
+        for (int i = 0; i < m; ++i) w[(size_t)i * m + j] = v[(size_t)i * m + ord[j]];
+    v.swap(w);
+}
+
+}  // namespace
+
+OriginBasis make_origin_basis(int n, int min_r, int R, float omax, float step, int n1, bool f8) {
+    OriginBasis ob;
+    ob.n1 = n1;
+    ob.R = R;
+    ob.mid = (float)(-(double)omax + 0.5 * (double)step * (n1 - 1));
+    const double w0 = 2.0 * 3.14159265358979323846 / n;
+    std::vector<double> u(n1);
+    for (int i = 0; i < n1; ++i) u[i] = (double)step * (i - 0.5 * (n1 - 1));
+    // even and odd eigenvectors apart: v(i) = +- v(n1 - 1 - i)
+    std::vector<std::vector<double>> fun;  // [function][n1], even and odd alternating
+    std::vector<double> vec[2];
+    const int he = (n1 + 1) / 2, ho = n1 / 2;
+    for (int odd = 0; odd < 2; ++odd) {
+        const int m = odd ? ho : he;
+        std::vector<double> a((size_t)m * m);
+        for (int i = 0; i < m; ++i)
+            for (int j = 0; j < m; ++j) {
+                double s = 0.0;
+                for (int h = -R; h <= R; ++h)
+                    s += odd ? std::sin(w0 * h * u[i]) * std::sin(w0 * h * u[j])
+                             : std::cos(w0 * h * u[i]) * std::cos(w0 * h * u[j]);
+                // orthonormal half-grid vectors (e_i +- e_mirror) / sqrt 2 (the middle one alone)
+                const double ci = (!odd && (n1 & 1) && i == m - 1) ? 1.0 : std::sqrt(2.0);
+                const double cj = (!odd && (n1 & 1) && j == m - 1) ? 1.0 : std::sqrt(2.0);
+                a[(size_t)i * m + j] = s * ci * cj;
+            }
+        eigenvectors(a, m, vec[odd]);
+    }
+    for (int k = 0; k < n1; ++k) {
+        const int odd = k & 1, m = odd ? ho : he, col = k / 2;
+        std::vector<double> g(n1, 0.0);
+        for (int i = 0; i < m; ++i) {
+            const bool middle = !odd && (n1 & 1) && i == m - 1;
+            const double x = vec[odd][(size_t)i * m + col] * (middle ? 1.0 : std::sqrt(0.5));
+            g[i] = x;
+            if (!middle) g[n1 - 1 - i] = odd ? -x : x;
+        }
+        fun.push_back(g);
+    }
+    // their transforms over the band
+    const int H = 2 * R + 1;
+    std::vector<double> f((size_t)n1 * H);
+    for (int k = 0; k < n1; ++k)
+        for (int h = -R; h <= R; ++h) {
+            double s = 0.0;
+            for (int i = 0; i < n1; ++i) s += fun[k][i] * ((k & 1) ? std::sin(w0 * h * u[i]) : std::cos(w0 * h * u[i]));
+            f[(size_t)k * H + h + R] = s;
+        }
+    // energy of each product over the half-plane band samples
+    std::vector<double> e((size_t)n1 * n1, 0.0);
+    double total = 0.0;
+    for (int ky = -R; ky <= R; ++ky)
+        for (int hx = 0; hx <= R; ++hx) {
+            const int d2 = hx * hx + ky * ky;
+            if ((hx == 0 && ky <= 0) || d2 < min_r * min_r || d2 > R * R) continue;
+            total += (double)n1 * n1;
+            for (int m = 0; m < n1; ++m) {
+                const double fm = f[(size_t)m * H + hx + R], fm2 = fm * fm;
+                if (fm2 < 1e-18) continue;
+                for (int k = 0; k < n1; ++k) {
+                    const double fk = f[(size_t)k * H + ky + R];
+                    e[(size_t)m * n1 + k] += fm2 * fk * fk;
+                }
+            }
+        }
+    // What is left out (tail, of total) acts on the score like a change of the particle's phases,
+    // the same for every sample that carries the signal, so it adds up where rounding averages
+    // out: its root mean square stays 5e-5 (BF16) or 4e-4 (e4m3), far below the operands' rounding
+    // (1e-3, 2e-2) and, in the score, below what thousands of rounded samples leave of that.
+    const double most = f8 ? 1.6e-7 : 2.5e-9;
+    auto at = [&](int m, int k) { return m < n1 && k < n1 ? e[(size_t)m * n1 + k] : 0.0; };
+    auto place = [&](int b, int m, int k, int part) {
+        ob.mx[b] = m;
+        ob.my[b] = k;
+        ob.part[b] = part;
+        ob.slot[((size_t)m * ob.nb + k) * 2 + part] = b;
+    };
+    auto clear = [&](int nb, int slots) {
+        ob.nb = nb;
+        ob.slots = slots;
+        ob.mx.assign(slots, -1);
+        ob.my.assign(slots, -1);
+        ob.part.assign(slots, 0);
+        ob.slot.assign(2 * (size_t)nb * nb, -1);
+    };
+    for (int l = 0; l < OB_LAYOUTS && ob.layout < 0; ++l) {
+        const OriginLayout& L = OB_LAYOUT[l];
+        // (summed from what is out: the difference of two nearly equal sums would not do)
+        double tail = 0.0;
+        for (int m = 0; m < n1; ++m)
+            for (int k = 0; k < n1; ++k)
+                if (!L.in(m, k)) tail += at(m, k);
+        if (tail > most * total) continue;
+        ob.layout = l;
+        clear(L.nb, L.rows);
+        int b = 0;
+        for (int part = 0; part < 2; ++part)
+            for (int m = 0; m < L.nb; ++m)
+                for (int k = 0; k < L.nb; ++k)
+                    if (L.in(m, k) && (part == 0 || m + k < L.second)) {
+                        if (m < n1 && k < n1) place(b, m, k, part);
+                        ++b;
+                    }
+    }
+    if (ob.layout < 0) {
+        // more functions: in the order of their energy, in as many units as it takes, and second
+        // rows (worth the energy of their function's rounding, the same order) in the rest
+        std::vector<int> ord((size_t)n1 * n1);
+        std::iota(ord.begin(), ord.end(), 0);
+        std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) { return e[x] > e[y]; });
+        size_t cnt = ord.size();
+        double tail = 0.0;
+        while (cnt > 1 && tail + e[ord[cnt - 1]] <= most * total) tail += e[ord[--cnt]];
+        ob.units = (int)((cnt + OB_UNIT - 1) / OB_UNIT);
+        int top = 0;
+        for (size_t b = 0; b < cnt; ++b) top = std::max(top, std::max(ord[b] / n1, ord[b] % n1) + 1);
+        clear(top, ob.units * OB_UNIT);
+        for (size_t b = 0; b < cnt; ++b) place((int)b, ord[b] / n1, ord[b] % n1, 0);
+        for (size_t b = cnt; b < (size_t)ob.slots && b < 2 * cnt; ++b)
+            place((int)b, ord[b - cnt] / n1, ord[b - cnt] % n1, 1);
+    }
+    ob.q.assign((size_t)ob.nb * n1, 0.0f);
+    ob.f.assign((size_t)ob.nb * H, 0.0f);
+    ob.ge.assign(ob.nb, 0);
+    for (int k = 0; k < std::min(ob.nb, n1); ++k) {
+        double fm = 0.0;
+        for (int h = 0; h < H; ++h) fm = std::max(fm, std::fabs(f[(size_t)k * H + h]));
+        if (f8 && fm > 0.0) ob.ge[k] = std::max(-60, std::min(60, -(int)std::ceil(std::log2(fm))));
+        for (int i = 0; i < n1; ++i) ob.q[(size_t)k * n1 + i] = (float)std::ldexp(fun[k][i], -ob.ge[k]);
+        for (int h = 0; h < H; ++h) ob.f[(size_t)k * H + h] = (float)std::ldexp(f[(size_t)k * H + h], ob.ge[k]);
+    }
+    return ob;
+}
+
+}  // namespace cryoim

@@ -302,6 +302,11 @@ struct Ctx {
     std::map<int, cufftHandle> plans;
     // reconstruction
     DBuf<float4> acc;
+    // splats under one operator per coset of the grid's rotations (ops5), zero between calls,
+    // and the octant they are summed in (launch_sym_add)
+    DBuf<float4> acc5, oct;
+    bool acc5_zero = false;
+    DBuf<float> ops5;
     DBuf<int2> samples;
     DBuf<float2> vol;
     bool rec_active = false;
@@ -409,7 +414,7 @@ struct Ctx {
         alpha.release(); imgs.release(); par.release(); fcut0.release(); ctf.release();
         tfcut.release(); state.release(); cand.release(); rpr.release(); rot.release();
         prbuf.release(); fft.release(); band.release(); ralpha.release(); best.release();
-        flag.release(); sel.release(); acc.release(); samples.release(); vol.release();
+        flag.release(); sel.release(); acc.release(); acc5.release(); oct.release(); ops5.release(); samples.release(); vol.release();
         mapcube.release(); mapreal.release(); csamples.release(); bmat.release(); amat.release(); corigins.release();
         topv.release(); kcc.release(); kcand.release(); topi.release(); gerr.release();
         kor.release(); korig.release(); pnorm.release(); kcc64.release(); pnorm0.release(); pctf.release();
@@ -774,6 +779,57 @@ int refine_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* part
     return CRYOIM_OK;
 }
 
+// One operator of each coset of the operators that permute and negate the axes (12: five
+// cosets) and of those that only negate them (4: fifteen) in the operator table: the table is
+// {g s}, g in the group, s among these.  ops5 holds the five, then the fifteen.
+int ensure_coset_ops(Ctx* c) {
+    if (c->ops5.n) return CRYOIM_OK;
+    const float* t = table_ops();
+    auto is = [](float a, float b) { return std::fabs(a - b) < 1e-4f; };
+    std::vector<float> rep;
+    for (int negate = 0; negate < 2; ++negate) {
+        std::vector<int> grid;
+        for (int k = 0; k < 60; ++k) {
+            bool ok = true;
+            for (int i = 0; i < 9; ++i) {
+                const float v = std::fabs(t[9 * k + i]);
+                ok = ok && (is(v, 0.0f) || is(v, 1.0f)) && (!negate || i % 4 == 0 || is(v, 0.0f));
+            }
+            if (ok) grid.push_back(k);
+        }
+        std::vector<char> done(60, 0);
+        size_t cosets = 0;
+        for (int k = 0; k < 60; ++k) {
+            if (done[k]) continue;
+            ++cosets;
+            rep.insert(rep.end(), t + 9 * k, t + 9 * k + 9);
+            for (int g : grid) {
+                float m[9];
+                for (int i = 0; i < 9; ++i) {
+                    m[i] = 0.0f;
+                    for (int q = 0; q < 3; ++q) m[i] += t[9 * g + i / 3 * 3 + q] * t[9 * k + 3 * q + i % 3];
+                }
+                for (int j = 0; j < 60; ++j) {
+                    bool same = true;
+                    for (int i = 0; i < 9; ++i) same = same && is(m[i], t[9 * j + i]);
+                    if (same) done[j] = 1;
+                }
+            }
+        }
+        if (cosets != (negate ? 15u : 5u)) return fail(CRYOIM_ERR_STATE, "operator table");
+    }
+    int r;
+    if ((r = c->ops5.ensure(rep.size()))) return r;
+    CK(cudaMemcpyAsync(c->ops5.p, rep.data(), sizeof(float) * rep.size(), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    return CRYOIM_OK;
+}
+
+// Selected particles of a call from which the coset path is the faster: its sum over the twelve
+// grid rotations costs about as much as one (maxR 64: 13 us against 12.9) to three (maxR 26: 9
+// against 3.1) particles under all 60 operators.
+constexpr int COSET_MIN = 4;
+
 int rec_insert_impl(Ctx* c, const float* imgs, bool on_device, const cryoim_particle* parts, int P,
                     int32_t* used) {
     int r = check_ready(c, false);
@@ -788,7 +844,21 @@ int rec_insert_impl(Ctx* c, const float* imgs, bool on_device, const cryoim_part
     const Angles an = host_angles();
     std::vector<float> hpar(8 * B), hrot(9 * B);
     std::vector<int> hsel(B);
-    int nused = 0;
+    auto selected = [&](const cryoim_particle& q) {
+        return q.pr <= c->p.pr_threshold && std::fabs(q.x) <= boundx && std::fabs(q.y) <= boundx;
+    };
+    int nused = 0, nsel = 0;
+    for (int i = 0; i < P; ++i) nsel += selected(parts[i]);
+    const bool coset = nsel >= COSET_MIN;
+    if (coset) {
+        // (the two planes of launch_insert_plane0 after the half box)
+        const long n5 = (long)c->bd.AW * c->bd.AW * (c->bd.max_r + 4), C = c->bd.max_r + 2;
+        if ((r = ensure_coset_ops(c)) || (r = c->oct.ensure(C * C * C)) || (r = c->acc5.ensure(n5))) return r;
+        if (!c->acc5_zero) {
+            CK(cudaMemsetAsync(c->acc5.p, 0, sizeof(float4) * n5, c->stream));
+            c->acc5_zero = true;
+        }
+    }
     for (int b0 = 0; b0 < P; b0 += B) {
         const int nb = std::min(B, P - b0);
         std::fill(hpar.begin(), hpar.end(), 0.0f);
@@ -797,7 +867,7 @@ int rec_insert_impl(Ctx* c, const float* imgs, bool on_device, const cryoim_part
             if (!c->rec_have_first) {  // reconstruct.f90:92 masks every image at particle(first)'s origin
                 c->rec_ox = q.x; c->rec_oy = q.y; c->rec_have_first = true;
             }
-            int s = (q.pr <= c->p.pr_threshold && std::fabs(q.x) <= boundx && std::fabs(q.y) <= boundx);
+            const int s = selected(q);
             hsel[i] = s;
             hpar[i] = c->rec_ox; hpar[B + i] = c->rec_oy;
             hpar[2 * B + i] = q.x; hpar[3 * B + i] = q.y;
@@ -822,7 +892,7 @@ int rec_insert_impl(Ctx* c, const float* imgs, bool on_device, const cryoim_part
                                cudaMemcpyHostToDevice, c->stream));
             d_src = c->imgs.p;
         }
-        if ((r = transform_batch(c, d_src, nb, B, hpar, c->p.use_imgmask, 1, true))) return r;
+        if ((r = transform_batch(c, d_src, nb, B, hpar, c->p.use_imgmask, 1, true, b0 > 0))) return r;
         ParView pv = par_view(c, B);
         const float* ctfp = nullptr;
         if (c->p.apply_ctf || c->p.imgstck) {
@@ -837,11 +907,27 @@ int rec_insert_impl(Ctx* c, const float* imgs, bool on_device, const cryoim_part
         InsertArgs a{};
         a.band = c->band.p; a.ctf = ctfp; a.rot = c->rot.p; a.ops = c->ops.p;
         a.samples = c->samples.p; a.nsamples = c->nsamples; a.nsym = c->p.nsym; a.sel = c->sel.p;
+        a.lim = c->rec_kind == REC_SUBSTEP ? c->p.max_r - 2 : c->p.max_r;
         a.off_xy = c->rec_off_xy; a.off_z = c->rec_off_z; a.base_xy = c->rec_base_xy;
         a.base_z = c->rec_base_z; a.bd = c->bd; a.acc = c->acc.p;
-        if (c->nsamples > 0) CK(launch_insert(a, nb, c->stream));
-        if ((r = check_flag(c))) return r;
+        if (c->nsamples > 0 && !coset) CK(launch_insert(a, nb, c->stream));
+        if (c->nsamples > 0 && coset) {
+            c->acc5_zero = false;
+            a.ops = c->ops5.p;
+            a.nsym = 5;
+            a.acc = c->acc5.p;
+            CK(launch_insert(a, nb, c->stream));
+            a.ops = c->ops5.p + 45;
+            a.nsym = 15;
+            a.acc = c->acc5.p + (long)c->bd.AW * c->bd.AW * (c->bd.max_r + 2);
+            CK(launch_insert_plane0(a, nb, c->stream));
+        }
     }
+    if (coset && c->nsamples > 0) {
+        CK(launch_sym_add(c->acc5.p, c->acc5.p + (long)c->bd.AW * c->bd.AW * (c->bd.max_r + 2), c->bd, c->oct.p, c->acc.p, c->stream));
+        c->acc5_zero = true;
+    }
+    if (P > 0 && (r = check_flag(c))) return r;  // (of every batch)
     c->rec_used += nused;
     if (used) *used = nused;
     return CRYOIM_OK;
@@ -2563,6 +2649,7 @@ int cryoim_set_params(void* ctx, const cryoim_params* p) {
         c->T = 0;  // templates depend on the band geometry
         c->grid_ready = false;
         c->rec_active = false;
+        c->acc5_zero = false;
         c->map_ready = false;
         c->cS = 0;
         c->bmat_ready = false;
@@ -2833,8 +2920,7 @@ static int rec_begin_impl(Ctx* c, int kind, const float* mask_origin) {
     // reconstruct.f90:26-28 (wg = 0.01), reconstruct_substep.f90:23-25 and
     // reconstruct_half.f90:17 (wg = 0)
     const float wg0 = kind == REC_FULL ? 0.01f : 0.0f;
-    std::vector<float4> init(nacc, make_float4(0.f, 0.f, wg0, 0.f));
-    CK(cudaMemcpyAsync(c->acc.p, init.data(), sizeof(float4) * nacc, cudaMemcpyHostToDevice, c->stream));
+    CK(launch_fill4(c->acc.p, nacc, make_float4(0.f, 0.f, wg0, 0.f), c->stream));
     // insertion samples: reconstruct.f90:103-106 and reconstruct_half.f90:95-96 (r <= maxR),
     // reconstruct_substep.f90:101-104 (r <= maxR-2)
     const float lim = kind == REC_SUBSTEP ? (float)(R - 2) : (float)R;

@@ -142,6 +142,7 @@ struct InsertArgs {
     const float* ops;        // [60][9]
     const int2* samples;     // (hx, ky) insertion samples
     int nsamples, nsym;
+    int lim;                 // the samples are hx >= 0, hx^2 + ky^2 <= lim^2
     const int* sel;          // [B] 1 = insert
     float off_xy, off_z;     // coordinate offsets added before int()
     int base_xy, base_z;     // accumulator index origin
@@ -149,6 +150,14 @@ struct InsertArgs {
     float4* acc;             // half box
 };
 cudaError_t launch_insert(const InsertArgs& a, int B, cudaStream_t st);
+// the cells of the plane z = 0 alone, under the a.nsym operators of a.ops, into two planes of
+// AW x AW at a.acc: of the samples off that plane and of those exactly on it
+cudaError_t launch_insert_plane0(const InsertArgs& a, int B, cudaStream_t st);
+// acc's cells z >= 1 += acc5 (a half box of splats under one operator per coset) summed over
+// the 12 rotations that permute and negate the axes, its cells z = 0 += plane0 (the two planes of
+// launch_insert_plane0) summed over the 4 that negate; both are left zero; oct: (maxR + 2)^3 scratch
+cudaError_t launch_sym_add(float4* acc5, float4* plane0, const Band& bd, float4* oct, float4* acc, cudaStream_t st);
+cudaError_t launch_fill4(float4* p, long n, float4 v, cudaStream_t st);
 
 // ---- gemm_tc.cu (tcgen05 BF16 contraction with fused per-tile argmax) --------
 // One independent product of a grouped launch: rows [a_row0, a_row0 + m_valid) of A

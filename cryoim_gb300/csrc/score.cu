@@ -667,11 +667,23 @@ __global__ void k_shift_band(const float2* __restrict__ band, const float* __res
     out[(long)p * W * W + m] = make_float4(v0.x, v0.y, v1.x, v1.y);
 }
 
-// reconstruct.f90:103-145: rotate each half-plane sample, apply the 60 operators,
+// reconstruct.f90:103-145: rotate each half-plane sample, apply the operators,
 // fold to z >= 0 and splat (a*ctf, b*ctf*signz, ctf^2) trilinearly.  One thread per
 // (operator, sample), consecutive threads on consecutive samples of one operator: the
 // samples run along hx, so a warp's splats land on neighbouring voxels and its float4
 // vector reductions share L2 sectors (the three sums of a voxel are one reduction).
+// Bound by those reductions in L2 (8 a splat).  All 60 operators of a particle cost 12.9 us at
+// maxR 64.  Twelve of them (the rotations that permute and negate the axes, the tetrahedral
+// group) take the voxel grid to itself, and a trilinear splat commutes with those: so the
+// particles of a call are splatted with one operator of each of their five cosets, 1.1 us a
+// particle, and the box is summed over the twelve once (k_sym_octant, k_sym_add: 18 us).  The
+// plane z = 0 of the half box is apart: which of v and -v a sample lands on there depends on
+// the sign of its own z, which the sums over the cyclic permutations no longer hold.  The half
+// turns about the axes keep it: after the fold a sample at (x, y, z > 0) is also one at
+// (-x, -y, z) and its conjugate at (-x, y, z) and (x, -y, z); one at z = 0 exactly is not folded,
+// so at all four it is itself.  So the plane's cells are splatted under one operator of each
+// coset of those (fifteen; k_insert_plane0, only the samples within 1 of the plane) and summed
+// over the four (k_sym_plane0).
 __device__ __forceinline__ void mv3_rn(const float* m, const float* v, float* o) {
     float t0 = __fmul_rn(m[0], v[0]); t0 = __fadd_rn(t0, __fmul_rn(m[1], v[1])); t0 = __fadd_rn(t0, __fmul_rn(m[2], v[2]));
     float t1 = __fmul_rn(m[3], v[0]); t1 = __fadd_rn(t1, __fmul_rn(m[4], v[1])); t1 = __fadd_rn(t1, __fmul_rn(m[5], v[2]));
@@ -679,21 +691,19 @@ __device__ __forceinline__ void mv3_rn(const float* m, const float* v, float* o)
     o[0] = t0; o[1] = t1; o[2] = t2;
 }
 
-__global__ void __launch_bounds__(256) k_insert(InsertArgs a) {
-    const int p = blockIdx.y;
-    if (!a.sel[p]) return;
-    const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= (long)a.nsamples * a.nsym) return;
-    const int k = (int)(q / a.nsamples), s = (int)(q - (long)k * a.nsamples);
+// PLANE0: only the cells of lz = 0, into a.acc as two planes: of samples off the plane z = 0,
+// and (a.acc + AW AW) of samples exactly on it
+template <bool PLANE0>
+__device__ __forceinline__ void splat(const InsertArgs& a, int p, int k, int2 hk) {
     const Band bd = a.bd;
     const int W = bd.W, R = bd.max_r;
-    const int2 hk = a.samples[s];
     const float* rot = a.rot + p * 9;
     float xv[3] = {(float)hk.x, (float)hk.y, 0.0f}, x00[3], x0[3];
     mv3_rn(rot, xv, x00);
     mv3_rn(a.ops + k * 9, x00, x0);
     float signz = 1.0f;
     if (x0[2] < 0.0f) { x0[0] = -x0[0]; x0[1] = -x0[1]; x0[2] = -x0[2]; signz = -1.0f; }
+    const float zfold = x0[2];
     x0[0] = __fadd_rn(x0[0], a.off_xy);
     x0[1] = __fadd_rn(x0[1], a.off_xy);
     x0[2] = __fadd_rn(x0[2], a.off_z);
@@ -716,16 +726,140 @@ __global__ void __launch_bounds__(256) k_insert(InsertArgs a) {
     const int AW = bd.AW;
     const int ix = lx - a.base_xy, iy = ly - a.base_xy, iz = lz - a.base_z;
     if (ix < 0 || iy < 0 || iz < 0 || ix > AW - 2 || iy > AW - 2 || iz > R) return;  // never taken
+    if (PLANE0 && iz != 0) return;
+    float4* acc = a.acc + (PLANE0 && zfold == 0.0f ? (long)AW * AW : 0L);
     const long base = ((long)iz * AW + iy) * AW + ix;
     const long offs[8] = {0, 1, AW, AW + 1, (long)AW * AW, (long)AW * AW + 1, (long)AW * AW + AW,
                           (long)AW * AW + AW + 1};
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < (PLANE0 ? 4 : 8); ++j) {
         float va = __fmul_rn(__fmul_rn(fv.x, dx[j]), c);
         float vb = __fmul_rn(__fmul_rn(__fmul_rn(fv.y, dx[j]), c), signz);
         float vw = __fmul_rn(dx[j], c2);
-        atomicAdd(a.acc + base + offs[j], make_float4(va, vb, vw, 0.0f));
+        atomicAdd(acc + base + offs[j], make_float4(va, vb, vw, 0.0f));
     }
+}
+
+__global__ void __launch_bounds__(256) k_insert(InsertArgs a) {
+    const int p = blockIdx.y;
+    if (!a.sel[p]) return;
+    const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= (long)a.nsamples * a.nsym) return;
+    const int k = (int)(q / a.nsamples), s = (int)(q - (long)k * a.nsamples);
+    splat<false>(a, p, k, a.samples[s]);
+}
+
+// One block per (operator, particle), a thread per row ky of samples in turn: the stretch of
+// hx whose rotated z, by the product of the two rotations, is within 1 (and a margin over the
+// rounding the two differ by) is splatted.  Bound by the reductions that meet on the cells around
+// the origin: under all 60 operators 81 us a 64-particle batch at maxR 64, under one of each of
+// the fifteen cosets of the half turns about the axes 42 us.
+__global__ void __launch_bounds__(160) k_insert_plane0(InsertArgs a) {
+    const int k = blockIdx.x, p = blockIdx.y;
+    if (!a.sel[p]) return;
+    const float* op = a.ops + k * 9 + 6;
+    const float* rot = a.rot + p * 9;
+    const float zx = op[0] * rot[0] + op[1] * rot[3] + op[2] * rot[6];
+    const float zy = op[0] * rot[1] + op[1] * rot[4] + op[2] * rot[7];
+    for (int r = threadIdx.x; r < 2 * a.lim + 1; r += blockDim.x) {
+        const int ky = r - a.lim;
+        int hmax = (int)sqrtf((float)(a.lim * a.lim - ky * ky));  // samples hx^2 + ky^2 <= lim^2
+        while (hmax * hmax + ky * ky > a.lim * a.lim) --hmax;
+        while ((hmax + 1) * (hmax + 1) + ky * ky <= a.lim * a.lim) ++hmax;
+        const float z0 = zy * (float)ky;
+        int h0 = 0, h1 = hmax;
+        if (fabsf(zx) * (float)hmax > 1.0e-3f) {  // else z is z0 all along
+            const float u = (-1.01f - z0) / zx, v = (1.01f - z0) / zx;
+            h0 = max(0, (int)ceilf(fmaxf(fminf(u, v), -1.0e6f)));
+            h1 = min(hmax, (int)floorf(fminf(fmaxf(u, v), 1.0e6f)));
+        } else if (fabsf(z0) > 1.02f) {
+            continue;
+        }
+        for (int hx = h0; hx <= h1; ++hx) splat<true>(a, p, k, make_int2(hx, ky));
+    }
+}
+
+// Sums over the tetrahedral group.  F(v) of a whole box is the half box acc5 for z > 0, its
+// conjugate at -v for z < 0 and acc5(v) + conj acc5(-v) on z = 0.  Over the four rotations by
+// half a turn about the axes, B(v) = F(x,y,z) + F(x,-y,-z) + F(-x,y,-z) + F(-x,-y,z) has
+// B = conj B under a sign change of any one axis, so the octant x, y, z >= 0 holds it:
+// k_sym_octant computes it and leaves acc5 zero (each thread owns the cells it reads).  The
+// three cyclic permutations of the axes give the rest: k_sym_add adds B(x,y,z) + B(y,z,x) +
+// B(z,x,y), conjugated for an odd number of negative axes, to the cells z >= 1 of acc.
+__device__ __forceinline__ long octant(int C, int x, int y, int z) { return ((long)z * C + y) * C + x; }
+__global__ void __launch_bounds__(256) k_sym_octant(float4* __restrict__ acc5, Band bd, float4* __restrict__ oct) {
+    const int C = bd.max_r + 2;
+    const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= (long)C * C * C) return;
+    const int x = (int)(q % C), y = (int)((q / C) % C), z = (int)(q / ((long)C * C));
+    const long c[4] = {acc_cell(bd, x, y, z), acc_cell(bd, -x, y, z), acc_cell(bd, x, -y, z), acc_cell(bd, -x, -y, z)};
+    const float4 v0 = acc5[c[0]], v1 = acc5[c[1]], v2 = acc5[c[2]], v3 = acc5[c[3]];
+    float4 s;
+    s.x = (v0.x + v3.x) + (v1.x + v2.x);
+    s.y = (v0.y + v3.y) - (v1.y + v2.y);
+    s.z = (v0.z + v3.z) + (v1.z + v2.z);
+    s.w = 0.0f;
+    if (z == 0) {  // F(v) + F(-v) is twice the real part
+        s.x *= 2.0f;
+        s.y = 0.0f;
+        s.z *= 2.0f;
+    }
+    oct[q] = s;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc5[c[i]] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+__global__ void __launch_bounds__(256) k_sym_add(const float4* __restrict__ oct, Band bd, float4* __restrict__ acc) {
+    const int C = bd.max_r + 2;
+    const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= (long)C * C * (C - 1)) return;
+    const int x = (int)(q % C), y = (int)((q / C) % C), z = 1 + (int)(q / ((long)C * C));
+    const float4 a = oct[octant(C, x, y, z)], b = oct[octant(C, y, z, x)], d = oct[octant(C, z, x, y)];
+    const float sx = a.x + b.x + d.x, sy = a.y + b.y + d.y, sz = a.z + b.z + d.z;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if ((i & 1 && x == 0) || (i & 2 && y == 0)) continue;
+        float4* o = acc + acc_cell(bd, i & 1 ? -x : x, i & 2 ? -y : y, z);
+        float4 v = *o;
+        v.x += sx;
+        v.y += (i == 1 || i == 2) ? -sy : sy;
+        v.z += sz;
+        *o = v;
+    }
+}
+
+// plane0: two planes of AW x AW (samples off and on z = 0), left zero; acc's cells of z = 0 are
+// the sums over the four half turns.
+__global__ void __launch_bounds__(256) k_sym_plane0(float4* __restrict__ plane0, Band bd, float4* __restrict__ acc) {
+    const int C = bd.max_r + 2;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= C * C) return;
+    const int x = q % C, y = q / C;
+    const long n = (long)bd.AW * bd.AW;
+    const long c[4] = {acc_cell(bd, x, y, 0), acc_cell(bd, -x, y, 0), acc_cell(bd, x, -y, 0), acc_cell(bd, -x, -y, 0)};
+    float4 a[4], b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { a[i] = plane0[c[i]]; b[i] = plane0[n + c[i]]; }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { plane0[c[i]] = make_float4(0.f, 0.f, 0.f, 0.f); plane0[n + c[i]] = make_float4(0.f, 0.f, 0.f, 0.f); }
+    // the same sums at the four cells, but for the sign of the folded ones' imaginary part
+    const float bx = (b[0].x + b[3].x) + (b[1].x + b[2].x), by = (b[0].y + b[3].y) + (b[1].y + b[2].y),
+                bz = (b[0].z + b[3].z) + (b[1].z + b[2].z);
+    const float ax = (a[0].x + a[3].x) + (a[1].x + a[2].x), ay = (a[0].y + a[3].y) - (a[1].y + a[2].y),
+                az = (a[0].z + a[3].z) + (a[1].z + a[2].z);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if ((i & 1 && x == 0) || (i & 2 && y == 0)) continue;
+        float4 v = acc[c[i]];
+        v.x += ax + bx;
+        v.y += (i == 1 || i == 2 ? -ay : ay) + by;
+        v.z += az + bz;
+        acc[c[i]] = v;
+    }
+}
+
+__global__ void k_fill4(float4* __restrict__ p, long n, float4 v) {
+    const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < n) p[q] = v;
 }
 
 Consts consts() {
@@ -832,6 +966,24 @@ bool pr_rescore_shared_band(const Band& bd, int T) {
                       sizeof(int) * T * 60;
     const size_t sm_s = sm + sizeof(float2) * (size_t)bd.W * rescore_pitch(bd.W);
     return sm_s + sizeof(double) * 2 * RG * (RS_THREADS / 32) <= 227 * 1024;
+}
+
+cudaError_t launch_insert_plane0(const InsertArgs& a, int B, cudaStream_t st) {
+    k_insert_plane0<<<dim3(a.nsym, B), 160, 0, st>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_sym_add(float4* acc5, float4* plane0, const Band& bd, float4* oct, float4* acc, cudaStream_t st) {
+    const long C = bd.max_r + 2, n = C * C * C;
+    k_sym_plane0<<<(unsigned)((C * C + 255) / 256), 256, 0, st>>>(plane0, bd, acc);
+    k_sym_octant<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(acc5, bd, oct);
+    k_sym_add<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(oct, bd, acc);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fill4(float4* p, long n, float4 v, cudaStream_t st) {
+    k_fill4<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(p, n, v);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_insert(const InsertArgs& a, int B, cudaStream_t st) {

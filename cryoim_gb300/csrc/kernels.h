@@ -86,7 +86,7 @@ struct PrOmegaArgs {
     float* pr_array;           // [B][per] or nullptr
     long per;
 };
-int pr_omega_smem_bytes(const Band& bd, int nomega, int* threads);
+int pr_omega_smem_bytes(const Band& bd, int nomega, float step, int* threads, int* groups);
 cudaError_t launch_pr_omega(const PrOmegaArgs& a, int B, cudaStream_t st);
 
 struct PrSingleArgs {

@@ -4,10 +4,10 @@
 // every asymmetric-unit view of every particle).  One CTA owns one (particle, view):
 //   * the particle's band-limited Fourier window (W x W float2) sits in shared memory
 //     for the whole CTA, so every bilinear tap is a shared-memory load;
-//   * thread (g, k) owns omega index k and accumulates PR1(k), PR2(k) in registers over
-//     the lines j = g, g+G, ... of every template (no cross-thread reduction until the
-//     end of the view), with per-line FP32 partial sums folded into Kahan-compensated
-//     running sums;
+//   * thread (g, k) owns omega index k (and k + half a turn where the grid has it) and
+//     accumulates PR1(k), PR2(k) in registers over the valid lines g, g+G, ... of every
+//     template (no cross-thread reduction until the end of the view), with per-line FP32
+//     partial sums folded into Kahan-compensated running sums;
 //   * per template, the 60 x nR template line samples (template x CTF, bilinear) are
 //     staged once into shared memory as (amplitude or -1 if below Fcut, phase);
 //   * the per-view argmin over omega is folded into a per-particle 64-bit key
@@ -127,7 +127,50 @@ __device__ __forceinline__ float angle_between_est(float cross, float dot, float
     return (dot < 0.0f) ? pi - r : r;
 }
 
-__global__ void __launch_bounds__(768, 1) k_pr_omega(PrOmegaArgs a, int nomp, Consts K) {
+// One PR term of a particle sample z (Re, -Im): the angle to the template sample e (a, b, half
+// amplitude) and the weight.
+struct OmegaTerm {
+    float2 z;
+    float amp, w;
+};
+// The particle's sample at radius fr in direction csn of the band in shared memory.
+__device__ __forceinline__ OmegaTerm omega_sample(const float2* sband, int W, int offW, float fr, float2 csn,
+                                                  float nxh, float half2) {
+    // sample position (x, y) = FR (cos, sin) + nx/2, then its cell
+    const float2 xy = __ffma2_rn(make_float2(fr, fr), csn, make_float2(nxh, nxh));
+    const int lx = (int)xy.x, ly = (int)xy.y;
+    const float2 f = __fadd2_rn(xy, make_float2(-(float)lx, -(float)ly));
+    const int b0 = ly * W + lx - offW;
+    const float2 t00 = sband[b0], t10 = sband[b0 + 1];
+    const float2 t01 = sband[b0 + W], t11 = sband[b0 + W + 1];
+    // bilinear on (re, im) pairs: lerp in x on both rows, then in y
+    const float2 ax2 = make_float2(f.x, f.x), ay2 = make_float2(f.y, f.y);
+    const float2 m1 = make_float2(-1.f, -1.f);
+    const float2 v0 = __ffma2_rn(ax2, __ffma2_rn(t00, m1, t10), t00);
+    const float2 v1 = __ffma2_rn(ax2, __ffma2_rn(t01, m1, t11), t01);
+    OmegaTerm r;
+    r.z = __ffma2_rn(ay2, __ffma2_rn(v0, m1, v1), v0);
+    const float2 zz = __fmul2_rn(r.z, r.z);
+    const float sq = zz.x + zz.y;
+    r.amp = sq * rsqrtf(sq);  // NaN for 0: fails the cut
+    r.w = fmaf(0.5f, r.amp, half2);
+    return r;
+}
+
+// HALF: thread (g, k) owns omega k and k + nomega / 2, half a turn apart.  The particle's
+// samples along a line and along its reverse are complex conjugates (the image is real), so one
+// sample, its amplitude, cut and weight serve both; the cross and dot products differ by the
+// sign of one of the two products each.  The two samples' positions round differently (2e-5
+// px), so where the amplitude lies within PAIR_MARGIN of its cut the second omega's sample is
+// taken by itself and every term passes or fails its cut as the search by single omegas has it.
+// Issue-bound (76 %; by single omegas 80 %, and the L1 data pipe 76 %): a particle of box 256 on
+// the 1-degree grid takes 13.1 ms in pairs, 17.8 by single omegas.  The margin's terms are marked
+// and taken after each 32 radii: inside the unrolled loop they cost more than the pairs gain (19
+// ms).  Cells by the add of 2^23 in place of conversions (which wait for the reciprocals'
+// quarter-rate pipe) gained nothing.
+constexpr float PAIR_MARGIN = 5.0e-4f;
+template <bool HALF>
+__global__ void __launch_bounds__(768, 1) k_pr_omega(PrOmegaArgs a, int nown, int G, Consts K) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const Band bd = a.bd;
     const int W = bd.W, nr = bd.nr, minR = bd.min_r;
@@ -135,13 +178,18 @@ __global__ void __launch_bounds__(768, 1) k_pr_omega(PrOmegaArgs a, int nomp, Co
     // per (line, radius): template sample (a2, b2), half amplitude (-1 below its cut),
     // particle cut at that radius
     float4* sline = reinterpret_cast<float4*>(sband + W * W);
-    float* sfc0 = reinterpret_cast<float*>(sline + 60 * nr);
-    float* salpha = sfc0 + ((nr + 3) & ~3);
-    float* sred = salpha + 64;
-    unsigned long long* skey = reinterpret_cast<unsigned long long*>(sred + 2 * blockDim.x);
+    float2* sred = reinterpret_cast<float2*>(sline);  // [1 or 2][threads], once a view's lines are done
+    float* sfc0 = reinterpret_cast<float*>(sline + max(60 * nr, (int)blockDim.x / (HALF ? 1 : 2)));
+    unsigned long long* skey = reinterpret_cast<unsigned long long*>(sfc0 + ((nr + 3) & ~3));
+    float* salpha = reinterpret_cast<float*>(skey + 32);  // particle line angles of the template's valid lines
+    int* sjl = reinterpret_cast<int*>(salpha + 64);       // and which lines they are
+    int* snv = sjl + 64;
 
     const int p = blockIdx.y, t = threadIdx.x;
-    const int G = blockDim.x / nomp, g = t / nomp, k = t - g * nomp;
+    // thread (g, k): group g's lines, omega k; no padding between groups (a warp may hold the end
+    // of one and the start of the next)
+    const int g = t / nown, k = t - g * nown;
+    const bool own = g < G;
     {
         const float4* gb = reinterpret_cast<const float4*>(a.band + (long)p * W * W);
         float4* sb4 = reinterpret_cast<float4*>(sband);
@@ -157,12 +205,25 @@ __global__ void __launch_bounds__(768, 1) k_pr_omega(PrOmegaArgs a, int nomp, Co
 
     for (int v = blockIdx.x; v < a.V; v += gridDim.x) {
         float pr1 = 0.f, pr2 = 0.f, c1 = 0.f, c2 = 0.f;
+        float qr1 = 0.f, qr2 = 0.f, d1 = 0.f, d2 = 0.f;  // HALF: of omega k + nomega / 2
         for (int i = 0; i < a.T; ++i) {
             __syncthreads();
             const float2* al = a.alpha + ((long)v * a.T + i) * 60;
-            if (t < 60) {
-                float2 aa = al[t];
-                salpha[t] = (aa.x < 999.0f && aa.y < 999.0f) ? aa.x : 1000.0f;
+            if (t < 32) {  // the valid lines, in order
+                int n = 0;
+                for (int h = 0; h < 2; ++h) {
+                    const int j = 32 * h + t;
+                    const float2 aa = j < 60 ? al[j] : make_float2(1000.f, 1000.f);
+                    const bool ok = aa.x < 999.0f && aa.y < 999.0f;
+                    const unsigned m = __ballot_sync(0xffffffffu, ok);
+                    if (ok) {
+                        const int at = n + __popc(m & ((1u << t) - 1u));
+                        salpha[at] = aa.x;
+                        sjl[at] = j;
+                    }
+                    n += __popc(m);
+                }
+                if (t == 0) *snv = n;
             }
             const float2* tb = a.tband + (long)i * W * W;
             const float* fct = tfc + (long)i * nr;
@@ -179,67 +240,89 @@ __global__ void __launch_bounds__(768, 1) k_pr_omega(PrOmegaArgs a, int nomp, Co
                 sline[q] = e;
             }
             __syncthreads();
-            if (k < a.nomega) {
-                for (int j = g; j < 60; j += G) {
-                    const float al1 = salpha[j];
-                    if (!(al1 < 999.0f)) continue;
-                    const float ang = __fmul_rn(__fsub_rn(al1, womega), K.d2r);
-                    float sn, cs;
-                    sincosf(ang, &sn, &cs);
-                    const float2 csn = make_float2(cs, sn), half2c = make_float2(nxh, nxh);
-                    const float4* sl = sline + j * nr;
-                    float2 acc = make_float2(0.f, 0.f);  // (sum diff*w, sum w) of this line
+            const int nv = *snv;
+            for (int jj = own ? g : nv; jj < nv; jj += G) {
+                const float al1 = salpha[jj];
+                const float ang = __fmul_rn(__fsub_rn(al1, womega), K.d2r);
+                float sn, cs;
+                sincosf(ang, &sn, &cs);
+                const float2 csn = make_float2(cs, sn);
+                const float4* sl = sline + sjl[jj] * nr;
+                float2 acc = make_float2(0.f, 0.f), acd = make_float2(0.f, 0.f);  // (sum diff*w, sum w) of this line
+for (int q0 = 0; q0 < nr; q0 += 32) {
+                    const int q1 = min(nr, q0 + 32);
+                    unsigned near = 0u, bit = 1u;  // HALF: radii whose amplitude is within the margin of its cut
 #pragma unroll 8
-                    for (int iq = 0; iq < nr; ++iq) {
+                    for (int iq = q0; iq < q1; ++iq, bit <<= 1) {
                         const float4 e = sl[iq];
                         if (e.z < 0.0f) continue;
-                        const float fr = (float)(minR + iq);
-                        // sample position (x, y) = FR (cos, sin) + nx/2, then its cell
-                        const float2 xy = __ffma2_rn(make_float2(fr, fr), csn, half2c);
-                        const int lx = (int)xy.x, ly = (int)xy.y;
-                        const float2 f = __fadd2_rn(xy, make_float2(-(float)lx, -(float)ly));
-                        const int b0 = ly * W + lx - offW;
-                        const float2 t00 = sband[b0], t10 = sband[b0 + 1];
-                        const float2 t01 = sband[b0 + W], t11 = sband[b0 + W + 1];
-                        // bilinear on (re, im) pairs: lerp in x on both rows, then in y
-                        const float2 ax2 = make_float2(f.x, f.x), ay2 = make_float2(f.y, f.y);
-                        const float2 m1 = make_float2(-1.f, -1.f);
-                        const float2 v0 = __ffma2_rn(ax2, __ffma2_rn(t00, m1, t10), t00);
-                        const float2 v1 = __ffma2_rn(ax2, __ffma2_rn(t01, m1, t11), t01);
-                        const float2 z = __ffma2_rn(ay2, __ffma2_rn(v0, m1, v1), v0);
-                        const float2 zz = __fmul2_rn(z, z);
-                        const float sq = zz.x + zz.y;
-                        const float amp1 = sq * rsqrtf(sq);  // NaN for 0: fails the cut
+                        const OmegaTerm u = omega_sample(sband, W, offW, (float)(minR + iq), csn, nxh, e.z);
                         // the particle's cut as a select: ~70 % of the lanes pass it, so a
                         // branch would run both sides anyway
-                        const float2 pd = __fmul2_rn(z, make_float2(e.x, e.y));
-                        const float2 pc = __fmul2_rn(z, make_float2(e.y, -e.x));
+                        const float2 pd = __fmul2_rn(u.z, make_float2(e.x, e.y));
+                        const float2 pc = __fmul2_rn(u.z, make_float2(e.y, -e.x));
                         const float d = angle_between_est(pc.x + pc.y, pd.x + pd.y, K.pi);
-                        const float w = fmaf(0.5f, amp1, e.z);
-                        const float2 na = __ffma2_rn(make_float2(d, 1.0f), make_float2(w, w), acc);
-                        const bool ok = amp1 >= e.w;
+                        const float2 na = __ffma2_rn(make_float2(d, 1.0f), make_float2(u.w, u.w), acc);
+                        const bool ok = u.amp >= e.w;
                         acc.x = ok ? na.x : acc.x;
                         acc.y = ok ? na.y : acc.y;
+                        if constexpr (HALF) {
+                            // conj z: (zx ey + zy ex, zx ex - zy ey)
+                            const float dc = angle_between_est(pc.x - pc.y, pd.x - pd.y, K.pi);
+                            const bool nr_cut = fabsf(u.amp - e.w) <= PAIR_MARGIN * e.w;
+                            const float2 nc = __ffma2_rn(make_float2(dc, 1.0f), make_float2(u.w, u.w), acd);
+                            near |= nr_cut ? bit : 0u;
+                            acd.x = ok && !nr_cut ? nc.x : acd.x;
+                            acd.y = ok && !nr_cut ? nc.y : acd.y;
+                        }
                     }
-                    kahan_add(pr1, c1, acc.x);
-                    kahan_add(pr2, c2, acc.y);
+                    if constexpr (HALF) {
+                        if (near) {  // (about one radius of a lane's line in 30)
+                            const float w2 = __fmul_rn(a.step, (float)(k + nown));
+                            float2 csn2;
+                            sincosf(__fmul_rn(__fsub_rn(al1, w2), K.d2r), &csn2.y, &csn2.x);
+                            do {
+                                const int iq = q0 + __ffs(near) - 1;
+                                near &= near - 1u;
+                                const float4 e = sl[iq];
+                                const OmegaTerm x = omega_sample(sband, W, offW, (float)(minR + iq), csn2, nxh, e.z);
+                                const float2 xd = __fmul2_rn(x.z, make_float2(e.x, e.y));
+                                const float2 xc = __fmul2_rn(x.z, make_float2(e.y, -e.x));
+                                const float dx = angle_between_est(xc.x + xc.y, xd.x + xd.y, K.pi);
+                                if (x.amp >= e.w) {
+                                    acd.x = fmaf(dx, x.w, acd.x);
+                                    acd.y += x.w;
+                                }
+                            } while (near);
+                        }
+                    }
+                }
+                kahan_add(pr1, c1, acc.x);
+                kahan_add(pr2, c2, acc.y);
+                if constexpr (HALF) {
+                    kahan_add(qr1, d1, acd.x);
+                    kahan_add(qr2, d2, acd.y);
                 }
             }
         }
-        sred[2 * t] = pr1;
-        sred[2 * t + 1] = pr2;
+        __syncthreads();
+        sred[t] = make_float2(pr1, pr2);
+        if constexpr (HALF) sred[blockDim.x + t] = make_float2(qr1, qr2);
         __syncthreads();
         unsigned long long key = ~0ull;
-        if (g == 0 && k < a.nomega) {
+        // omega t (both halves: nown (HALF ? 2 : 1) of them)
+        for (int o = t; o < a.nomega; o += blockDim.x) {
+            const float2* sr = sred + (o >= nown ? blockDim.x + o - nown : o);
             float s1 = 0.f, s2 = 0.f;
             for (int gg = 0; gg < G; ++gg) {
-                s1 += sred[2 * (gg * nomp + k)];
-                s2 += sred[2 * (gg * nomp + k) + 1];
+                s1 += sr[gg * nown].x;
+                s2 += sr[gg * nown].y;
             }
             const float pr = (s2 > 1.0e-10f) ? s1 / s2 * K.r2d : 999.0f;
             const int base = __float_as_int(a.views[(long)v * 4 + 2]);
-            if (a.pr_array) a.pr_array[(long)p * a.per + base + k] = pr;
-            key = ((unsigned long long)__float_as_uint(pr) << 32) | (unsigned)(base + k);
+            if (a.pr_array) a.pr_array[(long)p * a.per + base + o] = pr;
+            const unsigned long long kk = ((unsigned long long)__float_as_uint(pr) << 32) | (unsigned)(base + o);
+            key = kk < key ? kk : key;
         }
         for (int o = 16; o > 0; o >>= 1) {
             unsigned long long other = __shfl_xor_sync(0xffffffffu, key, o);
@@ -874,27 +957,34 @@ Consts consts() {
 
 }  // namespace
 
-int pr_omega_smem_bytes(const Band& bd, int nomega, int* threads) {
-    int nomp = (nomega + 31) / 32 * 32;
-    if (nomp > 768) return -1;
-    int G = 768 / nomp;
-    if (G < 1) G = 1;
-    int nt = G * nomp;
+// omega + nomega / 2 is half a turn on
+static bool omega_half(int nomega, float step) {
+    return nomega % 2 == 0 && fabsf(step * (float)(nomega / 2) - 180.0f) < 1e-3f;
+}
+
+int pr_omega_smem_bytes(const Band& bd, int nomega, float step, int* threads, int* groups) {
+    if (nomega < 1 || nomega > 768) return -1;
+    const bool half = omega_half(nomega, step);
+    const int nown = half ? nomega / 2 : nomega;
+    // groups of lines: as many as fit 768 threads, and no more than there are lines
+    const int G = std::min(60, 768 / nown), nt = (G * nown + 31) / 32 * 32;
     if (threads) *threads = nt;
-    size_t b = (size_t)bd.W * bd.W * 8 + (size_t)60 * bd.nr * 16 + (size_t)((bd.nr + 3) & ~3) * 4 +
-               64 * 4 + (size_t)2 * nt * 4 + 32 * 8;
+    if (groups) *groups = G;
+    size_t b = (size_t)bd.W * bd.W * 8 + (size_t)std::max(60 * bd.nr, nt / (half ? 1 : 2)) * 16 +
+               (size_t)((bd.nr + 3) & ~3) * 4 + 32 * 8 + 64 * 4 + 64 * 4 + 16;
     return (int)b;
 }
 
 cudaError_t launch_pr_omega(const PrOmegaArgs& a, int B, cudaStream_t st) {
-    int nt = 0;
-    int sm = pr_omega_smem_bytes(a.bd, a.nomega, &nt);
+    int nt = 0, G = 0;
+    int sm = pr_omega_smem_bytes(a.bd, a.nomega, a.step, &nt, &G);
     if (sm < 0) return cudaErrorInvalidValue;
-    int nomp = (a.nomega + 31) / 32 * 32;
-    cudaError_t e = cudaFuncSetAttribute(k_pr_omega, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    const bool half = omega_half(a.nomega, a.step);
+    auto kern = half ? k_pr_omega<true> : k_pr_omega<false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e != cudaSuccess) return e;
     dim3 grid(a.V, B);
-    k_pr_omega<<<grid, nt, sm, st>>>(a, nomp, consts());
+    kern<<<grid, nt, sm, st>>>(a, half ? a.nomega / 2 : a.nomega, G, consts());
     return cudaGetLastError();
 }
 

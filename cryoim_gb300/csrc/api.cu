@@ -299,6 +299,11 @@ struct Ctx {
     DBuf<float2> fft, band, ralpha;
     DBuf<unsigned long long> best;
     DBuf<int> flag, sel;
+    // rings of the amplitude-cut fits (ensure_rings)
+    RingTable rings{};
+    DBuf<short2> rpix;
+    DBuf<int> rint;
+    DBuf<double> rsum;
     std::map<int, cufftHandle> plans;
     // reconstruction
     DBuf<float4> acc;
@@ -414,6 +419,7 @@ struct Ctx {
         alpha.release(); imgs.release(); par.release(); fcut0.release(); ctf.release();
         tfcut.release(); state.release(); cand.release(); rpr.release(); rot.release();
         prbuf.release(); fft.release(); band.release(); ralpha.release(); best.release();
+        rpix.release(); rint.release(); rsum.release();
         flag.release(); sel.release(); acc.release(); acc5.release(); oct.release(); ops5.release(); samples.release(); vol.release();
         mapcube.release(); mapreal.release(); csamples.release(); bmat.release(); amat.release(); corigins.release();
         topv.release(); kcc.release(); kcand.release(); topi.release(); gerr.release();
@@ -453,13 +459,47 @@ int plan2d(Ctx* c, int nb, cufftHandle* out) {
     return CRYOIM_OK;
 }
 
+// The pixels, their number and radius sum of every ring int(|h| + 1/2) = minR .. maxR on the
+// half plane ky >= 0 (FT_amp_expfit.f90:13-25).
+int ensure_rings(Ctx* c) {
+    if (c->rings.pix) return CRYOIM_OK;
+    const int r0 = c->bd.min_r, R = c->bd.max_r, nr = c->bd.nr;
+    std::vector<std::vector<short2>> px(nr);
+    std::vector<double> sum(nr, 0.0);
+    for (int ky = 0; ky <= R; ++ky)
+        for (int hx = -R; hx <= R; ++hx) {
+            const int d2 = hx * hx + ky * ky;
+            int ir = (int)std::sqrt((double)d2);
+            if (d2 > ir * ir + ir) ++ir;  // ring ir: ir^2 - ir + 1 .. ir^2 + ir
+            if (ir < r0 || ir > R || d2 == 0) continue;
+            px[ir - r0].push_back(make_short2((short)hx, (short)ky));
+            sum[ir - r0] += (double)std::sqrt((float)d2);
+        }
+    std::vector<short2> all;
+    std::vector<int> tab(2 * (size_t)nr + 1);  // start [nr + 1], num [nr]
+    for (int k = 0; k < nr; ++k) {
+        tab[k] = (int)all.size();
+        tab[nr + 1 + k] = (int)px[k].size();
+        all.insert(all.end(), px[k].begin(), px[k].end());
+    }
+    tab[nr] = (int)all.size();
+    int r;
+    if ((r = c->rpix.ensure(all.size() + 1)) || (r = c->rint.ensure(tab.size())) || (r = c->rsum.ensure(nr))) return r;
+    CK(cudaMemcpyAsync(c->rpix.p, all.data(), sizeof(short2) * all.size(), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->rint.p, tab.data(), sizeof(int) * tab.size(), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->rsum.p, sum.data(), sizeof(double) * nr, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    c->rings = RingTable{c->rpix.p, c->rint.p, c->rint.p + nr + 1, c->rsum.p};
+    return CRYOIM_OK;
+}
+
 int check_ready(Ctx* c, bool need_templates) {
     if (!c) return fail(CRYOIM_ERR_ARG, "null context");
     if (!c->have_params) return fail(CRYOIM_ERR_STATE, "cryoim_set_params has not been called");
     if (need_templates && c->T <= 0)
         return fail(CRYOIM_ERR_STATE, "cryoim_load_templates has not been called");
     CK(cudaSetDevice(c->device));
-    return CRYOIM_OK;
+    return ensure_rings(c);
 }
 
 int ensure_batch(Ctx* c, int B) {
@@ -507,7 +547,7 @@ int transform_batch(Ctx* c, const float* d_src, int nb, int B, const std::vector
     int r = plan2d(c, nb, &h);
     if (r) return r;
     CKF(cufftExecC2C(h, (cufftComplex*)c->fft.p, (cufftComplex*)c->fft.p, CUFFT_FORWARD));
-    launch_post_fft(c->fft.p, nb, c->bd, shift ? pv.sx : nullptr, shift ? pv.sy : nullptr,
+    launch_post_fft(c->fft.p, nb, c->bd, c->rings, shift ? pv.sx : nullptr, shift ? pv.sy : nullptr,
                     c->band.p, need_fcut ? c->fcut0.p : nullptr, c->stream);
     CK(cudaGetLastError());
     return CRYOIM_OK;
@@ -640,7 +680,7 @@ int globesearch_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle*
         if (c->p.apply_ctf) {
             launch_ctf_band(nb, c->bd, pv.dfs, c->p.apix, c->p.vol, c->p.cs, c->p.ampwg, c->ctf.p,
                             c->stream);
-            launch_tmpl_fcut(c->tband.p, c->T, c->ctf.p, nb, c->bd, c->tfcut.p, c->stream);
+            launch_tmpl_fcut(c->tband.p, c->T, c->ctf.p, nb, c->bd, &c->rings, c->tfcut.p, c->stream);
             CK(cudaGetLastError());
             ctfp = c->ctf.p;
             tfc = c->tfcut.p;
@@ -742,7 +782,7 @@ int refine_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* part
         if (c->p.apply_ctf) {
             launch_ctf_band(nb, c->bd, pv.dfs, c->p.apix, c->p.vol, c->p.cs, c->p.ampwg, c->ctf.p,
                             c->stream);
-            launch_tmpl_fcut(c->tband.p, T, c->ctf.p, nb, c->bd, c->tfcut.p, c->stream);
+            launch_tmpl_fcut(c->tband.p, T, c->ctf.p, nb, c->bd, &c->rings, c->tfcut.p, c->stream);
             ctfp = c->ctf.p;
             tfc = c->tfcut.p;
             tfs = (long)T * c->bd.nr;
@@ -1725,6 +1765,7 @@ int refresh_lane(Ctx* c, int i) {
     h->p = c->p;
     h->have_params = c->have_params;
     h->bd = c->bd;
+    h->rings = c->rings;
     h->batch = c->batch;
     h->ops.borrow(c->ops);
     h->T = c->T;
@@ -1958,7 +1999,7 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
                 launch_ctf_band(nb, L->bd, pv.dfs, L->p.apix, L->p.vol, L->p.cs, L->p.ampwg, L->ctf.p, L->stream);
                 ctfp = L->ctf.p;
                 if (T > 0 && !local) {
-                    launch_tmpl_fcut(L->tband.p, T, L->ctf.p, nb, L->bd, L->tfcut.p, L->stream);
+                    launch_tmpl_fcut(L->tband.p, T, L->ctf.p, nb, L->bd, &L->rings, L->tfcut.p, L->stream);
                     tfc = L->tfcut.p;
                     tfs = (long)T * L->bd.nr;
                 }
@@ -2644,6 +2685,7 @@ int cryoim_set_params(void* ctx, const cryoim_params* p) {
     c->bd = make_band(p->fftsize, p->min_r, p->max_r);
     c->have_params = true;
     if (geom_changed) {
+        c->rings = RingTable{};
         for (auto& kv : c->plans) cufftDestroy(kv.second);
         c->plans.clear();
         c->T = 0;  // templates depend on the band geometry
@@ -2806,7 +2848,7 @@ int cryoim_prscore_omega(void* ctx, const float* ft_a, const float* ft_b, const 
     const float* ctfp = nullptr;
     if (ctf) {
         CK(cudaMemcpyAsync(c->ctf.p, cband.data(), sizeof(float) * W * W, cudaMemcpyHostToDevice, c->stream));
-        launch_tmpl_fcut(c->tband.p, T, c->ctf.p, 1, c->bd, c->tfcut.p, c->stream);
+        launch_tmpl_fcut(c->tband.p, T, c->ctf.p, 1, c->bd, &c->rings, c->tfcut.p, c->stream);
         ctfp = c->ctf.p;
         tfc = c->tfcut.p;
         tfs = (long)T * nr;
@@ -2861,7 +2903,7 @@ int cryoim_prscore(void* ctx, const float* ft_a, const float* ft_b, const float*
     const float* ctfp = nullptr;
     if (ctf) {
         CK(cudaMemcpyAsync(c->ctf.p, cband.data(), sizeof(float) * W * W, cudaMemcpyHostToDevice, c->stream));
-        launch_tmpl_fcut(c->tband.p, T, c->ctf.p, 1, c->bd, c->tfcut.p, c->stream);
+        launch_tmpl_fcut(c->tband.p, T, c->ctf.p, 1, c->bd, &c->rings, c->tfcut.p, c->stream);
         ctfp = c->ctf.p;
         tfc = c->tfcut.p;
         tfs = (long)T * nr;

@@ -38,16 +38,24 @@ __host__ __device__ inline long acc_cell(const Band& b, int hx, int ky, int lz) 
 void launch_prep_images(const float* imgs, int B, int nx, const float* ox, const float* oy,
                         int use_mask, float mask_px, int normalize, float2* fft, int* flag,
                         cudaStream_t st);
-// scale 1/nx^2, b = -Im, Fcut fit, optional origin shift (sx/sy per image, may be null),
-// band extraction.
-void launch_post_fft(const float2* fft, int B, Band bd, const float* sx, const float* sy,
+// The rings of the amplitude-cut fits over the ky >= 0 half plane, on the device: the pixels
+// (hx, ky) of ring k (minR + k) at pix[start[k] .. start[k + 1]), their number and radius sum.
+struct RingTable {
+    const short2* pix;
+    const int* start;    // [nr + 1]
+    const int* num;      // [nr]
+    const double* rsum;  // [nr]
+};
+// scale 1/nx^2, b = -Im, Fcut fit (if fcut), optional origin shift (sx/sy per image, may be
+// null), band extraction.
+void launch_post_fft(const float2* fft, int B, Band bd, const RingTable& rt, const float* sx, const float* sy,
                      float2* band, float* fcut, cudaStream_t st);
 // getCTF2d over the band for B images (per-image defocus triples in dfs: df1, df2, astig)
 void launch_ctf_band(int B, Band bd, const float* dfs, float apix, float vol, float cs,
                      float ampwg, float* ctf, cudaStream_t st);
-// Fcut of template x CTF for every (image, template)
-void launch_tmpl_fcut(const float2* tband, int T, const float* ctf, int B, Band bd, float* tfcut,
-                      cudaStream_t st);
+// Fcut of template x CTF for every (image, template); rt null: without the list of ring pixels
+void launch_tmpl_fcut(const float2* tband, int T, const float* ctf, int B, Band bd, const RingTable* rt,
+                      float* tfcut, cudaStream_t st);
 // common-line angle pairs for every (view, template, operator); views: V x 2 (theta, phi)
 void launch_alpha_table(const float* views, int V, const float* tort, int T, const float* ops,
                         float2* alpha, cudaStream_t st);

@@ -120,7 +120,7 @@ extern "C" int cryoim_prscore_noalloc(int32_t nx, int32_t min_r, int32_t max_r,
     }
     const float* tfc = d_tmpl_fcut;
     if (e == cudaSuccess && d_ctf_band) {
-        launch_tmpl_fcut(reinterpret_cast<const float2*>(d_tmpl_band), T, d_ctf_band, 1, bd, cuts, st);
+        launch_tmpl_fcut(reinterpret_cast<const float2*>(d_tmpl_band), T, d_ctf_band, 1, bd, nullptr, cuts, st);
         e = cudaGetLastError();
         tfc = cuts;
     }

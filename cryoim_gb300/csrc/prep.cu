@@ -54,7 +54,8 @@ __device__ __forceinline__ void two_sum_acc(float& h, float& l, float x) {
 }
 
 // One block of 1024 threads per image; warp w walks rows w, w + 32, ..., its lanes the
-// columns, so no pixel index is split by a division.  The image sums the reference takes
+// columns, so no pixel index is split by a division.  Issue-bound on its one SM: the distance to
+// the mask's centre decides most pixels by its square (the root only near the two radii).  The image sums the reference takes
 // in FP64 are FP32 TwoSum pairs per thread (exact to far below FP32 rounding), combined
 // in FP64 across the block.
 __global__ void k_prep_images(const float* __restrict__ imgs, int nx,
@@ -90,6 +91,8 @@ __global__ void k_prep_images(const float* __restrict__ imgs, int nx,
     float R2 = mask + 3.0f;
     if (R2 > (float)hh) R2 = (float)hh;
     const float x0 = ox[p] + (float)hh, y0 = oy[p] + (float)hh;
+    // squares that are certainly at or inside R1 and certainly beyond R2 (the root rounds by 2^-24)
+    const float in2 = R1 * R1 * 0.999999f, out2 = R2 * R2 * 1.000001f;
     double summ = 0;
     if (use_mask) {
         float h = 0.f, l = 0.f;
@@ -98,7 +101,9 @@ __global__ void k_prep_images(const float* __restrict__ imgs, int nx,
             const float yy = (-y0 + (float)iy) * (-y0 + (float)iy);
             for (int ix = lane; ix < nx; ix += 32) {
                 const float xx = (-x0 + (float)ix) * (-x0 + (float)ix);
-                const float ra = sqrtf(yy + xx);
+                const float r2 = yy + xx;
+                if (r2 <= in2 || r2 > out2) continue;
+                const float ra = sqrtf(r2);
                 if (ra > R1 && ra <= R2) {
                     float v = img[(long)iy * nx + ix];
                     if (normalize) v = (v - avg) / nd;
@@ -120,7 +125,8 @@ __global__ void k_prep_images(const float* __restrict__ imgs, int nx,
             if (normalize) v = (v - avg) / nd;
             if (use_mask) {
                 const float xx = (-x0 + (float)ix) * (-x0 + (float)ix);
-                const float ra = sqrtf(yy + xx);
+                const float r2 = yy + xx;
+                const float ra = r2 <= in2 ? R1 : r2 > out2 ? R2 + 1.0f : sqrtf(r2);
                 if (ra > R1 && ra <= R2) {
                     float edge = (1.0f + cosf(pi * (ra - R1) / 6.0f)) / 2.0f;
                     v = (float)((double)(v * edge) + (double)(1.0f - edge) * summ);
@@ -146,112 +152,108 @@ __device__ __forceinline__ int isqrt_ceil(int v) {
     return s * s < v ? s + 1 : s;
 }
 
-// FT_amp_expfit.f90:27-46: per-ring means, log, 2x2 least squares, Fcut.
-__device__ void expfit_finish(const double* sfav, const double* sres, const int* snum, int nr,
+// FT_amp_expfit.f90:27-46: per-ring means, log, 2x2 least squares, Fcut.  Called by the whole
+// block: the rings' logarithms, means and exponentials a thread each, the least-squares sums by one
+// thread in ring order.  sres: (double) radius sums, snum: pixels of each ring; fit: 2 nr floats.
+__device__ void expfit_finish(const double* sfav, const double* sres, const int* snum, int nr, float* fit,
                               float* out) {
-    float aa11 = 0.f, aa12 = 0.f, aa22 = 0.f, bb1 = 0.f, bb2 = 0.f;
-    for (int k = 0; k < nr; ++k) {
-        float fa = (float)sfav[k], rl = (float)sres[k];
-        int num = snum[k];
-        float fl;
+    __shared__ float x12[2];
+    float* srl = fit;
+    float* sfl = fit + nr;
+    __syncthreads();
+    for (int k = threadIdx.x; k < nr; k += blockDim.x) {
+        const float fa = (float)sfav[k];
+        float rl = (float)sres[k], fl = 0.0f;
+        const int num = snum[k];
         if (num > 0 && fa > 0.0f) {
             rl = rl / (float)num;
             fl = logf(fa / (float)num);
-        } else {
-            fl = 0.0f;
         }
-        aa11 = aa11 + rl * rl;
-        aa12 = aa12 + rl * 1.0f;
-        aa22 = aa22 + 1.0f * 1.0f;
-        bb1 = bb1 + rl * fl;
-        bb2 = bb2 + 1.0f * fl;
+        srl[k] = rl;
+        sfl[k] = fl;
     }
-    float aa21 = aa12;
-    float x2 = (bb2 - bb1 * aa21 / aa11) / (aa22 - aa12 * aa21 / aa11);
-    float x1 = (bb1 - aa12 * x2) / aa11;
-    for (int k = 0; k < nr; ++k) {
-        float rl = (float)sres[k];
-        int num = snum[k];
-        if (num > 0 && (float)sfav[k] > 0.0f) rl = rl / (float)num;
-        out[k] = expf(rl * x1 + x2) * 0.8f;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float aa11 = 0.f, aa12 = 0.f, aa22 = 0.f, bb1 = 0.f, bb2 = 0.f;
+        for (int k = 0; k < nr; ++k) {
+            const float rl = srl[k], fl = sfl[k];
+            aa11 = aa11 + rl * rl;
+            aa12 = aa12 + rl * 1.0f;
+            aa22 = aa22 + 1.0f * 1.0f;
+            bb1 = bb1 + rl * fl;
+            bb2 = bb2 + 1.0f * fl;
+        }
+        const float aa21 = aa12;
+        const float x2 = (bb2 - bb1 * aa21 / aa11) / (aa22 - aa12 * aa21 / aa11);
+        x12[1] = x2;
+        x12[0] = (bb1 - aa12 * x2) / aa11;
+    }
+    __syncthreads();
+    const float x1 = x12[0], x2 = x12[1];
+    for (int k = threadIdx.x; k < nr; k += blockDim.x) out[k] = expf(srl[k] * x1 + x2) * 0.8f;
+}
+
+// Sums of the amplitudes amp(hx, ky) of each ring's pixels, a warp per ring in turn (FP32 TwoSum
+// pairs per lane, then FP64), into sfav (shared), by the context's list of each ring's pixels.
+template <class Amp>
+__device__ __forceinline__ void ring_sums(const RingTable& rt, int nr, double* sfav, Amp amp) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    for (int k = warp; k < nr; k += nw) {
+        float fh = 0.f, fl = 0.f;
+        const int e = rt.start[k + 1];
+        for (int q = rt.start[k] + lane; q < e; q += 32) {
+            const short2 hk = rt.pix[q];
+            two_sum_acc(fh, fl, amp(hk.x, hk.y));
+        }
+        double fa = (double)fh + (double)fl;
+        for (int o = 16; o > 0; o >>= 1) fa += __shfl_xor_sync(0xffffffffu, fa, o);
+        if (lane == 0) sfav[k] = fa;
     }
 }
 
 // ---------------------------------------------------------------------------
 // after the forward FFT: 1/nx^2, b = -Im (img2d_FFT.f90:18-19, FFTW.f90:185),
 // Fcut fit (FT_amp_expfit.f90:13-25), optional origin shift (img2d_FT_centshift.f90:8-16)
-// and extraction of the band window.
+// and extraction of the band window.  Blocks (x, p): x = 0 the fit of image p if fcut is asked
+// for, the others 256 pixels of its band each.
 // ---------------------------------------------------------------------------
-__global__ void k_post_fft(const float2* __restrict__ fft, Band bd, const float* __restrict__ sx,
-                           const float* __restrict__ sy, float pi, float2* __restrict__ band,
-                           float* __restrict__ fcut) {
-    extern __shared__ double dsm[];
-    const int nr = bd.nr, R = bd.max_r, nx = bd.nx, h = nx / 2;
-    double* sfav = dsm;
-    double* sres = dsm + nr;
-    int* snum = (int*)(dsm + 2 * nr);
-    const int p = blockIdx.x;
+__global__ void __launch_bounds__(256) k_post_fft(const float2* __restrict__ fft, Band bd, RingTable rt,
+                                                  const float* __restrict__ sx, const float* __restrict__ sy,
+                                                  float pi, float2* __restrict__ band, float* __restrict__ fcut) {
+    const int nr = bd.nr, nx = bd.nx, h = nx / 2;
+    const int p = blockIdx.y;
     const long nn = (long)nx * nx;
     const float2* f = fft + p * nn;
     const float s = (float)nn;
-    if (fcut) {  // (no amplitude cut asked: the band only)
-        // ring sums over the ky >= 0 half plane, one warp per ring as in k_tmpl_fcut
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-        for (int ir = bd.min_r + warp; ir <= R; ir += nw) {
-            float fh = 0.f, fl = 0.f, rh = 0.f, rl = 0.f;
-            int n = 0;
-            const int lo = ir * ir - ir + 1, hi = ir * ir + ir;
-            for (int ky = lane; ky <= ir; ky += 32) {
-                const int k2 = ky * ky;
-                if (k2 > hi) continue;
-                const int hmax = isqrt_floor(hi - k2);
-                const int hmin = lo - k2 <= 0 ? 0 : isqrt_ceil(lo - k2);
-                for (int hx = hmin; hx <= hmax; ++hx) {
-                    const float rad = sqrtf((float)(hx * hx + k2));
-                    for (int sgn = (hx == 0 ? 1 : -1); sgn <= 1; sgn += 2) {
-                        const float2 v = f[(long)(ky + h) * nx + (sgn * hx + h)];
-                        const float a = v.x / s, b = -(v.y / s);
-                        two_sum_acc(fh, fl, sqrtf(a * a + b * b));
-                        two_sum_acc(rh, rl, rad);
-                        ++n;
-                    }
-                }
-            }
-            double fa = (double)fh + (double)fl, rs = (double)rh + (double)rl;
-            for (int o = 16; o > 0; o >>= 1) {
-                fa += __shfl_xor_sync(0xffffffffu, fa, o);
-                rs += __shfl_xor_sync(0xffffffffu, rs, o);
-                n += __shfl_xor_sync(0xffffffffu, n, o);
-            }
-            if (lane == 0) {
-                sfav[ir - bd.min_r] = fa;
-                sres[ir - bd.min_r] = rs;
-                snum[ir - bd.min_r] = n;
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) expfit_finish(sfav, sres, snum, nr, fcut + (long)p * nr);
+    if (fcut && blockIdx.x == 0) {
+        extern __shared__ double dsm[];
+        ring_sums(rt, nr, dsm, [&](int hx, int ky) {
+            const float2 v = f[(long)(ky + h) * nx + (hx + h)];
+            const float a = v.x / s, b = -(v.y / s);
+            return sqrtf(a * a + b * b);
+        });
+        expfit_finish(dsm, rt.rsum, rt.num, nr, reinterpret_cast<float*>(dsm + nr), fcut + (long)p * nr);
+        return;
     }
     const int W = bd.W;
     const bool shift = (sx != nullptr);
     const float xs = shift ? sx[p] + (float)h : 0.f, ys = shift ? sy[p] + (float)h : 0.f;
-    float2* ob = band + (long)p * W * W;
-    for (int q = threadIdx.x; q < W * W; q += blockDim.x) {
-        int by = q / W, bx = q % W;
-        int hi = bd.off + bx, ki = bd.off + by;
-        float2 v = f[(long)ki * nx + hi];
-        float a = v.x / s, b = -(v.y / s);
-        if (shift) {
-            int hx = hi - h, ky = ki - h;
-            float phase = 2.0f * pi * (xs * (float)hx + ys * (float)ky) / (float)nx;
-            float c = cosf(phase), sn = sinf(phase);
-            float fr = (a * c + b * sn);
-            float fi = (-a * sn + b * c);
-            a = fr;
-            b = fi;
-        }
-        ob[q] = make_float2(a, b);
+    const int q = (blockIdx.x - (fcut ? 1 : 0)) * blockDim.x + threadIdx.x;
+    if (q >= W * W) return;
+    const int by = q / W, bx = q % W;
+    const int hi = bd.off + bx, ki = bd.off + by;
+    float2 v = f[(long)ki * nx + hi];
+    float a = v.x / s, b = -(v.y / s);
+    if (shift) {
+        int hx = hi - h, ky = ki - h;
+        float phase = 2.0f * pi * (xs * (float)hx + ys * (float)ky) / (float)nx;
+        float c = cosf(phase), sn = sinf(phase);
+        float fr = (a * c + b * sn);
+        float fi = (-a * sn + b * c);
+        a = fr;
+        b = fi;
     }
+    band[(long)p * W * W + q] = make_float2(a, b);
 }
 
 // getCTF2d.f90:2-29 evaluated over the band window.
@@ -282,22 +284,44 @@ __global__ void k_ctf_band(Band bd, const float* __restrict__ dfs, float apix, f
 // Template amplitude cuts under each particle's CTF (FT_amp_expfit.f90 on template x
 // CTF over the ky >= 0 half plane): one block per (template, particle), one warp per
 // ring at a time.  Ring ir holds the pixels with int(|h| + 1/2) = ir, i.e. the integer
-// range ir^2 - ir + 1 <= hx^2 + ky^2 <= ir^2 + ir; lane l takes rows ky = l, l + 32, ...
-// and the ring's hx on them, summing |t c|, the radius and the count in FP64 (then a
-// warp reduction: no atomics, a fixed order).
-__global__ void k_tmpl_fcut(const float2* __restrict__ tband, int T, const float* __restrict__ ctf,
-                            Band bd, float* __restrict__ tfcut) {
+// range ir^2 - ir + 1 <= hx^2 + ky^2 <= ir^2 + ir.  The radius sums and counts do not depend on
+// the images and come with the list of the rings' pixels, whose lanes are full where a walk of
+// the rows ky leaves most of a warp waiting for the rows near the ring's top (64 particles x 20
+// templates at maxR 64: 165 us by rows, 59 by the list).
+__global__ void __launch_bounds__(256) k_tmpl_fcut(const float2* __restrict__ tband, int T,
+                                                   const float* __restrict__ ctf, Band bd, RingTable rt,
+                                                   float* __restrict__ tfcut) {
+    extern __shared__ double dsm[];
+    const int nr = bd.nr, R = bd.max_r, W = bd.W;
+    const int i = blockIdx.x, p = blockIdx.y;
+    const float2* tb = tband + (long)i * W * W;
+    const float* cb = ctf + (long)p * W * W;
+    ring_sums(rt, nr, dsm, [&](int hx, int ky) {
+        const int b = (ky + R) * W + (hx + R);
+        const float c = cb[b];
+        const float2 t = tb[b];
+        const float a2 = t.x * c, b2 = t.y * c;
+        return sqrtf(a2 * a2 + b2 * b2);
+    });
+    expfit_finish(dsm, rt.rsum, rt.num, nr, reinterpret_cast<float*>(dsm + nr), tfcut + ((long)p * T + i) * nr);
+}
+
+// The same without the list, for the allocation-free entry point: lane l takes rows ky = l,
+// l + 32, ... and the ring's hx on them.
+__global__ void __launch_bounds__(256) k_tmpl_fcut_rows(const float2* __restrict__ tband, int T,
+                                                        const float* __restrict__ ctf, Band bd,
+                                                        float* __restrict__ tfcut) {
     extern __shared__ double dsm[];
     const int nr = bd.nr, R = bd.max_r, W = bd.W;
     double* sfav = dsm;
     double* sres = dsm + nr;
-    int* snum = (int*)(dsm + 2 * nr);
+    float* fit = reinterpret_cast<float*>(dsm + 2 * nr);
+    int* snum = reinterpret_cast<int*>(fit + 2 * nr);
     const int i = blockIdx.x, p = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const float2* tb = tband + (long)i * W * W;
     const float* cb = ctf + (long)p * W * W;
     for (int ir = bd.min_r + warp; ir <= R; ir += nw) {
-        // per lane an FP32 pair (two_sum_acc), to FP64 once per lane
         float fh = 0.f, fl = 0.f, rh = 0.f, rl = 0.f;
         int n = 0;
         const int lo = ir * ir - ir + 1, hi = ir * ir + ir;
@@ -331,8 +355,7 @@ __global__ void k_tmpl_fcut(const float2* __restrict__ tband, int T, const float
             snum[ir - bd.min_r] = n;
         }
     }
-    __syncthreads();
-    if (threadIdx.x == 0) expfit_finish(sfav, sres, snum, nr, tfcut + ((long)p * T + i) * nr);
+    expfit_finish(sfav, sres, snum, nr, fit, tfcut + ((long)p * T + i) * nr);
 }
 
 // icos_crosslin_angle.f90 for every (view, template, operator).
@@ -579,10 +602,11 @@ void launch_prep_images(const float* imgs, int B, int nx, const float* ox, const
                                       fft, flag);
 }
 
-void launch_post_fft(const float2* fft, int B, Band bd, const float* sx, const float* sy,
+void launch_post_fft(const float2* fft, int B, Band bd, const RingTable& rt, const float* sx, const float* sy,
                      float2* band, float* fcut, cudaStream_t st) {
-    size_t sm = (size_t)bd.nr * (2 * sizeof(double) + sizeof(int)) + 16;
-    k_post_fft<<<B, 1024, sm, st>>>(fft, bd, sx, sy, angles().pi, band, fcut);
+    const size_t sm = (size_t)bd.nr * (sizeof(double) + 2 * sizeof(float));
+    k_post_fft<<<dim3(cdiv((long)bd.W * bd.W, 256) + (fcut ? 1 : 0), B), 256, sm, st>>>(fft, bd, rt, sx, sy,
+                                                                                       angles().pi, band, fcut);
 }
 
 void launch_ctf_band(int B, Band bd, const float* dfs, float apix, float vol, float cs,
@@ -591,11 +615,14 @@ void launch_ctf_band(int B, Band bd, const float* dfs, float apix, float vol, fl
     k_ctf_band<<<g, 256, 0, st>>>(bd, dfs, apix, vol, cs, ampwg, angles().pi, ctf);
 }
 
-void launch_tmpl_fcut(const float2* tband, int T, const float* ctf, int B, Band bd, float* tfcut,
-                      cudaStream_t st) {
-    size_t sm = (size_t)bd.nr * (2 * sizeof(double) + sizeof(int)) + 16;
-    dim3 g(T, B);
-    k_tmpl_fcut<<<g, 256, sm, st>>>(tband, T, ctf, bd, tfcut);
+void launch_tmpl_fcut(const float2* tband, int T, const float* ctf, int B, Band bd, const RingTable* rt,
+                      float* tfcut, cudaStream_t st) {
+    const dim3 g(T, B);
+    if (rt)
+        k_tmpl_fcut<<<g, 256, (size_t)bd.nr * (sizeof(double) + 2 * sizeof(float)), st>>>(tband, T, ctf, bd, *rt, tfcut);
+    else
+        k_tmpl_fcut_rows<<<g, 256, (size_t)bd.nr * (2 * sizeof(double) + 2 * sizeof(float) + sizeof(int)), st>>>(
+            tband, T, ctf, bd, tfcut);
 }
 
 void launch_alpha_table(const float* views, int V, const float* tort, int T, const float* ops,

@@ -297,6 +297,7 @@ struct Ctx {
     // per-batch scratch
     DBuf<float> imgs, par, fcut0, ctf, tfcut, state, cand, rpr, rot, prbuf;
     DBuf<float2> fft, band, ralpha;
+    DBuf<double2> rpart;
     DBuf<unsigned long long> best;
     DBuf<int> flag, sel;
     // rings of the amplitude-cut fits (ensure_rings)
@@ -418,7 +419,7 @@ struct Ctx {
         ops.release(); tband.release(); tfcut0.release(); tort.release(); d_views.release();
         alpha.release(); imgs.release(); par.release(); fcut0.release(); ctf.release();
         tfcut.release(); state.release(); cand.release(); rpr.release(); rot.release();
-        prbuf.release(); fft.release(); band.release(); ralpha.release(); best.release();
+        prbuf.release(); fft.release(); band.release(); ralpha.release(); rpart.release(); best.release();
         rpix.release(); rint.release(); rsum.release();
         flag.release(); sel.release(); acc.release(); acc5.release(); oct.release(); ops5.release(); samples.release(); vol.release();
         mapcube.release(); mapreal.release(); csamples.release(); bmat.release(); amat.release(); corigins.release();
@@ -750,12 +751,17 @@ int refine_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* part
     const long nn = (long)nx * nx;
     if ((r = ensure_batch(c, B))) return r;
     if ((r = c->state.ensure((size_t)B * 6))) return r;
-    if ((r = c->cand.ensure((size_t)B * 55))) return r;
-    if ((r = c->rpr.ensure((size_t)B * 11))) return r;
-    if ((r = c->ralpha.ensure((size_t)B * 11 * T * 60))) return r;
+    if ((r = c->cand.ensure(2 * (size_t)B * 55))) return r;  // this cycle's and the last one's
+    if ((r = c->ralpha.ensure((size_t)std::min(B, P) * 11 * T * 60))) return r;
+    if (c->num_sms == 0) CK(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, c->device));
+    const long w2 = (long)c->bd.W * c->bd.W;
     std::vector<float> hpar(8 * B), hstate(6 * B);
     for (int b0 = 0; b0 < P; b0 += B) {
         const int nb = std::min(B, P - b0);
+        // blocks per candidate; 0: the band does not fit shared memory (k_pr_single, one block)
+        const int splits = pr_refine_splits(c->bd, T, nb, c->num_sms), S = std::max(1, splits);
+        if ((r = c->rpart.ensure((size_t)nb * 11 * S))) return r;
+        if (splits && c->p.apply_ctf && (r = c->tbandc.ensure((size_t)std::min(B, P) * T * w2))) return r;
         const float* d_src;
         if (on_device) {
             d_src = imgs + b0 * nn;
@@ -789,20 +795,32 @@ int refine_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* part
         }
         CK(cudaMemcpyAsync(c->state.p, hstate.data(), sizeof(float) * 6 * nb, cudaMemcpyHostToDevice,
                            c->stream));
+        if (splits && ctfp) CK(launch_tband_ctf(c->tband.p, T, ctfp, c->bd, nb, c->tbandc.p, c->stream));
         float fac = 1.0f;
+        float* cand = c->cand.p;
+        const float* prev = nullptr;
         for (int cyc = 1; cyc <= c->p.ncycle; ++cyc) {
             float dang = c->p.delta_angle * fac, dtran = c->p.delta_trans * fac;
             fac = fac * 0.8f;
-            launch_refine_candidates(c->state.p, nb, dang, dtran, c->ops.p, c->cand.p, c->stream);
-            launch_refine_alpha(c->cand.p, nb, c->tort.p, T, c->ops.p, c->ralpha.p, c->stream);
+            launch_refine_step(c->state.p, prev, c->rpart.p, S, nb, dang, dtran, c->tort.p, T, c->ops.p, cand,
+                               c->ralpha.p, c->stream);
             PrSingleArgs a{};
             a.band = c->band.p; a.fcut0 = c->fcut0.p; a.tband = c->tband.p; a.tfcut = tfc;
-            a.tfcut_pstride = tfs; a.ctf = ctfp; a.cand = c->cand.p; a.alpha = c->ralpha.p;
-            a.T = T; a.bd = c->bd; a.pr = c->rpr.p;
-            CK(launch_pr_single(a, nb, c->stream));
-            launch_refine_select(c->cand.p, c->rpr.p, nb, c->state.p, c->stream);
+            a.tfcut_pstride = tfs; a.ctf = ctfp; a.cand = cand; a.alpha = c->ralpha.p;
+            a.T = T; a.bd = c->bd;
+            if (splits) {
+                a.tbandc = ctfp ? c->tbandc.p : nullptr;
+                CK(launch_pr_refine(a, nb, S, c->rpart.p, c->stream));
+            } else {
+                a.part = c->rpart.p;
+                CK(launch_pr_single(a, nb, c->stream));
+            }
             CK(cudaGetLastError());
+            prev = cand;
+            cand = cand == c->cand.p ? c->cand.p + (size_t)B * 55 : c->cand.p;
         }
+        if (prev) launch_refine_last(prev, c->rpart.p, S, nb, c->state.p, c->stream);
+        CK(cudaGetLastError());
         CK(cudaMemcpyAsync(hstate.data(), c->state.p, sizeof(float) * 6 * nb, cudaMemcpyDeviceToHost,
                            c->stream));
         if ((r = check_flag(c))) return r;

@@ -59,13 +59,17 @@ void launch_tmpl_fcut(const float2* tband, int T, const float* ctf, int B, Band 
 // common-line angle pairs for every (view, template, operator); views: V x 2 (theta, phi)
 void launch_alpha_table(const float* views, int V, const float* tort, int T, const float* ops,
                         float2* alpha, cudaStream_t st);
-// refinement: the 11 candidates of every image (ort_cent_11) and their angle pairs
-void launch_refine_candidates(float* state, int B, float dang, float dtran, const float* ops,
-                              float* cand, cudaStream_t st);
+// refinement, a step up to the scores: cand [B][11][5] <- the candidates (ort_cent_11) around the
+// first minimum of prev's scores (S partial sums (PR numerator, weight) each at prev_part
+// [B][11][S]; prev null: around state [B][6]), alpha <- their angle pairs
+void launch_refine_step(const float* state, const float* prev, const double2* prev_part, int S, int B, float dang,
+                        float dtran, const float* tort, int T, const float* ops, float* cand, float2* alpha,
+                        cudaStream_t st);
+// state <- the first minimum of the last candidates and its score
+void launch_refine_last(const float* cand, const double2* part, int S, int B, float* state, cudaStream_t st);
+// common-line angle pairs of ncand candidates of every image
 void launch_refine_alpha(const float* cand, int B, const float* tort, int T, const float* ops,
                          float2* alpha, cudaStream_t st, int ncand = 11);
-void launch_refine_select(const float* cand, const float* pr, int B, float* state,
-                          cudaStream_t st);
 // reconstruction finish: fold / divide / sign into the full complex grid
 // int_shell: 0 keeps |h| <= maxR (reconstruct.f90), 1 keeps int(|h|) <= maxR
 // (merge_reconstruct.f90)
@@ -109,6 +113,7 @@ struct PrSingleArgs {
     int T;
     Band bd;
     float* pr;               // [B][ncand]
+    double2* part = nullptr; // instead of pr: the two sums [B][ncand]
     int ncand = 11;          // 11 for the refinement step (ort_cent_11.f90)
     // rescoring by groups (launch_pr_rescore_groups) only:
     const float4* sband = nullptr;  // [B][W*W] band shifted to the candidates' common origin, in
@@ -125,6 +130,11 @@ struct PrSingleArgs {
     int nom = 0;
     float step = 0.0f;
 };
+// Scoring of a refinement step's 11 candidates per particle: the terms of each in S blocks, whose
+// sums (PR numerator, weight) go to part [B][11][S].  Where the band fits shared memory (and
+// with tbandc if there is a CTF); else one block each, S = 1.
+int pr_refine_splits(const Band& bd, int T, int B, int num_sms);
+cudaError_t launch_pr_refine(const PrSingleArgs& a, int B, int S, double2* part, cudaStream_t st);
 // cal_crosslin_PR for each candidate, its origin shift applied to every tap (k_pr_single)
 cudaError_t launch_pr_single(const PrSingleArgs& a, int B, cudaStream_t st);
 // rescoring by groups of candidates sharing a view: groups[g] = (particle, first

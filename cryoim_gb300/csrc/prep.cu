@@ -376,17 +376,77 @@ __global__ void k_alpha_table(const float* __restrict__ views, int V, const floa
     alpha[q] = make_float2(a1, a2);
 }
 
-// ort_cent_11.f90:1-94 (state = theta, phi, omega, x, y, pr per image).
-__global__ void k_refine_candidates(float* __restrict__ state, int B, float dang, float dtran,
-                                    const float* __restrict__ ops, float d2r,
-                                    float* __restrict__ cand) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= B) return;
-    float* st = state + p * 6;
-    float th0 = st[0], ph0 = st[1], om0 = st[2], x0 = st[3], y0 = st[4];
-    asu_fold(&th0, &ph0, &om0, ops, d2r);
-    st[0] = th0; st[1] = ph0; st[2] = om0;
-    for (int jj = 0; jj <= 10; ++jj) {
+// return_icos_asymmetry_unit.f90 by one warp: the lanes try two operators each, the first (table
+// order) that brings the view into the asymmetric unit decides, the last one if none does.
+__device__ void asu_fold_warp(float* theta, float* phi, float* omega, const float* ops, float d2r) {
+    const int lane = threadIdx.x & 31;
+    const AsuPlanes pl = asu_planes(d2r);
+    float e[9];
+    euler_mat(*theta, *phi, *omega, d2r, e);
+    float th[2], ph[2], om[2];
+    bool in[2];
+    for (int u = 0; u < 2; ++u) {
+        const int i = lane + 32 * u;
+        float m[9];
+        mm3(ops + (i < 60 ? i : 59) * 9, e, m);
+        const float m33 = fminf(1.0f, fmaxf(-1.0f, m[8]));
+        th[u] = acosf(m33);
+        ph[u] = atan2f(m[5], m[2]);
+        om[u] = atan2f(m[7], -m[6]);
+        const float x = sinf(th[u]) * cosf(ph[u]), y = sinf(th[u]) * sinf(ph[u]), z = cosf(th[u]);
+        in[u] = i < 60 && asu_inside(pl, x, y, z);
+    }
+    const unsigned m0 = __ballot_sync(0xffffffffu, in[0]), m1 = __ballot_sync(0xffffffffu, in[1]);
+    const int u = m0 ? 0 : 1, src = m0 ? __ffs(m0) - 1 : m1 ? __ffs(m1) - 1 : 59 - 32;
+    *theta = __shfl_sync(0xffffffffu, th[u], src) / d2r;
+    *phi = __shfl_sync(0xffffffffu, ph[u], src) / d2r;
+    *omega = __shfl_sync(0xffffffffu, om[u], src) / d2r;
+}
+
+// Phase residual of a candidate from the S partial sums of its scoring blocks, in their order.
+__device__ float refine_pr(const double2* part, int S, float pi) {
+    double s1 = 0, s2 = 0;
+    for (int s = 0; s < S; ++s) { s1 += part[s].x; s2 += part[s].y; }
+    const float f1 = (float)s1, f2 = (float)s2;
+    return f2 > 1.0e-10f ? f1 / f2 * 180.0f / pi : 1000.0f;
+}
+// ort_refinement.f90:85-91 on the last cycle's candidates: the first minimum of the 11 scores.
+__device__ void refine_pick(const float* pr, const float* cand, float* st) {
+    int mn = 0;
+    for (int jj = 1; jj <= 10; ++jj)
+        if (pr[jj] < pr[mn]) mn = jj;
+    for (int v = 0; v < 5; ++v) st[v] = cand[5 * mn + v];
+    st[5] = pr[mn];
+}
+
+// One step of the descent up to the scores: block (candidate, particle) picks the last cycle's
+// minimum (prev, prev_part; the first cycle starts from state), folds it, forms its candidate of
+// ort_cent_11.f90:1-94, folds that and writes it with its common-line angles.  The eleven blocks
+// of a particle each do the pick and the fold: they are a warp's work of a few us, which a
+// kernel of their own with a thread a particle took 50-75 us over.
+__global__ void __launch_bounds__(256) k_refine_step(const float* __restrict__ state, const float* __restrict__ prev,
+                                                     const double2* __restrict__ prev_part, int S, float dang,
+                                                     float dtran, const float* __restrict__ tort, int T,
+                                                     const float* __restrict__ ops, float d2r, float r2d, float pi,
+                                                     float* __restrict__ cand, float2* __restrict__ alpha) {
+    extern __shared__ float em[];  // [9] candidate, then [T][9] templates
+    __shared__ float spr[11], sst[6];
+    const int jj = blockIdx.x, p = blockIdx.y;
+    const long pc = (long)p * 11 + jj;
+    for (int i = threadIdx.x; i < T; i += blockDim.x)
+        euler_mat(tort[i * 3], tort[i * 3 + 1], tort[i * 3 + 2], d2r, em + 9 + 9 * i);
+    if (threadIdx.x < 32) {
+        if (prev) {
+            if (threadIdx.x < 11) spr[threadIdx.x] = refine_pr(prev_part + ((long)p * 11 + threadIdx.x) * S, S, pi);
+            __syncwarp();
+            if (threadIdx.x == 0) refine_pick(spr, prev + (long)p * 55, sst);
+        } else if (threadIdx.x < 6) {
+            sst[threadIdx.x] = state[6 * p + threadIdx.x];
+        }
+        __syncwarp();
+        float th0 = sst[0], ph0 = sst[1], om0 = sst[2];
+        const float x0 = sst[3], y0 = sst[4];
+        asu_fold_warp(&th0, &ph0, &om0, ops, d2r);
         float th = th0, ph = ph0, om = om0, x = x0, y = y0;
         switch (jj) {
             case 1: th = th0 - dang; break;
@@ -401,10 +461,29 @@ __global__ void k_refine_candidates(float* __restrict__ state, int B, float dang
             case 10: y = y0 + dtran; break;
             default: break;
         }
-        asu_fold(&th, &ph, &om, ops, d2r);
-        float* o = cand + ((long)p * 11 + jj) * 5;
-        o[0] = th; o[1] = ph; o[2] = om; o[3] = x; o[4] = y;
+        asu_fold_warp(&th, &ph, &om, ops, d2r);
+        if (threadIdx.x == 0) {
+            float* o = cand + pc * 5;
+            o[0] = th; o[1] = ph; o[2] = om; o[3] = x; o[4] = y;
+            euler_mat(th, ph, om, d2r, em);
+        }
     }
+    __syncthreads();
+    float2* out = alpha + pc * T * 60;
+    for (int q = threadIdx.x; q < T * 60; q += blockDim.x) {
+        const int i = q / 60, j = q - 60 * i;
+        float a1, a2;
+        crosslin_pair(em, em + 9 + 9 * i, ops + j * 9, r2d, &a1, &a2);
+        out[q] = make_float2(a1, a2);
+    }
+}
+__global__ void k_refine_last(const float* __restrict__ cand, const double2* __restrict__ part, int S, int B, float pi,
+                              float* __restrict__ state) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= B) return;
+    float pr[11];
+    for (int jj = 0; jj < 11; ++jj) pr[jj] = refine_pr(part + ((long)p * 11 + jj) * S, S, pi);
+    refine_pick(pr, cand + (long)p * 55, state + 6 * p);
 }
 
 // One block per candidate row: its Euler matrix and the T template matrices once in shared
@@ -427,20 +506,6 @@ __global__ void k_refine_alpha(const float* __restrict__ cand, long ncand_rows,
         crosslin_pair(em, em + 9 + 9 * i, ops + j * 9, r2d, &a1, &a2);
         out[q] = make_float2(a1, a2);
     }
-}
-
-// ort_refinement.f90:85-91: first minimum of the 11 scores.
-__global__ void k_refine_select(const float* __restrict__ cand, const float* __restrict__ pr, int B,
-                                float* __restrict__ state) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= B) return;
-    const float* v = pr + p * 11;
-    int mn = 0;
-    for (int jj = 1; jj <= 10; ++jj)
-        if (v[jj] < v[mn]) mn = jj;
-    const float* c = cand + ((long)p * 11 + mn) * 5;
-    float* st = state + p * 6;
-    st[0] = c[0]; st[1] = c[1]; st[2] = c[2]; st[3] = c[3]; st[4] = c[4]; st[5] = v[mn];
 }
 
 // ---------------------------------------------------------------------------
@@ -632,9 +697,18 @@ void launch_alpha_table(const float* views, int V, const float* tort, int T, con
     k_alpha_table<<<cdiv(total, 128), 128, 0, st>>>(views, V, tort, T, ops, a.d2r, a.r2d, alpha);
 }
 
-void launch_refine_candidates(float* state, int B, float dang, float dtran, const float* ops,
-                              float* cand, cudaStream_t st) {
-    k_refine_candidates<<<cdiv(B, 64), 64, 0, st>>>(state, B, dang, dtran, ops, angles().d2r, cand);
+void launch_refine_step(const float* state, const float* prev, const double2* prev_part, int S, int B, float dang,
+                        float dtran, const float* tort, int T, const float* ops, float* cand, float2* alpha,
+                        cudaStream_t st) {
+    const size_t sm = sizeof(float) * 9 * (T + 1);
+    if (sm > 48 * 1024) cudaFuncSetAttribute(k_refine_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    const HostAngles a = angles();
+    k_refine_step<<<dim3(11, B), 256, sm, st>>>(state, prev, prev_part, S, dang, dtran, tort, T, ops, a.d2r, a.r2d,
+                                                a.pi, cand, alpha);
+}
+
+void launch_refine_last(const float* cand, const double2* part, int S, int B, float* state, cudaStream_t st) {
+    k_refine_last<<<cdiv(B, 64), 64, 0, st>>>(cand, part, S, B, angles().pi, state);
 }
 
 void launch_refine_alpha(const float* cand, int B, const float* tort, int T, const float* ops,
@@ -644,11 +718,6 @@ void launch_refine_alpha(const float* cand, int B, const float* tort, int T, con
     if (sm > 48 * 1024) cudaFuncSetAttribute(k_refine_alpha, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     HostAngles a = angles();
     k_refine_alpha<<<(unsigned)rows, 256, sm, st>>>(cand, rows, tort, T, ops, a.d2r, a.r2d, alpha);
-}
-
-void launch_refine_select(const float* cand, const float* pr, int B, float* state,
-                          cudaStream_t st) {
-    k_refine_select<<<cdiv(B, 64), 64, 0, st>>>(cand, pr, B, state);
 }
 
 void launch_rec_fold(const float4* acc, Band bd, int int_shell, float2* vol, cudaStream_t st) {

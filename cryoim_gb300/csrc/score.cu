@@ -15,8 +15,9 @@
 //     minloc's first-occurrence rule.
 // The sampling positions x = FR*cos + nx/2 are rounded exactly as the reference
 // rounds them (separate multiply and add), so the bilinear taps and weights match it.
+#include <algorithm>
+#include <cmath>
 #include <cstdio>
-
 #include <type_traits>
 
 #include "geom.cuh"
@@ -430,6 +431,10 @@ __global__ void __launch_bounds__(512) k_pr_single(PrSingleArgs a, Consts K) {
     if (threadIdx.x == 0) {
         double s1 = 0, s2 = 0;
         for (int q = 0; q < nw; ++q) { s1 += sh[0][q]; s2 += sh[1][q]; }
+        if (a.part) {
+            a.part[(long)p * a.ncand + c] = make_double2(s1, s2);
+            return;
+        }
         float f1 = (float)s1, f2 = (float)s2;
         a.pr[(long)p * a.ncand + c] = (f2 > 1.0e-10f) ? f1 / f2 * 180.0f / K.pi : 1000.0f;
     }
@@ -715,6 +720,110 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pr_rescore_s(PrSingleArgs a, 
         for (int q = 0; q < RS_THREADS / 32; ++q) { s1 += sh[0][g][q]; s2 += sh[1][g][q]; }
         const float g1 = (float)s1, g2 = (float)s2;
         a.pr[(long)p * a.ncand + c0 + g] = (g2 > 1.0e-10f) ? g1 / g2 * 180.0f / K.pi : 1000.0f;
+    }
+}
+
+// A refinement step's candidates: block (candidate, particle, split) scores its share of the
+// templates.  cal_crosslin_PR.f90's terms as k_pr_single has them, arranged for the work they
+// repeat: the band is shifted to the candidate's origin once per pixel into shared memory (four
+// sincos a term before), the valid lines of the templates are listed with their directions, the
+// templates come multiplied by the CTF, and the phase difference is one arctangent of the cross
+// and dot products (two and a fold before; error 1e-7 rad either way).  Sums are TwoSum pairs per
+// thread as there, FP64 across the block and the splits.  Issue-bound.  64 particles of box
+// 256, 20 templates: 861 us a step by k_pr_single, 468 so.
+__device__ __forceinline__ float2 shifted_pixel(const float2* band, int m, int W, int off, int nx, float xs,
+                                                float ys, float twopi);
+constexpr int RF_THREADS = 1024;
+__global__ void __launch_bounds__(RF_THREADS, 1) k_pr_refine(PrSingleArgs a, Consts K, double2* __restrict__ part) {
+    extern __shared__ __align__(16) float rsm[];
+    __shared__ double sh[2][RF_THREADS / 32];
+    __shared__ int snv;
+    const Band bd = a.bd;
+    const int W = bd.W, nr = bd.nr, minR = bd.min_r, nx = bd.nx;
+    const int SP = rescore_pitch(W);
+    const int c = blockIdx.x, p = blockIdx.y, S = gridDim.z;
+    const int t0 = a.T * (int)blockIdx.z / S, t1 = a.T * ((int)blockIdx.z + 1) / S, nt = t1 - t0;
+    float2* sbd = reinterpret_cast<float2*>(rsm);                        // [W][SP] shifted particle band
+    float4* sln = reinterpret_cast<float4*>(rsm + ((2L * W * SP + 3) & ~3L));  // listed lines: cos, sin of particle, of template
+    int* stm = reinterpret_cast<int*>(sln + nt * 60);                    // and their templates (of this share)
+    float* sfc = reinterpret_cast<float*>(stm + nt * 60);                // [nt + 1][nr]: template cuts, the particle's
+    const float* cd = a.cand + ((long)p * a.ncand + c) * 5;
+    const float nxh = (float)(nx / 2);
+    const float xs = __fadd_rn(cd[3], nxh), ys = __fadd_rn(cd[4], nxh);
+    const float2* pb = a.band + (long)p * W * W;
+    const float twopi = __fmul_rn(2.0f, K.pi);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == 0) {  // the valid lines in order
+        const float2* al = a.alpha + (((long)p * a.ncand + c) * a.T + t0) * 60;
+        int n = 0;
+        for (int q0 = 0; q0 < nt * 60; q0 += 32) {
+            const int q = q0 + lane;
+            const float2 aa = q < nt * 60 ? al[q] : make_float2(1000.f, 1000.f);
+            const bool ok = aa.x < 999.0f && aa.y < 999.0f;
+            const unsigned m = __ballot_sync(0xffffffffu, ok);
+            if (ok) {
+                const int at = n + __popc(m & ((1u << lane) - 1u));
+                const float a1 = __fmul_rn(aa.x, K.d2r), a2 = __fmul_rn(aa.y, K.d2r);
+                sln[at] = make_float4(cosf(a1), sinf(a1), cosf(a2), sinf(a2));
+                stm[at] = q / 60;
+            }
+            n += __popc(m);
+        }
+        if (lane == 0) snv = n;
+    } else {
+        for (int row = warp - 1; row < W; row += RF_THREADS / 32 - 1)
+            for (int col = lane; col < W; col += 32)
+                sbd[row * SP + col] = shifted_pixel(pb, row * W + col, W, bd.off, nx, xs, ys, twopi);
+    }
+    const float* tfc = a.tfcut + (long)p * a.tfcut_pstride + (long)t0 * nr;
+    for (int q = threadIdx.x; q < nt * nr; q += RF_THREADS) sfc[q] = tfc[q];
+    for (int q = threadIdx.x; q < nr; q += RF_THREADS) sfc[nt * nr + q] = a.fcut0[(long)p * nr + q];
+    __syncthreads();
+    const int offW = bd.off * W + bd.off, offS = bd.off * SP + bd.off;
+    const float4* tbc = a.tbandc ? a.tbandc + ((long)p * a.T + t0) * W * W : nullptr;
+    const int total = snv * nr;
+    const int step_l = RF_THREADS / nr, step_iq = RF_THREADS - step_l * nr;
+    int l = (int)threadIdx.x / nr, iq = (int)threadIdx.x - l * nr;
+    float h1 = 0.f, l1 = 0.f, h2 = 0.f, l2 = 0.f;  // per-thread sums as TwoSum pairs
+    for (int q = threadIdx.x; q < total; q += RF_THREADS) {
+        const float4 ln = sln[l];
+        const int i = stm[l];
+        const float fr = (float)(minR + iq);
+        float re2, im2;
+        if (tbc)
+            tmpl_sample_pairs(tbc + (long)i * W * W, W, offW, nxh, ln.z, ln.w, fr, &re2, &im2);
+        else
+            tmpl_sample_cs(a.tband + (long)(t0 + i) * W * W, nullptr, W, offW, nxh, ln.z, ln.w, fr, &re2, &im2);
+        const float x = __fadd_rn(__fmul_rn(fr, ln.x), nxh), y = __fadd_rn(__fmul_rn(fr, ln.y), nxh);
+        const int lx = (int)x, ly = (int)y;
+        const float ax = __fsub_rn(x, (float)lx), ay = __fsub_rn(y, (float)ly);
+        const float2* tp = sbd + (ly * SP + lx - offS);
+        const float2 t00 = tp[0], t10 = tp[1], t01 = tp[SP], t11 = tp[SP + 1];
+        const float re1 = bilerp(ax, ay, t00.x, t10.x, t01.x, t11.x);
+        const float im1 = bilerp(ax, ay, t00.y, t10.y, t01.y, t11.y);
+        const float amp1 = sqrtf(re1 * re1 + im1 * im1);
+        const float amp2 = sqrtf(re2 * re2 + im2 * im2);
+        if (amp1 >= sfc[nt * nr + iq] && amp2 >= sfc[i * nr + iq]) {
+            const float d = atan2f(fabsf(re1 * im2 - im1 * re2), re1 * re2 + im1 * im2);
+            const float w = 0.5f * (amp1 + amp2);
+            two_sum_acc(h1, l1, d * w);
+            two_sum_acc(h2, l2, w);
+        }
+        iq += step_iq;
+        l += step_l;
+        if (iq >= nr) { iq -= nr; ++l; }
+    }
+    double p1 = (double)h1 + (double)l1, p2 = (double)h2 + (double)l2;
+    for (int o = 16; o > 0; o >>= 1) {
+        p1 += __shfl_xor_sync(0xffffffffu, p1, o);
+        p2 += __shfl_xor_sync(0xffffffffu, p2, o);
+    }
+    if (lane == 0) { sh[0][warp] = p1; sh[1][warp] = p2; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s1 = 0, s2 = 0;
+        for (int q = 0; q < RF_THREADS / 32; ++q) { s1 += sh[0][q]; s2 += sh[1][q]; }
+        part[((long)p * a.ncand + c) * S + blockIdx.z] = make_double2(s1, s2);
     }
 }
 
@@ -1026,6 +1135,33 @@ cudaError_t launch_tband_ctf(const float2* tband, int T, const float* ctf, const
 cudaError_t launch_pr_single(const PrSingleArgs& a, int B, cudaStream_t st) {
     dim3 grid(a.ncand, B);
     k_pr_single<<<grid, 512, 0, st>>>(a, consts());
+    return cudaGetLastError();
+}
+
+static size_t pr_refine_smem(const Band& bd, int nt) {
+    return sizeof(float) * ((2 * (size_t)bd.W * rescore_pitch(bd.W) + 3) & ~(size_t)3) +
+           (sizeof(float4) + sizeof(int)) * (size_t)nt * 60 + sizeof(float) * (size_t)(nt + 1) * bd.nr;
+}
+static bool pr_refine_fits(const Band& bd, int nt) { return pr_refine_smem(bd, nt) + 1024 <= 227 * 1024; }
+
+int pr_refine_splits(const Band& bd, int T, int B, int num_sms) {
+    // blocks of one SM each: the fewest rounds of them, counting the shift of the band (about a
+    // seventh of 20 templates' terms) that every split repeats; 0: not even a split's lines fit
+    int best = 0;
+    double cost = 1e30;
+    for (int S = 1; S <= std::min(T, 16); ++S) {
+        if (!pr_refine_fits(bd, (T + S - 1) / S)) continue;
+        const double rounds = std::ceil(11.0 * B * S / num_sms) * (1.0 / S + 0.15);
+        if (rounds < cost) { cost = rounds; best = S; }
+    }
+    return best;
+}
+
+cudaError_t launch_pr_refine(const PrSingleArgs& a, int B, int S, double2* part, cudaStream_t st) {
+    const size_t sm = pr_refine_smem(a.bd, (a.T + S - 1) / S);
+    cudaError_t e = cudaFuncSetAttribute(k_pr_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    k_pr_refine<<<dim3(a.ncand, B, S), RF_THREADS, sm, st>>>(a, consts(), part);
     return cudaGetLastError();
 }
 

@@ -240,6 +240,7 @@ struct LearnModel {
     long oW[5] = {0}, ob[5] = {0}, oT = 0;  // parameter offsets (conv 1-4, mix)
     int steps = 0;      // Adam steps taken
     int cap = 0, capV = 0;  // batch capacity of the activations, views they were sized for
+    bool cap_full = false;  // the full-resolution rows of layers 2-4 too (FP32 convolutions)
     DBuf<float> w, gr, m, v, vview, wflip;
     DBuf<float> feat, a1, a2, p2, a3, p3, a4, p4, g, sc, dsc, dg, dp4, da4, dp3, da3, dp2, da2, da1, loss, truth;
     DBuf<int> cell;
@@ -247,10 +248,17 @@ struct LearnModel {
     DBuf<float2> hscr;  // the head's frequency-domain scratch
     bool conv_tc = true;  // convolutions on the tensor cores (TF32) or on the CUDA cores (FP32)
     DBuf<int> cerr;       // set by a tensor-core convolution whose wait timed out
+    // tensor-core convolutions: where the ReLUs of layers 1 to 4 pass (a bit per channel), and
+    // the weight gradients' partial sums
+    DBuf<unsigned int> gate1, gate[3];
+    DBuf<float> wpart;
     void release() {
         for (DBuf<float>* b : {&w, &gr, &m, &v, &vview, &wflip, &feat, &a1, &a2, &p2, &a3, &p3, &a4, &p4, &g, &sc,
-                               &dsc, &dg, &dp4, &da4, &dp3, &da3, &dp2, &da2, &da1, &loss, &truth, &cellv})
+                               &dsc, &dg, &dp4, &da4, &dp3, &da3, &dp2, &da2, &da1, &loss, &truth, &cellv,
+                               &wpart})
             b->release();
+        gate1.release();
+        for (DBuf<unsigned int>& g : gate) g.release();
         cell.release();
         hscr.release();
         cerr.release();
@@ -1314,41 +1322,31 @@ int learn_layout(Ctx* c, int V) {
 
 int learn_activations(Ctx* c, int B) {
     LearnModel& L = c->lm;
-    if (B <= L.cap && L.V == L.capV) return CRYOIM_OK;
+    if (B <= L.cap && L.V == L.capV && (L.conv_tc || L.cap_full)) return CRYOIM_OK;
     B = std::max(B, L.cap);
     const size_t b = (size_t)B, P = LP_NT;
     int r;
     if ((r = L.feat.ensure(b * LP_NR * P)) || (r = L.a1.ensure(b * LP_C1 * LP_NR * P)) ||
-        (r = L.a2.ensure(b * LP_C2 * LP_NR * P)) || (r = L.p2.ensure(b * LP_C2 * (LP_NR / 2) * P)) ||
-        (r = L.a3.ensure(b * LP_C3 * (LP_NR / 2) * P)) || (r = L.p3.ensure(b * LP_C3 * (LP_NR / 4) * P)) ||
-        (r = L.a4.ensure(b * LP_C4 * (LP_NR / 4) * P)) || (r = L.p4.ensure(b * LP_MIXK * P)) ||
-        (r = L.g.ensure(b * LP_CM * P)) || (r = L.sc.ensure(b * L.V * P)) || (r = L.dsc.ensure(b * L.V * P)) ||
-        (r = L.dg.ensure(b * LP_CM * P)) || (r = L.dp4.ensure(b * LP_MIXK * P)) ||
-        (r = L.da4.ensure(b * LP_C4 * (LP_NR / 4) * P)) || (r = L.dp3.ensure(b * LP_C3 * (LP_NR / 4) * P)) ||
-        (r = L.da3.ensure(b * LP_C3 * (LP_NR / 2) * P)) || (r = L.dp2.ensure(b * LP_C2 * (LP_NR / 2) * P)) ||
-        (r = L.da2.ensure(b * LP_C2 * LP_NR * P)) || (r = L.da1.ensure(b * LP_C1 * LP_NR * P)) ||
+        (r = L.p2.ensure(b * LP_C2 * (LP_NR / 2) * P)) || (r = L.p3.ensure(b * LP_C3 * (LP_NR / 4) * P)) ||
+        (r = L.p4.ensure(b * LP_MIXK * P)) || (r = L.g.ensure(b * LP_CM * P)) || (r = L.sc.ensure(b * L.V * P)) ||
+        (r = L.dsc.ensure(b * L.V * P)) || (r = L.dg.ensure(b * LP_CM * P)) || (r = L.dp4.ensure(b * LP_MIXK * P)) ||
+        (r = L.dp3.ensure(b * LP_C3 * (LP_NR / 4) * P)) || (r = L.dp2.ensure(b * LP_C2 * (LP_NR / 2) * P)) ||
+        (r = L.da1.ensure(b * LP_C1 * LP_NR * P)) || (r = L.gate1.ensure(b * LP_NR * P)) ||
+        (r = L.gate[0].ensure(b * LP_NR * P)) || (r = L.gate[1].ensure(b * (LP_NR / 2) * P)) ||
+        (r = L.gate[2].ensure(b * (LP_NR / 4) * P)) || (r = L.wpart.ensure((size_t)lp_wgrad_scratch())) ||
         (r = L.loss.ensure(b)) || (r = L.truth.ensure(4 * b)) || (r = L.cell.ensure(b * 64)) ||
         (r = L.cellv.ensure(b * 64)) || (r = L.hscr.ensure((size_t)lp_head_scratch(B, L.V))))
+        return r;
+    if ((L.cap_full = !L.conv_tc) &&
+        ((r = L.a2.ensure(b * LP_C2 * LP_NR * P)) || (r = L.a3.ensure(b * LP_C3 * (LP_NR / 2) * P)) ||
+         (r = L.a4.ensure(b * LP_C4 * (LP_NR / 4) * P)) || (r = L.da4.ensure(b * LP_C4 * (LP_NR / 4) * P)) ||
+         (r = L.da3.ensure(b * LP_C3 * (LP_NR / 2) * P)) || (r = L.da2.ensure(b * LP_C2 * LP_NR * P))))
         return r;
     L.cap = B;
     L.capV = L.V;
     return CRYOIM_OK;
 }
 
-// The proposer's 3x3 convolutions: TF32 on the tensor cores (conv_tc.cu, the default) or
-// FP32 on the CUDA cores (learn.cu).
-cudaError_t lp_conv(Ctx* c, const float* in, int B, int Cin, int H, const float* W, const float* bias, int Cout,
-                    bool relu, float* out) {
-    LearnModel& L = c->lm;
-    if (L.conv_tc) return launch_lp_conv3_tc(in, B, Cin, H, W, bias, Cout, relu, out, L.cerr.p, c->stream);
-    return launch_lp_conv3(in, B, Cin, H, W, bias, Cout, relu, out, c->stream);
-}
-cudaError_t lp_wgrad(Ctx* c, const float* in, const float* dpre, int B, int Cin, int H, int Cout, float* dW,
-                     float* db) {
-    LearnModel& L = c->lm;
-    if (L.conv_tc) return launch_lp_conv3_wgrad_tc(in, dpre, B, Cin, H, Cout, dW, db, L.cerr.p, c->stream);
-    return launch_lp_conv3_wgrad(in, dpre, B, Cin, H, Cout, dW, db, c->stream);
-}
 // After the stream has drained: did a tensor-core convolution give up waiting?
 int learn_conv_status(Ctx* c) {
     LearnModel& L = c->lm;
@@ -1360,53 +1358,93 @@ int learn_conv_status(Ctx* c) {
     return CRYOIM_OK;
 }
 
-// scores L.sc [B][V][NT] of the features in L.feat
-int learn_forward(Ctx* c, int B) {
+// The layers up to the pooled rows of layer 4 (L.p4) from the features.  The 3x3 convolutions
+// run in TF32 on the tensor cores with the pooling in their epilogue (conv_tc.cu, the default;
+// train: the gates that the backward pass reads are kept) or in FP32 on the CUDA cores
+// (learn.cu).
+int learn_convs(Ctx* c, int B, bool train) {
     LearnModel& L = c->lm;
     const float* w = L.w.p;
     cudaStream_t st = c->stream;
-    CK(lp_conv(c, L.feat.p, B, 1, LP_NR, w + L.oW[0], w + L.ob[0], LP_C1, true, L.a1.p));
-    CK(lp_conv(c, L.a1.p, B, LP_C1, LP_NR, w + L.oW[1], w + L.ob[1], LP_C2, true, L.a2.p));
-    launch_lp_pool(L.a2.p, B, LP_C2, LP_NR / 2, L.p2.p, st);
-    CK(lp_conv(c, L.p2.p, B, LP_C2, LP_NR / 2, w + L.oW[2], w + L.ob[2], LP_C3, true, L.a3.p));
-    launch_lp_pool(L.a3.p, B, LP_C3, LP_NR / 4, L.p3.p, st);
-    CK(lp_conv(c, L.p3.p, B, LP_C3, LP_NR / 4, w + L.oW[3], w + L.ob[3], LP_C4, true, L.a4.p));
-    launch_lp_pool(L.a4.p, B, LP_C4, LP_NR / 8, L.p4.p, st);
+    const float* in[3] = {L.a1.p, L.p2.p, L.p3.p};
+    float *full[3] = {L.a2.p, L.a3.p, L.a4.p}, *pooled[3] = {L.p2.p, L.p3.p, L.p4.p};
+    if (L.conv_tc)
+        CK(launch_lp_conv3_tc(L.feat.p, B, 1, LP_NR, w + L.oW[0], w + L.ob[0], LP_C1, true, L.a1.p, L.cerr.p, st,
+                              train ? L.gate1.p : nullptr));
+    else
+        CK(launch_lp_conv3(L.feat.p, B, 1, LP_NR, w + L.oW[0], w + L.ob[0], LP_C1, true, L.a1.p, st));
+    for (int l = 1; l < 4; ++l) {
+        const int H = LP_NR >> (l - 1);
+        const float *W = w + L.oW[l], *bias = w + L.ob[l];
+        if (L.conv_tc) {
+            CK(launch_lp_conv3_pool_tc(in[l - 1], B, LP_CIN[l], H, W, bias, pooled[l - 1],
+                                       train ? L.gate[l - 1].p : nullptr, L.cerr.p, st));
+        } else {
+            CK(launch_lp_conv3(in[l - 1], B, LP_CIN[l], H, W, bias, LP_COUT[l], true, full[l - 1], st));
+            launch_lp_pool(full[l - 1], B, LP_COUT[l], H / 2, pooled[l - 1], st);
+        }
+    }
+    return CRYOIM_OK;
+}
+
+// the gradients of those layers from L.dp4, the gradient of L.p4
+int learn_convs_grad(Ctx* c, int B) {
+    LearnModel& L = c->lm;
+    const float* w = L.w.p;
+    float* gr = L.gr.p;
+    cudaStream_t st = c->stream;
+    const float *in[3] = {L.a1.p, L.p2.p, L.p3.p}, *full[3] = {L.a2.p, L.a3.p, L.a4.p};
+    float *dfull[3] = {L.da2.p, L.da3.p, L.da4.p}, *din[4] = {L.da1.p, L.dp2.p, L.dp3.p, L.dp4.p};
+    for (int l = 3; l >= 1; --l) {
+        const int H = LP_NR >> (l - 1), cin = LP_CIN[l], cout = LP_COUT[l];
+        const float* W = w + L.oW[l];
+        float *dW = gr + L.oW[l], *db = gr + L.ob[l];
+        if (L.conv_tc) {
+            CK(launch_lp_conv3_wgrad_pool_tc(in[l - 1], din[l], L.gate[l - 1].p, B, cin, H, dW, db, L.wpart.p,
+                                             L.cerr.p, st));
+            CK(launch_lp_conv3_back_tc(din[l], L.gate[l - 1].p, B, H, W, cin, l == 1 ? L.gate1.p : nullptr,
+                                       din[l - 1], L.cerr.p, st));
+        } else {
+            launch_lp_pool_grad(din[l], B, cout, H / 2, full[l - 1], dfull[l - 1], st);
+            CK(launch_lp_conv3_wgrad(in[l - 1], dfull[l - 1], B, cin, H, cout, dW, db, st));
+            launch_lp_flip(W, cout, cin, L.wflip.p, st);
+            CK(launch_lp_conv3(dfull[l - 1], B, cout, H, L.wflip.p, nullptr, cin, false, din[l - 1], st));
+        }
+    }
+    float *dW = gr + L.oW[0], *db = gr + L.ob[0];
+    if (L.conv_tc) {
+        CK(launch_lp_conv3_wgrad_tc(L.feat.p, L.da1.p, B, 1, LP_NR, LP_C1, dW, db, L.wpart.p, L.cerr.p, st));
+    } else {
+        launch_lp_relu_grad(L.a1.p, L.da1.p, (long)B * LP_C1 * LP_NR * LP_NT, L.da1.p, st);
+        CK(launch_lp_conv3_wgrad(L.feat.p, L.da1.p, B, 1, LP_NR, LP_C1, dW, db, st));
+    }
+    return CRYOIM_OK;
+}
+
+// scores L.sc [B][V][NT] of the features in L.feat
+int learn_forward(Ctx* c, int B, bool train) {
+    LearnModel& L = c->lm;
+    const float* w = L.w.p;
+    cudaStream_t st = c->stream;
+    int r;
+    if ((r = learn_convs(c, B, train))) return r;
     launch_lp_mix(L.p4.p, B, w + L.oW[4], w + L.ob[4], L.g.p, st);
     CK(launch_lp_head(L.g.p, w + L.oT, B, L.V, L.sc.p, L.hscr.p, st));
     return CRYOIM_OK;
 }
 
-// loss (L.loss [B]) and parameter gradients (L.gr) of the last forward, targets in L.truth
+// loss (L.loss [B]) and parameter gradients (L.gr) of the last forward (run with train set),
+// targets in L.truth
 int learn_backward(Ctx* c, int B) {
     LearnModel& L = c->lm;
     const float* w = L.w.p;
     float* gr = L.gr.p;
     cudaStream_t st = c->stream;
-    const long nt = LP_NT;
     CK(cudaMemsetAsync(gr, 0, sizeof(float) * L.nparam, st));
     launch_lp_loss(L.sc.p, B, L.V, L.vview.p, L.truth.p, 2.0f * c->p.searchstep, 1.0f, L.dsc.p, L.loss.p, st);
     launch_lp_head_grad(L.g.p, w + L.oT, L.dsc.p, B, L.V, L.dg.p, gr + L.oT, L.hscr.p, st);
     launch_lp_mix_grad(L.p4.p, L.dg.p, B, w + L.oW[4], L.dp4.p, gr + L.oW[4], gr + L.ob[4], st);
-    // layer 4
-    launch_lp_pool_grad(L.dp4.p, B, LP_C4, LP_NR / 8, L.a4.p, L.da4.p, st);
-    CK(lp_wgrad(c, L.p3.p, L.da4.p, B, LP_C3, LP_NR / 4, LP_C4, gr + L.oW[3], gr + L.ob[3]));
-    launch_lp_flip(w + L.oW[3], LP_C4, LP_C3, L.wflip.p, st);
-    CK(lp_conv(c, L.da4.p, B, LP_C4, LP_NR / 4, L.wflip.p, nullptr, LP_C3, false, L.dp3.p));
-    // layer 3
-    launch_lp_pool_grad(L.dp3.p, B, LP_C3, LP_NR / 4, L.a3.p, L.da3.p, st);
-    CK(lp_wgrad(c, L.p2.p, L.da3.p, B, LP_C2, LP_NR / 2, LP_C3, gr + L.oW[2], gr + L.ob[2]));
-    launch_lp_flip(w + L.oW[2], LP_C3, LP_C2, L.wflip.p, st);
-    CK(lp_conv(c, L.da3.p, B, LP_C3, LP_NR / 2, L.wflip.p, nullptr, LP_C2, false, L.dp2.p));
-    // layer 2
-    launch_lp_pool_grad(L.dp2.p, B, LP_C2, LP_NR / 2, L.a2.p, L.da2.p, st);
-    CK(lp_wgrad(c, L.a1.p, L.da2.p, B, LP_C1, LP_NR, LP_C2, gr + L.oW[1], gr + L.ob[1]));
-    launch_lp_flip(w + L.oW[1], LP_C2, LP_C1, L.wflip.p, st);
-    CK(lp_conv(c, L.da2.p, B, LP_C2, LP_NR, L.wflip.p, nullptr, LP_C1, false, L.da1.p));
-    // layer 1
-    launch_lp_relu_grad(L.a1.p, L.da1.p, (long)B * LP_C1 * LP_NR * nt, L.da1.p, st);
-    CK(lp_wgrad(c, L.feat.p, L.da1.p, B, 1, LP_NR, LP_C1, gr + L.oW[0], gr + L.ob[0]));
-    return CRYOIM_OK;
+    return learn_convs_grad(c, B);
 }
 
 // Haar-uniform rotation (unit quaternion) as ZYZ Euler angles in degrees
@@ -1648,7 +1686,7 @@ int learn_train_impl(Ctx* c, const float* map3d, const cryoim_learn_opts* o, flo
             draw(sidx + 1);
             if ((r = generate(sidx + 1))) return r;
         }
-        if ((r = learn_forward(c, B)) || (r = learn_backward(c, B))) return r;
+        if ((r = learn_forward(c, B, true)) || (r = learn_backward(c, B))) return r;
         // the learning rate ramps up linearly over the first tenth of the steps (from 10 %),
         // then stays at o->lr: Adam's first steps at the full rate sent some seeds' runs
         // to a poor minimum (the proposals' agreement with the exhaustive search ranged over
@@ -1688,7 +1726,7 @@ int learned_lists(Ctx* c, int nb, int kl, int nbf, std::vector<Proposals>& lists
     int r;
     if ((r = learn_activations(c, nb))) return r;
     launch_lp_features(c->band.p, c->bd, nb, L.feat.p, c->stream);
-    if ((r = learn_forward(c, nb))) return r;
+    if ((r = learn_forward(c, nb, false))) return r;
     launch_lp_topk(L.sc.p, nb, L.V, kl, L.cell.p, L.cellv.p, c->stream);
     CK(cudaGetLastError());
     std::vector<int> cell((size_t)nb * kl);
@@ -3856,7 +3894,7 @@ int cryoim_learn_forward(void* ctx, const float* feat, const float* truth, int32
     if (!feat || B < 1 || ((loss || grads) && !truth)) return fail(CRYOIM_ERR_ARG, "bad arguments");
     if ((r = learn_activations(c, B))) return r;
     CK(cudaMemcpyAsync(L.feat.p, feat, sizeof(float) * B * LP_NR * LP_NT, cudaMemcpyHostToDevice, c->stream));
-    if ((r = learn_forward(c, B))) return r;
+    if ((r = learn_forward(c, B, truth != nullptr))) return r;
     if (scores)
         CK(cudaMemcpyAsync(scores, L.sc.p, sizeof(float) * B * L.V * LP_NT, cudaMemcpyDeviceToHost, c->stream));
     if (truth) {
@@ -3879,14 +3917,15 @@ int cryoim_conv3_check(int32_t tensor_cores, const float* x, int32_t B, int32_t 
         (dpre && (!dW || !db)))
         return fail(CRYOIM_ERR_ARG, "bad arguments");
     const size_t nx = (size_t)B * Cin * H * LP_NT, ny = (size_t)B * Cout * H * LP_NT, nw = (size_t)Cout * Cin * 9;
-    DBuf<float> dx, dy, dwt, dbias, dg, dgw, dgb;
+    DBuf<float> dx, dy, dwt, dbias, dg, dgw, dgb, dpart;
     DBuf<int> derr;
     int r;
     if ((r = dx.ensure(nx)) || (r = dy.ensure(ny)) || (r = dwt.ensure(nw)) || (r = dbias.ensure(Cout)) ||
-        (r = derr.ensure(1)) || (dpre && ((r = dg.ensure(ny)) || (r = dgw.ensure(nw)) || (r = dgb.ensure(Cout)))))
+        (r = derr.ensure(1)) || (dpre && ((r = dg.ensure(ny)) || (r = dgw.ensure(nw)) || (r = dgb.ensure(Cout)) ||
+                                          (r = dpart.ensure((size_t)lp_wgrad_scratch())))))
         return r;
     auto done = [&](int code) {
-        for (DBuf<float>* b : {&dx, &dy, &dwt, &dbias, &dg, &dgw, &dgb}) b->release();
+        for (DBuf<float>* b : {&dx, &dy, &dwt, &dbias, &dg, &dgw, &dgb, &dpart}) b->release();
         derr.release();
         return code;
     };
@@ -3906,7 +3945,7 @@ int cryoim_conv3_check(int32_t tensor_cores, const float* x, int32_t B, int32_t 
         ok(cudaMemset(dgw.p, 0, nw * 4));
         ok(cudaMemset(dgb.p, 0, Cout * 4));
         if (e == cudaSuccess)
-            ok(tensor_cores ? launch_lp_conv3_wgrad_tc(dx.p, dg.p, B, Cin, H, Cout, dgw.p, dgb.p, derr.p, 0)
+            ok(tensor_cores ? launch_lp_conv3_wgrad_tc(dx.p, dg.p, B, Cin, H, Cout, dgw.p, dgb.p, dpart.p, derr.p, 0)
                             : launch_lp_conv3_wgrad(dx.p, dg.p, B, Cin, H, Cout, dgw.p, dgb.p, 0));
     }
     ok(cudaDeviceSynchronize());

@@ -334,11 +334,26 @@ cudaError_t launch_lp_conv3(const float* in, int B, int Cin, int H, const float*
 cudaError_t launch_lp_conv3_wgrad(const float* in, const float* dpre, int B, int Cin, int H, int Cout, float* dW,
                                   float* db, cudaStream_t st);
 // The same two convolutions on the tensor cores (conv_tc.cu, tcgen05 kind::tf32): Cin <= 32
-// (wgrad: 1 or a multiple of 8), Cout 16 or 32; *err is set if a wait timed out.
+// (wgrad: 1 or a multiple of 8), Cout 16 or 32; *err is set if a wait timed out.  gate_out
+// (Cout = 16, or null): [B][H][128], bit 8 (co / 4) + co % 4 set where the output is positive.
+// The weight gradients' scratch holds lp_wgrad_scratch() floats.
 cudaError_t launch_lp_conv3_tc(const float* in, int B, int Cin, int H, const float* W, const float* bias, int Cout,
-                               bool relu, float* out, int* err, cudaStream_t st);
+                               bool relu, float* out, int* err, cudaStream_t st, unsigned int* gate_out = nullptr);
+long lp_wgrad_scratch();
 cudaError_t launch_lp_conv3_wgrad_tc(const float* in, const float* dpre, int B, int Cin, int H, int Cout, float* dW,
-                                     float* db, int* err, cudaStream_t st);
+                                     float* db, float* scratch, int* err, cudaStream_t st);
+// Convolution (Cin 16 or 32, 32 output channels, even H), ReLU and average of radius pairs in
+// one: pooled [B][32][H / 2][128] and, unless null, gate [B][H][128], bit co set where the
+// ReLU's output is positive.
+cudaError_t launch_lp_conv3_pool_tc(const float* in, int B, int Cin, int H, const float* W, const float* bias,
+                                    float* pooled, unsigned int* gate, int* err, cudaStream_t st);
+// Its gradients from dp, the gradient of pooled: of the input (W: the forward's weights
+// [32][Cin][3][3]; gate_in, Cin = 16: kept only where a gate_out of launch_lp_conv3_tc has channel ci set) and of the
+// weights and bias (accumulated).
+cudaError_t launch_lp_conv3_back_tc(const float* dp, const unsigned int* gate, int B, int H, const float* W, int Cin,
+                                    const unsigned int* gate_in, float* din, int* err, cudaStream_t st);
+cudaError_t launch_lp_conv3_wgrad_pool_tc(const float* in, const float* dp, const unsigned int* gate, int B, int Cin,
+                                          int H, float* dW, float* db, float* scratch, int* err, cudaStream_t st);
 void launch_lp_relu_grad(const float* out, const float* dout, long n, float* dpre, cudaStream_t st);
 void launch_lp_flip(const float* W, int Cout, int Cin, float* Wf, cudaStream_t st);
 void launch_lp_pool(const float* a, int B, int C, int Hout, float* p, cudaStream_t st);

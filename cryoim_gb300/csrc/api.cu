@@ -248,7 +248,7 @@ struct LearnModel {
     DBuf<float2> hscr;  // the head's frequency-domain scratch
     bool conv_tc = true;  // convolutions on the tensor cores (TF32) or on the CUDA cores (FP32)
     DBuf<int> cerr;       // set by a tensor-core convolution whose wait timed out
-    // tensor-core convolutions: where the ReLUs of layers 1 to 4 pass (a bit per channel), and
+    // where the ReLUs of layers 1 to 4 pass (a bit per channel; tensor-core convolutions), and
     // the weight gradients' partial sums
     DBuf<unsigned int> gate1, gate[3];
     DBuf<float> wpart;
@@ -1333,7 +1333,7 @@ int learn_activations(Ctx* c, int B) {
         (r = L.dp3.ensure(b * LP_C3 * (LP_NR / 4) * P)) || (r = L.dp2.ensure(b * LP_C2 * (LP_NR / 2) * P)) ||
         (r = L.da1.ensure(b * LP_C1 * LP_NR * P)) || (r = L.gate1.ensure(b * LP_NR * P)) ||
         (r = L.gate[0].ensure(b * LP_NR * P)) || (r = L.gate[1].ensure(b * (LP_NR / 2) * P)) ||
-        (r = L.gate[2].ensure(b * (LP_NR / 4) * P)) || (r = L.wpart.ensure((size_t)lp_wgrad_scratch())) ||
+        (r = L.gate[2].ensure(b * (LP_NR / 4) * P)) || (r = L.wpart.ensure((size_t)std::max(lp_wgrad_scratch(), lp_mix_scratch()))) ||
         (r = L.loss.ensure(b)) || (r = L.truth.ensure(4 * b)) || (r = L.cell.ensure(b * 64)) ||
         (r = L.cellv.ensure(b * 64)) || (r = L.hscr.ensure((size_t)lp_head_scratch(B, L.V))))
         return r;
@@ -1443,7 +1443,8 @@ int learn_backward(Ctx* c, int B) {
     CK(cudaMemsetAsync(gr, 0, sizeof(float) * L.nparam, st));
     launch_lp_loss(L.sc.p, B, L.V, L.vview.p, L.truth.p, 2.0f * c->p.searchstep, 1.0f, L.dsc.p, L.loss.p, st);
     launch_lp_head_grad(L.g.p, w + L.oT, L.dsc.p, B, L.V, L.dg.p, gr + L.oT, L.hscr.p, st);
-    launch_lp_mix_grad(L.p4.p, L.dg.p, B, w + L.oW[4], L.dp4.p, gr + L.oW[4], gr + L.ob[4], st);
+    launch_lp_mix_grad(L.p4.p, L.dg.p, B, w + L.oW[4], L.dp4.p, gr + L.oW[4], gr + L.ob[4], L.wpart.p,
+                       st);
     return learn_convs_grad(c, B);
 }
 

@@ -360,8 +360,10 @@ void launch_lp_pool(const float* a, int B, int C, int Hout, float* p, cudaStream
 // with a (the pooled layer's ReLU output, or nullptr): the ReLU gate applied too
 void launch_lp_pool_grad(const float* dp, int B, int C, int Hout, const float* a, float* da, cudaStream_t st);
 void launch_lp_mix(const float* x, int B, const float* W5, const float* b5, float* g, cudaStream_t st);
+// scratch: lp_mix_scratch() floats
+long lp_mix_scratch();
 void launch_lp_mix_grad(const float* x, const float* dg, int B, const float* W5, float* dx, float* dW5, float* db5,
-                        cudaStream_t st);
+                        float* scratch, cudaStream_t st);
 // the head through 128-point real transforms; scratch of lp_head_scratch(B, V) float2,
 // kept between a forward and its backward
 long lp_head_scratch(int B, int V);

@@ -411,23 +411,36 @@ __global__ void k_pool_grad(const float4* __restrict__ dp, long nout4, const flo
     }
 }
 
-// g[b][o][t] = b5[o] + sum_k W5[o][k] x[b][k][t], K = LP_MIXK
-__global__ void __launch_bounds__(NT) k_mix(const float* __restrict__ x, const float* __restrict__ W5,
-                                           const float* __restrict__ b5, float* __restrict__ g) {
-    __shared__ float sw[CM * LP_MIXK];
-    const int b = blockIdx.x, t = threadIdx.x;
-    for (int q = t; q < CM * LP_MIXK; q += NT) sw[q] = W5[q];
+// g[b][o][t] = b5[o] + sum_k W5[o][k] x[b][k][t], K = LP_MIXK.  Half h of the block sums half of
+// the outputs; the weights lie [k][o], so that four outputs' are one broadcast load.  Bound: the
+// shared-memory and L2 loads of a chain of K steps (one load a weight: 72 us for a batch of 256,
+// now 33 us; 10 us at the bandwidth of its reads).
+constexpr int MIX_LD = CM + 4;  // row of the staged weights: 16-byte aligned, spread over the banks
+__global__ void __launch_bounds__(2 * NT) k_mix(const float* __restrict__ x, const float* __restrict__ W5,
+                                               const float* __restrict__ b5, float* __restrict__ g) {
+    extern __shared__ float sw[];  // [LP_MIXK][MIX_LD]
+    constexpr int CO = CM / 2;
+    const int b = blockIdx.x, t = threadIdx.x % NT, o0 = CO * (threadIdx.x / NT);
+    for (int q = threadIdx.x; q < CM * LP_MIXK; q += 2 * NT) sw[q % LP_MIXK * MIX_LD + q / LP_MIXK] = W5[q];
     __syncthreads();
-    float acc[CM];
+    float acc[CO];
 #pragma unroll
-    for (int o = 0; o < CM; ++o) acc[o] = b5[o];
+    for (int o = 0; o < CO; ++o) acc[o] = b5[o0 + o];
+    const float* src = x + (long)b * LP_MIXK * NT + t;
+#pragma unroll 16
     for (int k = 0; k < LP_MIXK; ++k) {
-        const float v = x[((long)b * LP_MIXK + k) * NT + t];
+        const float v = src[k * NT];
 #pragma unroll
-        for (int o = 0; o < CM; ++o) acc[o] = fmaf(sw[o * LP_MIXK + k], v, acc[o]);
+        for (int o = 0; o < CO; o += 4) {
+            const float4 w = *(const float4*)(sw + k * MIX_LD + o0 + o);
+            acc[o] = fmaf(w.x, v, acc[o]);
+            acc[o + 1] = fmaf(w.y, v, acc[o + 1]);
+            acc[o + 2] = fmaf(w.z, v, acc[o + 2]);
+            acc[o + 3] = fmaf(w.w, v, acc[o + 3]);
+        }
     }
 #pragma unroll
-    for (int o = 0; o < CM; ++o) g[((long)b * CM + o) * NT + t] = acc[o];
+    for (int o = 0; o < CO; ++o) g[((long)b * CM + o0 + o) * NT + t] = acc[o];
 }
 // dx[b][k][t] = sum_o W5[o][k] dg[b][o][t]
 __global__ void __launch_bounds__(NT) k_mix_dx(const float* __restrict__ dg, const float* __restrict__ W5,
@@ -446,32 +459,87 @@ __global__ void __launch_bounds__(NT) k_mix_dx(const float* __restrict__ dg, con
         dx[((long)b * LP_MIXK + k) * NT + t] = a;
     }
 }
-// dW5[o][k] = sum_{b,t} dg[b][o][t] x[b][k][t]; db5[o] = sum dg (block k = 0 adds it)
+// dW5[o][k] = sum_{b,t} dg[b][o][t] x[b][k][t]; db5[o] = sum dg.  A block takes 32 k and every
+// gridDim.y-th sample: dg and x of a sample in shared memory, 4 x 4 sums a thread at an eighth
+// of the angles.  part[blockIdx.y]: its sums, [o][k] then the bias (of the blocks of k = 0).
+// Bound: the read of x (67 MB for a batch of 256, 10 us).  A block per k, which read dg 512
+// times over, took 81 us; now 17 and 4 of k_mix_sum.
+constexpr int MW_K = 32, MW_LD = NT + 4, MW_SPLIT = 32;
 __global__ void __launch_bounds__(256) k_mix_dw(const float* __restrict__ x, const float* __restrict__ dg, int B,
-                                               float* __restrict__ dW5, float* __restrict__ db5) {
-    __shared__ float sh[32];
-    const int k = blockIdx.x;
-    float acc[CM], accb[CM];
+                                               float* __restrict__ part) {
+    __shared__ __align__(16) float sd[CM * MW_LD], sx[MW_K * MW_LD];
+    static_assert(CM == 16 && MW_K == 32 && NT == 128, "tile of the block");
+    const int k0 = MW_K * blockIdx.x;
+    const int tg = threadIdx.x & 7, o0 = 4 * (threadIdx.x >> 3 & 3), q0 = 4 * (threadIdx.x >> 5);
+    float acc[4][4], bias[4];
 #pragma unroll
-    for (int o = 0; o < CM; ++o) { acc[o] = 0.f; accb[o] = 0.f; }
-    const int t = threadIdx.x % NT;  // blockDim is a multiple of NT
-    for (long b = threadIdx.x / NT; b < B; b += blockDim.x / NT) {
-        const float v = x[(b * LP_MIXK + k) * NT + t];
+    for (int i = 0; i < 4; ++i) {
+        bias[i] = 0.f;
 #pragma unroll
-        for (int o = 0; o < CM; ++o) {
-            const float d = dg[(b * CM + o) * NT + t];
-            acc[o] = fmaf(d, v, acc[o]);
-            accb[o] += d;
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    }
+    // the next sample's rows are loaded while this one's are summed
+    constexpr int ND = CM * NT / 4 / 256, NX = MW_K * NT / 4 / 256;
+    float4 pd[ND], px[NX];
+    auto load = [&](long b) {
+#pragma unroll
+        for (int k = 0; k < ND; ++k) pd[k] = ((const float4*)dg)[b * (CM * NT / 4) + threadIdx.x + 256 * k];
+#pragma unroll
+        for (int k = 0; k < NX; ++k)
+            px[k] = ((const float4*)x)[(b * LP_MIXK + k0) * (NT / 4) + threadIdx.x + 256 * k];
+    };
+    auto at = [](int q) { return q / (NT / 4) * MW_LD + q % (NT / 4) * 4; };
+    load(blockIdx.y);  // gridDim.y <= B
+    for (int b = blockIdx.y; b < B; b += gridDim.y) {
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < ND; ++k) *(float4*)(sd + at(threadIdx.x + 256 * k)) = pd[k];
+#pragma unroll
+        for (int k = 0; k < NX; ++k) *(float4*)(sx + at(threadIdx.x + 256 * k)) = px[k];
+        __syncthreads();
+        if (b + (int)gridDim.y < B) load(b + gridDim.y);
+#pragma unroll
+        for (int t = 4 * tg; t < NT; t += 32) {
+            float4 d[4], v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                d[i] = *(const float4*)(sd + (o0 + i) * MW_LD + t);
+                v[i] = *(const float4*)(sx + (q0 + i) * MW_LD + t);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                bias[i] += (d[i].x + d[i].y) + (d[i].z + d[i].w);
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    acc[i][j] = fmaf(d[i].x, v[j].x, fmaf(d[i].y, v[j].y, fmaf(d[i].z, v[j].z,
+                                fmaf(d[i].w, v[j].w, acc[i][j]))));
+            }
         }
     }
-    for (int o = 0; o < CM; ++o) {
-        const float s = block_sum(acc[o], sh);
-        if (threadIdx.x == 0) dW5[o * LP_MIXK + k] = s;
-        if (k == 0) {
-            const float sb = block_sum(accb[o], sh);
-            if (threadIdx.x == 0) db5[o] = sb;
+    float* dst = part + (long)blockIdx.y * (CM * LP_MIXK + CM);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+            float v = j < 4 ? acc[i][j & 3] : bias[i];
+            for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (tg) continue;
+            if (j < 4)
+                dst[(o0 + i) * LP_MIXK + k0 + q0 + j] = v;
+            else if (k0 + q0 == 0)
+                dst[CM * LP_MIXK + o0 + i] = v;
         }
     }
+}
+__global__ void k_mix_sum(const float* __restrict__ part, int n, float* __restrict__ dW5, float* __restrict__ db5) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= CM * LP_MIXK + CM) return;
+    float s = 0.f;
+    for (int k = 0; k < n; ++k) s += part[(long)k * (CM * LP_MIXK + CM) + q];
+    if (q < CM * LP_MIXK)
+        dW5[q] = s;
+    else
+        db5[q - CM * LP_MIXK] = s;
 }
 
 // Head in the frequency domain.  With X^(f) = sum_t x(t) e^{-2 pi i f t / NT} (the real
@@ -481,196 +549,338 @@ __global__ void __launch_bounds__(256) k_mix_dw(const float* __restrict__ x, con
 // 128-point sums against a twiddle table (NT^2 / 2 operations each, a few per particle
 // and view), products over the NT / 2 + 1 frequencies.
 constexpr int NF = NT / 2 + 1;
-constexpr int DR = 8;  // rows per block step of the real transforms
+constexpr int DR = 8;          // rows a warp transforms at once
+constexpr int DR_LD = DR + 4;  // staged rows lie [t][row]: a load takes four of them
+constexpr int DI_LD = DR + 2;  // and [f][row] complex: a load takes two
+constexpr int DW = 4;          // warps of a block
 
+// the twiddles, entry k at k + k / 16: the strides f of a transform then spread over the banks
+__device__ __forceinline__ int tw_at(int k) { return k + (k >> 4); }
+constexpr int TW_N = NT + NT / 16;
 __device__ __forceinline__ void twiddles(float2* tw) {
     for (int k = threadIdx.x; k < NT; k += blockDim.x) {
         float sn, cs;
         sincospif(2.0f * (float)k / (float)NT, &sn, &cs);
-        tw[k] = make_float2(cs, sn);
+        tw[tw_at(k)] = make_float2(cs, sn);
     }
 }
 
-// X[r][f] = sum_t x[r][t] e^{-2 pi i f t / NT} for rows r < n; block of NT threads,
-// rows in a grid-stride loop
-__global__ void __launch_bounds__(NT) k_rdft(const float* __restrict__ x, long n, float2* __restrict__ X) {
-    __shared__ float2 tw[NT];
-    __shared__ float sx[DR][NT];
+// X[r][f] = sum_t x[r][t] e^{-2 pi i f t / NT} for rows r < n, in a grid-stride loop, DR rows a
+// warp.  Lane l has the frequencies l and NT/2 - l, whose twiddles differ by the sign of the sine
+// and by (-1)^t, so that a staged value serves four FMA; frequency NT/4, whose twiddles are
+// 0 and +-1, is left to the lanes by rows.  Bound: the loads from shared memory (a broadcast
+// costs a lane's width: 10 cycles of the SM for the 32 FMA, 8 cycles, of a t).  A frequency a
+// thread, a load a row and two FMA, took 60 us for 44,544 rows; now 43.
+__global__ void __launch_bounds__(32 * DW) k_rdft(const float* __restrict__ x, long n, float2* __restrict__ X) {
+    __shared__ float2 tw[TW_N];
+    __shared__ __align__(16) float sx[DW][NT][DR_LD];
     twiddles(tw);
-    for (long r0 = (long)blockIdx.x * DR; r0 < n; r0 += (long)gridDim.x * DR) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (long r0 = (long)blockIdx.x * DW * DR; r0 < n; r0 += (long)gridDim.x * DW * DR) {
         __syncthreads();
-#pragma unroll
-        for (int i = 0; i < DR; ++i) sx[i][threadIdx.x] = r0 + i < n ? x[(r0 + i) * NT + threadIdx.x] : 0.f;
+        for (int q = threadIdx.x; q < DW * DR * NT; q += 32 * DW) {
+            const int i = q / NT, t = q % NT;
+            sx[i / DR][t][i % DR] = r0 + i < n ? x[(r0 + i) * NT + t] : 0.f;
+        }
         __syncthreads();
-        const int f = threadIdx.x;
-        if (f < NF) {
-            float re[DR], im[DR];
+        float re[2][DR], im[2][DR];
 #pragma unroll
-            for (int i = 0; i < DR; ++i) re[i] = im[i] = 0.f;
-            for (int t = 0; t < NT; ++t) {
-                const float2 w = tw[(f * t) & (NT - 1)];
+        for (int i = 0; i < DR; ++i) re[0][i] = re[1][i] = im[0][i] = im[1][i] = 0.f;
+        for (int t0 = 0; t0 < NT; t0 += 2) {
 #pragma unroll
-                for (int i = 0; i < DR; ++i) {
-                    re[i] = fmaf(sx[i][t], w.x, re[i]);
-                    im[i] = fmaf(-sx[i][t], w.y, im[i]);
+            for (int h = 0; h < 2; ++h) {
+                const int t = t0 + h;
+                const float2 w = tw[tw_at((lane * t) & (NT - 1))];
+                const float c2 = h ? -w.x : w.x, s2 = h ? w.y : -w.y;  // of frequency NT/2 - lane
+#pragma unroll
+                for (int i = 0; i < DR; i += 4) {
+                    const float4 q = *(const float4*)&sx[warp][t][i];
+                    const float v[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        re[0][i + e] = fmaf(v[e], w.x, re[0][i + e]);
+                        im[0][i + e] = fmaf(-v[e], w.y, im[0][i + e]);
+                        re[1][i + e] = fmaf(v[e], c2, re[1][i + e]);
+                        im[1][i + e] = fmaf(-v[e], s2, im[1][i + e]);
+                    }
                 }
             }
+        }
+        const long r1 = r0 + warp * DR;
 #pragma unroll
-            for (int i = 0; i < DR; ++i)
-                if (r0 + i < n) X[(r0 + i) * NF + f] = make_float2(re[i], im[i]);
+        for (int i = 0; i < DR; ++i)
+            if (r1 + i < n) {
+                X[(r1 + i) * NF + lane] = make_float2(re[0][i], im[0][i]);
+                X[(r1 + i) * NF + NT / 2 - lane] = make_float2(re[1][i], im[1][i]);
+            }
+        if (lane < DR && r1 + lane < n) {  // frequency NT / 4
+            float a = 0.f, b = 0.f;
+            for (int t = 0; t < NT; t += 4) {
+                a += sx[warp][t][lane];
+                b -= sx[warp][t + 1][lane];
+                a -= sx[warp][t + 2][lane];
+                b += sx[warp][t + 3][lane];
+            }
+            X[(r1 + lane) * NF + NT / 4] = make_float2(a, b);
         }
     }
 }
 
 // x[r][t] = (1/NT) sum over all f of X e^{+2 pi i f t / NT} for Hermitian spectra given
-// on f = 0 .. NT/2; beta: x = inverse + beta * x (0 or 1)
-__global__ void __launch_bounds__(NT) k_irdft(const float2* __restrict__ X, long n, float* __restrict__ x) {
-    __shared__ float2 tw[NT];
-    __shared__ float2 sX[DR][NF];
+// on f = 0 .. NT/2, DR rows a warp.  Lane l has the angles l, NT/2 - l, NT/2 + l and NT - l, whose
+// twiddles differ by signs ((-1)^f and the sine's), so that a staged value serves four FMA; the
+// angles NT/4 and 3 NT/4, whose twiddles are 0 and +-1, are left to the lanes by rows.  Bound as
+// k_rdft (67 us for the same rows with an angle a thread; now 42).
+__global__ void __launch_bounds__(32 * DW) k_irdft(const float2* __restrict__ X, long n, float* __restrict__ x) {
+    __shared__ float2 tw[TW_N];
+    __shared__ __align__(16) float2 sX[DW][NF][DI_LD];
     twiddles(tw);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float inv = 1.0f / (float)NT;
-    for (long r0 = (long)blockIdx.x * DR; r0 < n; r0 += (long)gridDim.x * DR) {
+    for (long r0 = (long)blockIdx.x * DW * DR; r0 < n; r0 += (long)gridDim.x * DW * DR) {
         __syncthreads();
-        if (threadIdx.x < NF) {
-#pragma unroll
-            for (int i = 0; i < DR; ++i)
-                sX[i][threadIdx.x] = r0 + i < n ? X[(r0 + i) * NF + threadIdx.x] : make_float2(0.f, 0.f);
+        for (int q = threadIdx.x; q < DW * DR * NF; q += 32 * DW) {
+            const int i = q / NF, f = q - i * NF;
+            sX[i / DR][f][i % DR] = r0 + i < n ? X[(r0 + i) * NF + f] : make_float2(0.f, 0.f);
         }
         __syncthreads();
-        const int t = threadIdx.x;
-        float acc[DR], a2[DR];
+        float a[4][DR];  // angles lane, NT - lane, NT/2 + lane, NT/2 - lane
 #pragma unroll
-        for (int i = 0; i < DR; ++i) {
-            acc[i] = sX[i][0].x + ((t & 1) ? -sX[i][NT / 2].x : sX[i][NT / 2].x);
-            a2[i] = 0.f;
-        }
-        for (int f = 1; f < NT / 2; ++f) {
-            const float2 w = tw[(f * t) & (NT - 1)];
+        for (int i = 0; i < DR; ++i) a[0][i] = a[1][i] = a[2][i] = a[3][i] = 0.f;
+        auto term = [&](int f, bool odd) {
+            const float2 w = tw[tw_at((f * lane) & (NT - 1))];
+            const float c2 = odd ? -w.x : w.x, s2 = odd ? -w.y : w.y;
 #pragma unroll
-            for (int i = 0; i < DR; ++i) {
-                a2[i] = fmaf(sX[i][f].x, w.x, a2[i]);
-                a2[i] = fmaf(-sX[i][f].y, w.y, a2[i]);
+            for (int i = 0; i < DR; i += 2) {
+                const float4 q = *(const float4*)&sX[warp][f][i];
+                const float vr[2] = {q.x, q.z}, vi[2] = {q.y, q.w};
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    a[0][i + e] = fmaf(-vi[e], w.y, fmaf(vr[e], w.x, a[0][i + e]));
+                    a[1][i + e] = fmaf(vi[e], w.y, fmaf(vr[e], w.x, a[1][i + e]));
+                    a[2][i + e] = fmaf(-vi[e], s2, fmaf(vr[e], c2, a[2][i + e]));
+                    a[3][i + e] = fmaf(vi[e], s2, fmaf(vr[e], c2, a[3][i + e]));
+                }
             }
+        };
+        for (int f = 1; f < NT / 2 - 1; f += 2) {
+            term(f, true);
+            term(f + 1, false);
         }
+        term(NT / 2 - 1, true);
+        const long r1 = r0 + warp * DR;
 #pragma unroll
         for (int i = 0; i < DR; ++i)
-            if (r0 + i < n) x[(r0 + i) * NT + t] = (acc[i] + 2.0f * a2[i]) * inv;
+            if (r1 + i < n) {
+                const float x0 = sX[warp][0][i].x, x1 = sX[warp][NT / 2][i].x;
+                const float acc = x0 + ((lane & 1) ? -x1 : x1);
+                float* dst = x + (r1 + i) * NT;
+                dst[lane] = (acc + 2.0f * a[0][i]) * inv;
+                if (lane) dst[NT - lane] = (acc + 2.0f * a[1][i]) * inv;
+                dst[NT / 2 + lane] = (acc + 2.0f * a[2][i]) * inv;
+                if (lane) dst[NT / 2 - lane] = (acc + 2.0f * a[3][i]) * inv;
+            }
+        // lanes 0 .. DR - 1: angle NT/4, DR .. 2 DR - 1: 3 NT/4
+        const int i = lane % DR;
+        if (lane < 2 * DR && r1 + i < n) {
+            float b = 0.f;
+            const float up = lane < DR ? 1.f : -1.f;
+            for (int f = 1; f < NT / 2; f += 2) {  // sin(pi f / 2) = 1, 0, -1, 0, ...
+                const float v = sX[warp][f][i].y;
+                b += (f & 2) ? up * v : -up * v;
+                if (f + 1 < NT / 2) b += ((f + 1) & 2) ? -sX[warp][f + 1][i].x : sX[warp][f + 1][i].x;
+            }
+            const float acc = sX[warp][0][i].x + sX[warp][NT / 2][i].x;  // NT/4 is even
+            x[(r1 + i) * NT + (lane < DR ? NT / 4 : 3 * NT / 4)] = (acc + 2.0f * b) * inv;
+        }
     }
 }
 
-// Xs[b][v][f] = sum_c G[b][c][f] conj(TT[v][c][f])
-__global__ void k_head_prod(const float2* __restrict__ G, const float2* __restrict__ TT, int B, int V,
-                            float2* __restrict__ Xs) {
-    const long n = (long)B * V * NF;
-    for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
-        const int f = (int)(q % NF);
-        const long bv = q / NF;
-        const int v = (int)(bv % V), b = (int)(bv / V);
-        float re = 0.f, im = 0.f;
+// The products of the head, frequency by frequency.  A block takes HF frequencies, so that the
+// spectra its sums share stay in shared memory (a warp loads whole 64-byte pieces of rows); the
+// terms of a sum keep their order.
+constexpr int HF = 8;  // frequencies of a block
+
+// Xs[b][v][f] = sum_c G[b][c][f] conj(TT[v][c][f]); 16 particles x 16 views a block, 2 x 4 sums a
+// thread.  Bound: the loads from shared memory (6 for 32 FMA) and the write of Xs.  A sum a thread,
+// two loads a term, took 37 us for 256 particles and 174 views; now 26.
+constexpr int HP_T = 16, HP_B = 2, HP_V = 4, HP_LD = CM * HF + HF;
+__global__ void __launch_bounds__(256) k_head_prod(const float2* __restrict__ G, const float2* __restrict__ TT, int B,
+                                                  int V, float2* __restrict__ Xs) {
+    __shared__ float2 sg[HP_T * HP_LD], st[HP_T * HP_LD];  // [particle or view][c][f]
+    const int f0 = HF * blockIdx.x, v0 = HP_T * blockIdx.y, b0 = HP_T * blockIdx.z;
+    for (int q = threadIdx.x; q < HP_T * CM * HF; q += 256) {
+        const int f = q % HF, c = q / HF % CM, i = q / (HF * CM);
+        const bool in = f0 + f < NF;
+        const float2 zero = make_float2(0.f, 0.f);
+        sg[i * HP_LD + c * HF + f] = in && b0 + i < B ? G[((long)(b0 + i) * CM + c) * NF + f0 + f] : zero;
+        st[i * HP_LD + c * HF + f] = in && v0 + i < V ? TT[((long)(v0 + i) * CM + c) * NF + f0 + f] : zero;
+    }
+    __syncthreads();
+    const int f = threadIdx.x % HF, vi = HP_V * (threadIdx.x / HF % (HP_T / HP_V)),
+              bi = HP_B * (threadIdx.x / (HF * HP_T / HP_V));
+    float re[HP_B][HP_V], im[HP_B][HP_V];
 #pragma unroll
-        for (int c = 0; c < CM; ++c) {
-            const float2 g = G[((long)b * CM + c) * NF + f], t = TT[((long)v * CM + c) * NF + f];
-            re = fmaf(g.x, t.x, fmaf(g.y, t.y, re));
-            im = fmaf(g.y, t.x, fmaf(-g.x, t.y, im));
-        }
-        Xs[q] = make_float2(re, im);
+    for (int i = 0; i < HP_B; ++i)
+#pragma unroll
+        for (int j = 0; j < HP_V; ++j) re[i][j] = im[i][j] = 0.f;
+#pragma unroll 4
+    for (int c = 0; c < CM; ++c) {
+        float2 g[HP_B], t[HP_V];
+#pragma unroll
+        for (int i = 0; i < HP_B; ++i) g[i] = sg[(bi + i) * HP_LD + c * HF + f];
+#pragma unroll
+        for (int j = 0; j < HP_V; ++j) t[j] = st[(vi + j) * HP_LD + c * HF + f];
+#pragma unroll
+        for (int i = 0; i < HP_B; ++i)
+#pragma unroll
+            for (int j = 0; j < HP_V; ++j) {
+                re[i][j] = fmaf(g[i].x, t[j].x, fmaf(g[i].y, t[j].y, re[i][j]));
+                im[i][j] = fmaf(g[i].y, t[j].x, fmaf(-g[i].x, t[j].y, im[i][j]));
+            }
     }
+    if (f0 + f >= NF) return;
+#pragma unroll
+    for (int i = 0; i < HP_B; ++i)
+#pragma unroll
+        for (int j = 0; j < HP_V; ++j)
+            if (b0 + bi + i < B && v0 + vi + j < V)
+                Xs[((long)(b0 + bi + i) * V + v0 + vi + j) * NF + f0 + f] = make_float2(re[i][j], im[i][j]);
 }
 
-// dTT[v][c][f] = sum_b conj(D[b][v][f]) G[b][c][f]
-__global__ void k_head_dTT(const float2* __restrict__ D, const float2* __restrict__ G, int B, int V,
-                           float2* __restrict__ dTT) {
-    const long n = (long)V * CM * NF;
-    for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
-        const int f = (int)(q % NF);
-        const long vc = q / NF;
-        const int c = (int)(vc % CM), v = (int)(vc / CM);
-        float re = 0.f, im = 0.f;
-        for (int b = 0; b < B; ++b) {
-            const float2 d = D[((long)b * V + v) * NF + f], g = G[((long)b * CM + c) * NF + f];
-            re = fmaf(d.x, g.x, fmaf(d.y, g.y, re));
-            im = fmaf(d.x, g.y, fmaf(-d.y, g.x, im));
-        }
-        dTT[q] = make_float2(re, im);
-    }
+// out[o][c][f] = sum_s D(o, s)[f] Y[s][c][f] over s < ns, with D(o, s) at row do_ o + ds s of D and
+// conjugated in D for CONJ: the gradients of the templates (o = view, s = particle, CONJ, Y = G)
+// and of g (o = particle, s = view, Y = TT).  A warp has one o, a lane a frequency and four
+// channels; HS_N terms at a time come by cp.async, HS_BUF - 1 such groups ahead.  Bound:
+// the loads from shared memory (5 for 16 FMA).  A sum a thread, straight from L2, took 114 and
+// 43 us for 256 particles and 174 views; now 37 and 41.
+constexpr int HS_O = 12, HS_N = 8, HS_C = 4, HS_BUF = 2;
+__device__ __forceinline__ void cp_async8(void* dst, const void* src, bool in) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(in ? 8 : 0)
+                 : "memory");
 }
-
-// dG[b][c][f] = sum_v D[b][v][f] TT[v][c][f]
-__global__ void k_head_dG(const float2* __restrict__ D, const float2* __restrict__ TT, int B, int V,
-                          float2* __restrict__ dG) {
-    const long n = (long)B * CM * NF;
-    for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
-        const int f = (int)(q % NF);
-        const long bc = q / NF;
-        const int c = (int)(bc % CM), b = (int)(bc / CM);
-        float re = 0.f, im = 0.f;
-        for (int v = 0; v < V; ++v) {
-            const float2 d = D[((long)b * V + v) * NF + f], t = TT[((long)v * CM + c) * NF + f];
-            re = fmaf(d.x, t.x, fmaf(-d.y, t.y, re));
-            im = fmaf(d.x, t.y, fmaf(d.y, t.x, im));
+template <bool CONJ>
+__global__ void __launch_bounds__(32 * HS_O) k_head_sum(const float2* __restrict__ D, const float2* __restrict__ Y,
+                                                       int no, int ns, int do_, int ds, float2* __restrict__ out) {
+    __shared__ float2 sd[HS_BUF][HS_N][HS_O][HF], sy[HS_BUF][HS_N][CM][HF];
+    static_assert(HF * (CM / HS_C) == 32, "a warp is the frequencies times the channel groups");
+    const int f0 = HF * blockIdx.x, o0 = HS_O * blockIdx.y;
+    const int warp = threadIdx.x >> 5, f = threadIdx.x % HF;
+    const int c = (threadIdx.x & 31) / HF;  // and every HS_C-th channel after it: no bank twice
+    auto fetch = [&](int s0, int buf) {  // terms beyond the last and rows outside are zeros
+        for (int q = threadIdx.x; q < HS_N * HS_O * HF; q += 32 * HS_O) {
+            const int ff = q % HF, o = q / HF % HS_O, s = q / (HF * HS_O);
+            const bool in = s0 + s < ns && o0 + o < no && f0 + ff < NF;
+            cp_async8(&sd[buf][s][o][ff],
+                      in ? D + ((long)(o0 + o) * do_ + (long)(s0 + s) * ds) * NF + f0 + ff : D, in);
         }
-        dG[q] = make_float2(re, im);
+        for (int q = threadIdx.x; q < HS_N * CM * HF; q += 32 * HS_O) {
+            const int ff = q % HF, k = q / HF % CM, s = q / (HF * CM);
+            const bool in = s0 + s < ns && f0 + ff < NF;
+            cp_async8(&sy[buf][s][k][ff], in ? Y + ((long)(s0 + s) * CM + k) * NF + f0 + ff : Y, in);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float re[HS_C], im[HS_C];
+#pragma unroll
+    for (int k = 0; k < HS_C; ++k) re[k] = im[k] = 0.f;
+    for (int k = 0; k < HS_BUF - 1; ++k) fetch(k * HS_N, k);
+    int buf = 0;
+    for (int s0 = 0; s0 < ns; s0 += HS_N, buf = (buf + 1) % HS_BUF) {
+        fetch(s0 + (HS_BUF - 1) * HS_N, (buf + HS_BUF - 1) % HS_BUF);  // zeros beyond the last
+        asm volatile("cp.async.wait_group %0;" ::"n"(HS_BUF - 1) : "memory");
+        __syncthreads();
+#pragma unroll
+        for (int s = 0; s < HS_N; ++s) {
+            const float2 d = sd[buf][s][warp][f];
+#pragma unroll
+            for (int k = 0; k < HS_C; ++k) {
+                const float2 y = sy[buf][s][c + CM / HS_C * k][f];
+                if (CONJ) {
+                    re[k] = fmaf(d.x, y.x, fmaf(d.y, y.y, re[k]));
+                    im[k] = fmaf(d.x, y.y, fmaf(-d.y, y.x, im[k]));
+                } else {
+                    re[k] = fmaf(d.x, y.x, fmaf(-d.y, y.y, re[k]));
+                    im[k] = fmaf(d.x, y.y, fmaf(d.y, y.x, im[k]));
+                }
+            }
+        }
+        __syncthreads();
     }
+    if (f0 + f < NF && o0 + warp < no)
+#pragma unroll
+        for (int k = 0; k < HS_C; ++k)
+            out[((long)(o0 + warp) * CM + c + CM / HS_C * k) * NF + f0 + f] = make_float2(re[k], im[k]);
 }
 
 // Soft-target cross entropy over the V x NT cells of each particle.  truth[b] = (view
 // unit vector, shift); target(v, s) = exp(-(angle(v, v*) / sv)^2 - (d(s, s*) / ss)^2),
 // normalised.  dsc = (softmax - target) / B; loss[b] = -sum target log softmax.
-__global__ void __launch_bounds__(256) k_loss(const float* __restrict__ sc, int B, int V,
-                                             const float* __restrict__ vview, const float* __restrict__ truth,
-                                             float sv, float ss, float* __restrict__ dsc, float* __restrict__ loss) {
-    __shared__ float sh[32];
+// Thread tid has the shift tid % NT of every second view, so the shift's distance is one value
+// a thread; the angles to the views are worked out 256 at a time, once for the block.  Bound:
+// the three passes over the scores and their exponentials.  With an arc cosine per cell and
+// pass it took 144 us for 256 particles and 174 views; now 36.
+constexpr int LOSS_TPB = 256;
+__global__ void __launch_bounds__(LOSS_TPB) k_loss(const float* __restrict__ sc, int B, int V,
+                                                  const float* __restrict__ vview, const float* __restrict__ truth,
+                                                  float sv, float ss, float* __restrict__ dsc,
+                                                  float* __restrict__ loss) {
+    static_assert(LOSS_TPB % NT == 0, "a thread keeps its shift");
+    __shared__ float sh[32], sav[LOSS_TPB];
     const int b = blockIdx.x;
     const long n = (long)V * NT;
     const float* x = sc + (long)b * n;
     const float* tr = truth + 4 * b;
     const float rad2deg = 57.29577951308232f;
+    const int s = threadIdx.x % NT;
+    int ds = abs(s - (int)tr[3]) % NT;
+    ds = min(ds, NT - ds);
+    const float as = (float)ds / ss;
+    // f(cell, angle to its view) over the thread's cells, in the order of the views
+    auto cells = [&](auto f) {
+        for (int v0 = 0; v0 < V; v0 += LOSS_TPB) {
+            __syncthreads();
+            const int v = v0 + threadIdx.x;
+            if (v < V) {
+                const float dot = vview[3 * v] * tr[0] + vview[3 * v + 1] * tr[1] + vview[3 * v + 2] * tr[2];
+                sav[threadIdx.x] = acosf(fminf(fmaxf(dot, -1.f), 1.f)) * rad2deg / sv;
+            }
+            __syncthreads();
+            const int nv = min(V - v0, LOSS_TPB);
+#pragma unroll 4
+            for (int i = threadIdx.x / NT; i < nv; i += LOSS_TPB / NT) f((long)(v0 + i) * NT + s, sav[i]);
+        }
+    };
     // the target's exponent -(av^2 + as^2) is taken relative to its largest value over the
     // cells (the normalised target is unchanged), so its sum is >= 1 even for a label far
     // from every view class (an orientation at an asymmetric-unit edge that no operator
     // folds inside in FP32)
     float mx = -3.0e38f, dmin = 3.0e38f;
-    for (long q = threadIdx.x; q < n; q += blockDim.x) {
+    cells([&](long q, float av) {
         mx = fmaxf(mx, x[q]);
-        const int v = (int)(q / NT), s = (int)(q % NT);
-        const float dot = vview[3 * v] * tr[0] + vview[3 * v + 1] * tr[1] + vview[3 * v + 2] * tr[2];
-        const float av = acosf(fminf(fmaxf(dot, -1.f), 1.f)) * rad2deg / sv;
-        int ds = abs(s - (int)tr[3]) % NT;
-        ds = min(ds, NT - ds);
-        const float as = (float)ds / ss;
         dmin = fminf(dmin, av * av + as * as);
-    }
+    });
     mx = block_max(mx, sh);
     dmin = -block_max(-dmin, sh);
     float se = 0.f, st = 0.f, stx = 0.f;
-    for (long q = threadIdx.x; q < n; q += blockDim.x) {
-        const int v = (int)(q / NT), s = (int)(q % NT);
-        se += expf(x[q] - mx);
-        const float dot = vview[3 * v] * tr[0] + vview[3 * v + 1] * tr[1] + vview[3 * v + 2] * tr[2];
-        const float av = acosf(fminf(fmaxf(dot, -1.f), 1.f)) * rad2deg / sv;
-        int ds = abs(s - (int)tr[3]) % NT;
-        ds = min(ds, NT - ds);
-        const float as = (float)ds / ss;
+    cells([&](long q, float av) {
+        const float d = x[q] - mx;
+        se += expf(d);
         const float tg = expf(dmin - av * av - as * as);
         st += tg;
-        stx += tg * (x[q] - mx);
-    }
+        stx += tg * d;
+    });
     se = block_sum(se, sh);
     st = block_sum(st, sh);
     stx = block_sum(stx, sh);
     const float lse = logf(se);
     if (threadIdx.x == 0) loss[b] = -(stx / st - lse);
     const float ist = 1.0f / st, ise = 1.0f / se, ib = 1.0f / (float)B;
-    for (long q = threadIdx.x; q < n; q += blockDim.x) {
-        const int v = (int)(q / NT), s = (int)(q % NT);
-        const float dot = vview[3 * v] * tr[0] + vview[3 * v + 1] * tr[1] + vview[3 * v + 2] * tr[2];
-        const float av = acosf(fminf(fmaxf(dot, -1.f), 1.f)) * rad2deg / sv;
-        int ds = abs(s - (int)tr[3]) % NT;
-        ds = min(ds, NT - ds);
-        const float as = (float)ds / ss;
+    cells([&](long q, float av) {
         const float tg = expf(dmin - av * av - as * as);
         dsc[(long)b * n + q] = (expf(x[q] - mx) * ise - tg * ist) * ib;
-    }
+    });
 }
 
 __global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
@@ -781,13 +991,20 @@ void launch_lp_pool_grad(const float* dp, int B, int C, int Hout, const float* a
                                                    reinterpret_cast<float4*>(da));
 }
 void launch_lp_mix(const float* x, int B, const float* W5, const float* b5, float* g, cudaStream_t st) {
-    k_mix<<<B, NT, 0, st>>>(x, W5, b5, g);
+    constexpr int smem = LP_MIXK * MIX_LD * (int)sizeof(float);
+    static_assert(smem <= 48 * 1024, "no opt-in needed");
+    k_mix<<<B, 2 * NT, smem, st>>>(x, W5, b5, g);
 }
+long lp_mix_scratch() { return (long)MW_SPLIT * (CM * LP_MIXK + CM); }
 void launch_lp_mix_grad(const float* x, const float* dg, int B, const float* W5, float* dx, float* dW5, float* db5,
-                        cudaStream_t st) {
+                        float* scratch, cudaStream_t st) {
     if (dx) k_mix_dx<<<B, NT, 0, st>>>(dg, W5, dx);
-    k_mix_dw<<<LP_MIXK, 256, 0, st>>>(x, dg, B, dW5, db5);
+    const int split = std::min(B, MW_SPLIT);
+    k_mix_dw<<<dim3(LP_MIXK / MW_K, split), 256, 0, st>>>(x, dg, B, scratch);
+    k_mix_sum<<<cdiv(CM * LP_MIXK + CM, 64), 64, 0, st>>>(scratch, split, dW5, db5);
 }
+// a few blocks per SM; the loop takes the rest
+int dft_grid(long rows) { return (int)std::min<long>((rows + DW * DR - 1) / (DW * DR), 152 * 12); }
 long lp_head_scratch(int B, int V) { return (long)NF * (2L * B * CM + 2L * V * CM + 2L * B * V); }
 
 // scratch (float2): G [B][CM][NF], TT [V][CM][NF], X [B][V][NF], then the backward's
@@ -796,11 +1013,10 @@ cudaError_t launch_lp_head(const float* g, const float* T, int B, int V, float* 
     float2* G = scratch;
     float2* TT = G + (long)B * CM * NF;
     float2* X = TT + (long)V * CM * NF;
-    const int gmax = 152 * 16;
-    k_rdft<<<(int)std::min<long>(((long)B * CM + DR - 1) / DR, gmax), NT, 0, st>>>(g, (long)B * CM, G);
-    k_rdft<<<(int)std::min<long>(((long)V * CM + DR - 1) / DR, gmax), NT, 0, st>>>(T, (long)V * CM, TT);
-    k_head_prod<<<grid_for((long)B * V * NF, 256), 256, 0, st>>>(G, TT, B, V, X);
-    k_irdft<<<(int)std::min<long>(((long)B * V + DR - 1) / DR, gmax), NT, 0, st>>>(X, (long)B * V, sc);
+    k_rdft<<<dft_grid((long)B * CM), 32 * DW, 0, st>>>(g, (long)B * CM, G);
+    k_rdft<<<dft_grid((long)V * CM), 32 * DW, 0, st>>>(T, (long)V * CM, TT);
+    k_head_prod<<<dim3(cdiv(NF, HF), cdiv(V, HP_T), cdiv(B, HP_T)), 256, 0, st>>>(G, TT, B, V, X);
+    k_irdft<<<dft_grid((long)B * V), 32 * DW, 0, st>>>(X, (long)B * V, sc);
     return cudaGetLastError();
 }
 void launch_lp_head_grad(const float* g, const float* T, const float* dsc, int B, int V, float* dg, float* dT,
@@ -811,16 +1027,15 @@ void launch_lp_head_grad(const float* g, const float* T, const float* dsc, int B
     float2* D = TT + (long)V * CM * NF;  // over X
     float2* dTT = D + (long)B * V * NF;
     float2* dG = dTT + (long)V * CM * NF;
-    const int gmax = 152 * 16;
-    k_rdft<<<(int)std::min<long>(((long)B * V + DR - 1) / DR, gmax), NT, 0, st>>>(dsc, (long)B * V, D);
-    k_head_dTT<<<grid_for((long)V * CM * NF, 128), 128, 0, st>>>(D, G, B, V, dTT);
-    k_head_dG<<<grid_for((long)B * CM * NF, 128), 128, 0, st>>>(D, TT, B, V, dG);
-    k_irdft<<<(int)std::min<long>(((long)V * CM + DR - 1) / DR, gmax), NT, 0, st>>>(dTT, (long)V * CM, dT);
-    k_irdft<<<(int)std::min<long>(((long)B * CM + DR - 1) / DR, gmax), NT, 0, st>>>(dG, (long)B * CM, dg);
+    k_rdft<<<dft_grid((long)B * V), 32 * DW, 0, st>>>(dsc, (long)B * V, D);
+    k_head_sum<true><<<dim3(cdiv(NF, HF), cdiv(V, HS_O)), 32 * HS_O, 0, st>>>(D, G, V, B, 1, V, dTT);
+    k_head_sum<false><<<dim3(cdiv(NF, HF), cdiv(B, HS_O)), 32 * HS_O, 0, st>>>(D, TT, B, V, V, 1, dG);
+    k_irdft<<<dft_grid((long)V * CM), 32 * DW, 0, st>>>(dTT, (long)V * CM, dT);
+    k_irdft<<<dft_grid((long)B * CM), 32 * DW, 0, st>>>(dG, (long)B * CM, dg);
 }
 void launch_lp_loss(const float* sc, int B, int V, const float* vview, const float* truth, float sv, float ss,
                     float* dsc, float* loss, cudaStream_t st) {
-    k_loss<<<B, 256, 0, st>>>(sc, B, V, vview, truth, sv, ss, dsc, loss);
+    k_loss<<<B, LOSS_TPB, 0, st>>>(sc, B, V, vview, truth, sv, ss, dsc, loss);
 }
 void launch_lp_adam(float* w, const float* g, float* m, float* v, long n, float lr, int step, cudaStream_t st) {
     const float b1 = 0.9f, b2 = 0.999f;

@@ -21,6 +21,7 @@
 #include <type_traits>
 
 #include "geom.cuh"
+#include "reduce.cuh"
 #include "kernels.h"
 #include "origin_basis.h"
 
@@ -43,6 +44,16 @@ __device__ double block_sum_double(double v, double* sh) {
     r = sh[0];
     __syncthreads();
     return r;
+}
+
+// 1 / sqrt of the block's FP64 sum of part (0 for 0); the root and the quotient by one thread: FP64
+// work of every warp would take longer than a row's samples
+__device__ float block_inv_norm(float part, double* sh) {
+    __shared__ float inv;
+    const double nrm = block_sum_double((double)part, sh);
+    if (threadIdx.x == 0) inv = nrm > 0.0 ? (float)(1.0 / sqrt(nrm)) : 0.0f;
+    __syncthreads();
+    return inv;
 }
 
 // map * (-1)^(x+y+z) as complex, so the forward FFT is centred at nx/2
@@ -159,8 +170,7 @@ __global__ void __launch_bounds__(512) k_slice_bf16(cudaTextureObject_t cube, in
         ssec[i] = val;
         part += val.x * val.x + val.y * val.y;
     }
-    const double nrm = block_sum_double((double)part, sh);
-    const float inv = nrm > 0.0 ? (float)(1.0 / sqrt(nrm)) : 0.0f;
+    const float inv = block_inv_norm(part, sh);
     __nv_bfloat16* row = B + (long)blockIdx.x * (2 * KH);
     for (int i = 2 * threadIdx.x; i < KH; i += 2 * blockDim.x) {
         const float2 a = i < S ? ssec[i] : make_float2(0.f, 0.f);
@@ -214,8 +224,7 @@ __global__ void __launch_bounds__(512) k_slice_bf16_local(cudaTextureObject_t cu
         const float cw = pctf ? pctf[(long)p * S + t] : 1.0f;
         part += cw * cw * (val.x * val.x + val.y * val.y);
     }
-    const double nrm = block_sum_double((double)part, sh);
-    const float inv = nrm > 0.0 ? (float)(1.0 / sqrt(nrm)) : 0.0f;
+    const float inv = block_inv_norm(part, sh);
     __nv_bfloat162* row = B + (long)blockIdx.x * (Kpad / 2);
     for (int t = threadIdx.x; t < Kpad / 2; t += blockDim.x) {
         float2 val = t < S ? ssec[t] : make_float2(0.f, 0.f);
@@ -224,19 +233,26 @@ __global__ void __launch_bounds__(512) k_slice_bf16_local(cudaTextureObject_t cu
 }
 
 // The same rows, one CTA per (particle p, i, j) cutting the n rows k = 0 .. n - 1 (the
-// omega steps) in turn: a thread holds its samples (h, k, CTF^2) in registers across the
-// rows and a row's values in registers until its norm is known, so the CTA needs no
-// shared-memory row and the SM's L1 stays large for the texture fetches, which
+// omega steps) LSR_ROWS at a time: a thread holds its SPT samples (h, k, CTF^2) in registers
+// across the rows and the rows' values in registers until their norms are known, so the CTA needs
+// no shared-memory row and the SM's L1 stays large for the texture fetches, which
 // neighbouring omegas share (0.25 degrees moves a sample by a fraction of a voxel).
 // Each row's values, norm and BF16 row are k_slice_bf16_local's; the norm's FP32
 // per-thread partials cover fewer samples (it agrees to FP32 rounding).
+// Bound: the texture pipe (60 % busy, FP64 16 %).  With a row at a time, every warp summing in five
+// FP64 steps and taking the root and the quotient for itself, the FP64 pipe was 70 % busy and
+// the 15,625 rows of each of 24 particles (25 steps a side, 1,600
+// samples a row) took 6.27 ms; now 3.66.  Two rows at a time 3.8 to 3.9, one 4.4, 512 threads 4.1.
 constexpr int LSR_THREADS = 256, LSR_SPT = 8;  // rows of up to 2,048 samples (pairs)
-__global__ void __launch_bounds__(LSR_THREADS) k_slice_bf16_local_rows(
+constexpr int LSR_ROWS = 4;
+template <int SPT>
+__global__ void __launch_bounds__(LSR_THREADS, 2) k_slice_bf16_local_rows(
     cudaTextureObject_t cube, int R, const int2* __restrict__ samples, int S, int Kpad,
     const float* __restrict__ centre, int m, float step, float d2r, __nv_bfloat162* __restrict__ B,
     const float2* __restrict__ lin, float gk, long lpitch, const float* __restrict__ pctf, float sc) {
     extern __shared__ float rots[];  // [n][9]
-    __shared__ double wsum[2][LSR_THREADS / 32];
+    __shared__ double wsum[LSR_ROWS][LSR_THREADS / 32];
+    __shared__ float sinv[LSR_ROWS];
     const int n = 2 * m + 1;
     const int p = blockIdx.y, ij = blockIdx.x;
     const int i = ij / n, j = ij % n;
@@ -246,9 +262,9 @@ __global__ void __launch_bounds__(LSR_THREADS) k_slice_bf16_local_rows(
                   centre[3 * p + 2] + step * (float)(k - m), d2r, rot);
         for (int e = 0; e < 9; ++e) rot[e] *= sc;  // cube voxels per frequency unit
     }
-    float hx[LSR_SPT], ky[LSR_SPT], cw2[LSR_SPT];
+    float hx[SPT], ky[SPT], cw2[SPT];
 #pragma unroll
-    for (int s = 0; s < LSR_SPT; ++s) {
+    for (int s = 0; s < SPT; ++s) {
         const int t = threadIdx.x + s * LSR_THREADS;
         hx[s] = 0.0f;
         ky[s] = 0.0f;
@@ -264,36 +280,51 @@ __global__ void __launch_bounds__(LSR_THREADS) k_slice_bf16_local_rows(
     __syncthreads();
     const float off = (float)(R + 1) + 0.5f;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int k = 0; k < n; ++k) {
-        const float* rot = rots + 9 * k;
-        const float r0 = rot[0], r1 = rot[1], r3 = rot[3], r4 = rot[4], r6 = rot[6], r7 = rot[7];
-        float2 val[LSR_SPT];
-        float part = 0.0f;
+    for (int k0 = 0; k0 < n; k0 += LSR_ROWS) {
+        float2 val[LSR_ROWS][SPT];
+        double sums[LSR_ROWS];
 #pragma unroll
-        for (int s = 0; s < LSR_SPT; ++s) {
-            val[s] = make_float2(0.f, 0.f);
-            if (threadIdx.x + s * LSR_THREADS < S) {
-                const float x = r0 * hx[s] + r1 * ky[s], y = r3 * hx[s] + r4 * ky[s], z = r6 * hx[s] + r7 * ky[s];
-                val[s] = gk > 0.0f ? gauss_sample(lin, 2 * R + 3, R + 1, x, y, z, gk)
-                                   : tex3D<float2>(cube, x + off, y + off, z + off);
-                part += cw2[s] * (val[s].x * val[s].x + val[s].y * val[s].y);
+        for (int q = 0; q < LSR_ROWS; ++q) {
+            const float* rot = rots + 9 * min(k0 + q, n - 1);  // a row beyond the last is not written
+            const float r0 = rot[0], r1 = rot[1], r3 = rot[3], r4 = rot[4], r6 = rot[6], r7 = rot[7];
+            float part = 0.0f;
+#pragma unroll
+            for (int s = 0; s < SPT; ++s) {
+                val[q][s] = make_float2(0.f, 0.f);
+                if (threadIdx.x + s * LSR_THREADS < S && k0 + q < n) {
+                    const float x = r0 * hx[s] + r1 * ky[s], y = r3 * hx[s] + r4 * ky[s], z = r6 * hx[s] + r7 * ky[s];
+                    val[q][s] = gk > 0.0f ? gauss_sample(lin, 2 * R + 3, R + 1, x, y, z, gk)
+                                          : tex3D<float2>(cube, x + off, y + off, z + off);
+                }
             }
+#pragma unroll
+            for (int s = 0; s < SPT; ++s)
+                if (threadIdx.x + s * LSR_THREADS < S)
+                    part += cw2[s] * (val[q][s].x * val[q][s].x + val[q][s].y * val[q][s].y);
+            sums[q] = (double)part;
         }
-        // norm: FP64 across the block in a fixed order (warps, then the warps' sums)
-        double d = (double)part;
-        for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-        if (lane == 0) wsum[k & 1][wid] = d;
-        __syncthreads();  // also orders this row's reads of wsum[k & 1] before row k + 2 writes it
-        double nrm = 0.0;
+        // norms: FP64 across the block in a fixed order (warps, then the warps' sums)
+        warp_sums<LSR_ROWS>(sums, lane);
+        if (lane % (32 / LSR_ROWS) == 0) wsum[warp_sum_index<LSR_ROWS>(lane)][wid] = sums[0];
+        __syncthreads();
+        if (threadIdx.x < LSR_ROWS) {
+            double nrm = 0.0;
 #pragma unroll
-        for (int w = 0; w < LSR_THREADS / 32; ++w) nrm += wsum[k & 1][w];
-        const float inv = nrm > 0.0 ? (float)(1.0 / sqrt(nrm)) : 0.0f;
-        const long q = (long)p * lpitch + (long)ij * n + k;
-        __nv_bfloat162* row = B + q * (Kpad / 2);
+            for (int w = 0; w < LSR_THREADS / 32; ++w) nrm += wsum[threadIdx.x][w];
+            sinv[threadIdx.x] = nrm > 0.0 ? (float)(1.0 / sqrt(nrm)) : 0.0f;
+        }
+        __syncthreads();
 #pragma unroll
-        for (int s = 0; s < LSR_SPT; ++s) {
-            const int t = threadIdx.x + s * LSR_THREADS;
-            if (t < Kpad / 2) row[bf16_pair_at(t, q)] = __floats2bfloat162_rn(val[s].x * inv, val[s].y * inv);
+        for (int q = 0; q < LSR_ROWS; ++q) {
+            if (k0 + q >= n) break;
+            const float inv = sinv[q];
+            const long r = (long)p * lpitch + (long)ij * n + k0 + q;
+            __nv_bfloat162* row = B + r * (Kpad / 2);
+#pragma unroll
+            for (int s = 0; s < SPT; ++s) {
+                const int t = threadIdx.x + s * LSR_THREADS;
+                if (t < Kpad / 2) row[bf16_pair_at(t, r)] = __floats2bfloat162_rn(val[q][s].x * inv, val[q][s].y * inv);
+            }
         }
     }
 }
@@ -1349,10 +1380,18 @@ cudaError_t launch_slice_bf16_local(cudaTextureObject_t cube, int R, const int2*
     if (Kpad / 2 <= LSR_THREADS * LSR_SPT && count % lpitch == 0 && n * n <= 65535 && count / lpitch <= 65535) {
         // the whole grid of each of count / lpitch particles: rows by (p, i, j) lines of omegas
         dim3 grid((unsigned)(n * n), (unsigned)(count / lpitch));
-        k_slice_bf16_local_rows<<<grid, LSR_THREADS, sizeof(float) * 9 * (size_t)n, st>>>(
-            cube, R, samples, S, Kpad, centre, m, step, host_angles().deg2rad, (__nv_bfloat162*)B, lin, gk, lpitch,
-            pctf, sc);
-        return cudaGetLastError();
+        auto rows = [&](auto spt) {
+            k_slice_bf16_local_rows<decltype(spt)::value><<<grid, LSR_THREADS, sizeof(float) * 9 * (size_t)n, st>>>(
+                cube, R, samples, S, Kpad, centre, m, step, host_angles().deg2rad, (__nv_bfloat162*)B, lin, gk, lpitch,
+                pctf, sc);
+            return cudaGetLastError();
+        };
+        // registers for the samples there are, to the next even number a thread
+        const int spt = (Kpad / 2 + LSR_THREADS - 1) / LSR_THREADS;
+        if (spt <= 2) return rows(std::integral_constant<int, 2>());
+        if (spt <= 4) return rows(std::integral_constant<int, 4>());
+        if (spt <= 6) return rows(std::integral_constant<int, 6>());
+        return rows(std::integral_constant<int, LSR_SPT>());
     }
     size_t sm = (size_t)S * sizeof(float2);
     cudaError_t e =

@@ -21,6 +21,7 @@
 #include <type_traits>
 
 #include "geom.cuh"
+#include "reduce.cuh"
 #include "kernels.h"
 
 namespace cryoim {
@@ -451,7 +452,7 @@ __global__ void __launch_bounds__(512) k_pr_single(PrSingleArgs a, Consts K) {
 constexpr int RG = 4;
 __global__ void __launch_bounds__(512) k_pr_rescore_g(PrSingleArgs a, const int4* __restrict__ groups, Consts K) {
     extern __shared__ float rsm[];
-    __shared__ double sh[2][RG][16];
+    __shared__ double sh[2 * RG][32];
     const Band bd = a.bd;
     const int W = bd.W, nr = bd.nr, minR = bd.min_r, nx = bd.nx, T = a.T;
     const int4 gr = groups[blockIdx.x];
@@ -536,22 +537,16 @@ __global__ void __launch_bounds__(512) k_pr_rescore_g(PrSingleArgs a, const int4
             }
         }
     }
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+    double sums[2 * RG];
 #pragma unroll
     for (int g = 0; g < RG; ++g) {
-        double p1 = (double)f1[g], p2 = (double)f2[g];
-        for (int o = 16; o > 0; o >>= 1) {
-            p1 += __shfl_xor_sync(0xffffffffu, p1, o);
-            p2 += __shfl_xor_sync(0xffffffffu, p2, o);
-        }
-        if (l == 0) { sh[0][g][w] = p1; sh[1][g][w] = p2; }
+        sums[2 * g] = (double)f1[g];
+        sums[2 * g + 1] = (double)f2[g];
     }
-    __syncthreads();
+    block_sums<2 * RG>(sums, sh);
     if (threadIdx.x < m) {
         const int g = threadIdx.x;
-        double s1 = 0, s2 = 0;
-        for (int q = 0; q < nw; ++q) { s1 += sh[0][g][q]; s2 += sh[1][g][q]; }
-        const float g1 = (float)s1, g2 = (float)s2;
+        const float g1 = (float)sh[2 * g][0], g2 = (float)sh[2 * g + 1][0];
         a.pr[(long)p * a.ncand + c0 + g] = (g2 > 1.0e-10f) ? g1 / g2 * 180.0f / K.pi : 1000.0f;
     }
 }
@@ -575,12 +570,14 @@ __global__ void __launch_bounds__(512) k_pr_rescore_g(PrSingleArgs a, const int4
 // candidate loop, but a longer shared-memory dependency chain) 1.36x, the template taps
 // fetched one iteration ahead 1.12x (no gain: not latency-bound), 768 threads 1.07x, 512
 // threads 1.34x, branch-free items or two items per iteration 1.07x.
+// The sums at the end: 10 us of a block's 90 as a butterfly and a serial sum per candidate (FP64
+// pipe), 4 so (block_sums): 443 -> 418 us a launch of 760 groups.
 constexpr int RS_THREADS = 1024;
 __host__ __device__ inline int rescore_pitch(int W) { return W + ((3 - W % 16) + 16) % 16; }
 __global__ void __launch_bounds__(RS_THREADS, 1) k_pr_rescore_s(PrSingleArgs a, const int4* __restrict__ groups,
                                                                   Consts K) {
     extern __shared__ __align__(16) float rsm[];
-    __shared__ double sh[2][RG][RS_THREADS / 32];
+    __shared__ double sh[2 * RG][32];
     const Band bd = a.bd;
     const int W = bd.W, nr = bd.nr, minR = bd.min_r, nx = bd.nx, T = a.T;
     const int SP = rescore_pitch(W);
@@ -640,7 +637,6 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pr_rescore_s(PrSingleArgs a, 
         while (j >= 60) { j -= 60; ++i; }
     };
     const float2 nxh2 = make_float2(nxh, nxh);
-    const int wi = threadIdx.x >> 5, l = threadIdx.x & 31;
     // The group's candidate count M is a compile-time constant of each instance of the
     // loop, so the M candidates' terms of one template sample are independent chains that
     // the compiler interleaves; the two amplitude cuts are selects, not branches (with
@@ -697,15 +693,14 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pr_rescore_s(PrSingleArgs a, 
                 fs[g].y = ok ? nf.y : fs[g].y;
             }
         }
+        constexpr int N = M == 1 ? 2 : M == 2 ? 4 : 8;
+        double sums[N];
 #pragma unroll
-        for (int g = 0; g < M; ++g) {
-            double p1 = (double)fs[g].x, p2 = (double)fs[g].y;
-            for (int o = 16; o > 0; o >>= 1) {
-                p1 += __shfl_xor_sync(0xffffffffu, p1, o);
-                p2 += __shfl_xor_sync(0xffffffffu, p2, o);
-            }
-            if (l == 0) { sh[0][g][wi] = p1; sh[1][g][wi] = p2; }
+        for (int g = 0; g < N / 2; ++g) {
+            sums[2 * g] = g < M ? (double)fs[g < M ? g : 0].x : 0.0;
+            sums[2 * g + 1] = g < M ? (double)fs[g < M ? g : 0].y : 0.0;
         }
+        block_sums<N>(sums, sh);
     };
     switch (m) {
         case 1: run(std::integral_constant<int, 1>()); break;
@@ -713,12 +708,9 @@ __global__ void __launch_bounds__(RS_THREADS, 1) k_pr_rescore_s(PrSingleArgs a, 
         case 3: run(std::integral_constant<int, 3>()); break;
         default: run(std::integral_constant<int, RG>()); break;
     }
-    __syncthreads();
     if (threadIdx.x < m) {
         const int g = threadIdx.x;
-        double s1 = 0, s2 = 0;
-        for (int q = 0; q < RS_THREADS / 32; ++q) { s1 += sh[0][g][q]; s2 += sh[1][g][q]; }
-        const float g1 = (float)s1, g2 = (float)s2;
+        const float g1 = (float)sh[2 * g][0], g2 = (float)sh[2 * g + 1][0];
         a.pr[(long)p * a.ncand + c0 + g] = (g2 > 1.0e-10f) ? g1 / g2 * 180.0f / K.pi : 1000.0f;
     }
 }
@@ -736,7 +728,7 @@ __device__ __forceinline__ float2 shifted_pixel(const float2* band, int m, int W
 constexpr int RF_THREADS = 1024;
 __global__ void __launch_bounds__(RF_THREADS, 1) k_pr_refine(PrSingleArgs a, Consts K, double2* __restrict__ part) {
     extern __shared__ __align__(16) float rsm[];
-    __shared__ double sh[2][RF_THREADS / 32];
+    __shared__ double sh[2][32];
     __shared__ int snv;
     const Band bd = a.bd;
     const int W = bd.W, nr = bd.nr, minR = bd.min_r, nx = bd.nx;
@@ -813,18 +805,9 @@ __global__ void __launch_bounds__(RF_THREADS, 1) k_pr_refine(PrSingleArgs a, Con
         l += step_l;
         if (iq >= nr) { iq -= nr; ++l; }
     }
-    double p1 = (double)h1 + (double)l1, p2 = (double)h2 + (double)l2;
-    for (int o = 16; o > 0; o >>= 1) {
-        p1 += __shfl_xor_sync(0xffffffffu, p1, o);
-        p2 += __shfl_xor_sync(0xffffffffu, p2, o);
-    }
-    if (lane == 0) { sh[0][warp] = p1; sh[1][warp] = p2; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double s1 = 0, s2 = 0;
-        for (int q = 0; q < RF_THREADS / 32; ++q) { s1 += sh[0][q]; s2 += sh[1][q]; }
-        part[((long)p * a.ncand + c) * S + blockIdx.z] = make_double2(s1, s2);
-    }
+    double sums[2] = {(double)h1 + (double)l1, (double)h2 + (double)l2};
+    block_sums<2>(sums, sh);
+    if (threadIdx.x == 0) part[((long)p * a.ncand + c) * S + blockIdx.z] = make_double2(sh[0][0], sh[1][0]);
 }
 
 // The particle transform shifted to the origin its candidates share (cand[p][0][3..4]):
@@ -1191,7 +1174,7 @@ bool pr_rescore_shared_band(const Band& bd, int T) {
     const size_t sm = sizeof(float) * ((size_t)RG * T * 120 + (size_t)T * 120 + (size_t)(T + 1) * bd.nr) +
                       sizeof(int) * T * 60;
     const size_t sm_s = sm + sizeof(float2) * (size_t)bd.W * rescore_pitch(bd.W);
-    return sm_s + sizeof(double) * 2 * RG * (RS_THREADS / 32) <= 227 * 1024;
+    return sm_s + sizeof(double) * 2 * RG * 32 <= 227 * 1024;
 }
 
 cudaError_t launch_insert_plane0(const InsertArgs& a, int B, cudaStream_t st) {

@@ -313,7 +313,7 @@ struct Ctx {
     DBuf<short2> rpix;
     DBuf<int> rint;
     DBuf<double> rsum;
-    std::map<int, cufftHandle> plans;
+    std::map<int, cufftHandle> plans;  // of batches of images, by their size; -1: of the map (finish_volume)
     // reconstruction
     DBuf<float4> acc;
     // splats under one operator per coset of the grid's rotations (ops5), zero between calls,
@@ -323,6 +323,7 @@ struct Ctx {
     DBuf<float> ops5;
     DBuf<int2> samples;
     DBuf<float2> vol;
+    DBuf<float> fmap;  // the finished map, kept between maps as vol and the 3D plan are
     bool rec_active = false;
     int rec_kind = 0;  // REC_FULL, REC_SUBSTEP or REC_HALF
     int nsamples = 0, rec_used = 0, rec_img_id0 = -100;
@@ -429,7 +430,7 @@ struct Ctx {
         tfcut.release(); state.release(); cand.release(); rpr.release(); rot.release();
         prbuf.release(); fft.release(); band.release(); ralpha.release(); rpart.release(); best.release();
         rpix.release(); rint.release(); rsum.release();
-        flag.release(); sel.release(); acc.release(); acc5.release(); oct.release(); ops5.release(); samples.release(); vol.release();
+        flag.release(); sel.release(); acc.release(); acc5.release(); oct.release(); ops5.release(); samples.release(); vol.release(); fmap.release();
         mapcube.release(); mapreal.release(); csamples.release(); bmat.release(); amat.release(); corigins.release();
         topv.release(); kcc.release(); kcand.release(); topi.release(); gerr.release();
         kor.release(); korig.release(); pnorm.release(); kcc64.release(); pnorm0.release(); pctf.release();
@@ -2985,24 +2986,24 @@ int cryoim_prscore(void* ctx, const float* ft_a, const float* ft_b, const float*
 static int finish_volume(Ctx* c, int dir, bool merge_mask, bool avg, float* map) {
     const int nx = c->p.fftsize;
     const long n3 = (long)nx * nx * nx;
-    cufftHandle h;
-    CKF(cufftPlan3d(&h, nx, nx, nx, CUFFT_C2C));
-    cufftResult fr = cufftSetStream(h, c->stream);
-    if (fr == CUFFT_SUCCESS) fr = cufftExecC2C(h, (cufftComplex*)c->vol.p, (cufftComplex*)c->vol.p, dir);
-    if (fr != CUFFT_SUCCESS) {
-        cufftDestroy(h);
-        return fail(CRYOIM_ERR_CUDA, "3D FFT failed: cufft %d", (int)fr);
-    }
-    DBuf<float> dmap, davg;
     int r;
-    if ((r = dmap.ensure(n3)) || (avg && (r = davg.ensure(n3)))) { cufftDestroy(h); return r; }
+    if (!c->plans.count(-1)) {
+        cufftHandle h;
+        CKF(cufftPlan3d(&h, nx, nx, nx, CUFFT_C2C));
+        c->plans[-1] = h;
+        CKF(cufftSetStream(h, c->stream));
+    }
+    const cufftResult fr = cufftExecC2C(c->plans[-1], (cufftComplex*)c->vol.p, (cufftComplex*)c->vol.p, dir);
+    if (fr != CUFFT_SUCCESS) return fail(CRYOIM_ERR_CUDA, "3D FFT failed: cufft %d", (int)fr);
+    DBuf<float>& dmap = c->fmap;
+    DBuf<float> davg;
+    if ((r = dmap.ensure(n3)) || (avg && (r = davg.ensure(n3)))) return r;
     cudaError_t e = merge_mask ? launch_merge_real(c->vol.p, nx, c->p.imgmask_px, dmap.p, c->stream)
                                : (launch_rec_real(c->vol.p, nx, dmap.p, c->stream), cudaGetLastError());
     if (e == cudaSuccess && avg) e = launch_icosavg(dmap.p, nx, c->p.imgmask_px, c->ops.p, 60, davg.p, c->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(map, avg ? davg.p : dmap.p, sizeof(float) * n3, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    cufftDestroy(h);
     if (e != cudaSuccess) return fail(CRYOIM_ERR_CUDA, "map finish: %s", cudaGetErrorString(e));
     return CRYOIM_OK;
 }

@@ -6,10 +6,14 @@
 // reference's preprocessing to the last bit of its expression order.  Reductions the
 // reference does sequentially in FP32 are done here in FP64 (then rounded), which is
 // closer to the exact value than the reference and independent of thread order.
+#include <cooperative_groups.h>
+
+#include <algorithm>
 #include <cstdio>
 
 #include "geom.cuh"
 #include "kernels.h"
+#include "reduce.cuh"
 
 namespace cryoim {
 namespace {
@@ -20,25 +24,6 @@ struct HostAngles {
 HostAngles angles() {
     Angles a = host_angles();
     return HostAngles{a.pi, a.deg2rad, a.rad2deg};
-}
-
-__device__ double block_sum_d(double v, double* sh) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    __syncthreads();
-    if (l == 0) sh[w] = v;
-    __syncthreads();
-    int nw = (blockDim.x + 31) >> 5;
-    double r = 0;
-    if (threadIdx.x < 32) {
-        r = (l < nw) ? sh[l] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-        if (l == 0) sh[0] = r;
-    }
-    __syncthreads();
-    r = sh[0];
-    __syncthreads();
-    return r;
 }
 
 // ---------------------------------------------------------------------------
@@ -53,28 +38,66 @@ __device__ __forceinline__ void two_sum_acc(float& h, float& l, float x) {
     h = s2;
 }
 
-// One block of 1024 threads per image; warp w walks rows w, w + 32, ..., its lanes the
-// columns, so no pixel index is split by a division.  Issue-bound on its one SM: the distance to
-// the mask's centre decides most pixels by its square (the root only near the two radii).  The image sums the reference takes
+// The sum of the threads' values (and of their counts) over the blocks of a cluster, in the order of
+// the blocks, for every thread.
+struct ClusterSum {
+    double sh[1][32];
+    double sum;
+    int cnt, all_cnt;
+};
+__device__ double cluster_sum(double v, int cnt, ClusterSum* cs, int* count) {
+    auto cluster = cooperative_groups::this_cluster();
+    if (count) {
+        if (threadIdx.x == 0) cs->cnt = 0;
+        __syncthreads();
+        const int n = __reduce_add_sync(0xffffffffu, cnt);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&cs->cnt, n);
+    }
+    double d[1] = {v};
+    block_sums<1>(d, cs->sh);
+    cluster.sync();
+    if (threadIdx.x == 0) {
+        double s = 0;
+        int n = 0;
+        for (unsigned r = 0; r < cluster.num_blocks(); ++r) {
+            const ClusterSum* o = cluster.map_shared_rank(cs, r);
+            s += o->sh[0][0];
+            if (count) n += o->cnt;
+        }
+        cs->sum = s;
+        cs->all_cnt = n;
+    }
+    cluster.sync();  // the others have read this block's sums, this block its total
+    if (count) *count = cs->all_cnt;
+    return cs->sum;
+}
+
+// A cluster of up to eight blocks of 1024 threads per image (prep_cluster): the warps of all blocks
+// walk the rows in turn, their lanes the columns, so no pixel index is split by a division.  Bound:
+// issue and FP64 (a block has an SM to itself: 65 us for 64 images of 256^2 with a block an image, and
+// 18 us for one of 64^2; now 44 and 13).  The distance to the mask's centre decides most pixels by its
+// square (the root only near the two radii).  The image sums the reference takes
 // in FP64 are FP32 TwoSum pairs per thread (exact to far below FP32 rounding), combined
-// in FP64 across the block.
+// in FP64 across the cluster.
 __global__ void k_prep_images(const float* __restrict__ imgs, int nx,
                               const float* __restrict__ ox, const float* __restrict__ oy,
                               int use_mask, float mask, int normalize, float pi,
                               float2* __restrict__ out, int* flag) {
-    __shared__ double sh[32];
-    const int p = blockIdx.x;
+    __shared__ ClusterSum cs;
+    auto cluster = cooperative_groups::this_cluster();
+    const int p = blockIdx.x / cluster.num_blocks();
     const long nn = (long)nx * nx;
     const float* img = imgs + p * nn;
     float2* o = out + p * nn;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = cluster.block_rank() * (blockDim.x >> 5) + (threadIdx.x >> 5),
+              nw = cluster.num_blocks() * (blockDim.x >> 5);
     int bad = 0;
     float avg = 0.f, nd = 1.f;
     if (normalize) {
         float h = 0.f, l = 0.f;
         for (int iy = warp; iy < nx; iy += nw)
             for (int ix = lane; ix < nx; ix += 32) two_sum_acc(h, l, img[(long)iy * nx + ix]);
-        const double s = block_sum_d((double)h + (double)l, sh);
+        const double s = cluster_sum((double)h + (double)l, 0, &cs, nullptr);
         avg = (float)s / (float)nn;
         h = 0.f, l = 0.f;
         for (int iy = warp; iy < nx; iy += nw)
@@ -82,7 +105,7 @@ __global__ void k_prep_images(const float* __restrict__ imgs, int nx,
                 const float d = img[(long)iy * nx + ix] - avg;
                 two_sum_acc(h, l, __fmul_rn(d, d));  // the square rounded to FP32, as the reference
             }
-        const double s2 = block_sum_d((double)h + (double)l, sh);
+        const double s2 = cluster_sum((double)h + (double)l, 0, &cs, nullptr);
         nd = sqrtf((float)s2 / (float)nn);
     }
     const int hh = nx / 2;
@@ -112,9 +135,9 @@ __global__ void k_prep_images(const float* __restrict__ imgs, int nx,
                 }
             }
         }
-        summ = block_sum_d((double)h + (double)l, sh);
-        const double c = block_sum_d((double)cnt, sh);
-        if (c != 0.0) summ = summ / (double)(float)c;
+        int c;
+        summ = cluster_sum((double)h + (double)l, cnt, &cs, &c);
+        if (c != 0) summ = summ / (double)(float)c;
     }
     for (int iy = warp; iy < nx; iy += nw) {
         const float yy = (-y0 + (float)iy) * (-y0 + (float)iy);
@@ -663,8 +686,20 @@ inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 void launch_prep_images(const float* imgs, int B, int nx, const float* ox, const float* oy,
                         int use_mask, float mask_px, int normalize, float2* fft, int* flag,
                         cudaStream_t st) {
-    k_prep_images<<<B, 1024, 0, st>>>(imgs, nx, ox, oy, use_mask, mask_px, normalize, angles().pi,
-                                      fft, flag);
+    // blocks per image: as many as leave every block an SM of its own (one holds no second), and a
+    // row for half of the warps
+    int c = 1;
+    while (c < 8 && 2L * c * B <= 152 && 32 * c <= nx) c *= 2;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(B * c));
+    cfg.blockDim = dim3(1024);
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim = {(unsigned)c, 1, 1};
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_prep_images, imgs, nx, ox, oy, use_mask, mask_px, normalize, angles().pi, fft, flag);
 }
 
 void launch_post_fft(const float2* fft, int B, Band bd, const RingTable& rt, const float* sx, const float* sy,

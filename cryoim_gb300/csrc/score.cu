@@ -171,8 +171,9 @@ __device__ __forceinline__ OmegaTerm omega_sample(const float2* sband, int W, in
 // ms).  Cells by the add of 2^23 in place of conversions (which wait for the reciprocals'
 // quarter-rate pipe) gained nothing.
 constexpr float PAIR_MARGIN = 5.0e-4f;
-template <bool HALF>
-__global__ void __launch_bounds__(768, 1) k_pr_omega(PrOmegaArgs a, int nown, int G, Consts K) {
+// SHARE: blockIdx.z takes its share of the omegas (an instance of its own: the indices cost the other 2 %).
+template <bool HALF, bool SHARE>
+__global__ void __launch_bounds__(768, 1) k_pr_omega(PrOmegaArgs a, int nall, int Gall, Consts K) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const Band bd = a.bd;
     const int W = bd.W, nr = bd.nr, minR = bd.min_r;
@@ -188,8 +189,14 @@ __global__ void __launch_bounds__(768, 1) k_pr_omega(PrOmegaArgs a, int nown, in
     int* snv = sjl + 64;
 
     const int p = blockIdx.y, t = threadIdx.x;
-    // thread (g, k): group g's lines, omega k; no padding between groups (a warp may hold the end
-    // of one and the start of the next)
+    // this block's omegas: k0 .. k0 + nown - 1 of nall (and, HALF, those half a turn on)
+    const int share = SHARE ? (nall + (int)gridDim.z - 1) / (int)gridDim.z : nall;
+    const int k0 = SHARE ? (int)blockIdx.z * share : 0;
+    const int nown = SHARE ? min(share, nall - k0) : nall;
+    if (SHARE && nown < 1) return;  // uniform over the block
+    // thread (g, k): group g's lines, omega k0 + k; as many groups as fit the block, and no more than
+    // there are lines; no padding between groups (a warp may hold the end of one and the start of the next)
+    const int G = SHARE ? min(60, (int)blockDim.x / nown) : Gall;
     const int g = t / nown, k = t - g * nown;
     const bool own = g < G;
     {
@@ -202,7 +209,7 @@ __global__ void __launch_bounds__(768, 1) k_pr_omega(PrOmegaArgs a, int nown, in
     const int offW = bd.off * W + bd.off;
     const float* ctfp = a.ctf ? a.ctf + (long)p * W * W : nullptr;
     const float* tfc = a.tfcut + (long)p * a.tfcut_pstride;
-    const float womega = __fmul_rn(a.step, (float)k);
+    const float womega = __fmul_rn(a.step, (float)(SHARE ? k0 + k : k));
     const int nwarps = blockDim.x >> 5;
 
     for (int v = blockIdx.x; v < a.V; v += gridDim.x) {
@@ -280,7 +287,7 @@ for (int q0 = 0; q0 < nr; q0 += 32) {
                     }
                     if constexpr (HALF) {
                         if (near) {  // (about one radius of a lane's line in 30)
-                            const float w2 = __fmul_rn(a.step, (float)(k + nown));
+                            const float w2 = __fmul_rn(a.step, (float)(SHARE ? k0 + k + nall : k + nown));
                             float2 csn2;
                             sincosf(__fmul_rn(__fsub_rn(al1, w2), K.d2r), &csn2.y, &csn2.x);
                             do {
@@ -312,9 +319,10 @@ for (int q0 = 0; q0 < nr; q0 += 32) {
         if constexpr (HALF) sred[blockDim.x + t] = make_float2(qr1, qr2);
         __syncthreads();
         unsigned long long key = ~0ull;
-        // omega t (both halves: nown (HALF ? 2 : 1) of them)
-        for (int o = t; o < a.nomega; o += blockDim.x) {
-            const float2* sr = sred + (o >= nown ? blockDim.x + o - nown : o);
+        // the block's omegas, then those half a turn on
+        for (int q = t; q < (SHARE ? (HALF ? 2 : 1) * nown : a.nomega); q += blockDim.x) {
+            const int o = SHARE ? (q >= nown ? k0 + q - nown + nall : k0 + q) : q;
+            const float2* sr = sred + (q >= nown ? blockDim.x + q - nown : q);
             float s1 = 0.f, s2 = 0.f;
             for (int gg = 0; gg < G; ++gg) {
                 s1 += sr[gg * nown].x;
@@ -1072,11 +1080,22 @@ cudaError_t launch_pr_omega(const PrOmegaArgs& a, int B, cudaStream_t st) {
     int sm = pr_omega_smem_bytes(a.bd, a.nomega, a.step, &nt, &G);
     if (sm < 0) return cudaErrorInvalidValue;
     const bool half = omega_half(a.nomega, a.step);
-    auto kern = half ? k_pr_omega<true> : k_pr_omega<false>;
+    // A block has an SM to itself: where a block a view and particle leave SMs idle, several share a view's omegas
+    // (each repeats the template's samples: 47 views of 90 omegas, one particle, 4 templates, box 64, 78 us by 47
+    // blocks, 51 by 94)
+    const int nall = half ? a.nomega / 2 : a.nomega;
+    auto rounds = [&](int zz) {  // of a template's 60 lines over the block's groups
+        const int Gz = std::min(60, nt / ((nall + zz - 1) / zz));
+        return (60 + Gz - 1) / Gz;
+    };
+    int z = 1;
+    for (int zz = 2; zz <= 8 && (long)a.V * B * zz <= 152; ++zz)
+        if (rounds(zz) < rounds(z)) z = zz;
+    auto kern = z > 1 ? (half ? k_pr_omega<true, true> : k_pr_omega<false, true>)
+                      : (half ? k_pr_omega<true, false> : k_pr_omega<false, false>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e != cudaSuccess) return e;
-    dim3 grid(a.V, B);
-    kern<<<grid, nt, sm, st>>>(a, half ? a.nomega / 2 : a.nomega, G, consts());
+    kern<<<dim3(a.V, B, z), nt, sm, st>>>(a, nall, G, consts());
     return cudaGetLastError();
 }
 

@@ -374,7 +374,7 @@ void launch_lp_head_grad(const float* g, const float* T, const float* dsc, int B
 void launch_lp_loss(const float* sc, int B, int V, const float* vview, const float* truth, float sv, float ss,
                     float* dsc, float* loss, cudaStream_t st);
 void launch_lp_adam(float* w, const float* g, float* m, float* v, long n, float lr, int step, cudaStream_t st);
-// sc is overwritten (taken cells set to -inf)
+// sc may be overwritten (taken cells set to -inf)
 void launch_lp_topk(float* sc, int B, int V, int k, int* cell, float* val, cudaStream_t st);
 
 // dst row r = src row idx[r] (row_bytes a multiple of 16), n rows

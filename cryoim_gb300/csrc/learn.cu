@@ -894,37 +894,64 @@ __global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float
     }
 }
 
-// The k best cells of each particle's V x NT scores (repeated block argmax; sc is
-// scratch: taken cells are set to -inf).
+// The k best cells of each particle's V x NT scores, ties to the first: each thread keeps the best
+// of its cells (tid, tid + blockDim, ...), a round picks the best of the threads', and only its
+// thread looks through its cells again.  SHARED: the scores in shared memory (else sc is scratch:
+// taken cells are set to -inf).  64 particles of 22,272 cells, 24 cells each: 75 us with every
+// thread reading all of its cells from L2 each round, now 45.
+template <bool SHARED>
 __global__ void __launch_bounds__(512) k_topk_cells(float* __restrict__ sc, long n, int k, int* __restrict__ cell,
                                                    float* __restrict__ val) {
+    extern __shared__ float srow[];
     __shared__ float sv[32];
-    __shared__ long si[32];
+    __shared__ long si[32], pi;
     const int b = blockIdx.x;
     float* x = sc + (long)b * n;
+    if (SHARED) {
+        for (long q = threadIdx.x; q < n; q += blockDim.x) srow[q] = x[q];  // a thread reads its own cells alone
+        x = srow;
+    }
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int r = 0; r < k; ++r) {
-        float bv = -3.0e38f;
-        long bi = -1;
-        for (long q = threadIdx.x; q < n; q += blockDim.x)
-            if (x[q] > bv) { bv = x[q]; bi = q; }
+    float bv;
+    long bi;
+    auto scan = [&]() {
+        bv = -3.0e38f;
+        bi = -1;
+#pragma unroll 8
+        for (long q = threadIdx.x; q < n; q += blockDim.x) {
+            const float v = x[q];
+            if (v > bv) { bv = v; bi = q; }
+        }
+    };
+    auto best = [&](float& v, long& i) {  // of the warp
         for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const long oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ov > bv || (ov == bv && oi >= 0 && (bi < 0 || oi < bi))) { bv = ov; bi = oi; }
+            const float ov = __shfl_xor_sync(0xffffffffu, v, o);
+            const long oi = __shfl_xor_sync(0xffffffffu, i, o);
+            if (ov > v || (ov == v && oi >= 0 && (i < 0 || oi < i))) { v = ov; i = oi; }
         }
-        if (l == 0) { sv[w] = bv; si[w] = bi; }
+    };
+    scan();
+    for (int r = 0; r < k; ++r) {
+        float v = bv;
+        long i = bi;
+        best(v, i);
+        if (l == 0) { sv[w] = v; si[w] = i; }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            float v0 = sv[0];
-            long i0 = si[0];
-            for (int q = 1; q < nw; ++q)
-                if (sv[q] > v0 || (sv[q] == v0 && si[q] >= 0 && (i0 < 0 || si[q] < i0))) { v0 = sv[q]; i0 = si[q]; }
-            cell[b * k + r] = (int)i0;
-            val[b * k + r] = v0;
-            if (i0 >= 0) x[i0] = -3.0e38f;
+        if (w == 0) {
+            v = l < nw ? sv[l] : -3.0e38f;
+            i = l < nw ? si[l] : -1;
+            best(v, i);
+            if (l == 0) {
+                cell[b * k + r] = (int)i;
+                val[b * k + r] = v;
+                pi = i;
+            }
         }
         __syncthreads();
+        if (pi >= 0 && pi == bi) {
+            x[bi] = -3.0e38f;
+            scan();
+        }
     }
 }
 
@@ -1043,7 +1070,13 @@ void launch_lp_adam(float* w, const float* g, float* m, float* v, long n, float 
     k_adam<<<grid_for(n, 256), 256, 0, st>>>(w, g, m, v, n, lr, b1, b2, 1.0e-8f, c1, c2);
 }
 void launch_lp_topk(float* sc, int B, int V, int k, int* cell, float* val, cudaStream_t st) {
-    k_topk_cells<<<B, 512, 0, st>>>(sc, (long)V * NT, k, cell, val);
+    const long n = (long)V * NT;
+    const size_t sm = sizeof(float) * (size_t)n;
+    if (sm <= 200 * 1024 &&
+        cudaFuncSetAttribute(k_topk_cells<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) == cudaSuccess)
+        k_topk_cells<true><<<B, 512, sm, st>>>(sc, n, k, cell, val);
+    else
+        k_topk_cells<false><<<B, 512, 0, st>>>(sc, n, k, cell, val);
 }
 
 }  // namespace cryoim

@@ -932,19 +932,22 @@ __global__ void __launch_bounds__(256) k_insert(InsertArgs a) {
     splat<false>(a, p, k, a.samples[s]);
 }
 
-// One block per (operator, particle), a thread per row ky of samples in turn: the stretch of
+// One block per (operator, particle), P0_LANES threads per row ky of samples in turn: the stretch of
 // hx whose rotated z, by the product of the two rotations, is within 1 (and a margin over the
-// rounding the two differ by) is splatted.  Bound by the reductions that meet on the cells around
-// the origin: under all 60 operators 81 us a 64-particle batch at maxR 64, under one of each of
-// the fifteen cosets of the half turns about the axes 42 us.
-__global__ void __launch_bounds__(160) k_insert_plane0(InsertArgs a) {
+// rounding the two differ by) is splatted.  Bound by the longest rows, along the plane, and the
+// reductions that meet on the cells around the origin: under all 60 operators 81 us a 64-particle
+// batch at maxR 64, under one of each of the fifteen cosets of the half turns about the axes 42 us
+// by a thread a row, 19 by eight.
+constexpr int P0_THREADS = 256, P0_LANES = 8;  // threads of a block, of a row
+__global__ void __launch_bounds__(P0_THREADS) k_insert_plane0(InsertArgs a) {
     const int k = blockIdx.x, p = blockIdx.y;
     if (!a.sel[p]) return;
     const float* op = a.ops + k * 9 + 6;
     const float* rot = a.rot + p * 9;
     const float zx = op[0] * rot[0] + op[1] * rot[3] + op[2] * rot[6];
     const float zy = op[0] * rot[1] + op[1] * rot[4] + op[2] * rot[7];
-    for (int r = threadIdx.x; r < 2 * a.lim + 1; r += blockDim.x) {
+    const int l = threadIdx.x % P0_LANES;
+    for (int r = threadIdx.x / P0_LANES; r < 2 * a.lim + 1; r += P0_THREADS / P0_LANES) {
         const int ky = r - a.lim;
         int hmax = (int)sqrtf((float)(a.lim * a.lim - ky * ky));  // samples hx^2 + ky^2 <= lim^2
         while (hmax * hmax + ky * ky > a.lim * a.lim) --hmax;
@@ -958,7 +961,7 @@ __global__ void __launch_bounds__(160) k_insert_plane0(InsertArgs a) {
         } else if (fabsf(z0) > 1.02f) {
             continue;
         }
-        for (int hx = h0; hx <= h1; ++hx) splat<true>(a, p, k, make_int2(hx, ky));
+        for (int hx = h0 + l; hx <= h1; hx += P0_LANES) splat<true>(a, p, k, make_int2(hx, ky));
     }
 }
 
@@ -1203,7 +1206,7 @@ bool pr_rescore_shared_band(const Band& bd, int T) {
 }
 
 cudaError_t launch_insert_plane0(const InsertArgs& a, int B, cudaStream_t st) {
-    k_insert_plane0<<<dim3(a.nsym, B), 160, 0, st>>>(a);
+    k_insert_plane0<<<dim3(a.nsym, B), P0_THREADS, 0, st>>>(a);
     return cudaGetLastError();
 }
 

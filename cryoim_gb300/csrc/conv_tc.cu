@@ -141,7 +141,7 @@ constexpr int conv_fwd_smem() {
 // channel, rows written in full and pooled by a pass of its own) took, for a batch of 256
 // samples, 184, 274, 149 and 85 us at layers 1 to 4 and 102 us of pooling; this one takes 89, 142, 94
 // and 53 us.  Data gradients of layers 4 to 2: 82, 141 and 191 us and 205 us for the gates and
-// the pooling; now 58, 102 and 189 us.
+// the pooling; now 55, 95 and 174 us.
 template <int CINP, int COUT, int MODE>
 __global__ void __launch_bounds__(CT_THREADS, 1) k_conv3_tc(ConvTcArgs a) {
     constexpr int N = 3 * COUT;                     // product columns (dt, co)
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_conv3_tc(ConvTcArgs a) {
             const int r1 = min(j + 1, S - 1);  // a row beyond the sample is gated off
 #pragma unroll
             for (int c = 0; c < CN; ++c) {
-                pre[0][c] = fresh ? __ldg(src + c * cs + j * CT_NT) : pre[1][c];
+                pre[0][c] = fresh ? tf32r(0.5f * __ldg(src + c * cs + j * CT_NT)) : pre[1][c];
                 pre[1][c] = __ldg(src + c * cs + r1 * CT_NT);
             }
             const unsigned char* g = a.gate_in + (((long)b * H + 2 * j) * CT_NT + t) * 4 + grp;
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_conv3_tc(ConvTcArgs a) {
             for (int e = 0; e < 4; ++e) {
                 const int c = 4 * k4 + e;
                 if constexpr (MODE == CONV_BACK)
-                    x[e] = (gate >> c) & 1u ? tf32r(0.5f * v[c]) : 0.f;
+                    x[e] = (gate >> c) & 1u ? v[c] : 0.f;
                 else
                     x[e] = tf32r(v[c]);
             }
@@ -239,9 +239,17 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_conv3_tc(ConvTcArgs a) {
         }
     };
     const float none[CN] = {};
+    // CONV_BACK: pooled row j + 1, as loaded, halved and rounded once for its two rows (pre[0] is so already)
+    auto halve = [&]() {
+        if constexpr (MODE == CONV_BACK) {
+#pragma unroll
+            for (int c = 0; c < CN; ++c) pre[1][c] = tf32r(0.5f * pre[1][c]);
+        }
+    };
     // lo, hi: ring pairs of the step's stages j and j + 1
     auto put = [&](int lo, int hi, bool fresh) {
         if (!stages) return;
+        halve();
         if (fresh) {
             put_row(2 * lo, none, 0u);
             if constexpr (MODE == CONV_BACK)
@@ -267,6 +275,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_conv3_tc(ConvTcArgs a) {
         // a block that starts inside a sample: rows 2j - 1 and 2j
         if constexpr (MODE == CONV_BACK) {
             load(b, j - 1, true);
+            halve();
             put_row(2 * lo, pre[0], gb[1]);
             put_row(2 * lo + 1, pre[1], gb[2]);
         } else {

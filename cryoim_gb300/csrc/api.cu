@@ -2178,9 +2178,9 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
                         q.topv_off = (int)toff;
                         q.c_off = poffs;
                         seg[i - i0] = make_int2((int)toff, ntp);
+                        up_tiles = std::max(up_tiles, ntp);
                         if (!local) {
                             ug[i - i0] = UpGroup{poffs, (nl + tn - 1) / tn, (int)moff, np, (int)toff, ntp};
-                            up_tiles = std::max(up_tiles, ntp);
                             poffs += prod_of(i);
                             moff += np;
                         }
@@ -2203,8 +2203,9 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
                     }
                     CK(cudaMemcpyAsync(L->gseg.p, seg.data(), sizeof(int2) * seg.size(), cudaMemcpyHostToDevice,
                                        L->stream));
-                    launch_select_distinct(L->topv.p, L->topi.p, O, L->gseg.p, i1 - i0, k, L->kor.p + (size_t)i0 * k,
-                                           L->korig.p + (size_t)i0 * k, L->kcc.p + (size_t)i0 * k, L->stream);
+                    launch_select_distinct(L->topv.p, L->topi.p, O, L->gseg.p, i1 - i0, up_tiles, k,
+                                           L->kor.p + (size_t)i0 * k, L->korig.p + (size_t)i0 * k,
+                                           L->kcc.p + (size_t)i0 * k, L->stream);
                     CK(cudaGetLastError());
                     // the cut-section buffer, the products and the row lists are reused by the next group
                     if (i1 < nb) CK(cudaStreamSynchronize(L->stream));

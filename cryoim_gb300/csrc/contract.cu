@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "geom.cuh"
@@ -574,11 +575,12 @@ template <int LY> struct UpCoef {
     }
 };
 template <int LY, class Emit>
-__device__ __forceinline__ void up_eval(const OriginDev& ob, const UpCoef<LY>& cf, const float* sm, Emit emit) {
+__device__ __forceinline__ void up_eval(const OriginDev& ob, const UpCoef<LY>& cf, const float* sm, Emit emit,
+                                        int jy0 = 0, int jy1 = 0x7fffffff) {
     constexpr int H = UpCoef<LY>::H;
     const int hn = (ob.n1 + 1) / 2;
     const float2* q2 = reinterpret_cast<const float2*>(sm);
-    for (int jy = 0; jy < hn; ++jy) {
+    for (int jy = jy0; jy < min(hn, jy1); ++jy) {
         float2 qy[H];
 #pragma unroll
         for (int k = 0; k < H; ++k) qy[k] = q2[jy * H + k];
@@ -808,7 +810,8 @@ __global__ void __launch_bounds__(128) k_up_origin(OriginDev ob, const float* __
 // else one warp works on the output itself); the maximum of 32 lanes by redux on the
 // order-preserving integer image of the value, up to 16 origins at a time so that their
 // latencies overlap (one origin at a time, with its update in between: 185 us a 64-particle
-// pass of the box-256 search; so: 137 us).
+// pass of the box-256 search; so: 137 us).  gridDim.z blocks share a tile's origins by rows (pairs of
+// y about the middle) where a call has few tiles: one particle's three, 625 origins, 60 -> 23 us.
 template <int LY>
 __global__ void __launch_bounds__(256, 1) k_up_list(OriginDev ob, const float* __restrict__ C, int parts,
                                                     const UpGroup* __restrict__ groups, const int* __restrict__ map,
@@ -831,6 +834,8 @@ __global__ void __launch_bounds__(256, 1) k_up_list(OriginDev ob, const float* _
         si = oi;
         stride = g.ntiles;
     }
+    const int hn = (ob.n1 + 1) / 2;
+    const int jy0 = hn * (int)blockIdx.z / (int)gridDim.z, jy1 = hn * ((int)blockIdx.z + 1) / (int)gridDim.z;
     if constexpr (LY >= 0) up_table<LY>(ob, smem);
     for (int o = lane; o < O; o += 32) { sv[o * stride] = -3.0e38f; si[o * stride] = -1; }
     __syncthreads();
@@ -883,7 +888,7 @@ __global__ void __launch_bounds__(256, 1) k_up_list(OriginDev ob, const float* _
                 const float u = __ldg(U + i * pitch);
                 return V ? fmaf(sgn, __ldg(V + i * pitch), u) : u;
             });
-            up_eval<LY>(ob, c, smem, emit);
+            up_eval<LY>(ob, c, smem, emit, jy0, jy1);
         } else {
             up_eval_gen(ob, U, V, sgn, pitch, emit);
         }
@@ -894,6 +899,8 @@ __global__ void __launch_bounds__(256, 1) k_up_list(OriginDev ob, const float* _
     sv = smem + up_table_floats<LY>(ob.n1);
     si = reinterpret_cast<int*>(sv + nw * O);
     for (int o = threadIdx.x; o < O; o += blockDim.x) {
+        const int y = o / ob.n1, jy = y >= ob.n1 / 2 ? y - ob.n1 / 2 : (ob.n1 - 1) / 2 - y;
+        if (jy < jy0 || jy >= jy1) continue;
         float bv = -3.0e38f;
         int bi = -1;
         for (int w = 0; w < nw; ++w) {
@@ -906,45 +913,62 @@ __global__ void __launch_bounds__(256, 1) k_up_list(OriginDev ob, const float* _
     }
 }
 
-// Per particle: the k best entries of cnt (value, orientation) pairs, by
-// repeated block argmax (selected values are set to -inf in v, a scratch array).
-__global__ void k_select_topk(float* __restrict__ v, const int* __restrict__ orient, int cnt_per_particle, int k,
-                              int* __restrict__ out_orient, float* __restrict__ out_cc) {
-    __shared__ float sv[32];
-    __shared__ long si[32];
-    const int p = blockIdx.x;
-    const long base = (long)p * cnt_per_particle, cnt = cnt_per_particle;
-    float* topv = v;
-    for (int r = 0; r < k; ++r) {
-        float bv = -3.0e38f;
-        long bi = -1;
-        for (long q = threadIdx.x; q < cnt; q += blockDim.x) {
-            float v = topv[base + q];
-            if (v > bv) { bv = v; bi = q; }
-        }
+// The larger (value, index) of a block's threads, the first of equal values, for every thread; index
+// -1: none.  sv, si: 32 each and a place for the result.
+__device__ __forceinline__ void block_best(float& v, int& i, float* sv, int* si) {
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
+    auto warp = [&]() {
         for (int off = 16; off > 0; off >>= 1) {
-            float ov = __shfl_xor_sync(0xffffffffu, bv, off);
-            long oi = __shfl_xor_sync(0xffffffffu, bi, off);
-            if (ov > bv || (ov == bv && oi < bi && oi >= 0)) { bv = ov; bi = oi; }
+            const float ov = __shfl_xor_sync(0xffffffffu, v, off);
+            const int oi = __shfl_xor_sync(0xffffffffu, i, off);
+            if (ov > v || (ov == v && oi >= 0 && (i < 0 || oi < i))) { v = ov; i = oi; }
         }
-        const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-        if (l == 0) { sv[w] = bv; si[w] = bi; }
-        __syncthreads();
+    };
+    warp();
+    if (l == 0) { sv[w] = v; si[w] = i; }
+    __syncthreads();
+    if (w == 0) {
+        v = l < nw ? sv[l] : -3.0e38f;
+        i = l < nw ? si[l] : -1;
+        warp();
+        if (l == 0) { sv[32] = v; si[32] = i; }
+    }
+    __syncthreads();
+    v = sv[32];
+    i = si[32];
+}
+
+// Per particle: the k best entries of cnt (value, orientation) pairs; a thread keeps the best of its
+// entries and looks through them again (taken ones set to -inf in v, a scratch array) once one is taken.
+__global__ void k_select_topk(float* __restrict__ v, const int* __restrict__ orient, int cnt, int k,
+                              int* __restrict__ out_orient, float* __restrict__ out_cc) {
+    __shared__ float sv[33];
+    __shared__ int si[33];
+    const int p = blockIdx.x;
+    const long base = (long)p * cnt;
+    float bv;
+    int bi;
+    auto scan = [&]() {
+        bv = -3.0e38f;
+        bi = -1;
+        for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
+            const float x = v[base + q];
+            if (x > bv) { bv = x; bi = q; }
+        }
+    };
+    scan();
+    for (int r = 0; r < k; ++r) {
+        float x = bv;
+        int i = bi;
+        block_best(x, i, sv, si);
         if (threadIdx.x == 0) {
-            float v0 = sv[0];
-            long i0 = si[0];
-            for (int q = 1; q < nw; ++q)
-                if (sv[q] > v0 || (sv[q] == v0 && si[q] < i0 && si[q] >= 0)) { v0 = sv[q]; i0 = si[q]; }
-            if (i0 >= 0 && v0 > -3.0e38f) {
-                out_orient[p * k + r] = orient[base + i0];
-                out_cc[p * k + r] = v0;
-                topv[base + i0] = -3.0e38f;
-            } else {
-                out_orient[p * k + r] = -1;
-                out_cc[p * k + r] = -3.0e38f;
-            }
+            out_orient[p * k + r] = i >= 0 ? orient[base + i] : -1;
+            out_cc[p * k + r] = i >= 0 ? x : -3.0e38f;
         }
-        __syncthreads();
+        if (i >= 0 && i == bi) {
+            v[base + i] = -3.0e38f;
+            scan();
+        }
     }
 }
 
@@ -953,13 +977,19 @@ __global__ void k_select_topk(float* __restrict__ v, const int* __restrict__ ori
 // col[...] its column in the gathered list; once a column is taken, every entry that
 // names it is retired, so the candidates are k distinct orientations, each at its best
 // origin.  Columns are remapped to orientations on the host.
-// One block per particle of a group: seg[b] = (offset of its entries, its ntiles).
-__global__ void k_select_distinct(float* __restrict__ v0, const int* __restrict__ col0, int O,
-                                  const int2* __restrict__ seg, int k, int* __restrict__ out_col0,
-                                  int* __restrict__ out_origin0, float* __restrict__ out_cc0) {
-    __shared__ float sv[32];
-    __shared__ int si[32];
-    __shared__ int taken;
+// One block per particle of a group: seg[b] = (offset of its entries, its ntiles).  SHARED: the
+// entries in shared memory (else v is scratch: retired entries are set to -inf).  Retiring a column
+// and finding a thread's next best is one pass over its entries.  One particle of 1,875 entries, 16
+// of them: 28 us with two passes over global memory and a serial comparison of the warps' bests a
+// round, now 23; the 17,918 entries of each of 24 local grids 95, now 78.
+template <bool SHARED>
+__global__ void __launch_bounds__(512) k_select_distinct(float* __restrict__ v0, const int* __restrict__ col0, int O,
+                                                        const int2* __restrict__ seg, int k,
+                                                        int* __restrict__ out_col0, int* __restrict__ out_origin0,
+                                                        float* __restrict__ out_cc0) {
+    extern __shared__ float sent[];  // values, then columns
+    __shared__ float sv[33];
+    __shared__ int si[33];
     const int2 sg = seg[blockIdx.x];
     const int ntiles = sg.y, cnt = O * ntiles;
     float* v = v0 + sg.x;
@@ -967,44 +997,35 @@ __global__ void k_select_distinct(float* __restrict__ v0, const int* __restrict_
     int* out_col = out_col0 + (long)blockIdx.x * k;
     int* out_origin = out_origin0 + (long)blockIdx.x * k;
     float* out_cc = out_cc0 + (long)blockIdx.x * k;
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+    if (SHARED) {  // a thread reads its own entries alone
+        int* sc = reinterpret_cast<int*>(sent + cnt);
+        for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
+            sent[q] = v[q];
+            sc[q] = col[q];
+        }
+        v = sent;
+        col = sc;
+    }
+    int taken = -1;
     for (int r = 0; r < k; ++r) {
         float bv = -3.0e38f;
         int bi = -1;
+#pragma unroll 4
         for (int q = threadIdx.x; q < cnt; q += blockDim.x) {
+            const int c = col[q];
             const float x = v[q];
-            if (col[q] >= 0 && x > bv) { bv = x; bi = q; }
+            if (c < 0) continue;
+            if (c == taken) v[q] = -3.0e38f;
+            else if (x > bv) { bv = x; bi = q; }
         }
-        for (int off = 16; off > 0; off >>= 1) {
-            float ov = __shfl_xor_sync(0xffffffffu, bv, off);
-            int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-            if (ov > bv || (ov == bv && oi >= 0 && (bi < 0 || oi < bi))) { bv = ov; bi = oi; }
-        }
-        if (l == 0) { sv[w] = bv; si[w] = bi; }
-        __syncthreads();
+        block_best(bv, bi, sv, si);
+        taken = -1;
+        if (bi >= 0) taken = SHARED ? reinterpret_cast<const int*>(sent + cnt)[bi] : col[bi];
         if (threadIdx.x == 0) {
-            float v0 = sv[0];
-            int i0 = si[0];
-            for (int q = 1; q < nw; ++q)
-                if (sv[q] > v0 || (sv[q] == v0 && si[q] >= 0 && (i0 < 0 || si[q] < i0))) { v0 = sv[q]; i0 = si[q]; }
-            if (i0 >= 0 && v0 > -3.0e38f) {
-                out_col[r] = col[i0];
-                out_origin[r] = i0 / ntiles;
-                out_cc[r] = v0;
-                taken = col[i0];
-            } else {
-                out_col[r] = -1;
-                out_origin[r] = 0;
-                out_cc[r] = -3.0e38f;
-                taken = -1;
-            }
+            out_col[r] = taken;
+            out_origin[r] = bi >= 0 ? bi / ntiles : 0;
+            out_cc[r] = bi >= 0 ? bv : -3.0e38f;
         }
-        __syncthreads();
-        const int t = taken;
-        if (t >= 0)
-            for (int q = threadIdx.x; q < cnt; q += blockDim.x)
-                if (col[q] == t) v[q] = -3.0e38f;
-        __syncthreads();
     }
 }
 
@@ -1310,7 +1331,12 @@ cudaError_t launch_up_list(const OriginDev& ob, const float* C, int parts, const
                 : ly == 3 ? k_up_list<3> : k_up_list<4>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    kern<<<dim3(max_tiles, ngroups), 32 * nw, sm, st>>>(ob, C, parts, groups, map, topv, topi, shm ? 1 : 0);
+    // blocks to a tile: as many as find an SM of their own (each reads its tile's products again, so that with
+    // the SMs filled, by this launch or by other lanes', the pass takes longer: 14.0 -> 14.5 ms of the box-256
+    // search with 192 tiles cut in three)
+    int z = 1;
+    if (shm && ly >= 0) z = std::max(1, std::min(std::min(8, (ob.n1 + 1) / 2), 152 / std::max(1, max_tiles * ngroups)));
+    kern<<<dim3(max_tiles, ngroups, z), 32 * nw, sm, st>>>(ob, C, parts, groups, map, topv, topi, shm ? 1 : 0);
     return cudaGetLastError();
 }
 
@@ -1423,9 +1449,15 @@ void launch_build_a(const float2* band, const float* ctf, Band bd, const int2* s
                                    (__nv_bfloat162*)A);
 }
 
-void launch_select_distinct(float* topv, const int* topi, int O, const int2* seg, int B, int k, int* col,
+void launch_select_distinct(float* topv, const int* topi, int O, const int2* seg, int B, int max_tiles, int k, int* col,
                             int* origin, float* cc, cudaStream_t st) {
-    k_select_distinct<<<B, 512, 0, st>>>(topv, topi, O, seg, k, col, origin, cc);
+    const size_t sm = (size_t)O * max_tiles * (sizeof(float) + sizeof(int));
+    if (sm <= 48 * 1024 ||
+        (sm <= 200 * 1024 && cudaFuncSetAttribute(k_select_distinct<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  (int)sm) == cudaSuccess))
+        k_select_distinct<true><<<B, 512, sm, st>>>(topv, topi, O, seg, k, col, origin, cc);
+    else
+        k_select_distinct<false><<<B, 512, 0, st>>>(topv, topi, O, seg, k, col, origin, cc);
 }
 
 long cc_fp64_scratch(int k, int B) { return (long)k * B * CC_SPLIT * 3; }

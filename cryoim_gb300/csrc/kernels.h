@@ -380,7 +380,7 @@ void launch_lp_topk(float* sc, int B, int V, int k, int* cell, float* val, cudaS
 // dst row r = src row idx[r] (row_bytes a multiple of 16), n rows
 // per particle b of B: the k best of its O x seg[b].y (value, column) entries at
 // topv/topi + seg[b].x with distinct columns -> col, origin, cc [B][k]
-void launch_select_distinct(float* topv, const int* topi, int O, const int2* seg, int B, int k, int* col,
+void launch_select_distinct(float* topv, const int* topi, int O, const int2* seg, int B, int max_tiles, int k, int* col,
                             int* origin, float* cc, cudaStream_t st);
 // FP8-e4m3 operands (contract.cu): per-band max |B| (R+1 bands, float bits) over every
 // stride-th row; B8 = e4m3(B x mulB) with KH8 bytes per part of a row.

@@ -55,41 +55,43 @@ FP32_PEAK_TFLOPS_NOMINAL = 152 * 128 * 2 * 2.07e9 / 1e12  # FMA lanes x 2 flop x
 FLOPS_PER_TERM = 30.0
 # this library's kernels launched per 64-particle pass of the headline form (ncu launch
 # list, cuFFT's own kernels not counted): prep, FFT post-processing, CTF, template cuts,
-# templates x CTF, particle norms, features, 4 convolutions, 3 poolings, mix, head (2
-# forward real transforms, the product, 1 inverse), cell top-k, operand A, grouped
-# contraction, distinct selection, and two rounds (candidates, neighbours of the best
-# four) of band shift and phase residual (the line angles come from the grid's view
-# table, built once per template set; the FP64 correlation is not computed for a
-# phase-residual pick without candidate output)
-LAUNCHES_PER_PASS = 27
-# DRAM bytes (read + write) of one GEMM launch (3 particles x 625 origins) from an ncu
-# capture at the 2-degree grid (1.483 GB for 31,320 orientations), scaled to the
-# orientation count: operand B streams once per launch.
-GEMM_TRAFFIC_PER_ORIENT = 1.483e9 / 31320
+# particle norms, operand A (the origin grid's basis), features, 4 convolutions with their
+# poolings, mix, head (2 forward real transforms, the product, 1 inverse), cell top-k,
+# grouped contraction, its expansion to all origins, distinct selection, templates x CTF,
+# and two rounds (candidates, neighbours of the best four) of band shift and phase residual
+# (the line angles come from the grid's view table, built once per template set; the FP64
+# correlation is not computed for a phase-residual pick without candidate output)
+LAUNCHES_PER_PASS = 25
+# DRAM bytes (read + write) of one exhaustive contraction launch (12 particles x 160 basis
+# rows against 15,660 bank rows, a section for two omegas) from an ncu capture at the
+# 2-degree grid, scaled to the orientation count: operand B streams, the products are written.
+GEMM_TRAFFIC_PER_ORIENT = (905.505536e6 + 226.131456e6) / 31320
 LANES = 6  # pass lanes of the contraction search (the library's default)
 # the L2's peak rate of float4 reductions (one sector per cycle per slice): ncu's
-# lts__t_sectors_srcunit_tex_op_red at 56.5 % of peak sustained = 2.136e11 / s in the
-# k_insert capture of profiles/k_insert_box256.md
+# lts__t_sectors_srcunit_tex_op_red at 56.5 % of peak sustained = 2.136e11 / s in a capture of
+# k_insert (profiles/k_insert_box256.md)
 L2_RED_PEAK = 3.779e11
-# sm__pipe_tensor_cycles_active of the FP8 contraction (profiles/k_gemm_argmax_e4m3_box256.md)
-TENSOR_PIPE_ACTIVE_E4M3 = 0.781
+# sm__pipe_tensor_cycles_active of the FP8 contraction (--profile-case exhaustive-fp8; it counts e4m3
+# and bf16 alike: the BF16 contraction at 0.97 of the measured rate reads 0.72 there)
+TENSOR_PIPE_ACTIVE_E4M3 = 0.679
 # dram__bytes_read.sum + dram__bytes_write.sum of one grouped fine-contraction launch over
 # a 64-particle pass of the box-256 workload (ncu capture of --profile-case learned: rows
-# copied from the section bank by index, +-1-step proposal neighbourhoods)
-GROUPED_GEMM_TRAFFIC_PER_PASS = 1.783445e9 + 4.284416e6
-# the same for the phase-residual rescoring (mean of the two launches of a pass,
-# profiles/k_pr_rescore_s_box256.md)
-RESCORE_TRAFFIC_PER_LAUNCH = 0.5 * (585.458432e6 + 3.246592e6 + 769.335296e6 + 3.527936e6)
+# copied from the section bank by index, +-1-step proposal neighbourhoods of 24 cells)
+GROUPED_GEMM_TRAFFIC_PER_PASS = 682.209536e6 + 28.097792e6
+# rows of operand A a particle: the basis of the 25 x 25 origins of +-6 px at 0.5 px
+BASIS_ROWS = 160
+# the same for the phase-residual rescoring (mean of the two launches of a pass)
+RESCORE_TRAFFIC_PER_LAUNCH = 0.5 * (587.134464e6 + 3.439872e6 + 795.0208e6 + 3.52768e6)
 # l1tex__throughput (pct of peak, active) of the same capture: the rescoring's limiter
-RESCORE_L1_ACTIVE = 0.5 * (0.806 + 0.824)
+RESCORE_L1_ACTIVE = 0.5 * (0.841 + 0.874)
 
 
 
 def grouped_algorithmic_bytes(g, origins, particles=64):
     """Algorithmic bytes of one grouped-contraction launch from the library's counters
-    (cryoim_contract_stats): operand A of the pass (particles x origins BF16 rows) plus
-    each listed bank row once, the listed rows from the counted FLOPs
-    (2 x origins x rows x K per particle).  None without a launch."""
+    (cryoim_contract_stats): operand A of the pass (particles x origins BF16 rows, origins
+    being the rows of A a particle) plus each listed bank row once, the listed rows from
+    the counted FLOPs (2 x origins x rows x K per particle).  None without a launch."""
     if not g.get("gemm_launches") or not g.get("kpad"):
         return None
     rows = g["gemm_flops"] / g["gemm_launches"] / (2.0 * origins * g["kpad"])
@@ -665,14 +667,13 @@ def run_ours(args):
                                 "overlapping kernels of the other lanes",
                                 traffic=GROUPED_GEMM_TRAFFIC_PER_PASS * min(1.0, B / 64.0),
                                 traffic_note="DRAM bytes of one launch (64-particle pass) from an ncu capture of "
-                                "--profile-case learned with 16 learned cells, whose lists hold fewer rows "
-                                "than this run's 24-cell lists (algorithmic_bytes_per_launch is this run's)",
-                                algorithmic_bytes_per_launch=grouped_algorithmic_bytes(
-                                    gst, (int(round(2 * w["origin"] / w["origin_step"])) + 1) ** 2),
+                                "--profile-case learned",
+                                algorithmic_bytes_per_launch=grouped_algorithmic_bytes(gst, BASIS_ROWS),
                                 note="the grouped fine contraction of the headline form; its launches are "
-                                "small (each particle's 625 origins x its few hundred listed "
-                                "orientations, copied from the section bank by index), and the step is "
-                                "shared with the rescoring kernels (profiles/ has the launch list)")
+                                "small (the 160 basis rows of each particle's 625 origins x its few hundred "
+                                "listed orientations, two omegas a bank row, copied from the section bank by "
+                                "index), and the step is shared with the rescoring kernels (profiles/ has the "
+                                "launch list)")
     bf_v, bf_st, bf_g, bf_q = forms["bf16"]
     f8_v, f8_st, f8_g, f8_q = forms["fp8"]
     passes = (B + 63) // 64
@@ -732,11 +733,12 @@ def run_ours(args):
                                "samples_x_operators_per_particle": "r <= maxR half plane x 60",
                                "finish_ms": fin_ms, "entry": "cryoim_rec_insert_device / cryoim_rec_finish",
                                "roofline": {"bound": "l2_reductions", "kernel": "k_insert",
-                                            "achieved": s_ins * 60 * 8 * Bs / (ins_ms / 1000.0),
+                                            "achieved": s_ins * 5 * 8 * Bs / (ins_ms / 1000.0),
                                             "peak": L2_RED_PEAK, "unit": "float4 reductions/s",
-                                            "frac": s_ins * 60 * 8 * Bs / (ins_ms / 1000.0) / L2_RED_PEAK,
+                                            "frac": s_ins * 5 * 8 * Bs / (ins_ms / 1000.0) / L2_RED_PEAK,
                                             "hbm_bytes_per_s": s_ins * 12 * Bs / (ins_ms / 1000.0),
-                                            "note": "S_ins x 60 operators x 8 corners float4 reductions per "
+                                            "note": "S_ins x 5 operators (one of each coset of the grid's own "
+                                                    "rotations among the 60) x 8 corners float4 reductions per "
                                                     "particle into the L2-resident accumulator; peak = the L2's "
                                                     "reduction sector rate from ncu (profiles/k_insert_box256.md); "
                                                     "the insertion call's time includes the H2D-free device path"}},

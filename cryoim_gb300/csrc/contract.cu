@@ -386,7 +386,8 @@ __global__ void __launch_bounds__(256) k_build_a(const float2* __restrict__ band
     // origins relative to the particle's own (poff) or absolute
     const float hx = (float)(bd.nx / 2) + (poff ? poff[2 * p] : 0.0f);
     const float hy = (float)(bd.nx / 2) + (poff ? poff[2 * p + 1] : 0.0f);
-    const float inv = norm[p] > 0.0 ? (float)(1.0 / sqrt(norm[p])) : 0.0f;
+    __shared__ float sinv;  // root and quotient once: FP64 by every warp outweighs a block's FP32 work
+    if (threadIdx.x == 0) sinv = norm[p] > 0.0 ? (float)(1.0 / sqrt(norm[p])) : 0.0f;
     for (int j = 0; j < no; ++j) {
         const float sx = origins[2 * (o0 + j)] + hx, sy = origins[2 * (o0 + j) + 1] + hy;
         for (int i = threadIdx.x; i < nt; i += blockDim.x) {
@@ -398,6 +399,7 @@ __global__ void __launch_bounds__(256) k_build_a(const float2* __restrict__ band
         }
     }
     __syncthreads();
+    const float inv = sinv;
     for (int i = threadIdx.x; i < Kpad / 2; i += blockDim.x) {
         if (i < S) {
             const int2 hk = samples[i];
@@ -446,7 +448,8 @@ __global__ void __launch_bounds__(256) k_build_basis(const float2* __restrict__ 
     const float* c = ctf ? ctf + (long)p * W * W : nullptr;
     const float sx = (float)(bd.nx / 2) + ob.mid + (poff ? poff[2 * p] : 0.0f);
     const float sy = (float)(bd.nx / 2) + ob.mid + (poff ? poff[2 * p + 1] : 0.0f);
-    const float inv = norm[p] > 0.0 ? (float)(1.0 / sqrt(norm[p])) : 0.0f;
+    __shared__ float sinv;  // root and quotient once: FP64 by every warp outweighs a block's FP32 work
+    if (threadIdx.x == 0) sinv = norm[p] > 0.0 ? (float)(1.0 / sqrt(norm[p])) : 0.0f;
     const float pscale = F8 ? ldexpf(1.0f, fexp[p]) : 1.0f;
     int rot[BO], part[BO];  // rot: quarter turns of i^(...), part: -1 for an empty row
 #pragma unroll
@@ -469,6 +472,7 @@ __global__ void __launch_bounds__(256) k_build_basis(const float2* __restrict__ 
         ptab[i] = make_float2(cs, sn);
     }
     __syncthreads();
+    const float inv = sinv;
     for (int i = 2 * threadIdx.x; i < KH; i += 2 * blockDim.x) {  // two samples a thread
         float2 z[2];
         int2 hk[2];
@@ -1044,14 +1048,18 @@ __global__ void k_cc_fp64(const float2* __restrict__ cube, const double2* __rest
                           double* __restrict__ part, double gk, const float* __restrict__ pctf, int Rq, double sc) {
     extern __shared__ double2 ctab[];  // [R + 1] per hx, then [2R + 1] per ky
     __shared__ double sh[32];
-    __shared__ double rot[9];
+    __shared__ double rot[9], trig[6];
     // R: the band; Rq: the cube's radius (its side C = 2 Rq + 3), sc cube voxels per frequency
     const int c = blockIdx.x, p = blockIdx.y, sp = blockIdx.z, R = bd.max_r, C = 2 * Rq + 3, off = Rq + 1;
     const float* cd = cand + ((long)p * k + c) * 5;
+    if (threadIdx.x < 6) {  // cosines and sines of phi, theta, omega, a lane each
+        const int e = threadIdx.x % 3;
+        const double d2r = 3.14159265358979323846 / 180.0, ang = cd[e == 0 ? 1 : e == 1 ? 0 : 2] * d2r;
+        trig[threadIdx.x] = threadIdx.x < 3 ? cos(ang) : sin(ang);
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
-        const double d2r = 3.14159265358979323846 / 180.0;
-        double t = cd[0] * d2r, ph = cd[1] * d2r, om = cd[2] * d2r;
-        double c1 = cos(ph), c2 = cos(t), c3 = cos(om), s1 = sin(ph), s2 = sin(t), s3 = sin(om);
+        const double c1 = trig[0], c2 = trig[1], c3 = trig[2], s1 = trig[3], s2 = trig[4], s3 = trig[5];
         rot[0] = c1 * c2 * c3 - s1 * s3; rot[1] = -c1 * c2 * s3 - c3 * s1; rot[2] = c1 * s2;
         rot[3] = c2 * c3 * s1 + c1 * s3; rot[4] = -c2 * s1 * s3 + c1 * c3; rot[5] = s1 * s2;
         rot[6] = -c3 * s2;               rot[7] = s2 * s3;                 rot[8] = c2;

@@ -1420,11 +1420,12 @@ cudaError_t launch_slice_bf16_local(cudaTextureObject_t cube, int R, const int2*
                 pctf, sc);
             return cudaGetLastError();
         };
-        // registers for the samples there are, to the next even number a thread
+        // registers for the samples there are, in steps of two a thread (7 for the 1,600 of maxR 32: 1-2 % of the form)
         const int spt = (Kpad / 2 + LSR_THREADS - 1) / LSR_THREADS;
         if (spt <= 2) return rows(std::integral_constant<int, 2>());
         if (spt <= 4) return rows(std::integral_constant<int, 4>());
         if (spt <= 6) return rows(std::integral_constant<int, 6>());
+        if (spt <= 7) return rows(std::integral_constant<int, 7>());
         return rows(std::integral_constant<int, LSR_SPT>());
     }
     size_t sm = (size_t)S * sizeof(float2);

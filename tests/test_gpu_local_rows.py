@@ -1,4 +1,4 @@
-"""Rows of the local grids at every number of samples a thread holds (2, 4, 6, 8), with a last
+"""Rows of the local grids at every number of samples a thread holds (2, 4, 6, 7, 8), with a last
 group of 1, 2 or 3 of the four rows that are normalised together: the BF16 score of every candidate
 follows its FP64 score (the bound of the other local tests: BF16 rows of a few hundred samples)."""
 import numpy as np
@@ -9,7 +9,7 @@ from _data import small_case
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,R,m", [(48, 12, 2), (64, 21, 3), (96, 29, 1), (96, 34, 4)])
+@pytest.mark.parametrize("n,R,m", [(48, 12, 2), (64, 21, 3), (96, 29, 1), (96, 32, 2), (96, 34, 4)])
 def test_scores_follow_fp64(built, n, R, m):
     import cryoim_gb300 as ci
     p, vol, tmpl, timgs, imgs, parts, truth = small_case(n=n, P=3, T=2, step=4.0, min_res=60.0,

@@ -141,9 +141,10 @@ def make_data(ci, nparticles: int, projector):
 
 
 class ClockSampler:
-    """nvidia-smi clocks and throttle reasons sampled every 100 ms.  The sampler is started
-    ahead of the timed region (nvidia-smi takes a moment to come up) and summary() keeps
-    the samples that arrived between begin() and end(): the timed region itself."""
+    """nvidia-smi clocks and throttle reasons sampled every 20 ms (a default run is timed for
+    0.2 s).  The sampler is started ahead of the timed region (nvidia-smi takes a moment to
+    come up) and summary() keeps the samples that arrived between begin() and end(): the
+    timed region itself."""
 
     Q = ("clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.hw_slowdown,"
          "clocks_event_reasons.hw_thermal_slowdown,clocks_event_reasons.sw_thermal_slowdown,"
@@ -152,7 +153,7 @@ class ClockSampler:
     def __init__(self, index: int, cmd=None):
         self.index, self.rows, self.proc = index, [], None
         self.cmd = cmd or ["nvidia-smi", "-i", str(index), f"--query-gpu={self.Q}",
-                           "--format=csv,noheader,nounits", "-lms", "100"]
+                           "--format=csv,noheader,nounits", "-lms", "20"]
         self.t0 = self.t1 = None
 
     def start(self):

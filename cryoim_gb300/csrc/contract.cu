@@ -24,6 +24,7 @@
 #include "geom.cuh"
 #include "reduce.cuh"
 #include "kernels.h"
+#include "launch.h"
 #include "origin_basis.h"
 
 namespace cryoim {
@@ -1461,9 +1462,7 @@ void launch_build_a(const float2* band, const float* ctf, Band bd, const int2* s
 void launch_select_distinct(float* topv, const int* topi, int O, const int2* seg, int B, int max_tiles, int k, int* col,
                             int* origin, float* cc, cudaStream_t st) {
     const size_t sm = (size_t)O * max_tiles * (sizeof(float) + sizeof(int));
-    if (sm <= 48 * 1024 ||
-        (sm <= 200 * 1024 && cudaFuncSetAttribute(k_select_distinct<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)sm) == cudaSuccess))
+    if (sm <= 200 * 1024 && allow_smem(k_select_distinct<true>, sm) == cudaSuccess)
         k_select_distinct<true><<<B, 512, sm, st>>>(topv, topi, O, seg, k, col, origin, cc);
     else
         k_select_distinct<false><<<B, 512, 0, st>>>(topv, topi, O, seg, k, col, origin, cc);

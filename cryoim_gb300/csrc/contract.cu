@@ -1277,10 +1277,8 @@ cudaError_t launch_build_basis(const float2* band, const float* ctf, Band bd, co
     const size_t sm = (sizeof(float2) + sizeof(float) * BO) * (3 * (size_t)bd.max_r + 2);
     if (f8) k_particle_exp8<<<B, 256, 0, st>>>(band, ctf, bd, samples, S, norm, mulA, fexp);
     auto kern = f8 ? k_build_basis<true> : k_build_basis<false>;
-    if (sm > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_smem(kern, sm);
+    if (e != cudaSuccess) return e;
     kern<<<g, 256, sm, st>>>(band, ctf, bd, samples, S, KH, ob, poff, norm, mulA, fexp, tpn, A);
     return cudaGetLastError();
 }
@@ -1300,7 +1298,7 @@ cudaError_t launch_up_topk(const OriginDev& ob, const float* C, long pitch, long
             const int cols = nom == nomr ? UP_THREADS : UP_THREADS / 2;
             const long tiles = (rows + cols - 1) / cols * B;
             const size_t sm = sizeof(float) * (up_table_floats<LY>(ob.n1) + (size_t)UP_THREADS * OB_LAYOUT[LY].rows);
-            e = cudaFuncSetAttribute(k_up_max<LY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            e = allow_smem(k_up_max<LY>, sm);
             if (e != cudaSuccess) return;
             k_up_max<LY><<<(unsigned)std::min<long>(tiles, num_sms), UP_THREADS, sm, st>>>(ob, C, pitch, rows, nom, nomr, B,
                                                                                           ccmax);
@@ -1338,7 +1336,7 @@ cudaError_t launch_up_list(const OriginDev& ob, const float* C, int parts, const
     const size_t sm = tab + (shm ? (size_t)nw * O * 8 : 0);
     auto kern = ly < 0 ? k_up_list<-1> : ly == 0 ? k_up_list<0> : ly == 1 ? k_up_list<1> : ly == 2 ? k_up_list<2>
                 : ly == 3 ? k_up_list<3> : k_up_list<4>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return e;
     // blocks to a tile: as many as find an SM of their own (each reads its tile's products again, so that with
     // the SMs filled, by this launch or by other lanes', the pass takes longer: 14.0 -> 14.5 ms of the box-256
@@ -1395,7 +1393,7 @@ cudaError_t launch_slice_bf16(cudaTextureObject_t cube, int R, const int2* sampl
                               cudaStream_t st, const float2* lin, float sigma, float sc) {
     const float gk = (lin && sigma > 0.0f) ? 1.0f / (2.0f * sigma * sigma) : 0.0f;
     size_t sm = (size_t)S * sizeof(float2);
-    cudaError_t e = cudaFuncSetAttribute(k_slice_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_smem(k_slice_bf16, sm);
     if (e != cudaSuccess) return e;
     k_slice_bf16<<<(unsigned)count, SLICE_THREADS, sm, st>>>(cube, R, samples, S, KH, views, nomr, step,
                                                              host_angles().deg2rad, n0, (__nv_bfloat16*)B, lin, gk,
@@ -1430,8 +1428,7 @@ cudaError_t launch_slice_bf16_local(cudaTextureObject_t cube, int R, const int2*
         return rows(std::integral_constant<int, LSR_SPT>());
     }
     size_t sm = (size_t)S * sizeof(float2);
-    cudaError_t e =
-        cudaFuncSetAttribute(k_slice_bf16_local, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_smem(k_slice_bf16_local, sm);
     if (e != cudaSuccess) return e;
     for (long c0 = 0; c0 < count; c0 += 65535) {
         long nb = count - c0 < 65535 ? count - c0 : 65535;
@@ -1454,7 +1451,7 @@ void launch_build_a(const float2* band, const float* ctf, Band bd, const int2* s
     const float tpn = 2.0f * host_angles().pi / (float)bd.nx;
     dim3 ga((O + AO - 1) / AO, B);
     const int sm = (int)(sizeof(float2) * AO * (3 * bd.max_r + 2));
-    if (sm > 48 * 1024) cudaFuncSetAttribute(k_build_a, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    allow_smem(k_build_a, sm);
     k_build_a<<<ga, 256, sm, st>>>(band, ctf, bd, samples, S, Kpad, origins, O, poff, norm, tpn,
                                    (__nv_bfloat162*)A);
 }

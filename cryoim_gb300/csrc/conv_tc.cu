@@ -31,6 +31,7 @@
 #include <cstdint>
 
 #include "kernels.h"
+#include "launch.h"
 #include "tc.cuh"
 
 namespace cryoim {
@@ -810,8 +811,7 @@ cudaError_t launch_fwd(ConvTcArgs a, cudaStream_t st) {
     if (steps > 0x7fffffffL) return cudaErrorInvalidValue;
     a.steps_per_cta = (int)((steps + ctas - 1) / ctas);
     const int grid = (int)((steps + a.steps_per_cta - 1) / a.steps_per_cta);
-    const cudaError_t e =
-        cudaFuncSetAttribute(k_conv3_tc<CINP, COUT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = allow_smem(k_conv3_tc<CINP, COUT, MODE>, smem);
     if (e != cudaSuccess) return e;
     k_conv3_tc<CINP, COUT, MODE><<<grid, CT_THREADS, smem, st>>>(a);
     return cudaGetLastError();
@@ -820,8 +820,7 @@ cudaError_t launch_fwd(ConvTcArgs a, cudaStream_t st) {
 template <int CINP, int COUT, bool GATED>
 cudaError_t launch_wgrad(const ConvWgTcArgs& a, int grid, cudaStream_t st) {
     constexpr int smem = WgGeom<CINP, COUT>::SMEM;
-    const cudaError_t e = cudaFuncSetAttribute(k_conv3_wgrad_tc<CINP, COUT, GATED>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = allow_smem(k_conv3_wgrad_tc<CINP, COUT, GATED>, smem);
     if (e != cudaSuccess) return e;
     k_conv3_wgrad_tc<CINP, COUT, GATED><<<grid, CT_THREADS, smem, st>>>(a);
     return cudaGetLastError();

@@ -32,6 +32,7 @@
 
 #include "../../include/cryoim.h"
 #include "kernels.h"
+#include "launch.h"
 #include "tc.cuh"
 
 namespace cryoim {
@@ -472,7 +473,7 @@ static cudaError_t gemm_kernel(bool f8, bool store, int smem,
                                void (**kern)(const CUtensorMap, const CUtensorMap, GemmArgmaxArgs)) {
     *kern = f8 ? (store ? k_gemm_argmax<true, true> : k_gemm_argmax<true, false>)
                : (store ? k_gemm_argmax<false, true> : k_gemm_argmax<false, false>);
-    return cudaFuncSetAttribute(*kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return allow_smem(*kern, smem);
 }
 // stored products: units of c_rows rows (whole 32-column reads of TMEM, two accumulators and a
 // stage's tiles within TMEM and shared memory), K in k_parts equal shares of whole stages

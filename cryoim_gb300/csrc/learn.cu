@@ -23,6 +23,7 @@
 
 #include "geom.cuh"
 #include "kernels.h"
+#include "launch.h"
 
 namespace cryoim {
 namespace {
@@ -1072,8 +1073,7 @@ void launch_lp_adam(float* w, const float* g, float* m, float* v, long n, float 
 void launch_lp_topk(float* sc, int B, int V, int k, int* cell, float* val, cudaStream_t st) {
     const long n = (long)V * NT;
     const size_t sm = sizeof(float) * (size_t)n;
-    if (sm <= 200 * 1024 &&
-        cudaFuncSetAttribute(k_topk_cells<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) == cudaSuccess)
+    if (sm <= 200 * 1024 && allow_smem(k_topk_cells<true>, sm) == cudaSuccess)
         k_topk_cells<true><<<B, 512, sm, st>>>(sc, n, k, cell, val);
     else
         k_topk_cells<false><<<B, 512, 0, st>>>(sc, n, k, cell, val);

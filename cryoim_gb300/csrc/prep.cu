@@ -13,6 +13,7 @@
 
 #include "geom.cuh"
 #include "kernels.h"
+#include "launch.h"
 #include "reduce.cuh"
 
 namespace cryoim {
@@ -736,7 +737,7 @@ void launch_refine_step(const float* state, const float* prev, const double2* pr
                         float dtran, const float* tort, int T, const float* ops, float* cand, float2* alpha,
                         cudaStream_t st) {
     const size_t sm = sizeof(float) * 9 * (T + 1);
-    if (sm > 48 * 1024) cudaFuncSetAttribute(k_refine_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    allow_smem(k_refine_step, sm);
     const HostAngles a = angles();
     k_refine_step<<<dim3(11, B), 256, sm, st>>>(state, prev, prev_part, S, dang, dtran, tort, T, ops, a.d2r, a.r2d,
                                                 a.pi, cand, alpha);
@@ -750,7 +751,7 @@ void launch_refine_alpha(const float* cand, int B, const float* tort, int T, con
                          float2* alpha, cudaStream_t st, int ncand) {
     const long rows = (long)B * ncand;
     const size_t sm = sizeof(float) * 9 * (T + 1);
-    if (sm > 48 * 1024) cudaFuncSetAttribute(k_refine_alpha, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    allow_smem(k_refine_alpha, sm);
     HostAngles a = angles();
     k_refine_alpha<<<(unsigned)rows, 256, sm, st>>>(cand, rows, tort, T, ops, a.d2r, a.r2d, alpha);
 }

@@ -23,6 +23,7 @@
 #include "geom.cuh"
 #include "reduce.cuh"
 #include "kernels.h"
+#include "launch.h"
 
 namespace cryoim {
 namespace {
@@ -1096,7 +1097,7 @@ cudaError_t launch_pr_omega(const PrOmegaArgs& a, int B, cudaStream_t st) {
         if (rounds(zz) < rounds(z)) z = zz;
     auto kern = z > 1 ? (half ? k_pr_omega<true, true> : k_pr_omega<false, true>)
                       : (half ? k_pr_omega<true, false> : k_pr_omega<false, false>);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return e;
     kern<<<dim3(a.V, B, z), nt, sm, st>>>(a, nall, G, consts());
     return cudaGetLastError();
@@ -1170,7 +1171,7 @@ int pr_refine_splits(const Band& bd, int T, int B, int num_sms) {
 
 cudaError_t launch_pr_refine(const PrSingleArgs& a, int B, int S, double2* part, cudaStream_t st) {
     const size_t sm = pr_refine_smem(a.bd, (a.T + S - 1) / S);
-    cudaError_t e = cudaFuncSetAttribute(k_pr_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_smem(k_pr_refine, sm);
     if (e != cudaSuccess) return e;
     k_pr_refine<<<dim3(a.ncand, B, S), RF_THREADS, sm, st>>>(a, consts(), part);
     return cudaGetLastError();
@@ -1184,13 +1185,13 @@ cudaError_t launch_pr_rescore_groups(const PrSingleArgs& a, const int4* groups, 
     const size_t sm_s = sm + sizeof(float2) * (size_t)a.bd.W * rescore_pitch(a.bd.W);
     if (pr_rescore_shared_band(a.bd, a.T)) {
         if (!a.valpha || !a.corient || a.nom < 1) return cudaErrorInvalidValue;
-        cudaError_t e = cudaFuncSetAttribute(k_pr_rescore_s, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_s);
+        cudaError_t e = allow_smem(k_pr_rescore_s, sm_s);
         if (e != cudaSuccess) return e;
         k_pr_rescore_s<<<ngroups, RS_THREADS, sm_s, st>>>(a, groups, consts());
         return cudaGetLastError();
     }
     if (sm > 200 * 1024) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(k_pr_rescore_g, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = allow_smem(k_pr_rescore_g, sm);
     if (e != cudaSuccess) return e;
     k_pr_rescore_g<<<ngroups, 512, sm, st>>>(a, groups, consts());
     return cudaGetLastError();

@@ -1,6 +1,7 @@
 """A kernel's shared-memory permission is one state of the device for all host threads (csrc/launch.h): a
-launch's request never lowers it and counts the kernel's static memory."""
+launch's request never lowers it, counts the kernel's static memory, and is the only place that sets it."""
 import ctypes as C
+import glob
 import os
 import subprocess
 
@@ -59,3 +60,9 @@ def test_static_memory_counts(fake):
     fake.reset(264)
     assert fake.ask(232448 - 264) == 0 and fake.launch(232448 - 264)
     assert fake.ask(232448 - 263) != 0
+
+
+def test_nothing_else_sets_it():
+    users = [os.path.basename(f) for f in glob.glob(os.path.join(CSRC, "**", "*.*"), recursive=True)
+             if "cudaFuncSetAttribute" in open(f).read()]
+    assert users == ["launch.h"]

@@ -710,7 +710,7 @@ int globesearch_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle*
             a.band = c->band.p; a.fcut0 = c->fcut0.p; a.tband = c->tband.p;
             a.tfcut = tfc; a.tfcut_pstride = tfs; a.ctf = ctfp; a.alpha = c->alpha.p;
             a.views = c->d_views.p; a.V = c->V; a.T = c->T; a.nomega = c->nom;
-            a.step = c->p.searchstep; a.bd = c->bd; a.best = c->best.p;
+            a.step = c->p.searchstep; a.real_image = true; a.bd = c->bd; a.best = c->best.p;
             a.pr_array = pr_array ? c->prbuf.p : nullptr; a.per = per;
             if (c->prof) CK(cudaEventRecord(c->pe0, c->stream));
             CK(launch_pr_omega(a, nb, c->stream));
@@ -2918,6 +2918,7 @@ int cryoim_prscore_omega(void* ctx, const float* ft_a, const float* ft_b, const 
     a.band = c->band.p; a.fcut0 = c->fcut0.p; a.tband = c->tband.p; a.tfcut = tfc;
     a.tfcut_pstride = tfs; a.ctf = ctfp; a.alpha = dal.p; a.views = dv.p; a.V = 1; a.T = T;
     a.nomega = nom; a.step = step; a.bd = c->bd; a.best = c->best.p; a.pr_array = dprs.p; a.per = nom;
+    a.real_image = false;  // any ft_a, ft_b: each omega from its own samples
     CK(launch_pr_omega(a, 1, c->stream));
     CK(cudaMemcpyAsync(pr_omega, dprs.p, sizeof(float) * nom, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));

@@ -93,12 +93,12 @@ struct PrOmegaArgs {
     const float* views;      // [V][4]: theta, phi, slot base (int bits), pad
     int V, T, nomega;
     float step;
+    bool real_image;           // band(-h) = conj band(h): two omegas half a turn apart share a sample
     Band bd;
     unsigned long long* best;  // [B]
     float* pr_array;           // [B][per] or nullptr
     long per;
 };
-int pr_omega_smem_bytes(const Band& bd, int nomega, float step, int* threads, int* groups);
 cudaError_t launch_pr_omega(const PrOmegaArgs& a, int B, cudaStream_t st);
 
 struct PrSingleArgs {

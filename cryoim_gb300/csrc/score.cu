@@ -1061,14 +1061,13 @@ Consts consts() {
 
 }  // namespace
 
-// omega + nomega / 2 is half a turn on
-static bool omega_half(int nomega, float step) {
-    return nomega % 2 == 0 && fabsf(step * (float)(nomega / 2) - 180.0f) < 1e-3f;
+// omega + nomega / 2 is half a turn on, and its samples are those at omega conjugated
+static bool omega_half(const PrOmegaArgs& a) {
+    return a.real_image && a.nomega % 2 == 0 && fabsf(a.step * (float)(a.nomega / 2) - 180.0f) < 1e-3f;
 }
 
-int pr_omega_smem_bytes(const Band& bd, int nomega, float step, int* threads, int* groups) {
+static int pr_omega_smem_bytes(const Band& bd, int nomega, bool half, int* threads, int* groups) {
     if (nomega < 1 || nomega > 768) return -1;
-    const bool half = omega_half(nomega, step);
     const int nown = half ? nomega / 2 : nomega;
     // groups of lines: as many as fit 768 threads, and no more than there are lines
     const int G = std::min(60, 768 / nown), nt = (G * nown + 31) / 32 * 32;
@@ -1081,9 +1080,9 @@ int pr_omega_smem_bytes(const Band& bd, int nomega, float step, int* threads, in
 
 cudaError_t launch_pr_omega(const PrOmegaArgs& a, int B, cudaStream_t st) {
     int nt = 0, G = 0;
-    int sm = pr_omega_smem_bytes(a.bd, a.nomega, a.step, &nt, &G);
+    const bool half = omega_half(a);
+    int sm = pr_omega_smem_bytes(a.bd, a.nomega, half, &nt, &G);
     if (sm < 0) return cudaErrorInvalidValue;
-    const bool half = omega_half(a.nomega, a.step);
     // A block has an SM to itself: where a block a view and particle leave SMs idle, several share a view's omegas
     // (each repeats the template's samples: 47 views of 90 omegas, one particle, 4 templates, box 64, 78 us by 47
     // blocks, 51 by 94)

@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <numeric>
 
 namespace cryoim {
@@ -61,23 +62,35 @@ OriginBasis make_origin_basis(int n, int min_r, int R, float omax, float step, i
     const double w0 = 2.0 * 3.14159265358979323846 / n;
     std::vector<double> u(n1);
     for (int i = 0; i < n1; ++i) u[i] = (double)step * (i - 0.5 * (n1 - 1));
+    // cos and sin of w0 h u_i for h = 0 .. R, [h][i] (u_{n1-1-i} = -u_i)
+    std::vector<double> cs((size_t)(R + 1) * n1), sn((size_t)(R + 1) * n1);
+    const int he = (n1 + 1) / 2, ho = n1 / 2;
+    for (int h = 0; h <= R; ++h)
+        for (int i = 0; i < he; ++i) {
+            const size_t q = (size_t)h * n1 + i, r = (size_t)h * n1 + n1 - 1 - i;
+            cs[q] = cs[r] = std::cos(w0 * h * u[i]);
+            sn[q] = std::sin(w0 * h * u[i]);
+            if (r != q) sn[r] = -sn[q];
+        }
     // even and odd eigenvectors apart: v(i) = +- v(n1 - 1 - i)
     std::vector<std::vector<double>> fun;  // [function][n1], even and odd alternating
     std::vector<double> vec[2];
-    const int he = (n1 + 1) / 2, ho = n1 / 2;
     for (int odd = 0; odd < 2; ++odd) {
         const int m = odd ? ho : he;
-        std::vector<double> a((size_t)m * m);
+        const std::vector<double>& t = odd ? sn : cs;
+        std::vector<double> a((size_t)m * m, 0.0);
+        for (int h = -R; h <= R; ++h) {
+            const double* th = t.data() + (size_t)std::abs(h) * n1;  // (the signs of a negative h cancel)
+            for (int i = 0; i < m; ++i)
+                for (int j = 0; j <= i; ++j) a[(size_t)i * m + j] += th[i] * th[j];
+        }
+        // orthonormal half-grid vectors (e_i +- e_mirror) / sqrt 2 (the middle one alone)
+        auto norm = [&](int i) { return (!odd && (n1 & 1) && i == m - 1) ? 1.0 : std::sqrt(2.0); };
         for (int i = 0; i < m; ++i)
-            for (int j = 0; j < m; ++j) {
-                double s = 0.0;
-                for (int h = -R; h <= R; ++h)
-                    s += odd ? std::sin(w0 * h * u[i]) * std::sin(w0 * h * u[j])
-                             : std::cos(w0 * h * u[i]) * std::cos(w0 * h * u[j]);
-                // orthonormal half-grid vectors (e_i +- e_mirror) / sqrt 2 (the middle one alone)
-                const double ci = (!odd && (n1 & 1) && i == m - 1) ? 1.0 : std::sqrt(2.0);
-                const double cj = (!odd && (n1 & 1) && j == m - 1) ? 1.0 : std::sqrt(2.0);
-                a[(size_t)i * m + j] = s * ci * cj;
+            for (int j = 0; j <= i; ++j) {
+                const double s = a[(size_t)i * m + j];
+                a[(size_t)i * m + j] = s * norm(i) * norm(j);
+                a[(size_t)j * m + i] = s * norm(j) * norm(i);
             }
         eigenvectors(a, m, vec[odd]);
     }
@@ -92,32 +105,40 @@ OriginBasis make_origin_basis(int n, int min_r, int R, float omax, float step, i
         }
         fun.push_back(g);
     }
-    // their transforms over the band
+    // their transforms over the band, even or odd in h as the function is
     const int H = 2 * R + 1;
-    std::vector<double> f((size_t)n1 * H);
-    for (int k = 0; k < n1; ++k)
-        for (int h = -R; h <= R; ++h) {
+    std::vector<double> f((size_t)n1 * H), sq((size_t)(R + 1) * n1);  // sq: their squares, [h][function]
+    for (int k = 0; k < n1; ++k) {
+        const std::vector<double>& t = (k & 1) ? sn : cs;
+        for (int h = 0; h <= R; ++h) {
+            const double* th = t.data() + (size_t)h * n1;
             double s = 0.0;
-            for (int i = 0; i < n1; ++i) s += fun[k][i] * ((k & 1) ? std::sin(w0 * h * u[i]) : std::cos(w0 * h * u[i]));
-            f[(size_t)k * H + h + R] = s;
+            for (int i = 0; i < n1; ++i) s += fun[k][i] * th[i];
+            f[(size_t)k * H + R + h] = s;
+            f[(size_t)k * H + R - h] = (k & 1) ? -s : s;
+            sq[(size_t)h * n1 + k] = s * s;
         }
-    // energy of each product over the half-plane band samples
-    std::vector<double> e((size_t)n1 * n1, 0.0);
+    }
+    // energy of each product over the half-plane band samples (hx > 0, or hx = 0 and ky > 0): row by
+    // row of hx, whose samples are minR^2 <= hx^2 + ky^2 <= R^2
+    std::vector<double> e((size_t)n1 * n1, 0.0), row(n1);
     double total = 0.0;
-    for (int ky = -R; ky <= R; ++ky)
-        for (int hx = 0; hx <= R; ++hx) {
+    for (int hx = 0; hx <= R; ++hx) {
+        std::fill(row.begin(), row.end(), 0.0);
+        long samples = 0;
+        for (int ky = 0; ky <= R; ++ky) {
             const int d2 = hx * hx + ky * ky;
-            if ((hx == 0 && ky <= 0) || d2 < min_r * min_r || d2 > R * R) continue;
-            total += (double)n1 * n1;
-            for (int m = 0; m < n1; ++m) {
-                const double fm = f[(size_t)m * H + hx + R], fm2 = fm * fm;
-                if (fm2 < 1e-18) continue;
-                for (int k = 0; k < n1; ++k) {
-                    const double fk = f[(size_t)k * H + ky + R];
-                    e[(size_t)m * n1 + k] += fm2 * fk * fk;
-                }
-            }
+            if ((hx == 0 && ky == 0) || d2 < min_r * min_r || d2 > R * R) continue;
+            const int both = hx > 0 && ky > 0 ? 2 : 1;  // ky and -ky
+            samples += both;
+            const double* sk = sq.data() + (size_t)ky * n1;
+            for (int k = 0; k < n1; ++k) row[k] += both * sk[k];
         }
+        total += (double)samples * n1 * n1;
+        const double* sm = sq.data() + (size_t)hx * n1;
+        for (int m = 0; m < n1; ++m)
+            for (int k = 0; k < n1; ++k) e[(size_t)m * n1 + k] += sm[m] * row[k];
+    }
     // What is left out (tail, of total) acts on the score like a change of the particle's phases,
     // the same for every sample that carries the signal, so it adds up where rounding averages
     // out: its root mean square stays 5e-5 (BF16) or 4e-4 (e4m3), far below the operands' rounding

@@ -267,14 +267,14 @@ struct LearnModel {
     }
 };
 
-// An origin grid's basis on the device, rebuilt when the grid, the band or the type changes.
+// An origin grid's basis on the device, and what it was made for (nx = 0: nothing).
 struct OriginPlan {
     OriginDev dev{};
-    DBuf<float> q, f;
-    DBuf<int> row;
-    DBuf<int2> slot;
-    int nx = 0, min_r = -1, R = -1, n1 = 0;
+    DBuf<unsigned char> mem;  // dev's tables
+    int nx = 0, min_r = -1, R = -1;
     float omax = -1.0f, step = -1.0f;
+    bool f8 = false;
+    long used = 0;  // when, for the least recently used one
 };
 
 struct Ctx {
@@ -350,8 +350,10 @@ struct Ctx {
     bool bmat8_ready = false;
     double bmat8_ms = 0.0;
     int cKH8 = 0, last_kpad = 0;
-    // bases of the origin grids (BF16, FP8, coarse) and the products of a sub-batch or pass
-    OriginPlan op, op8, op_c;
+    // bases of the last origin grids (a call uses two at most, its fine and its coarse level's) and the
+    // products of a sub-batch or pass
+    OriginPlan oplans[8];
+    long oplan_calls = 0;
     DBuf<float> cprod, ccmax;
     DBuf<int> lmap;
     DBuf<UpGroup> upg;
@@ -1031,28 +1033,47 @@ int bank_omegas(int nom, float step) {
     return nom % 2 == 0 && std::fabs(step * (float)(nom / 2) - 180.0f) < 1e-3f ? nom / 2 : nom;
 }
 
-int ensure_origin_plan(Ctx* c, OriginPlan& o, int R, float omax, float step, bool f8) {
-    const int n1 = (int)(2.0f * omax / step + 0.5f) + 1;
-    if (o.nx == c->p.fftsize && o.min_r == c->p.min_r && o.R == R && o.omax == omax && o.step == step)
-        return CRYOIM_OK;
+// The basis of an origin grid over the band |h| <= R: one of the context's last ones, or made in place
+// of the least recently used (0.2 ms of host work at 25 x 25 origins and R = 64, 0.9 ms at 41 x 41, beside
+// searches of a millisecond: two grids in turn do not make it anew).
+int ensure_origin_plan(Ctx* c, int R, float omax, float step, bool f8, OriginDev* out) {
+    OriginPlan* at = &c->oplans[0];
+    for (OriginPlan& o : c->oplans) {
+        if (o.nx == c->p.fftsize && o.min_r == c->p.min_r && o.R == R && o.omax == omax && o.step == step && o.f8 == f8) {
+            o.used = ++c->oplan_calls;
+            *out = o.dev;
+            return CRYOIM_OK;
+        }
+        if (o.used < at->used) at = &o;
+    }
+    OriginPlan& o = *at;
     o.nx = 0;
+    const int n1 = (int)(2.0f * omax / step + 0.5f) + 1;
     const OriginBasis b = make_origin_basis(c->p.fftsize, c->p.min_r, R, omax, step, n1, f8);
     if (b.nb > 512) return fail(CRYOIM_ERR_SIZE, "origin grid of %d x %d", n1, n1);
-    std::vector<int> row(b.slots);
-    std::vector<int2> slot((size_t)b.nb * b.nb);
-    for (int i = 0; i < b.slots; ++i) row[i] = b.mx[i] < 0 ? -1 : b.mx[i] | b.my[i] << 12 | b.part[i] << 24;
-    for (size_t i = 0; i < slot.size(); ++i) slot[i] = make_int2(b.slot[2 * i], b.slot[2 * i + 1]);
+    // one block of memory and one copy: slot (8-byte elements), row, q, f
+    std::vector<int> h;
+    auto put = [&](const void* p, size_t n) {
+        const size_t at = h.size();
+        h.resize(at + n);
+        std::memcpy(h.data() + at, p, sizeof(int) * n);
+        return at;
+    };
+    std::vector<int> rows(b.slots);
+    for (int i = 0; i < b.slots; ++i) rows[i] = b.mx[i] < 0 ? -1 : b.mx[i] | b.my[i] << 12 | b.part[i] << 24;
+    const size_t slot = put(b.slot.data(), b.slot.size()), row = put(rows.data(), rows.size());
+    const size_t q = put(b.q.data(), b.q.size()), f = put(b.f.data(), b.f.size()), words = h.size();
     int r;
-    if ((r = o.q.ensure(b.q.size())) || (r = o.f.ensure(b.f.size())) || (r = o.row.ensure(b.slots)) || (r = o.slot.ensure(slot.size())))
-        return r;
-    CK(cudaMemcpyAsync(o.q.p, b.q.data(), sizeof(float) * b.q.size(), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(o.f.p, b.f.data(), sizeof(float) * b.f.size(), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(o.row.p, row.data(), sizeof(int) * b.slots, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(o.slot.p, slot.data(), sizeof(int2) * slot.size(), cudaMemcpyHostToDevice, c->stream));
+    if ((r = o.mem.ensure(sizeof(int) * words))) return r;
+    CK(cudaMemcpyAsync(o.mem.p, h.data(), sizeof(int) * words, cudaMemcpyHostToDevice, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    o.dev = OriginDev{o.q.p, o.f.p, o.row.p, o.slot.p, b.n1, b.nb, b.slots, b.units, b.R, b.layout, b.mid,
+    const int* d = reinterpret_cast<const int*>(o.mem.p);
+    o.dev = OriginDev{reinterpret_cast<const float*>(d + q), reinterpret_cast<const float*>(d + f), d + row,
+                      reinterpret_cast<const int2*>(d + slot), b.n1, b.nb, b.slots, b.units, b.R, b.layout, b.mid,
                       f8 ? 0.0625f : 1.0f};
-    o.nx = c->p.fftsize; o.min_r = c->p.min_r; o.R = R; o.n1 = n1; o.omax = omax; o.step = step;
+    o.nx = c->p.fftsize; o.min_r = c->p.min_r; o.R = R; o.omax = omax; o.step = step; o.f8 = f8;
+    o.used = ++c->oplan_calls;
+    *out = o.dev;
     return CRYOIM_OK;
 }
 
@@ -1097,8 +1118,8 @@ int ensure_bmat(Ctx* c) {
 
 // The coarse level of the proposal form: views at twice the search step, the band
 // minR <= |h| <= maxR/2, BF16 unit-norm sections (built as the fine ones), origins at
-// twice the origin step over the same range.
-int ensure_coarse(Ctx* c, float omax, float ostep) {
+// twice the origin step over the same range, whose basis goes to ob.
+int ensure_coarse(Ctx* c, float omax, float ostep, OriginDev* ob) {
     int r;
     if ((r = ensure_grid(c))) return r;
     if (!c->bmat_c_ready) {
@@ -1137,7 +1158,7 @@ int ensure_coarse(Ctx* c, float omax, float ostep) {
         c->n_orient_c = n;
         c->bmat_c_ready = true;
     }
-    return ensure_origin_plan(c, c->op_c, std::max(c->p.min_r + 1, c->p.max_r / 2), omax, 2.0f * ostep, false);
+    return ensure_origin_plan(c, std::max(c->p.min_r + 1, c->p.max_r / 2), omax, 2.0f * ostep, false, ob);
 }
 
 // A particle's proposed orientations: fine-grid indices, each once, in the order first
@@ -1916,7 +1937,8 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
     }
     if (P == 0) return CRYOIM_OK;
     if ((r = local ? ensure_samples(c) : (f8 ? ensure_bmat8(c) : ensure_bmat(c)))) return r;
-    if (kc > 0 && (r = ensure_coarse(c, opts->origin_max, opts->origin_step))) return r;
+    OriginDev ob{}, ob_c{};
+    if (kc > 0 && (r = ensure_coarse(c, opts->origin_max, opts->origin_step, &ob_c))) return r;
     const int kpad = local ? c->cKpad : 2 * (f8 ? c->cKH8 : c->cKH);
     c->last_kpad = kpad;
     c->last_slice_ms = c->bmat_ms + (f8 ? c->bmat8_ms : 0.0);
@@ -1943,9 +1965,7 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
     // rows are the particle's own (no half turn to share), the BF16 score of every origin
     // decides which one the FP64 rescoring sees, and 289 origins of a 128 box are 3 row tiles
     // against 1: 8 % of its time, the sections' cut 83 %
-    OriginPlan& plan = f8 ? c->op8 : c->op;
-    if (!local && (r = ensure_origin_plan(c, plan, c->p.max_r, opts->origin_max, opts->origin_step, f8))) return r;
-    const OriginDev ob = plan.dev, ob_c = c->op_c.dev;
+    if (!local && (r = ensure_origin_plan(c, c->p.max_r, opts->origin_max, opts->origin_step, f8, &ob))) return r;
     const int parts_k = local ? 1 : c->nom / c->nomr;
     // Particles per pass (transform, rescoring: large grids, two host waits per pass);
     // operand A is built for the whole pass.

@@ -12,6 +12,7 @@ namespace cryoim {
 // the most that a block of this kernel can have: with each launch's own size, one thread could lower
 // it between another's call and its launch, which the device would then refuse.
 inline cudaError_t allow_smem_of(const void* kern, size_t bytes) {
+    if (bytes <= 16 * 1024) return cudaSuccess;  // (no kernel with dynamic memory has 32 KB of its own beside it)
     cudaFuncAttributes fa;
     cudaError_t e = cudaFuncGetAttributes(&fa, kern);
     if (e != cudaSuccess) return e;

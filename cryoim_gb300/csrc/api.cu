@@ -1050,9 +1050,8 @@ int ensure_origin_plan(Ctx* c, int R, float omax, float step, bool f8, OriginDev
     o.nx = 0;
     const int n1 = (int)(2.0f * omax / step + 0.5f) + 1;
     const OriginBasis b = make_origin_basis(c->p.fftsize, c->p.min_r, R, omax, step, n1, f8);
-    if (b.nb > 512) return fail(CRYOIM_ERR_SIZE, "origin grid of %d x %d", n1, n1);
-    // one block of memory and one copy: slot (8-byte elements), row, q, f
-    std::vector<int> h;
+    // one block of memory and one copy: ent, qx, qy (16-byte elements), slot (8), row, ent_off, q, f
+    std::vector<int> h(b.ent);
     auto put = [&](const void* p, size_t n) {
         const size_t at = h.size();
         h.resize(at + n);
@@ -1061,7 +1060,9 @@ int ensure_origin_plan(Ctx* c, int R, float omax, float step, bool f8, OriginDev
     };
     std::vector<int> rows(b.slots);
     for (int i = 0; i < b.slots; ++i) rows[i] = b.mx[i] < 0 ? -1 : b.mx[i] | b.my[i] << 12 | b.part[i] << 24;
+    const size_t qx = put(b.qx.data(), b.qx.size()), qy = put(b.qy.data(), b.qy.size());
     const size_t slot = put(b.slot.data(), b.slot.size()), row = put(rows.data(), rows.size());
+    const size_t off = put(b.ent_off.data(), b.ent_off.size());
     const size_t q = put(b.q.data(), b.q.size()), f = put(b.f.data(), b.f.size()), words = h.size();
     int r;
     if ((r = o.mem.ensure(sizeof(int) * words))) return r;
@@ -1069,8 +1070,10 @@ int ensure_origin_plan(Ctx* c, int R, float omax, float step, bool f8, OriginDev
     CK(cudaStreamSynchronize(c->stream));
     const int* d = reinterpret_cast<const int*>(o.mem.p);
     o.dev = OriginDev{reinterpret_cast<const float*>(d + q), reinterpret_cast<const float*>(d + f), d + row,
-                      reinterpret_cast<const int2*>(d + slot), b.n1, b.nb, b.slots, b.units, b.R, b.layout, b.mid,
-                      f8 ? 0.0625f : 1.0f};
+                      reinterpret_cast<const int2*>(d + slot), reinterpret_cast<const int4*>(d), d + off,
+                      reinterpret_cast<const float4*>(d + qx), reinterpret_cast<const float4*>(d + qy),
+                      b.n1, b.nb, b.slots, b.units, b.R, b.ent_off.back(),
+                      (int)b.qx.size() / 4, (int)b.qy.size() / 4, b.layout, b.mid, f8 ? 0.0625f : 1.0f};
     o.nx = c->p.fftsize; o.min_r = c->p.min_r; o.R = R; o.omax = omax; o.step = step; o.f8 = f8;
     o.used = ++c->oplan_calls;
     *out = o.dev;

@@ -533,16 +533,15 @@ __global__ void __launch_bounds__(256) k_build_basis(const float2* __restrict__ 
 // (m even) or odd, so a pair of mirror origins costs one pass: per pair of y the sums over
 // even and odd k apart give T_m at both, per pair of x the same over m; (even, odd) sums ride
 // in packed FP32x2 operations.  In one of origin_basis.h's fixed layouts the c_mk sit in
-// registers; more functions (origin ranges beyond ~7 px at maxR n/4) are read from C again for
-// every y (up_eval_gen).
+// registers; more functions (BF16 origin ranges beyond 6 px at maxR n/4, e4m3 beyond 7) lie in
+// shared memory (UpAny below).
 // emit(N, jy, jx, h[N], l[N]): (even, odd) sums over x at y hi and y lo for the pairs of x
 // jx .. jx + N - 1; the value at x hi is their sum, at x lo their difference, where hi =
 // n1/2 + j, lo = (n1-1)/2 - j.
-constexpr int UP_THREADS = 256, UP_GEN = 512, UP_N1 = 1024;
+constexpr int UP_THREADS = 256, UP_N1 = 1024;
 // q at the upper half of the origins, [(n1 + 1) / 2][nb rounded up to even], zero beyond nb
 template <int LY> __host__ __device__ inline int up_table_floats(int n1) {
-    constexpr int NP = LY < 0 ? 0 : (OB_LAYOUT[LY < 0 ? 0 : LY].nb + 1) / 2 * 2;
-    return (n1 + 1) / 2 * NP;
+    return (n1 + 1) / 2 * ((OB_LAYOUT[LY].nb + 1) / 2 * 2);
 }
 template <int LY> __device__ __forceinline__ void up_table(const OriginDev& ob, float* sm) {
     constexpr int NP = (OB_LAYOUT[LY].nb + 1) / 2 * 2;
@@ -641,30 +640,84 @@ __device__ __forceinline__ float up_coef(const OriginDev& ob, const float* U, co
     }
     return s;
 }
-template <class Emit>
-__device__ __forceinline__ void up_eval_gen(const OriginDev& ob, const float* U, const float* V, float sgn, long pitch,
-                                            Emit emit) {
-    const int hn = (ob.n1 + 1) / 2;
-    float2 t[UP_GEN];  // (T_m at y hi, at y lo)
-    for (int jy = 0; jy < hn; ++jy) {
-        const int iy = ob.n1 / 2 + jy;
-        for (int m = 0; m < ob.nb; ++m) {
-            float e = 0.0f, o = 0.0f;
-            for (int k = 0; k < ob.nb; ++k) {
-                const float cq = up_coef(ob, U, V, sgn, pitch, m, k) * __ldg(ob.q + (long)k * ob.n1 + iy);
-                if (k & 1) o += cq;
-                else e += cq;
-            }
-            t[m] = make_float2(e + o, e - o);
+// Any number of functions.  A warp has 32 columns (a lane each) and a pair of y: for UM_X or UL_X pairs
+// of x at a time it goes through the functions m in (even, odd) couples, forms T_m at its y from the
+// couple's products and adds T_m q_m(x) to the sums in registers, so that neither T nor the products
+// need registers of their own and nothing bounds the number of functions.  The products are combined
+// (u +- v, second rows) once for all warps of a block and lie in shared memory four to a 16-byte entry
+// (OriginBasis::ent), in chunks of entries where they are too many.  Bound: shared memory, five 128-byte
+// reads (an entry of 32 lanes and its q) for each four functions, and the instructions of few warps.
+constexpr int UM_X = 16, UM_SHARES = 4, UL_X = 8, UL_THREADS = 256;  // exhaustive, lists
+struct UpAny {
+    const float4* c;        // the chunk's products: entry e of the chunk of this lane's column at c[e * cols]
+    int cols;
+    const float4 *qx, *qy;  // OriginBasis::qx, qy
+    const int* off;         // [h + 1] entries
+    int h;                  // (nb + 1) / 2
+};
+// q's tables (QSH: into shared memory; else they are read where they are) and the entry offsets, by the
+// whole block: qx, qy, offsets from sm
+template <bool QSH>
+__device__ __forceinline__ UpAny up_any_tables(const OriginDev& ob, unsigned char* sm) {
+    const int h = (ob.nb + 1) / 2;
+    float4* q = reinterpret_cast<float4*>(sm);
+    int* off = reinterpret_cast<int*>(q + (QSH ? ob.nqx + ob.nqy : 0));
+    if (QSH) {
+        for (int i = threadIdx.x; i < ob.nqx; i += blockDim.x) q[i] = ob.qx[i];
+        for (int i = threadIdx.x; i < ob.nqy; i += blockDim.x) q[ob.nqx + i] = ob.qy[i];
+    }
+    for (int i = threadIdx.x; i <= h; i += blockDim.x) off[i] = ob.ent_off[i];
+    return UpAny{nullptr, 0, QSH ? q : ob.qx, QSH ? q + ob.nqx : ob.qy, off, h};
+}
+// shared memory of the tables, a multiple of 16 bytes
+__host__ __device__ inline size_t up_any_table_bytes(const OriginDev& ob, bool qsh) {
+    const int h = (ob.nb + 1) / 2;
+    return (qsh ? sizeof(float4) * (ob.nqx + ob.nqy) : 0) + (sizeof(int) * (h + 1) + 15) / 16 * 16;
+}
+// The rows of entry i: part 0, part 1 of its four functions.
+__device__ __forceinline__ void up_any_rows(const OriginDev& ob, int i, int (&rows)[8]) {
+    const int4 a = __ldg(ob.ent + 2 * i), b = __ldg(ob.ent + 2 * i + 1);
+    rows[0] = a.x, rows[1] = a.y, rows[2] = a.z, rows[3] = a.w;
+    rows[4] = b.x, rows[5] = b.y, rows[6] = b.z, rows[7] = b.w;
+}
+// the four functions' products of one sign of v
+__device__ __forceinline__ float4 up_any_four(const float* u, const float* v, float sgn, float lo) {
+    float c[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c[k] = fmaf(fmaf(sgn, v[2 * k + 1], u[2 * k + 1]), lo, fmaf(sgn, v[2 * k], u[2 * k]));
+    return make_float4(c[0], c[1], c[2], c[3]);
+}
+// adds the chunk e0 .. e1 (even) to the sums of the pair of y jy over the N pairs of x from x0 (up to UM_X
+// beyond the last: zeros): (even, odd) sums h, l at y hi, lo
+template <int N>
+__device__ __forceinline__ void up_any_add(const UpAny& A, int e0, int e1, int jy, int x0, float2 (&h)[N], float2 (&l)[N]) {
+    const float4* qy = A.qy + jy * ((A.h + 1) / 2);
+    for (int a = 0; a < A.h; ++a) {
+        const int o = A.off[a], i0 = max(o, e0), i1 = min(A.off[a + 1], e1);
+        if (i0 >= i1) continue;
+        float2 e[2], d[2];  // (sums over even k, over odd k) of functions 2a and 2a + 1, of every other entry
+        e[0] = e[1] = d[0] = d[1] = make_float2(0.f, 0.f);
+        const float4* c = A.c + (i0 - e0) * A.cols;
+        const float4* q = qy + (i0 - o) / 2;
+#pragma unroll 2
+        for (int i = i0; i < i1; i += 2, c += 2 * A.cols, ++q) {
+            const float4 c0 = c[0], c1 = c[A.cols], v = *q;
+            e[0] = __ffma2_rn(make_float2(c0.x, c0.y), make_float2(v.x, v.y), e[0]);
+            d[0] = __ffma2_rn(make_float2(c0.z, c0.w), make_float2(v.x, v.y), d[0]);
+            e[1] = __ffma2_rn(make_float2(c1.x, c1.y), make_float2(v.z, v.w), e[1]);
+            d[1] = __ffma2_rn(make_float2(c1.z, c1.w), make_float2(v.z, v.w), d[1]);
         }
-        for (int jx = 0; jx < hn; ++jx) {
-            float2 h = make_float2(0.f, 0.f), l = make_float2(0.f, 0.f);
-            for (int m = 0; m < ob.nb; ++m) {
-                const float q = __ldg(ob.q + (long)m * ob.n1 + ob.n1 / 2 + jx);
-                if (m & 1) { h.y = fmaf(t[m].x, q, h.y); l.y = fmaf(t[m].y, q, l.y); }
-                else { h.x = fmaf(t[m].x, q, h.x); l.x = fmaf(t[m].y, q, l.x); }
-            }
-            emit(std::integral_constant<int, 1>(), jy, jx, &h, &l);
+        e[0] = __fadd2_rn(e[0], e[1]);
+        d[0] = __fadd2_rn(d[0], d[1]);
+        const float2 th = make_float2(e[0].x + e[0].y, d[0].x + d[0].y), tl = make_float2(e[0].x - e[0].y, d[0].x - d[0].y);
+        const float4* qx = A.qx + x0 / 2 * A.h + a;
+#pragma unroll
+        for (int u = 0; u < N; u += 2) {
+            const float4 v = qx[u / 2 * A.h];
+            h[u] = __ffma2_rn(th, make_float2(v.x, v.y), h[u]);
+            l[u] = __ffma2_rn(tl, make_float2(v.x, v.y), l[u]);
+            h[u + 1] = __ffma2_rn(th, make_float2(v.z, v.w), h[u + 1]);
+            l[u + 1] = __ffma2_rn(tl, make_float2(v.z, v.w), l[u + 1]);
         }
     }
 }
@@ -725,19 +778,93 @@ __global__ void __launch_bounds__(UP_THREADS, 1) k_up_max(OriginDev ob, const fl
         if (r < rows) ccmax[p * (rows / nomr * nom) + r / nomr * nom + r % nomr + (long)half * nomr] = best;
     }
 }
-// Any number of rows and functions: one thread per (bank row, particle, half turn).
-__global__ void __launch_bounds__(128) k_up_max_gen(OriginDev ob, const float* __restrict__ C, long pitch, long rows,
-                                                    int nom, int nomr, float* __restrict__ ccmax) {
-    const long r = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    const int p = blockIdx.y, parts = nom / nomr;
-    const float* U = C + (long)p * parts * ob.slots * pitch + r;
-    const float* V = parts > 1 ? U + ob.slots * pitch : nullptr;
+// Any number of functions: blocks of 64 orientations (32 bank rows and the half turn, or 64 bank rows) by 4
+// shares of y.  Issue 50 %, shared memory 60 %, the rest waits for the block's products.  A particle of
+// box 256 on the 1-degree grid at +-6.5 px (320 rows): 0.23 ms, at +-10 px 0.68, its contraction 0.59;
+// with every product read from C again for every pair of y 2.4 and 3.8 ms.  Two shares of y 0.19 and 0.90; two
+// pairs of y a warp (fewer reads, half the warps) 0.26; pairs of x 8 at a time 0.26.
+constexpr int UM_COLS = 64, UM_THREADS = UM_COLS * UM_SHARES;
+template <bool QSH, int W>
+__global__ void __launch_bounds__(UM_THREADS, 2) k_up_max_any(OriginDev ob, const float* __restrict__ C, long pitch,
+                                                              long rows, int nom, int nomr, int chunk,
+                                                              float* __restrict__ ccmax) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ float sbest[UM_SHARES - 1][UM_COLS];
+    const int hn = (ob.n1 + 1) / 2, ne = ob.nent;
+    float4* sc = reinterpret_cast<float4*>(smraw + up_any_table_bytes(ob, QSH));  // [chunk][UM_COLS]
+    const bool two = nom != nomr;
+    const int cols = two ? UM_COLS / 2 : UM_COLS;
+    const int p = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long r0 = (long)blockIdx.x * cols;
+    const float* U = C + (long)p * (two ? 2 : 1) * ob.slots * pitch + r0;  // (pitch: whole tiles of 256)
+    const float* V = U + ob.slots * pitch;
+    const int col = 32 * (warp & 1) + lane, share = warp >> 1;
+    UpAny A = up_any_tables<QSH>(ob, smraw);
+    A.c = sc + col;
+    A.cols = UM_COLS;
+    auto load = [&](int e0, int e1) {
+        __syncthreads();
+        // four columns of an entry a thread, 16 bytes a load
+        const int lg = two ? 3 : 4;  // threads an entry
+        for (int i = threadIdx.x; i < (e1 - e0) << lg; i += UM_THREADS) {
+            const int e = i >> lg, c = 4 * (i & ((1 << lg) - 1));
+            int row[8];
+            up_any_rows(ob, e0 + e, row);
+            float w[2][4][4];  // [sign][column][function]
+#pragma unroll
+            for (int f = 0; f < 4; ++f) {
+                float4 u[2], v[2];
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    u[k] = v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    const int at = row[2 * f + k];
+                    if (at < 0) continue;
+                    u[k] = __ldg(reinterpret_cast<const float4*>(U + at * pitch + c));
+                    if (two) v[k] = __ldg(reinterpret_cast<const float4*>(V + at * pitch + c));
+                }
+                const float4 a = make_float4(fmaf(u[1].x, ob.lo, u[0].x), fmaf(u[1].y, ob.lo, u[0].y),
+                                             fmaf(u[1].z, ob.lo, u[0].z), fmaf(u[1].w, ob.lo, u[0].w));
+                const float4 b = make_float4(fmaf(v[1].x, ob.lo, v[0].x), fmaf(v[1].y, ob.lo, v[0].y),
+                                             fmaf(v[1].z, ob.lo, v[0].z), fmaf(v[1].w, ob.lo, v[0].w));
+                w[0][0][f] = a.x + b.x, w[0][1][f] = a.y + b.y, w[0][2][f] = a.z + b.z, w[0][3][f] = a.w + b.w;
+                w[1][0][f] = a.x - b.x, w[1][1][f] = a.y - b.y, w[1][2][f] = a.z - b.z, w[1][3][f] = a.w - b.w;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float4* at = sc + e * UM_COLS + c + j;
+                at[0] = make_float4(w[0][j][0], w[0][j][1], w[0][j][2], w[0][j][3]);
+                if (two) at[UM_COLS / 2] = make_float4(w[1][j][0], w[1][j][1], w[1][j][2], w[1][j][3]);
+            }
+        }
+        __syncthreads();
+    };
+    if (chunk >= ne) load(0, ne);
     float best = -3.0e38f;
-    up_eval_gen(ob, U, V, blockIdx.z ? -1.0f : 1.0f, pitch, [&](auto, int, int, const float2* h, const float2* l) {
-        best = fmaxf(best, fmaxf(h->x + fabsf(h->y), l->x + fabsf(l->y)));
-    });
-    ccmax[(long)p * (rows / nomr * nom) + r / nomr * nom + r % nomr + (long)blockIdx.z * nomr] = best;
+    for (int x0 = 0; x0 < hn; x0 += W)
+        for (int j0 = 0; j0 < hn; j0 += UM_SHARES) {
+            float2 ah[W], al[W];
+#pragma unroll
+            for (int u = 0; u < W; ++u) ah[u] = al[u] = make_float2(0.f, 0.f);
+            const int jy = j0 + share;
+            for (int e0 = 0; e0 < ne; e0 += chunk) {
+                const int e1 = min(ne, e0 + chunk);
+                if (chunk < ne) load(e0, e1);
+                if (jy >= hn) continue;
+                up_any_add(A, e0, e1, jy, x0, ah, al);
+            }
+            if (jy >= hn) continue;
+#pragma unroll
+            for (int u = 0; u < W; ++u)
+                if (x0 + u < hn) best = fmaxf(best, fmaxf(ah[u].x + fabsf(ah[u].y), al[u].x + fabsf(al[u].y)));
+        }
+    if (share) sbest[share - 1][col] = best;
+    __syncthreads();
+    if (share) return;
+#pragma unroll
+    for (int i = 0; i < UM_SHARES - 1; ++i) best = fmaxf(best, sbest[i][col]);
+    const int half = two ? warp & 1 : 0;
+    const long r = r0 + (two ? lane : col);
+    if (r < rows) ccmax[(long)p * (rows / nomr * nom) + r / nomr * nom + r % nomr + (long)half * nomr] = best;
 }
 
 // Per (particle, block of 256 orientations): the best value and its orientation.
@@ -766,6 +893,7 @@ __global__ void __launch_bounds__(256) k_tile_best(const float* __restrict__ ccm
 
 // Best origin (index iy n1 + ix) of the selected orientations: one block per (candidate,
 // particle), a thread per row of origins in turn.
+constexpr int UO_X = 32;  // origins of a row at a time
 __global__ void __launch_bounds__(128) k_up_origin(OriginDev ob, const float* __restrict__ C, long pitch, int nom,
                                                    int nomr, const int* __restrict__ orient, int k,
                                                    int* __restrict__ origin) {
@@ -779,20 +907,24 @@ __global__ void __launch_bounds__(128) k_up_origin(OriginDev ob, const float* __
         const long r = (long)(n / nom) * nomr + io % nomr;
         const float* U = C + (long)p * parts * ob.slots * pitch + r;
         const float* V = parts > 1 ? U + ob.slots * pitch : nullptr;
-        float t[UP_GEN];
-        for (int iy = threadIdx.x; iy < ob.n1; iy += blockDim.x) {
-            for (int m = 0; m < ob.nb; ++m) {
-                float s = 0.0f;
-                for (int q = 0; q < ob.nb; ++q)
-                    s = fmaf(up_coef(ob, U, V, io >= nomr ? -1.0f : 1.0f, pitch, m, q), ob.q[(long)q * ob.n1 + iy], s);
-                t[m] = s;
+        for (int iy = threadIdx.x; iy < ob.n1; iy += blockDim.x)
+            for (int x0 = 0; x0 < ob.n1; x0 += UO_X) {
+                float s[UO_X];
+#pragma unroll
+                for (int j = 0; j < UO_X; ++j) s[j] = 0.0f;
+                for (int m = 0; m < ob.nb; ++m) {
+                    float t = 0.0f;
+                    for (int q = 0; q < ob.nb; ++q)
+                        t = fmaf(up_coef(ob, U, V, io >= nomr ? -1.0f : 1.0f, pitch, m, q), ob.q[(long)q * ob.n1 + iy], t);
+                    const float* qx = ob.q + (long)m * ob.n1 + x0;
+#pragma unroll
+                    for (int j = 0; j < UO_X; ++j)
+                        if (x0 + j < ob.n1) s[j] = fmaf(t, qx[j], s[j]);
+                }
+#pragma unroll
+                for (int j = 0; j < UO_X; ++j)
+                    if (x0 + j < ob.n1 && s[j] > bv) { bv = s[j]; bi = iy * ob.n1 + x0 + j; }
             }
-            for (int ix = 0; ix < ob.n1; ++ix) {
-                float s = 0.0f;
-                for (int m = 0; m < ob.nb; ++m) s = fmaf(t[m], ob.q[(long)m * ob.n1 + ix], s);
-                if (s > bv) { bv = s; bi = iy * ob.n1 + ix; }
-            }
-        }
     }
     for (int off = 16; off > 0; off >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, bv, off);
@@ -811,38 +943,57 @@ __global__ void __launch_bounds__(128) k_up_origin(OriginDev ob, const float* __
 // Listed orientations (the proposal forms): one block per (block of 256 list positions,
 // particle) gives, per origin, the best of its positions and which it is (the first of
 // equal ones), as the argmax contraction does for a local grid's columns.  A warp takes 32
-// positions at a time and keeps its running maxima over the origins in shared memory (shm;
-// else one warp works on the output itself); the maximum of 32 lanes by redux on the
+// positions at a time and keeps its running maxima over the origins in shared memory; the
+// maximum of 32 lanes by redux on the
 // order-preserving integer image of the value, up to 16 origins at a time so that their
 // latencies overlap (one origin at a time, with its update in between: 185 us a 64-particle
 // pass of the box-256 search; so: 137 us).  gridDim.z blocks share a tile's origins by rows (pairs of
 // y about the middle) where a call has few tiles: one particle's three, 625 origins, 60 -> 23 us.
+
+// The maxima of 4 N origins (up_eval's pairs of x jx .. jx + N - 1 at the pair of y jy) over a
+// warp's 32 positions: they are independent, lane i keeps the i-th and hands it to put(y, x, value, lane of the
+// maximum).
+template <int N, class Put>
+__device__ __forceinline__ void list_max(const float2* h, const float2* l, bool valid, int n1, int jy, int jx, Put put) {
+    const int lane = threadIdx.x & 31;
+    float mine = 0.0f;
+    int who = -1;
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        const float v[4] = {h[u].x + h[u].y, h[u].x - h[u].y, l[u].x + l[u].y, l[u].x - l[u].y};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const unsigned x = __float_as_uint(v[q]);
+            const unsigned key = valid ? ((x & 0x80000000u) ? ~x : (x | 0x80000000u)) : 0u;
+            const unsigned mx = __reduce_max_sync(0xffffffffu, key);
+            const unsigned eq = __ballot_sync(0xffffffffu, key == mx);
+            if (lane == 4 * u + q) {
+                mine = __uint_as_float((mx & 0x80000000u) ? (mx & 0x7fffffffu) : ~mx);
+                who = __ffs(eq) - 1;
+            }
+        }
+    }
+    const int jj = jx + (lane >> 2);
+    if (who >= 0 && jj < (n1 + 1) / 2)
+        put((lane & 2) ? (n1 - 1) / 2 - jy : n1 / 2 + jy, (lane & 1) ? (n1 - 1) / 2 - jj : n1 / 2 + jj, mine, who);
+}
 template <int LY>
 __global__ void __launch_bounds__(256, 1) k_up_list(OriginDev ob, const float* __restrict__ C, int parts,
                                                     const UpGroup* __restrict__ groups, const int* __restrict__ map,
-                                                    float* __restrict__ topv, int* __restrict__ topi, int shm) {
+                                                    float* __restrict__ topv, int* __restrict__ topi) {
     extern __shared__ __align__(16) float smem[];
     const UpGroup g = groups[blockIdx.y];
     const int tile = blockIdx.x;
     if (tile >= g.ntiles) return;
     const int O = ob.n1 * ob.n1, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    float* sv = smem + up_table_floats<LY>(ob.n1);
-    int* si = reinterpret_cast<int*>(sv + nw * O);
+    float* sv = smem + up_table_floats<LY>(ob.n1) + warp * O;
+    int* si = reinterpret_cast<int*>(smem + up_table_floats<LY>(ob.n1) + nw * O) + warp * O;
     float* ov = topv + g.topv_off + tile;  // stride ntiles
     int* oi = topi + g.topv_off + tile;
-    long stride = 1;
-    if (shm) {
-        sv += warp * O;
-        si += warp * O;
-    } else {
-        sv = ov;
-        si = oi;
-        stride = g.ntiles;
-    }
     const int hn = (ob.n1 + 1) / 2;
     const int jy0 = hn * (int)blockIdx.z / (int)gridDim.z, jy1 = hn * ((int)blockIdx.z + 1) / (int)gridDim.z;
-    if constexpr (LY >= 0) up_table<LY>(ob, smem);
-    for (int o = lane; o < O; o += 32) { sv[o * stride] = -3.0e38f; si[o * stride] = -1; }
+    up_table<LY>(ob, smem);
+    for (int o = lane; o < O; o += 32) { sv[o] = -3.0e38f; si[o] = -1; }
     __syncthreads();
     const long pitch = 256L * g.n_tiles;
     for (int c = warp; c < 8; c += nw) {
@@ -854,52 +1005,26 @@ __global__ void __launch_bounds__(256, 1) k_up_list(OriginDev ob, const float* _
         const float* U = C + g.c_off + (mp >> 1);
         const float* V = parts > 1 ? U + ob.slots * pitch : nullptr;
         const float sgn = (mp & 1) ? -1.0f : 1.0f;
-        // 4 N origins at a time: their warp maxima are independent, lane i keeps the i-th and
-        // updates its running maximum
-        auto emit = [&](auto nc, int jy, int jx, const float2* h, const float2* l) {
-            constexpr int N = decltype(nc)::value;
-            float mine = 0.0f;
-            int who = -1;
-#pragma unroll
-            for (int u = 0; u < N; ++u) {
-                const float v[4] = {h[u].x + h[u].y, h[u].x - h[u].y, l[u].x + l[u].y, l[u].x - l[u].y};
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const unsigned x = __float_as_uint(v[q]);
-                    const unsigned key = valid ? ((x & 0x80000000u) ? ~x : (x | 0x80000000u)) : 0u;
-                    const unsigned mx = __reduce_max_sync(0xffffffffu, key);
-                    const unsigned eq = __ballot_sync(0xffffffffu, key == mx);
-                    if (lane == 4 * u + q) {
-                        mine = __uint_as_float((mx & 0x80000000u) ? (mx & 0x7fffffffu) : ~mx);
-                        who = __ffs(eq) - 1;
-                    }
-                }
-            }
-            if (who >= 0) {
-                const int jj = jx + (lane >> 2);
-                const int y = (lane & 2) ? (ob.n1 - 1) / 2 - jy : ob.n1 / 2 + jy;
-                const int x = (lane & 1) ? (ob.n1 - 1) / 2 - jj : ob.n1 / 2 + jj;
-                const long o = (long)(y * ob.n1 + x) * stride;
-                if (mine > sv[o]) {
-                    sv[o] = mine;
-                    si[o] = j0 + who;
-                }
+        // (neighbouring list positions mostly stand for neighbouring columns)
+        UpCoef<LY> cf;
+        cf.load(ob.lo, [&](int i) {
+            const float u = __ldg(U + i * pitch);
+            return V ? fmaf(sgn, __ldg(V + i * pitch), u) : u;
+        });
+        auto keep = [&](int y, int x, float v, int who) {
+            const int o = y * ob.n1 + x;
+            if (v > sv[o]) {
+                sv[o] = v;
+                si[o] = j0 + who;
             }
         };
-        if constexpr (LY >= 0) {
-            // (neighbouring list positions mostly stand for neighbouring columns)
-            UpCoef<LY> c;
-            c.load(ob.lo, [&](int i) {
-                const float u = __ldg(U + i * pitch);
-                return V ? fmaf(sgn, __ldg(V + i * pitch), u) : u;
-            });
-            up_eval<LY>(ob, c, smem, emit, jy0, jy1);
-        } else {
-            up_eval_gen(ob, U, V, sgn, pitch, emit);
-        }
+        up_eval<LY>(ob, cf, smem,
+                    [&](auto nc, int jy, int jx, const float2* h, const float2* l) {
+                        list_max<decltype(nc)::value>(h, l, valid, ob.n1, jy, jx, keep);
+                    },
+                    jy0, jy1);
         __syncwarp();  // the next 32 positions update these maxima from other lanes
     }
-    if (!shm) return;
     __syncthreads();
     sv = smem + up_table_floats<LY>(ob.n1);
     si = reinterpret_cast<int*>(sv + nw * O);
@@ -915,6 +1040,99 @@ __global__ void __launch_bounds__(256, 1) k_up_list(OriginDev ob, const float* _
         }
         ov[(long)o * g.ntiles] = bv;
         oi[(long)o * g.ntiles] = bi;
+    }
+}
+
+// The same for any number of functions and origins.  A task is a pair of y and UL_X pairs of x: 32 origins, a
+// lane each.  A warp's tasks are its own for all positions of the tile, which the block goes through 32 at a
+// time, so that an origin's maximum is one warp's alone.  blockIdx.z blocks share a tile's tasks.  One particle's
+// lists of box 256 at +-8 px (33 x 33 origins): 73 us, 64 particles' 356; with every product read from C
+// again for every pair of y 1.4 and 3.1 ms.  Two pairs of y and 16 of x a task 188 and 380 us.
+template <bool QSH>
+__global__ void __launch_bounds__(UL_THREADS, 2) k_up_list_any(OriginDev ob, const float* __restrict__ C, int parts,
+                                                               const UpGroup* __restrict__ groups,
+                                                               const int* __restrict__ map, int chunk,
+                                                               float* __restrict__ topv, int* __restrict__ topi) {
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const UpGroup g = groups[blockIdx.y];
+    const int tile = blockIdx.x;
+    if (tile >= g.ntiles) return;
+    const int hn = (ob.n1 + 1) / 2, ne = ob.nent, n1 = ob.n1;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int NW = UL_THREADS / 32;
+    const int nx = (hn + UL_X - 1) / UL_X, tasks = hn * nx;
+    const int t0 = (int)((long)tasks * blockIdx.z / gridDim.z), t1 = (int)((long)tasks * (blockIdx.z + 1) / gridDim.z);
+    float4* sc = reinterpret_cast<float4*>(smraw + up_any_table_bytes(ob, QSH));  // [chunk][32]
+    float* sv = reinterpret_cast<float*>(sc + chunk * 32);                        // [t1 - t0][32]
+    int* si = reinterpret_cast<int*>(sv + (t1 - t0) * 32);
+    for (int t = t0 + warp; t < t1; t += NW) {
+        sv[(t - t0) * 32 + lane] = -3.0e38f;
+        si[(t - t0) * 32 + lane] = -1;
+    }
+    const long pitch = 256L * g.n_tiles;
+    UpAny A = up_any_tables<QSH>(ob, smraw);
+    A.c = sc + lane;
+    A.cols = 32;
+    for (int c = 0; c < 8; ++c) {
+        const int j0 = tile * 256 + c * 32;
+        if (j0 >= g.n_list) break;
+        const bool valid = j0 + lane < g.n_list;
+        const int mp = map[g.map_off + (valid ? j0 + lane : 0)];  // (of this lane's column, which it also loads)
+        const float* U = C + g.c_off + (mp >> 1);
+        const float* V = U + ob.slots * pitch;
+        const float sgn = (mp & 1) ? -1.0f : 1.0f;
+        auto load = [&](int e0, int e1) {
+            __syncthreads();
+            // an entry a warp, two at a time: up to 32 loads in flight
+            for (int e = e0 + warp; e < e1; e += 2 * NW) {
+                float u[2][8], v[2][8];
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    int row[8];
+                    up_any_rows(ob, min(e + t * NW, e1 - 1), row);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const bool in = row[k] >= 0 && e + t * NW < e1;
+                        u[t][k] = in ? __ldg(U + row[k] * pitch) : 0.0f;
+                        v[t][k] = in && parts > 1 ? __ldg(V + row[k] * pitch) : 0.0f;
+                    }
+                }
+#pragma unroll
+                for (int t = 0; t < 2; ++t)
+                    if (e + t * NW < e1) sc[(e + t * NW - e0) * 32 + lane] = up_any_four(u[t], v[t], sgn, ob.lo);
+            }
+            __syncthreads();
+        };
+        if (chunk >= ne) load(0, ne);
+        for (int tb = t0; tb < t1; tb += NW) {
+            const int t = tb + warp, jy = t / nx, x0 = (t - jy * nx) * UL_X;
+            float2 ah[UL_X], al[UL_X];
+#pragma unroll
+            for (int u = 0; u < UL_X; ++u) ah[u] = al[u] = make_float2(0.f, 0.f);
+            for (int e0 = 0; e0 < ne; e0 += chunk) {
+                const int e1 = min(ne, e0 + chunk);
+                if (chunk < ne) load(e0, e1);
+                if (t < t1) up_any_add(A, e0, e1, jy, x0, ah, al);
+            }
+            if (t >= t1) continue;
+            const int at = (t - t0) * 32 + lane;
+            list_max<UL_X>(ah, al, valid, n1, jy, x0, [&](int, int, float v, int who) {
+                if (v > sv[at]) {
+                    sv[at] = v;
+                    si[at] = j0 + who;
+                }
+            });
+        }
+    }
+    float* ov = topv + g.topv_off + tile;  // stride ntiles
+    int* oi = topi + g.topv_off + tile;
+    for (int t = t0 + warp; t < t1; t += NW) {
+        const int jy = t / nx, jx = (t - jy * nx) * UL_X + (lane >> 2), at = (t - t0) * 32 + lane;
+        if (jx >= hn) continue;
+        // (hi and lo are the same row, or column, in the middle of an odd grid: equal values)
+        const int y = (lane & 2) ? (n1 - 1) / 2 - jy : n1 / 2 + jy, x = (lane & 1) ? (n1 - 1) / 2 - jx : n1 / 2 + jx;
+        ov[((long)y * n1 + x) * g.ntiles] = sv[at];
+        oi[((long)y * n1 + x) * g.ntiles] = si[at];
     }
 }
 
@@ -1286,6 +1504,24 @@ cudaError_t launch_build_basis(const float2* band, const float* ctf, Band bd, co
 // the register kernels: a fixed layout, and origins whose table leaves room for the products
 static int up_layout(const OriginDev& ob) { return ob.n1 <= UP_N1 ? ob.layout : -1; }
 
+// Shared memory of the kernels for any number of functions: q's table where it is small, then as many
+// entries of cols columns as leave two blocks an SM (113 KB each), at least 16.
+struct UpAnyShape {
+    bool qsh;
+    int chunk;
+    size_t smem;
+};
+static UpAnyShape up_any_shape(const OriginDev& ob, int cols, size_t more) {
+    UpAnyShape s;
+    const size_t room = 110 * 1024 - more, entry = sizeof(float4) * cols;
+    s.qsh = up_any_table_bytes(ob, true) <= 32 * 1024;
+    const size_t tab = up_any_table_bytes(ob, s.qsh);
+    const size_t fit = room > tab + 16 * entry ? (room - tab) / entry : 16;
+    s.chunk = (int)std::min<size_t>(fit / 2 * 2, std::max(2, ob.nent));
+    s.smem = tab + s.chunk * entry + more;
+    return s;
+}
+
 cudaError_t launch_up_topk(const OriginDev& ob, const float* C, long pitch, long rows, int nom, int nomr, int B, int k,
                            float* ccmax, int ntiles, float* tile_v, int* tile_o, int* orient, int* origin, float* cc,
                            bool want_origin, int num_sms, cudaStream_t st) {
@@ -1312,8 +1548,19 @@ cudaError_t launch_up_topk(const OriginDev& ob, const float* C, long pitch, long
         }
         if (e != cudaSuccess) return e;
     } else {
-        const dim3 g((unsigned)((rows + 127) / 128), B, nom / nomr);
-        k_up_max_gen<<<g, 128, 0, st>>>(ob, C, pitch, rows, nom, nomr, ccmax);
+        const int cols = nom == nomr ? UM_COLS : UM_COLS / 2;
+        const UpAnyShape sh = up_any_shape(ob, UM_COLS, 0);
+        // pairs of x at a time: as few turns as UM_X allows, in turns of one width
+        const int hn = (ob.n1 + 1) / 2, turns = (hn + UM_X - 1) / UM_X, w = ((hn + turns - 1) / turns + 1) / 2 * 2;
+        auto kern = !sh.qsh   ? k_up_max_any<false, UM_X>
+                    : w <= 8  ? k_up_max_any<true, 8>
+                    : w <= 10 ? k_up_max_any<true, 10>
+                    : w <= 12 ? k_up_max_any<true, 12>
+                    : w <= 14 ? k_up_max_any<true, 14>
+                              : k_up_max_any<true, UM_X>;
+        if ((e = allow_smem(kern, sh.smem)) != cudaSuccess) return e;
+        kern<<<dim3((unsigned)((rows + cols - 1) / cols), B), UM_THREADS, sh.smem, st>>>(ob, C, pitch, rows, nom, nomr,
+                                                                                        sh.chunk, ccmax);
     }
     k_tile_best<<<dim3(ntiles, B), 256, 0, st>>>(ccmax, n_orient, ntiles, tile_v, tile_o);
     k_select_topk<<<B, 512, 0, st>>>(tile_v, tile_o, ntiles, k, orient, cc);
@@ -1327,23 +1574,34 @@ cudaError_t launch_up_topk(const OriginDev& ob, const float* C, long pitch, long
 cudaError_t launch_up_list(const OriginDev& ob, const float* C, int parts, const UpGroup* groups, int ngroups,
                            int max_tiles, const int* map, float* topv, int* topi, cudaStream_t st) {
     const int O = ob.n1 * ob.n1, ly = up_layout(ob);
-    // warps per block: the running maxima of each over the origins in shared memory; one warp
-    // on the output itself where a single one does not fit
-    const size_t tab = sizeof(float) * (ly >= 0 ? (ob.n1 + 1) / 2 * ((ob.nb + 1) / 2 * 2) : 0);
+    // warps per block: the running maxima of each over the origins in shared memory
+    const size_t tab = sizeof(float) * ((ob.n1 + 1) / 2 * ((ob.nb + 1) / 2 * 2));
     int nw = 8;
     while (nw > 1 && tab + (size_t)nw * O * 8 > 220 * 1024) nw /= 2;
-    const bool shm = tab + (size_t)nw * O * 8 <= 220 * 1024;
-    const size_t sm = tab + (shm ? (size_t)nw * O * 8 : 0);
-    auto kern = ly < 0 ? k_up_list<-1> : ly == 0 ? k_up_list<0> : ly == 1 ? k_up_list<1> : ly == 2 ? k_up_list<2>
-                : ly == 3 ? k_up_list<3> : k_up_list<4>;
+    const size_t sm = tab + (size_t)nw * O * 8;
+    if (ly < 0 || sm > 220 * 1024) {
+        // blocks to a tile: as many as find an SM (each combines its positions' products again), and as
+        // hold the maxima of their tasks in 48 KB
+        const int hn = (ob.n1 + 1) / 2, tasks = hn * ((hn + UL_X - 1) / UL_X), nw = UL_THREADS / 32;
+        const int most = 48 * 1024 / (32 * 8), fill = 2 * 152 / std::max(1, max_tiles * ngroups);
+        const int z = std::max((tasks + most - 1) / most, std::min(fill, (tasks + nw - 1) / nw));
+        const UpAnyShape sh = up_any_shape(ob, 32, (size_t)((tasks + z - 1) / z) * 32 * (sizeof(float) + sizeof(int)));
+        auto kern = sh.qsh ? k_up_list_any<true> : k_up_list_any<false>;
+        const cudaError_t e = allow_smem(kern, sh.smem);
+        if (e != cudaSuccess) return e;
+        kern<<<dim3(max_tiles, ngroups, z), UL_THREADS, sh.smem, st>>>(ob, C, parts, groups, map, sh.chunk, topv, topi);
+        return cudaGetLastError();
+    }
+    auto kern = ly == 0 ? k_up_list<0> : ly == 1 ? k_up_list<1> : ly == 2 ? k_up_list<2> : ly == 3 ? k_up_list<3>
+                                                                                                    : k_up_list<4>;
     cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return e;
     // blocks to a tile: as many as find an SM of their own (each reads its tile's products again, so that with
     // the SMs filled, by this launch or by other lanes', the pass takes longer: 14.0 -> 14.5 ms of the box-256
     // search with 192 tiles cut in three)
     int z = 1;
-    if (shm && ly >= 0) z = std::max(1, std::min(std::min(8, (ob.n1 + 1) / 2), 152 / std::max(1, max_tiles * ngroups)));
-    kern<<<dim3(max_tiles, ngroups, z), 32 * nw, sm, st>>>(ob, C, parts, groups, map, topv, topi, shm ? 1 : 0);
+    z = std::max(1, std::min(std::min(8, (ob.n1 + 1) / 2), 152 / std::max(1, max_tiles * ngroups)));
+    kern<<<dim3(max_tiles, ngroups, z), 32 * nw, sm, st>>>(ob, C, parts, groups, map, topv, topi);
     return cudaGetLastError();
 }
 

@@ -272,7 +272,13 @@ struct OriginDev {
     const float* f;     // [nb][2 R + 1]
     const int* row;     // [slots]: mx | my << 12 | part << 24, -1 empty
     const int2* slot;   // [nb nb]: row of part 0, of part 1, -1 none
+    const int4* ent;    // [ent_off[h]][2]: the same, four functions an entry (OriginBasis::ent)
+    const int* ent_off; // [h + 1], h = (nb + 1) / 2
+    const float4* qx;   // OriginBasis::qx
+    const float4* qy;   // OriginBasis::qy
     int n1, nb, slots, units, R;
+    int nent;           // ent_off[h]
+    int nqx, nqy;       // float4s of qx, qy
     int layout;         // fixed places of the rows (OB_LAYOUT), -1: by slot alone
     float mid;
     float lo;           // scale of a second row's products (1, FP8 1/16)

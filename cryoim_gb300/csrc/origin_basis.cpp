@@ -195,6 +195,26 @@ OriginBasis make_origin_basis(int n, int min_r, int R, float omax, float step, i
         for (size_t b = cnt; b < (size_t)ob.slots && b < 2 * cnt; ++b)
             place((int)b, ord[b - cnt] / n1, ord[b - cnt] % n1, 1);
     }
+    for (int a = 0; 2 * a < ob.nb; ++a) {
+        ob.ent_off.push_back((int)ob.ent.size() / 8);
+        size_t used = ob.ent.size();
+        for (int b = 0; 2 * b < ob.nb; ++b) {
+            bool any = false;
+            for (int i = 0; i < 4; ++i) {
+                const int m = 2 * a + i / 2, k = 2 * b + i % 2;
+                const bool in = m < ob.nb && k < ob.nb;
+                for (int part = 0; part < 2; ++part) {
+                    const int v = in ? ob.slot[((size_t)m * ob.nb + k) * 2 + part] : -1;
+                    any = any || v >= 0;
+                    ob.ent.push_back(v);
+                }
+            }
+            if (any) used = ob.ent.size();
+        }
+        ob.ent.resize(used);
+        if ((used / 8 - ob.ent_off.back()) & 1) ob.ent.resize(used + 8, -1);
+    }
+    ob.ent_off.push_back((int)ob.ent.size() / 8);
     ob.q.assign((size_t)ob.nb * n1, 0.0f);
     ob.f.assign((size_t)ob.nb * H, 0.0f);
     ob.ge.assign(ob.nb, 0);
@@ -205,6 +225,13 @@ OriginBasis make_origin_basis(int n, int min_r, int R, float omax, float step, i
         for (int i = 0; i < n1; ++i) ob.q[(size_t)k * n1 + i] = (float)std::ldexp(fun[k][i], -ob.ge[k]);
         for (int h = 0; h < H; ++h) ob.f[(size_t)k * H + h] = (float)std::ldexp(f[(size_t)k * H + h], ob.ge[k]);
     }
+    auto hi = [&](int m, int j) { return m < ob.nb && j < he ? ob.q[(size_t)m * n1 + n1 / 2 + j] : 0.0f; };
+    const int couples = (ob.nb + 1) / 2;
+    for (int j = 0; j < he + 16; j += 2)
+        for (int a = 0; a < couples; ++a)
+            for (int i = 0; i < 4; ++i) ob.qx.push_back(hi(2 * a + i % 2, j + i / 2));
+    for (int j = 0; j < he; ++j)
+        for (int m = 0; m < 2 * ((couples + 1) / 2 * 2); ++m) ob.qy.push_back(hi(m, j));
     return ob;
 }
 

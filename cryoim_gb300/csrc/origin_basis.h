@@ -45,6 +45,14 @@ struct OriginBasis {
     // part 1: what part 0's rounding left (times 16 for FP8); -1: an empty row
     std::vector<int> mx, my, part;
     std::vector<int> slot;   // [nb * nb][2]: row of part 0, of part 1 of function mx * nb + my, -1: none
+    // the functions four at a time: entry i of ent_off[a] .. ent_off[a + 1] has (2a, 2b), (2a, 2b + 1),
+    // (2a + 1, 2b), (2a + 1, 2b + 1) with b = i - ent_off[a]: row of part 0, of part 1 of each, -1: none;
+    // an even number for each a
+    std::vector<int> ent, ent_off;
+    // q at the upper half of the origins, hi(j) = n1/2 + j, by couples of functions, zero beyond: qy
+    // [hn][h rounded up to even][2] = q_2a(hi j), q_2a+1(hi j); qx [hn / 2 rounded up, and 8 more][h][4] =
+    // the couple at j = 2i, then at 2i + 1 (h = (nb + 1) / 2, hn = (n1 + 1) / 2)
+    std::vector<float> qx, qy;
 };
 
 // Origins i = 0 .. n1-1 at -omax + step i on both axes, frequencies |h| <= R (minR <= |h|)

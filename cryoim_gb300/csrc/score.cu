@@ -50,6 +50,7 @@ __device__ __forceinline__ float bilerp(float ax, float ay, float v00, float v10
 
 struct Consts {
     float d2r, r2d, pi, tpi;
+    float margin;  // k_pr_omega in pairs: share of a cut within which an amplitude is in doubt
 };
 
 // Template line sample (template x CTF, bilinear) at angle alpha2, radius fr.
@@ -163,17 +164,21 @@ __device__ __forceinline__ OmegaTerm omega_sample(const float2* sband, int W, in
 // HALF: thread (g, k) owns omega k and k + nomega / 2, half a turn apart.  The particle's
 // samples along a line and along its reverse are complex conjugates (the image is real), so one
 // sample, its amplitude, cut and weight serve both; the cross and dot products differ by the
-// sign of one of the two products each.  The two samples' positions round differently (2e-5
-// px), so where the amplitude lies within PAIR_MARGIN of its cut the second omega's sample is
-// taken by itself and every term passes or fails its cut as the search by single omegas has it.
+// sign of one of the two products each.  The two samples' positions round differently (at box 256 and
+// maxR 64 by 1e-5 px, 8e-5 at most), so where the amplitude lies within a margin of its cut the second
+// omega's sample is taken by itself.  The margin is a rule of thumb: the amplitudes near a cut
+// were seen to differ by up to 3e-4 of it for noise and particles at box 256, 6e-4 beside lattice peaks, and
+// by as much more in a larger box as its positions round more.  A term in doubt beyond it may count
+// at one omega of the pair and not in the search by single omegas, which is then 1 / terms off (2e-5 at
+// 60,000 terms), as the other rounding of a position can have it anyway.
 // Issue-bound (76 %; by single omegas 80 %, and the L1 data pipe 76 %): a particle of box 256 on
 // the 1-degree grid takes 13.1 ms in pairs, 17.8 by single omegas.  The margin's terms are marked
 // and taken after each 32 radii: inside the unrolled loop they cost more than the pairs gain (19
 // ms).  Cells by the add of 2^23 in place of conversions (which wait for the reciprocals'
 // quarter-rate pipe) gained nothing.
-constexpr float PAIR_MARGIN = 5.0e-4f;
+constexpr float PAIR_MARGIN = 5.0e-4f;  // of the cut, up to box 256; beyond (LARGE) as the box
 // SHARE: blockIdx.z takes its share of the omegas (an instance of its own: the indices cost the other 2 %).
-template <bool HALF, bool SHARE>
+template <bool HALF, bool SHARE, bool LARGE>
 __global__ void __launch_bounds__(768, 1) k_pr_omega(PrOmegaArgs a, int nall, int Gall, Consts K) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const Band bd = a.bd;
@@ -259,7 +264,7 @@ __global__ void __launch_bounds__(768, 1) k_pr_omega(PrOmegaArgs a, int nall, in
                 const float2 csn = make_float2(cs, sn);
                 const float4* sl = sline + sjl[jj] * nr;
                 float2 acc = make_float2(0.f, 0.f), acd = make_float2(0.f, 0.f);  // (sum diff*w, sum w) of this line
-for (int q0 = 0; q0 < nr; q0 += 32) {
+                for (int q0 = 0; q0 < nr; q0 += 32) {
                     const int q1 = min(nr, q0 + 32);
                     unsigned near = 0u, bit = 1u;  // HALF: radii whose amplitude is within the margin of its cut
 #pragma unroll 8
@@ -279,7 +284,7 @@ for (int q0 = 0; q0 < nr; q0 += 32) {
                         if constexpr (HALF) {
                             // conj z: (zx ey + zy ex, zx ex - zy ey)
                             const float dc = angle_between_est(pc.x - pc.y, pd.x - pd.y, K.pi);
-                            const bool nr_cut = fabsf(u.amp - e.w) <= PAIR_MARGIN * e.w;
+                            const bool nr_cut = fabsf(u.amp - e.w) <= (LARGE ? K.margin : PAIR_MARGIN) * e.w;
                             const float2 nc = __ffma2_rn(make_float2(dc, 1.0f), make_float2(u.w, u.w), acd);
                             near |= nr_cut ? bit : 0u;
                             acd.x = ok && !nr_cut ? nc.x : acd.x;
@@ -1056,6 +1061,7 @@ Consts consts() {
     K.pi = an.pi;
     K.tpi = an.tpi;
     K.r2d = 180.0f / an.pi;
+    K.margin = 0.0f;
     return K;
 }
 
@@ -1094,11 +1100,14 @@ cudaError_t launch_pr_omega(const PrOmegaArgs& a, int B, cudaStream_t st) {
     int z = 1;
     for (int zz = 2; zz <= 8 && (long)a.V * B * zz <= 152; ++zz)
         if (rounds(zz) < rounds(z)) z = zz;
-    auto kern = z > 1 ? (half ? k_pr_omega<true, true> : k_pr_omega<false, true>)
-                      : (half ? k_pr_omega<true, false> : k_pr_omega<false, false>);
+    const bool large = a.bd.nx > 256;  // (an instance of its own: a margin in a register costs 0.5 %)
+    auto kern = z > 1 ? (!half ? k_pr_omega<false, true, false> : large ? k_pr_omega<true, true, true> : k_pr_omega<true, true, false>)
+                      : (!half ? k_pr_omega<false, false, false> : large ? k_pr_omega<true, false, true> : k_pr_omega<true, false, false>);
     cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return e;
-    kern<<<dim3(a.V, B, z), nt, sm, st>>>(a, nall, G, consts());
+    Consts K = consts();
+    K.margin = PAIR_MARGIN * (float)a.bd.nx / 256.0f;
+    kern<<<dim3(a.V, B, z), nt, sm, st>>>(a, nall, G, K);
     return cudaGetLastError();
 }
 

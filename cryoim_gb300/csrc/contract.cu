@@ -1677,13 +1677,18 @@ cudaError_t launch_slice_bf16_local(cudaTextureObject_t cube, int R, const int2*
                 pctf, sc);
             return cudaGetLastError();
         };
-        // registers for the samples there are, in steps of two a thread (7 for the 1,600 of maxR 32: 1-2 % of the form)
-        const int spt = (Kpad / 2 + LSR_THREADS - 1) / LSR_THREADS;
-        if (spt <= 2) return rows(std::integral_constant<int, 2>());
-        if (spt <= 4) return rows(std::integral_constant<int, 4>());
-        if (spt <= 6) return rows(std::integral_constant<int, 6>());
-        if (spt <= 7) return rows(std::integral_constant<int, 7>());
-        return rows(std::integral_constant<int, LSR_SPT>());
+        // registers for the samples there are (24 grids of 25 steps a side: at maxR 32, 7 a thread, 1-2 % of the
+        // form against 8)
+        switch ((Kpad / 2 + LSR_THREADS - 1) / LSR_THREADS) {
+            case 1: return rows(std::integral_constant<int, 1>());
+            case 2: return rows(std::integral_constant<int, 2>());
+            case 3: return rows(std::integral_constant<int, 3>());
+            case 4: return rows(std::integral_constant<int, 4>());
+            case 5: return rows(std::integral_constant<int, 5>());
+            case 6: return rows(std::integral_constant<int, 6>());
+            case 7: return rows(std::integral_constant<int, 7>());
+            default: return rows(std::integral_constant<int, LSR_SPT>());
+        }
     }
     size_t sm = (size_t)S * sizeof(float2);
     cudaError_t e = allow_smem(k_slice_bf16_local, sm);

@@ -1261,8 +1261,9 @@ int exhaustive_topk(Ctx* c, const OriginDev& ob, const void* A, const void* bank
 
 // Coarse level for nb prepared particles (c->band, ctfp): the best kc distinct coarse
 // orientations of each, mapped onto the fine grid (twice the coarse indices) with their
-// fine neighbours within nbf steps in theta, phi and omega -> lists[i].
-int coarse_lists(Ctx* c, int nb, const float* ctfp, const float* poff, const OriginDev& ob, int kc, int nbf,
+// fine neighbours within nbf steps in theta, phi and omega -> lists[i].  Its origins are about the
+// image's centre also where the fine level's are centred on the particle's own.
+int coarse_lists(Ctx* c, int nb, const float* ctfp, const OriginDev& ob, int kc, int nbf,
                  std::vector<Proposals>& lists) {
     const ViewGrid& g = c->cgrid;
     const int ntc = (int)((c->n_orient_c + gemm_tile_n() - 1) / gemm_tile_n());
@@ -1274,7 +1275,7 @@ int coarse_lists(Ctx* c, int nb, const float* ctfp, const float* poff, const Ori
         return r;
     launch_particle_norm(c->band.p, ctfp, c->bd, c->csamples_c.p, c->cS_c, nb, c->pnorm_c.p, c->stream);
     CK(launch_build_basis(c->band.p, ctfp, c->bd, c->csamples_c.p, c->cS_c, c->cKH_c, ob, c->pnorm_c.p, nb, c->amat_c.p,
-                          false, nullptr, nullptr, c->stream, poff));
+                          false, nullptr, nullptr, c->stream));
     CK(cudaMemsetAsync(c->gerr.p, 0, sizeof(int), c->stream));
     if ((r = exhaustive_topk(c, ob, c->amat_c.p, c->bmat_c.p, c->n_orient_c / g.nom * c->nomr_c, g.nom, c->nomr_c,
                              2 * c->cKH_c, false, nb, kc, ntc, c->tilev_c.p, c->tileo_c.p, c->kor_c.p, c->korig_c.p,
@@ -2116,7 +2117,7 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
                 // proposal forms: the coarse contraction or the learned proposer names each
                 // particle's candidate orientations, the fine contraction runs on their
                 // sections only; the local form cuts each particle's local grid
-                if (!local && (r = kc > 0 ? coarse_lists(L, nb, ctfp, nullptr, ob_c, kc, nbf, lists)
+                if (!local && (r = kc > 0 ? coarse_lists(L, nb, ctfp, ob_c, kc, nbf, lists)
                                           : learned_lists(L, nb, kl, nbf, lists)))
                     return r;
                 CK(cudaMemsetAsync(L->gerr.p, 0, sizeof(int), L->stream));

@@ -1583,7 +1583,7 @@ cudaError_t launch_up_list(const OriginDev& ob, const float* C, int parts, const
         // blocks to a tile: as many as find an SM (each combines its positions' products again), and as
         // hold the maxima of their tasks in 48 KB
         const int hn = (ob.n1 + 1) / 2, tasks = hn * ((hn + UL_X - 1) / UL_X), nw = UL_THREADS / 32;
-        const int most = 48 * 1024 / (32 * 8), fill = 2 * 152 / std::max(1, max_tiles * ngroups);
+        const int most = 48 * 1024 / (32 * 8), fill = 2 * sm_count() / std::max(1, max_tiles * ngroups);
         const int z = std::max((tasks + most - 1) / most, std::min(fill, (tasks + nw - 1) / nw));
         const UpAnyShape sh = up_any_shape(ob, 32, (size_t)((tasks + z - 1) / z) * 32 * (sizeof(float) + sizeof(int)));
         auto kern = sh.qsh ? k_up_list_any<true> : k_up_list_any<false>;
@@ -1600,7 +1600,7 @@ cudaError_t launch_up_list(const OriginDev& ob, const float* C, int parts, const
     // the SMs filled, by this launch or by other lanes', the pass takes longer: 14.0 -> 14.5 ms of the box-256
     // search with 192 tiles cut in three)
     int z = 1;
-    z = std::max(1, std::min(std::min(8, (ob.n1 + 1) / 2), 152 / std::max(1, max_tiles * ngroups)));
+    z = std::max(1, std::min(std::min(8, (ob.n1 + 1) / 2), sm_count() / std::max(1, max_tiles * ngroups)));
     kern<<<dim3(max_tiles, ngroups, z), 32 * nw, sm, st>>>(ob, C, parts, groups, map, topv, topi);
     return cudaGetLastError();
 }

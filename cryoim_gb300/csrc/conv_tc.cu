@@ -791,19 +791,6 @@ __global__ void __launch_bounds__(256) k_wgrad_sum(const float* __restrict__ par
     dW[((co * Cin + ci) * 3 + dh) * 3 + dt] += s;
 }
 
-int sm_count() {
-    static int n = 0;
-    if (!n) {
-        int dev = 0, v = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess &&
-            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0)
-            n = v;
-        else
-            return 1;
-    }
-    return n;
-}
-
 template <int CINP, int COUT, int MODE>
 cudaError_t launch_fwd(ConvTcArgs a, cudaStream_t st) {
     constexpr int smem = conv_fwd_smem<COUT>();

@@ -17,17 +17,25 @@ inline cudaError_t allow_smem_of(const void* kern, size_t bytes) {
     cudaError_t e = cudaFuncGetAttributes(&fa, kern);
     if (e != cudaSuccess) return e;
     if (bytes + fa.sharedSizeBytes <= 48 * 1024) return cudaSuccess;
+    if (fa.maxDynamicSharedSizeBytes > 48 * 1024 && bytes <= (size_t)fa.maxDynamicSharedSizeBytes) return cudaSuccess;
     int dev = 0, most = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
     const int room = most - (int)fa.sharedSizeBytes;
     if (room < 0 || bytes > (size_t)room) return cudaErrorInvalidValue;
-    if (fa.maxDynamicSharedSizeBytes == room) return cudaSuccess;
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, room);
 }
 template <class... A>
 cudaError_t allow_smem(void (*kern)(A...), size_t bytes) {
     return allow_smem_of(reinterpret_cast<const void*>(kern), bytes);
+}
+
+// the current device's SMs (152 where it cannot be asked: the launch will say why)
+inline int sm_count() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 152;
+    return n;
 }
 
 }  // namespace cryoim

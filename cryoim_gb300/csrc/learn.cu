@@ -1032,7 +1032,7 @@ void launch_lp_mix_grad(const float* x, const float* dg, int B, const float* W5,
     k_mix_sum<<<cdiv(CM * LP_MIXK + CM, 64), 64, 0, st>>>(scratch, split, dW5, db5);
 }
 // a few blocks per SM; the loop takes the rest
-int dft_grid(long rows) { return (int)std::min<long>((rows + DW * DR - 1) / (DW * DR), 152 * 12); }
+int dft_grid(long rows) { return (int)std::min<long>((rows + DW * DR - 1) / (DW * DR), sm_count() * 12); }
 long lp_head_scratch(int B, int V) { return (long)NF * (2L * B * CM + 2L * V * CM + 2L * B * V); }
 
 // scratch (float2): G [B][CM][NF], TT [V][CM][NF], X [B][V][NF], then the backward's

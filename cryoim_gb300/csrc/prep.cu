@@ -690,7 +690,8 @@ void launch_prep_images(const float* imgs, int B, int nx, const float* ox, const
     // blocks per image: as many as leave every block an SM of its own (one holds no second), and a
     // row for half of the warps
     int c = 1;
-    while (c < 8 && 2L * c * B <= 152 && 32 * c <= nx) c *= 2;
+    const int sms = sm_count();
+    while (c < 8 && 2L * c * B <= sms && 32 * c <= nx) c *= 2;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(B * c));
     cfg.blockDim = dim3(1024);

@@ -1098,7 +1098,8 @@ cudaError_t launch_pr_omega(const PrOmegaArgs& a, int B, cudaStream_t st) {
         return (60 + Gz - 1) / Gz;
     };
     int z = 1;
-    for (int zz = 2; zz <= 8 && (long)a.V * B * zz <= 152; ++zz)
+    const int sms = sm_count();
+    for (int zz = 2; zz <= 8 && (long)a.V * B * zz <= sms; ++zz)
         if (rounds(zz) < rounds(z)) z = zz;
     const bool large = a.bd.nx > 256;  // (an instance of its own: a margin in a register costs 0.5 %)
     auto kern = z > 1 ? (!half ? k_pr_omega<false, true, false> : large ? k_pr_omega<true, true, true> : k_pr_omega<true, true, false>)

@@ -1072,7 +1072,7 @@ int ensure_origin_plan(Ctx* c, int R, float omax, float step, bool f8, OriginDev
     o.dev = OriginDev{reinterpret_cast<const float*>(d + q), reinterpret_cast<const float*>(d + f), d + row,
                       reinterpret_cast<const int2*>(d + slot), reinterpret_cast<const int4*>(d), d + off,
                       reinterpret_cast<const float4*>(d + qx), reinterpret_cast<const float4*>(d + qy),
-                      b.n1, b.nb, b.slots, b.units, b.R, b.ent_off.back(),
+                      b.n1, b.nb, b.slots, b.used, b.units, b.R, b.ent_off.back(),
                       (int)b.qx.size() / 4, (int)b.qy.size() / 4, b.layout, b.mid, f8 ? 0.0625f : 1.0f};
     o.nx = c->p.fftsize; o.min_r = c->p.min_r; o.R = R; o.omax = omax; o.step = step; o.f8 = f8;
     o.used = ++c->oplan_calls;
@@ -1218,41 +1218,52 @@ void expand_seeds(Ctx* c, const std::vector<std::vector<int3>>& seeds, int nbf, 
     }
 }
 
-// Particles per exhaustive product: its FP32 products (122 MB a particle at 119,520 rows)
-// within 1.25 GB, equal sub-batches
-int product_batch(int nb, int parts, int slots, long pitch) {
-    const long each = (long)parts * slots * pitch * 4;
+// How an exhaustive product of np particles packs their rows: a unit of the contraction takes up to 160
+// rows (whole 32s), so grids of few origins (2 to 73 rows in use) share one, evenly; grids of more
+// have a particle to a block.
+OriginPack pack_rows(const OriginDev& ob, int np) {
+    const int most = ob.units > 1 ? 1 : 160 / ob.used;
+    if (most < 2 || np < 2) return OriginPack{1, ob.slots};
+    const int blocks = (np + most - 1) / most, per = (np + blocks - 1) / blocks;
+    return per < 2 ? OriginPack{1, ob.slots} : OriginPack{per, (per * ob.used + 31) / 32 * 32};
+}
+
+// Blocks of a pack per exhaustive product: its FP32 products (122 MB for 128 rows at 119,520
+// orientations) within 1.25 GB, equal sub-batches
+int product_batch(int blocks, int parts, int rows, long pitch) {
+    const long each = (long)parts * rows * pitch * 4;
     const int most = (int)std::max(1L, std::min(64L, (5L << 28) / std::max(1L, each)));
-    const int cuts = (nb + most - 1) / most;
-    return (nb + cuts - 1) / cuts;
+    const int cuts = (blocks + most - 1) / most;
+    return (blocks + cuts - 1) / cuts;
 }
 
 // The k best orientations (one per block of 256) of np particles against every row of a
-// bank: A of np x ob.slots rows, products and their expansion in sub-batches, queued back to
+// bank: A packed by pk (pack_rows), products and their expansion in sub-batches, queued back to
 // back on c's stream.  mark (profiling) is called before and after every contraction launch.
-int exhaustive_topk(Ctx* c, const OriginDev& ob, const void* A, const void* bank, long rows, int nom, int nomr, int K,
-                    bool f8, int np, int k, int ntiles, float* tilev, int* tileo, int* kor, int* korig, float* kcc,
-                    bool want_origin, const std::function<int()>& mark = nullptr) {
+int exhaustive_topk(Ctx* c, const OriginDev& ob, OriginPack pk, const void* A, const void* bank, long rows, int nom,
+                    int nomr, int K, bool f8, int np, int k, int ntiles, float* tilev, int* tileo, int* kor, int* korig,
+                    float* kcc, bool want_origin, const std::function<int()>& mark = nullptr) {
     const int parts = nom / nomr, tn = gemm_tile_n();
     const long n_orient = rows / nomr * nom, pitch = (rows + tn - 1) / tn * tn;
-    const int pb = product_batch(np, parts, ob.slots, pitch);
+    const int blocks = (int)pk.blocks(np), bb = product_batch(blocks, parts, pk.rows, pitch);
     int r;
-    if ((r = c->cprod.ensure((size_t)pb * parts * ob.slots * pitch)) || (r = c->ccmax.ensure((size_t)pb * n_orient)))
+    if ((r = c->cprod.ensure((size_t)bb * parts * pk.rows * pitch)) ||
+        (r = c->ccmax.ensure((size_t)std::min(np, bb * pk.per) * n_orient)))
         return r;
-    for (int s0 = 0; s0 < np; s0 += pb) {
-        const int ns = std::min(pb, np - s0);
+    for (int b0 = 0; b0 < blocks; b0 += bb) {
+        const int nb = std::min(bb, blocks - b0), s0 = b0 * pk.per, ns = std::min(nb * pk.per, np - s0);
         GemmArgmaxArgs g{};
         g.b_mode = 1;  // the banks' rows are pre-swizzled
         g.err = c->gerr.p;
         g.cstore = c->cprod.p;
         g.k_parts = parts;
         g.c_units = ob.units;
-        g.c_rows = ob.slots / ob.units;
+        g.c_rows = pk.rows / ob.units;
         if (mark && (r = mark())) return r;
-        CK(launch_gemm_argmax((const char*)A + (size_t)s0 * ob.slots * K * (f8 ? 1 : 2), bank, ns * ob.slots, (int)rows,
+        CK(launch_gemm_argmax((const char*)A + (size_t)b0 * pk.rows * K * (f8 ? 1 : 2), bank, nb * pk.rows, (int)rows,
                               K, f8, g, c->num_sms, c->stream));
         if (mark && (r = mark())) return r;
-        CK(launch_up_topk(ob, c->cprod.p, pitch, rows, nom, nomr, ns, k, c->ccmax.p, ntiles, tilev, tileo,
+        CK(launch_up_topk(ob, pk, c->cprod.p, pitch, rows, nom, nomr, ns, k, c->ccmax.p, ntiles, tilev, tileo,
                           kor + (size_t)s0 * k, korig + (size_t)s0 * k, kcc + (size_t)s0 * k, want_origin, c->num_sms,
                           c->stream));
     }
@@ -1268,16 +1279,17 @@ int coarse_lists(Ctx* c, int nb, const float* ctfp, const OriginDev& ob, int kc,
     const ViewGrid& g = c->cgrid;
     const int ntc = (int)((c->n_orient_c + gemm_tile_n() - 1) / gemm_tile_n());
     int r;
-    if ((r = c->amat_c.ensure((size_t)nb * ob.slots * 2 * c->cKH_c)) || (r = c->tilev_c.ensure((size_t)nb * ntc)) ||
+    const OriginPack pk = pack_rows(ob, nb);
+    if ((r = c->amat_c.ensure((size_t)pk.blocks(nb) * pk.rows * 2 * c->cKH_c)) || (r = c->tilev_c.ensure((size_t)nb * ntc)) ||
         (r = c->tileo_c.ensure((size_t)nb * ntc)) || (r = c->kor_c.ensure((size_t)nb * kc)) ||
         (r = c->korig_c.ensure((size_t)nb * kc)) || (r = c->kcc_c.ensure((size_t)nb * kc)) ||
         (r = c->pnorm_c.ensure(nb)))
         return r;
     launch_particle_norm(c->band.p, ctfp, c->bd, c->csamples_c.p, c->cS_c, nb, c->pnorm_c.p, c->stream);
-    CK(launch_build_basis(c->band.p, ctfp, c->bd, c->csamples_c.p, c->cS_c, c->cKH_c, ob, c->pnorm_c.p, nb, c->amat_c.p,
-                          false, nullptr, nullptr, c->stream));
+    CK(launch_build_basis(c->band.p, ctfp, c->bd, c->csamples_c.p, c->cS_c, c->cKH_c, ob, pk, c->pnorm_c.p, nb,
+                          c->amat_c.p, false, nullptr, nullptr, c->stream));
     CK(cudaMemsetAsync(c->gerr.p, 0, sizeof(int), c->stream));
-    if ((r = exhaustive_topk(c, ob, c->amat_c.p, c->bmat_c.p, c->n_orient_c / g.nom * c->nomr_c, g.nom, c->nomr_c,
+    if ((r = exhaustive_topk(c, ob, pk, c->amat_c.p, c->bmat_c.p, c->n_orient_c / g.nom * c->nomr_c, g.nom, c->nomr_c,
                              2 * c->cKH_c, false, nb, kc, ntc, c->tilev_c.p, c->tileo_c.p, c->kor_c.p, c->korig_c.p,
                              c->kcc_c.p, false)))
         return r;
@@ -1974,7 +1986,7 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
     // Particles per pass (transform, rescoring: large grids, two host waits per pass);
     // operand A is built for the whole pass.
     const int PB = std::max(1, c->batch);
-    const int arows = local ? O : ob.slots;  // rows of A per particle
+    const int arows = local ? O : ob.slots;  // rows of A per particle, but in exhaustive passes (pack_rows)
     const int ntiles = (int)(((local ? nloc : c->n_orient) + gemm_tile_n() - 1) / gemm_tile_n());
     // list positions of a particle in the proposal forms, at most: seeds x neighbourhood
     const long nlist = std::min((long)c->n_orient,
@@ -2013,8 +2025,10 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
         int r;
         if ((r = ensure_batch(L, PB))) return r;
         const int ps = std::min(PB, P);  // particles of the largest pass
-        if (f8 ? ((r = L->amat8.ensure((size_t)ps * arows * kpad)) || (r = L->fexp.ensure(PB)))
-               : (r = L->amat.ensure((size_t)ps * arows * kpad)))
+        // (a unit has up to 160 rows: no smaller pass needs more than the largest one's units of that)
+        const OriginPack most = local || listed ? OriginPack{1, arows} : pack_rows(ob, ps);
+        const size_t na = (size_t)most.blocks(ps) * (most.per > 1 ? 160 : most.rows);
+        if (f8 ? ((r = L->amat8.ensure(na * kpad)) || (r = L->fexp.ensure(PB))) : (r = L->amat.ensure(na * kpad)))
             return r;
         if ((r = L->topv.ensure((size_t)ps * O * toptiles)) || (r = L->topi.ensure((size_t)ps * O * toptiles)))
             return r;
@@ -2094,13 +2108,14 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
                 CK(cudaMemcpyAsync(L->poff.p, po.data(), sizeof(float) * po.size(), cudaMemcpyHostToDevice, L->stream));
             }
             const float* po = centred ? L->poff.p : nullptr;
+            const OriginPack pk = local || listed ? OriginPack{1, arows} : pack_rows(ob, nb);
             // operand A of the pass: the basis rows of every particle, or (local) its origins,
             // normalised by |P| there (the sections by |CTF S|)
             if (local)
                 launch_build_a(L->band.p, ctfp, L->bd, L->csamples.p, L->cS, L->cKpad, L->corigins.p, O, L->pnorm0.p,
                                nb, L->amat.p, L->stream, po);
             else
-                CK(launch_build_basis(L->band.p, ctfp, L->bd, L->csamples.p, L->cS, kpad / 2, ob, L->pnorm.p, nb,
+                CK(launch_build_basis(L->band.p, ctfp, L->bd, L->csamples.p, L->cS, kpad / 2, ob, pk, L->pnorm.p, nb,
                                       f8 ? (void*)L->amat8.p : (void*)L->amat.p, f8, L->mulA.p, L->fexp.p, L->stream,
                                       po));
             CK(cudaGetLastError());
@@ -2237,7 +2252,7 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
                 }
             } else {
                 // exhaustive: every particle of the pass against every row of the bank
-                if ((r = exhaustive_topk(L, ob, f8 ? (const void*)L->amat8.p : (const void*)L->amat.p,
+                if ((r = exhaustive_topk(L, ob, pk, f8 ? (const void*)L->amat8.p : (const void*)L->amat.p,
                                          f8 ? (const void*)L->bmat8.p : (const void*)L->bmat.p,
                                          L->n_orient / L->nom * L->nomr, L->nom, L->nomr, kpad, f8, nb, k, ntiles,
                                          L->tilev.p, L->tileo.p, L->kor.p, L->korig.p, L->kcc.p, need_cc64,
@@ -2245,7 +2260,7 @@ int contract_impl(Ctx* c, const float* imgs, bool on_device, cryoim_particle* pa
                     return r;
                 if (L->prof)
                     L->prof_gemm_flops +=
-                        2.0 * (double)nb * ob.slots * (double)(L->n_orient / L->nom * L->nomr) * (double)kpad;
+                        2.0 * (double)nb * ob.used * (double)(L->n_orient / L->nom * L->nomr) * (double)kpad;
             }
             int gerr = 0;
             CK(cudaMemcpyAsync(&gerr, L->gerr.p, sizeof(int), cudaMemcpyDeviceToHost, L->stream));

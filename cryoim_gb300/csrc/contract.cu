@@ -438,12 +438,13 @@ constexpr int BO = 8;  // rows per block: a sample's transform, CTF and phase on
 template <bool F8>
 __global__ void __launch_bounds__(256) k_build_basis(const float2* __restrict__ band, const float* __restrict__ ctf,
                                                      Band bd, const int2* __restrict__ samples, int S, int KH,
-                                                     OriginDev ob, const float* __restrict__ poff,
+                                                     OriginDev ob, OriginPack pk, const float* __restrict__ poff,
                                                      const double* __restrict__ norm, const float* __restrict__ mulA,
                                                      const int* __restrict__ fexp, float two_pi_over_n,
                                                      void* __restrict__ Aout) {
     extern __shared__ float2 ptab[];  // [3 R + 2] origin phasors, then per row f_m [R + 1], f_k [2 R + 1]
     const int b0 = blockIdx.x * BO, p = blockIdx.y, W = bd.W, R = bd.max_r, nt = 3 * R + 2, R1 = ob.R;
+    const int nrow = pk.per > 1 ? ob.used : ob.slots;
     float* ft = reinterpret_cast<float*>(ptab + nt);
     const float2* b = band + (long)p * W * W;
     const float* c = ctf ? ctf + (long)p * W * W : nullptr;
@@ -455,7 +456,7 @@ __global__ void __launch_bounds__(256) k_build_basis(const float2* __restrict__ 
     int rot[BO], part[BO];  // rot: quarter turns of i^(...), part: -1 for an empty row
 #pragma unroll
     for (int j = 0; j < BO; ++j) {
-        const int rw = ob.row[b0 + j];
+        const int rw = b0 + j < ob.slots ? ob.row[b0 + j] : -1;
         const int m = rw & 0xfff, k = (rw >> 12) & 0xfff;
         part[j] = rw < 0 ? -1 : (rw >> 24) & 1;
         rot[j] = rw < 0 ? 0 : (m & 1) + (k & 1);
@@ -502,7 +503,8 @@ __global__ void __launch_bounds__(256) k_build_basis(const float2* __restrict__ 
                 re[u] = rot[j] == 0 ? x : (rot[j] == 1 ? -y : -x);
                 im[u] = rot[j] == 0 ? y : (rot[j] == 1 ? x : -y);
             }
-            const long row = (long)p * ob.slots + b0 + j;
+            if (b0 + j >= nrow) continue;
+            const long row = pk.at(ob.used, p) + b0 + j;
             if constexpr (F8) {
                 unsigned char* A = (unsigned char*)Aout + row * (2 * KH);
                 float2 vr = make_float2(re[0], re[1]), vi = make_float2(im[0], im[1]);
@@ -554,6 +556,7 @@ template <int LY> struct UpCoef {
     static constexpr int NB = OB_LAYOUT[LY].nb, CUT = OB_LAYOUT[LY].cut, L2 = OB_LAYOUT[LY].second,
                          ROWS = OB_LAYOUT[LY].rows, H = (NB + 1) / 2;
     static __host__ __device__ constexpr bool in(int m, int k) { return m < NB && k < NB && m + k <= CUT; }
+    static __host__ __device__ constexpr bool twice(int m, int k) { return in(m, k) && m + k < L2; }
     static __host__ __device__ constexpr bool pair(int m, int k) { return in(m, 2 * k) || in(m, 2 * k + 1); }
     float2 c[2 * H][H];  // (k even, k odd) pairs; zero outside the layout
     // get(i): product of row i; lo: scale of the second rows
@@ -571,7 +574,7 @@ template <int LY> struct UpCoef {
         for (int m = 0; m < L2; ++m)
 #pragma unroll
             for (int k = 0; k < L2; ++k)
-                if (m + k < L2) {
+                if (twice(m, k)) {
                     const float v = get(b++);
                     if (k & 1) c[m][k / 2].y = fmaf(v, lo, c[m][k / 2].y);
                     else c[m][k / 2].x = fmaf(v, lo, c[m][k / 2].x);
@@ -730,10 +733,13 @@ __device__ __forceinline__ void up_any_add(const UpAny& A, int e0, int e1, int j
 // issued and land under the expansion.  FP32-issue-bound.  Measured at 625 origins and 2 x
 // 119,520 orientations: 87 us a particle; 480 us with each function's row looked up and
 // fetched by its thread (the loads' latency exposed), 118 us without the prefetch.
+// blocks an SM: what the coefficients' registers leave (one where there are 96 of them and more)
+constexpr int up_blocks(int ly) { return OB_LAYOUT[ly].rows <= 18 ? 4 : OB_LAYOUT[ly].rows < 96 ? 2 : 1; }
 template <int LY>
-__global__ void __launch_bounds__(UP_THREADS, 1) k_up_max(OriginDev ob, const float* __restrict__ C, long pitch,
-                                                          long rows, int nom, int nomr, int B,
-                                                          float* __restrict__ ccmax) {
+__global__ void __launch_bounds__(UP_THREADS, up_blocks(LY)) k_up_max(OriginDev ob, OriginPack pk,
+                                                                     const float* __restrict__ C, long pitch, long rows,
+                                                                     int nom, int nomr, int B,
+                                                                     float* __restrict__ ccmax) {
     constexpr int ROWS = OB_LAYOUT[LY].rows;
     extern __shared__ __align__(16) float smem[];  // [share][row of A][columns], then the table of q
     float* sq = smem + UP_THREADS * ROWS;
@@ -744,12 +750,13 @@ __global__ void __launch_bounds__(UP_THREADS, 1) k_up_max(OriginDev ob, const fl
     const long ntile = (rows + cols - 1) / cols, total = ntile * B;
     auto fetch = [&](long t) {
         const long p = t / ntile, r0 = (t - p * ntile) * cols;
-        const float* src = C + p * (two ? 2 : 1) * ROWS * pitch + r0;  // (the shares' rows follow one another)
+        const float* src = C + pk.at_c(ROWS, (int)p, two ? 2 : 1) * pitch + r0;
         const int n = UP_THREADS * ROWS / 4;
         for (int i = threadIdx.x; i < n; i += UP_THREADS) {
             const int row = i / ch, c = i - row * ch;
             const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem + 4 * i);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src + row * pitch + 4 * c) : "memory");
+            const long at = row < ROWS ? row : row - ROWS + pk.rows;  // (the second share's)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src + at * pitch + 4 * c) : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -785,8 +792,8 @@ __global__ void __launch_bounds__(UP_THREADS, 1) k_up_max(OriginDev ob, const fl
 // pairs of y a warp (fewer reads, half the warps) 0.26; pairs of x 8 at a time 0.26.
 constexpr int UM_COLS = 64, UM_THREADS = UM_COLS * UM_SHARES;
 template <bool QSH, int W>
-__global__ void __launch_bounds__(UM_THREADS, 2) k_up_max_any(OriginDev ob, const float* __restrict__ C, long pitch,
-                                                              long rows, int nom, int nomr, int chunk,
+__global__ void __launch_bounds__(UM_THREADS, 2) k_up_max_any(OriginDev ob, OriginPack pk, const float* __restrict__ C,
+                                                              long pitch, long rows, int nom, int nomr, int chunk,
                                                               float* __restrict__ ccmax) {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ float sbest[UM_SHARES - 1][UM_COLS];
@@ -796,8 +803,8 @@ __global__ void __launch_bounds__(UM_THREADS, 2) k_up_max_any(OriginDev ob, cons
     const int cols = two ? UM_COLS / 2 : UM_COLS;
     const int p = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long r0 = (long)blockIdx.x * cols;
-    const float* U = C + (long)p * (two ? 2 : 1) * ob.slots * pitch + r0;  // (pitch: whole tiles of 256)
-    const float* V = U + ob.slots * pitch;
+    const float* U = C + pk.at_c(ob.used, p, two ? 2 : 1) * pitch + r0;  // (pitch: whole tiles of 256)
+    const float* V = U + pk.rows * pitch;
     const int col = 32 * (warp & 1) + lane, share = warp >> 1;
     UpAny A = up_any_tables<QSH>(ob, smraw);
     A.c = sc + col;
@@ -894,8 +901,8 @@ __global__ void __launch_bounds__(256) k_tile_best(const float* __restrict__ ccm
 // Best origin (index iy n1 + ix) of the selected orientations: one block per (candidate,
 // particle), a thread per row of origins in turn.
 constexpr int UO_X = 32;  // origins of a row at a time
-__global__ void __launch_bounds__(128) k_up_origin(OriginDev ob, const float* __restrict__ C, long pitch, int nom,
-                                                   int nomr, const int* __restrict__ orient, int k,
+__global__ void __launch_bounds__(128) k_up_origin(OriginDev ob, OriginPack pk, const float* __restrict__ C, long pitch,
+                                                   int nom, int nomr, const int* __restrict__ orient, int k,
                                                    int* __restrict__ origin) {
     __shared__ float sv[4];
     __shared__ int si[4];
@@ -905,8 +912,8 @@ __global__ void __launch_bounds__(128) k_up_origin(OriginDev ob, const float* __
     if (n >= 0) {
         const int io = n % nom;
         const long r = (long)(n / nom) * nomr + io % nomr;
-        const float* U = C + (long)p * parts * ob.slots * pitch + r;
-        const float* V = parts > 1 ? U + ob.slots * pitch : nullptr;
+        const float* U = C + pk.at_c(ob.used, p, parts) * pitch + r;
+        const float* V = parts > 1 ? U + pk.rows * pitch : nullptr;
         for (int iy = threadIdx.x; iy < ob.n1; iy += blockDim.x)
             for (int x0 = 0; x0 < ob.n1; x0 += UO_X) {
                 float s[UO_X];
@@ -1488,21 +1495,28 @@ cudaError_t launch_b_to_e4m3(const void* B, long n, int KH, int S, const float* 
 }
 
 cudaError_t launch_build_basis(const float2* band, const float* ctf, Band bd, const int2* samples, int S, int KH,
-                               const OriginDev& ob, const double* norm, int B, void* A, bool f8, const float* mulA,
-                               int* fexp, cudaStream_t st, const float* poff) {
+                               const OriginDev& ob, OriginPack pk, const double* norm, int B, void* A, bool f8,
+                               const float* mulA, int* fexp, cudaStream_t st, const float* poff) {
     const float tpn = 2.0f * host_angles().pi / (float)bd.nx;
-    const dim3 g((ob.slots + BO - 1) / BO, B);
+    const dim3 g(((pk.per > 1 ? ob.used : ob.slots) + BO - 1) / BO, B);
     const size_t sm = (sizeof(float2) + sizeof(float) * BO) * (3 * (size_t)bd.max_r + 2);
     if (f8) k_particle_exp8<<<B, 256, 0, st>>>(band, ctf, bd, samples, S, norm, mulA, fexp);
     auto kern = f8 ? k_build_basis<true> : k_build_basis<false>;
     const cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return e;
-    kern<<<g, 256, sm, st>>>(band, ctf, bd, samples, S, KH, ob, poff, norm, mulA, fexp, tpn, A);
+    kern<<<g, 256, sm, st>>>(band, ctf, bd, samples, S, KH, ob, pk, poff, norm, mulA, fexp, tpn, A);
     return cudaGetLastError();
 }
 
 // the register kernels: a fixed layout, and origins whose table leaves room for the products
 static int up_layout(const OriginDev& ob) { return ob.n1 <= UP_N1 ? ob.layout : -1; }
+
+// f with the layout ly as a constant
+template <int LY, class F>
+static void up_dispatch(int ly, F& f) {
+    if (ly == LY) f(std::integral_constant<int, LY>());
+    else if constexpr (LY + 1 < OB_LAYOUTS) up_dispatch<LY + 1>(ly, f);
+}
 
 // Shared memory of the kernels for any number of functions: q's table where it is small, then as many
 // entries of cols columns as leave two blocks an SM (113 KB each), at least 16.
@@ -1522,8 +1536,8 @@ static UpAnyShape up_any_shape(const OriginDev& ob, int cols, size_t more) {
     return s;
 }
 
-cudaError_t launch_up_topk(const OriginDev& ob, const float* C, long pitch, long rows, int nom, int nomr, int B, int k,
-                           float* ccmax, int ntiles, float* tile_v, int* tile_o, int* orient, int* origin, float* cc,
+cudaError_t launch_up_topk(const OriginDev& ob, OriginPack pk, const float* C, long pitch, long rows, int nom, int nomr,
+                           int B, int k, float* ccmax, int ntiles, float* tile_v, int* tile_o, int* orient, int* origin, float* cc,
                            bool want_origin, int num_sms, cudaStream_t st) {
     const long n_orient = rows / nomr * nom;
     cudaError_t e = cudaSuccess;
@@ -1536,16 +1550,10 @@ cudaError_t launch_up_topk(const OriginDev& ob, const float* C, long pitch, long
             const size_t sm = sizeof(float) * (up_table_floats<LY>(ob.n1) + (size_t)UP_THREADS * OB_LAYOUT[LY].rows);
             e = allow_smem(k_up_max<LY>, sm);
             if (e != cudaSuccess) return;
-            k_up_max<LY><<<(unsigned)std::min<long>(tiles, num_sms), UP_THREADS, sm, st>>>(ob, C, pitch, rows, nom, nomr, B,
+            k_up_max<LY><<<(unsigned)std::min<long>(tiles, num_sms * up_blocks(LY)), UP_THREADS, sm, st>>>(ob, pk, C, pitch, rows, nom, nomr, B,
                                                                                           ccmax);
         };
-        switch (ly) {
-            case 0: run(std::integral_constant<int, 0>()); break;
-            case 1: run(std::integral_constant<int, 1>()); break;
-            case 2: run(std::integral_constant<int, 2>()); break;
-            case 3: run(std::integral_constant<int, 3>()); break;
-            default: run(std::integral_constant<int, 4>()); break;
-        }
+        up_dispatch<0>(ly, run);
         if (e != cudaSuccess) return e;
     } else {
         const int cols = nom == nomr ? UM_COLS : UM_COLS / 2;
@@ -1559,13 +1567,13 @@ cudaError_t launch_up_topk(const OriginDev& ob, const float* C, long pitch, long
                     : w <= 14 ? k_up_max_any<true, 14>
                               : k_up_max_any<true, UM_X>;
         if ((e = allow_smem(kern, sh.smem)) != cudaSuccess) return e;
-        kern<<<dim3((unsigned)((rows + cols - 1) / cols), B), UM_THREADS, sh.smem, st>>>(ob, C, pitch, rows, nom, nomr,
+        kern<<<dim3((unsigned)((rows + cols - 1) / cols), B), UM_THREADS, sh.smem, st>>>(ob, pk, C, pitch, rows, nom, nomr,
                                                                                         sh.chunk, ccmax);
     }
     k_tile_best<<<dim3(ntiles, B), 256, 0, st>>>(ccmax, n_orient, ntiles, tile_v, tile_o);
     k_select_topk<<<B, 512, 0, st>>>(tile_v, tile_o, ntiles, k, orient, cc);
     if (want_origin)
-        k_up_origin<<<dim3(k, B), 128, 0, st>>>(ob, C, pitch, nom, nomr, orient, k, origin);
+        k_up_origin<<<dim3(k, B), 128, 0, st>>>(ob, pk, C, pitch, nom, nomr, orient, k, origin);
     else
         return cudaMemsetAsync(origin, 0, sizeof(int) * (size_t)B * k, st);
     return cudaGetLastError();
@@ -1592,8 +1600,9 @@ cudaError_t launch_up_list(const OriginDev& ob, const float* C, int parts, const
         kern<<<dim3(max_tiles, ngroups, z), UL_THREADS, sh.smem, st>>>(ob, C, parts, groups, map, sh.chunk, topv, topi);
         return cudaGetLastError();
     }
-    auto kern = ly == 0 ? k_up_list<0> : ly == 1 ? k_up_list<1> : ly == 2 ? k_up_list<2> : ly == 3 ? k_up_list<3>
-                                                                                                    : k_up_list<4>;
+    void (*kern)(OriginDev, const float*, int, const UpGroup*, const int*, float*, int*) = nullptr;
+    auto pick = [&](auto lyc) { kern = k_up_list<decltype(lyc)::value>; };
+    up_dispatch<0>(ly, pick);
     cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return e;
     // blocks to a tile: as many as find an SM of their own (each reads its tile's products again, so that with

@@ -276,26 +276,36 @@ struct OriginDev {
     const int* ent_off; // [h + 1], h = (nb + 1) / 2
     const float4* qx;   // OriginBasis::qx
     const float4* qy;   // OriginBasis::qy
-    int n1, nb, slots, units, R;
+    int n1, nb, slots, used, units, R;  // used: rows in use, the first of slots
     int nent;           // ent_off[h]
     int nqx, nqy;       // float4s of qx, qy
     int layout;         // fixed places of the rows (OB_LAYOUT), -1: by slot alone
     float mid;
     float lo;           // scale of a second row's products (1, FP8 1/16)
 };
-// Operand A of the global forms: ob.slots rows per particle (the basis instead of the origin
-// grid), split as the banks are: BF16 with KH elements per part, or (f8) e4m3 with KH bytes,
+// Where the particles' rows lie in A, and in each K share of the products: per particles to a block of
+// `rows` rows, the rows in use of each after the other's (one to a block: all its slots).
+struct OriginPack {
+    int per, rows;
+    __host__ __device__ long at(int used, int p) const { return (long)(p / per) * rows + (long)(p % per) * used; }
+    // its first row in a product of `parts` shares
+    __host__ __device__ long at_c(int used, int p, int parts) const {
+        return (long)(p / per) * parts * rows + (long)(p % per) * used;
+    }
+    long blocks(int np) const { return (np + per - 1) / per; }
+};
+// Operand A of the global forms: a particle's rows of the basis (instead of the origin grid), split as the banks are: BF16 with KH elements per part, or (f8) e4m3 with KH bytes,
 // sample scales mulA and a power of two 2^fexp[p] per particle.  poff as in launch_build_a.
 cudaError_t launch_build_basis(const float2* band, const float* ctf, Band bd, const int2* samples, int S, int KH,
-                               const OriginDev& ob, const double* norm, int B, void* A, bool f8, const float* mulA,
-                               int* fexp, cudaStream_t st, const float* poff = nullptr);
+                               const OriginDev& ob, OriginPack pk, const double* norm, int B, void* A, bool f8,
+                               const float* mulA, int* fexp, cudaStream_t st, const float* poff = nullptr);
 // Exhaustive product C of B particles (GemmArgmaxArgs::cstore, pitch columns, nom / nomr K
 // shares; rows of the bank: nomr of the nom omegas per view): the best origin's value of every
 // orientation (ccmax: B x orientations), the best orientation of each of the ntiles blocks of
 // 256 (tile_v, tile_o: B x ntiles), the k best of those with their value and, if wanted,
 // origin (else 0).
-cudaError_t launch_up_topk(const OriginDev& ob, const float* C, long pitch, long rows, int nom, int nomr, int B, int k,
-                           float* ccmax, int ntiles, float* tile_v, int* tile_o, int* orient, int* origin, float* cc,
+cudaError_t launch_up_topk(const OriginDev& ob, OriginPack pk, const float* C, long pitch, long rows, int nom, int nomr,
+                           int B, int k, float* ccmax, int ntiles, float* tile_v, int* tile_o, int* orient, int* origin, float* cc,
                            bool want_origin, int num_sms, cudaStream_t st);
 // Listed products, one group per particle: list position j of group g stands for column
 // map[map_off + j] >> 1 of its block of C (parts K shares), conjugated if map & 1.  topv / topi

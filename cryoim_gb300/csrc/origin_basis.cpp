@@ -162,18 +162,28 @@ OriginBasis make_origin_basis(int n, int min_r, int R, float omax, float step, i
     for (int l = 0; l < OB_LAYOUTS && ob.layout < 0; ++l) {
         const OriginLayout& L = OB_LAYOUT[l];
         // (summed from what is out: the difference of two nearly equal sums would not do)
-        double tail = 0.0;
+        // likewise the functions that the layouts of few rows leave without the second row that the others
+        // give them: 5e-4 of total, 2 % of the rounding of A as it would be with none
+        double tail = 0.0, single = 0.0;
+        bool whole = true;
         for (int m = 0; m < n1; ++m)
             for (int k = 0; k < n1; ++k)
-                if (!L.in(m, k)) tail += at(m, k);
-        if (tail > most * total) continue;
+                if (!L.in(m, k)) {
+                    tail += at(m, k);
+                    whole = false;
+                } else if (l < OB_FEW && !L.twice(m, k) && m + k < 5) {
+                    single += at(m, k);
+                }
+        if (tail > most * total || single > 5e-4 * total) continue;
+        if (n1 <= OB_WHOLE && !whole && 8.0 * R * (double)step > n) continue;
         ob.layout = l;
-        clear(L.nb, L.rows);
+        clear(L.nb, (L.rows + 31) / 32 * 32);
+        ob.used = L.rows;
         int b = 0;
         for (int part = 0; part < 2; ++part)
             for (int m = 0; m < L.nb; ++m)
                 for (int k = 0; k < L.nb; ++k)
-                    if (L.in(m, k) && (part == 0 || m + k < L.second)) {
+                    if (part ? L.twice(m, k) : L.in(m, k)) {
                         if (m < n1 && k < n1) place(b, m, k, part);
                         ++b;
                     }
@@ -191,6 +201,7 @@ OriginBasis make_origin_basis(int n, int min_r, int R, float omax, float step, i
         int top = 0;
         for (size_t b = 0; b < cnt; ++b) top = std::max(top, std::max(ord[b] / n1, ord[b] % n1) + 1);
         clear(top, ob.units * OB_UNIT);
+        ob.used = ob.slots;
         for (size_t b = 0; b < cnt; ++b) place((int)b, ord[b] / n1, ord[b] % n1, 0);
         for (size_t b = cnt; b < (size_t)ob.slots && b < 2 * cnt; ++b)
             place((int)b, ord[b - cnt] / n1, ord[b - cnt] % n1, 1);

@@ -5,13 +5,24 @@
 namespace cryoim {
 
 // Rows of a particle with fixed places: functions (m, k) with m, k < nb and m + k <= cut,
-// m-major, then second rows (see below) for the functions with m + k < second, m-major.
+// m-major, then second rows (see below) for the functions with m + k < second, m-major.  The first
+// fourteen are of grids of few origins, whose rows an exhaustive search packs several particles to a unit
+// (64 particles of box 256 on the 1-degree grid, 1, 25 and 49 origins: 21 ms with 96 rows each, now 3.5, 7.2
+// and 12.5; a row per origin took 4.2, 8.8 and 15.2).
 struct OriginLayout {
     int nb, cut, second, rows;
     constexpr bool in(int m, int k) const { return m < nb && k < nb && m + k <= cut; }
+    constexpr bool twice(int m, int k) const { return in(m, k) && m + k < second; }
 };
-constexpr OriginLayout OB_LAYOUT[] = {{9, 16, 5, 96}, {10, 14, 3, 96}, {11, 15, 6, 128}, {12, 17, 7, 160}, {13, 19, 3, 160}};
-constexpr int OB_LAYOUTS = 5;
+constexpr OriginLayout OB_LAYOUT[] = {{1, 0, 1, 2},     {3, 3, 2, 11},    {4, 3, 2, 13},   {3, 4, 3, 15},
+                                      {3, 4, 5, 18},    {4, 4, 3, 19},    {5, 4, 3, 21},   {5, 6, 4, 32},
+                                      {5, 8, 5, 40},    {6, 7, 5, 45},    {7, 8, 5, 54},   {8, 9, 5, 64},
+                                      {7, 12, 5, 64},   {8, 11, 5, 73},   {9, 16, 5, 96},  {10, 14, 3, 96},
+                                      {11, 15, 6, 128}, {12, 17, 7, 160}, {13, 19, 3, 160}};
+constexpr int OB_LAYOUTS = 19, OB_FEW = 14;
+// grids of up to OB_WHOLE origins an axis keep all their functions, unless their step is at most a quarter of
+// the band's sampling distance n / 2R (most of such a grid's functions are below the tail)
+constexpr int OB_WHOLE = 8;
 constexpr int OB_UNIT = 160;  // rows come in units of this many where no layout is enough
 
 // The cross-correlation of one (particle, orientation) as a function of the origin is
@@ -31,7 +42,8 @@ constexpr int OB_UNIT = 160;  // rows come in units of this many where no layout
 struct OriginBasis {
     int n1 = 0;        // origins per axis: origin_i = mid + step (i - (n1 - 1) / 2)
     int nb = 0;        // functions per axis, even and odd ones alternating
-    int slots = 0;     // rows of A per particle, in units of equal size
+    int slots = 0;     // rows of A per particle, in units of equal size (a multiple of 32)
+    int used = 0;      // the first of them that hold something
     int units = 1;
     int layout = -1;   // the fixed places above, -1: rows by worth, any number of units
     int R = 0;

@@ -93,8 +93,8 @@ struct PrOmegaArgs {
     const float* views;      // [V][4]: theta, phi, slot base (int bits), pad
     int V, T, nomega;
     float step;
-    bool real_image;           // band(-h) = conj band(h): two omegas half a turn apart share a sample
     Band bd;
+    bool real_image;           // band(-h) = conj band(h): two omegas half a turn apart share a sample
     unsigned long long* best;  // [B]
     float* pr_array;           // [B][per] or nullptr
     long per;

@@ -435,7 +435,8 @@ __global__ void __launch_bounds__(256) k_build_a(const float2* __restrict__ band
 // HBM-write-bound: 160 rows x 25.6 KB a particle at box 256 (the origin grid is 625 rows:
 // 247 us a 64-particle pass against 82).
 constexpr int BO = 8;  // rows per block: a sample's transform, CTF and phase once for eight rows
-template <bool F8>
+// PACK: several particles to a block of rows (pack_rows), the rows in use alone.
+template <bool F8, bool PACK>
 __global__ void __launch_bounds__(256) k_build_basis(const float2* __restrict__ band, const float* __restrict__ ctf,
                                                      Band bd, const int2* __restrict__ samples, int S, int KH,
                                                      OriginDev ob, OriginPack pk, const float* __restrict__ poff,
@@ -444,7 +445,8 @@ __global__ void __launch_bounds__(256) k_build_basis(const float2* __restrict__ 
                                                      void* __restrict__ Aout) {
     extern __shared__ float2 ptab[];  // [3 R + 2] origin phasors, then per row f_m [R + 1], f_k [2 R + 1]
     const int b0 = blockIdx.x * BO, p = blockIdx.y, W = bd.W, R = bd.max_r, nt = 3 * R + 2, R1 = ob.R;
-    const int nrow = pk.per > 1 ? ob.used : ob.slots;
+    const long row0 = pk.at(ob.used, p) + b0;
+    const int nrow = ob.used - b0;  // PACK: of this block's
     float* ft = reinterpret_cast<float*>(ptab + nt);
     const float2* b = band + (long)p * W * W;
     const float* c = ctf ? ctf + (long)p * W * W : nullptr;
@@ -456,7 +458,7 @@ __global__ void __launch_bounds__(256) k_build_basis(const float2* __restrict__ 
     int rot[BO], part[BO];  // rot: quarter turns of i^(...), part: -1 for an empty row
 #pragma unroll
     for (int j = 0; j < BO; ++j) {
-        const int rw = b0 + j < ob.slots ? ob.row[b0 + j] : -1;
+        const int rw = ob.row[b0 + j];  // (slots is a multiple of BO)
         const int m = rw & 0xfff, k = (rw >> 12) & 0xfff;
         part[j] = rw < 0 ? -1 : (rw >> 24) & 1;
         rot[j] = rw < 0 ? 0 : (m & 1) + (k & 1);
@@ -503,8 +505,8 @@ __global__ void __launch_bounds__(256) k_build_basis(const float2* __restrict__ 
                 re[u] = rot[j] == 0 ? x : (rot[j] == 1 ? -y : -x);
                 im[u] = rot[j] == 0 ? y : (rot[j] == 1 ? x : -y);
             }
-            if (b0 + j >= nrow) continue;
-            const long row = pk.at(ob.used, p) + b0 + j;
+            if (PACK && j >= nrow) continue;
+            const long row = row0 + j;
             if constexpr (F8) {
                 unsigned char* A = (unsigned char*)Aout + row * (2 * KH);
                 float2 vr = make_float2(re[0], re[1]), vi = make_float2(im[0], im[1]);
@@ -1498,10 +1500,12 @@ cudaError_t launch_build_basis(const float2* band, const float* ctf, Band bd, co
                                const OriginDev& ob, OriginPack pk, const double* norm, int B, void* A, bool f8,
                                const float* mulA, int* fexp, cudaStream_t st, const float* poff) {
     const float tpn = 2.0f * host_angles().pi / (float)bd.nx;
-    const dim3 g(((pk.per > 1 ? ob.used : ob.slots) + BO - 1) / BO, B);
+    const bool pack = pk.per > 1;
+    const dim3 g(((pack ? ob.used : ob.slots) + BO - 1) / BO, B);
     const size_t sm = (sizeof(float2) + sizeof(float) * BO) * (3 * (size_t)bd.max_r + 2);
     if (f8) k_particle_exp8<<<B, 256, 0, st>>>(band, ctf, bd, samples, S, norm, mulA, fexp);
-    auto kern = f8 ? k_build_basis<true> : k_build_basis<false>;
+    auto kern = f8 ? (pack ? k_build_basis<true, true> : k_build_basis<true, false>)
+                   : (pack ? k_build_basis<false, true> : k_build_basis<false, false>);
     const cudaError_t e = allow_smem(kern, sm);
     if (e != cudaSuccess) return e;
     kern<<<g, 256, sm, st>>>(band, ctf, bd, samples, S, KH, ob, pk, poff, norm, mulA, fexp, tpn, A);

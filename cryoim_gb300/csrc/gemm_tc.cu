@@ -336,25 +336,25 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     aph = a1 + 1 == nacc ? aph1 ^ 1u : aph1;
                 }
             } else {
-            for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++lt) {
-                const int b = lt & 1;
-                const uint32_t aph = (uint32_t)(lt >> 1) & 1u;
-                if (!mbar_wait(acce + b, aph ^ 1u, g.err, true, g.wait_ns)) break;
-                tc_fence_after();
-                const uint32_t d = tmem + (uint32_t)(b * GN);
-                for (int kb = 0; kb < g.kblocks; ++kb) {
-                    if (!mbar_wait(full + s, ph, g.err, true, g.wait_ns)) { ok = false; break; }
+                for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++lt) {
+                    const int b = lt & 1;
+                    const uint32_t aph = (uint32_t)(lt >> 1) & 1u;
+                    if (!mbar_wait(acce + b, aph ^ 1u, g.err, true, g.wait_ns)) break;
                     tc_fence_after();
-                    const uint32_t a0 = su32(sA + s * A_BYTES), b0 = su32(sB + s * B_BYTES);
+                    const uint32_t d = tmem + (uint32_t)(b * GN);
+                    for (int kb = 0; kb < g.kblocks; ++kb) {
+                        if (!mbar_wait(full + s, ph, g.err, true, g.wait_ns)) { ok = false; break; }
+                        tc_fence_after();
+                        const uint32_t a0 = su32(sA + s * A_BYTES), b0 = su32(sB + s * B_BYTES);
 #pragma unroll
-                    for (int kk = 0; kk < GKB / 32; ++kk)
-                        tc_mma<F8>(d, sdesc(a0 + kk * 32), sdesc(b0 + kk * 32), (kb | kk) != 0,
-                                   F8 ? IDESC_E4M3 : IDESC_BF16);
-                    tc_commit(empty + s);
-                    if (++s == NSTAGE) { s = 0; ph ^= 1u; }
+                        for (int kk = 0; kk < GKB / 32; ++kk)
+                            tc_mma<F8>(d, sdesc(a0 + kk * 32), sdesc(b0 + kk * 32), (kb | kk) != 0,
+                                       F8 ? IDESC_E4M3 : IDESC_BF16);
+                        tc_commit(empty + s);
+                        if (++s == NSTAGE) { s = 0; ph ^= 1u; }
+                    }
+                    if (ok) tc_commit(accf + b);
                 }
-                if (ok) tc_commit(accf + b);
-            }
             }
             // all issued MMAs complete before TMEM is released
             tc_commit(drain);
@@ -390,37 +390,37 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 }
             }
         } else {
-        int lt = 0;
-        for (int t = blockIdx.x; t < total; t += gridDim.x, ++lt) {
-            const int b = lt & 1;
-            const uint32_t aph = (uint32_t)(lt >> 1) & 1u;
-            if (!mbar_wait(accf + b, aph, g.err, true, g.wait_ns)) break;
-            tc_fence_after();
-            const TileAt ta = tile_at(g, t);
-            const long row = (long)ta.mt * GM + row_in_tile;
-            float best = -3.0e38f;
-            int bi = -1;
-            for (int c = 0; c < GN / 32; ++c) {
-                float v[32];
-                tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(b * GN + c * 32), v);
-                const int col0 = ta.nt * GN + c * 32;
+            int lt = 0;
+            for (int t = blockIdx.x; t < total; t += gridDim.x, ++lt) {
+                const int b = lt & 1;
+                const uint32_t aph = (uint32_t)(lt >> 1) & 1u;
+                if (!mbar_wait(accf + b, aph, g.err, true, g.wait_ns)) break;
+                tc_fence_after();
+                const TileAt ta = tile_at(g, t);
+                const long row = (long)ta.mt * GM + row_in_tile;
+                float best = -3.0e38f;
+                int bi = -1;
+                for (int c = 0; c < GN / 32; ++c) {
+                    float v[32];
+                    tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(b * GN + c * 32), v);
+                    const int col0 = ta.nt * GN + c * 32;
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const int col = col0 + j;
-                    if (col < ta.n_valid && v[j] > best) { best = v[j]; bi = col; }
+                    for (int j = 0; j < 32; ++j) {
+                        const int col = col0 + j;
+                        if (col < ta.n_valid && v[j] > best) { best = v[j]; bi = col; }
+                    }
+                    if (g.cfull && row < ta.m_valid) {
+                        for (int j = 0; j < 32; ++j)
+                            if (col0 + j < ta.n_valid) g.cfull[row * g.ldc + col0 + j] = v[j];
+                    }
                 }
-                if (g.cfull && row < ta.m_valid) {
-                    for (int j = 0; j < 32; ++j)
-                        if (col0 + j < ta.n_valid) g.cfull[row * g.ldc + col0 + j] = v[j];
+                tc_fence_before();
+                mbar_arrive(acce + b);
+                if (row < ta.m_valid) {
+                    g.topv[ta.topv_off + row * ta.n_tiles + ta.nt] = best;
+                    g.topi[ta.topv_off + row * ta.n_tiles + ta.nt] = bi;
                 }
             }
-            tc_fence_before();
-            mbar_arrive(acce + b);
-            if (row < ta.m_valid) {
-                g.topv[ta.topv_off + row * ta.n_tiles + ta.nt] = best;
-                g.topi[ta.topv_off + row * ta.n_tiles + ta.nt] = bi;
-            }
-        }
         }
     }
     tc_fence_before();

@@ -35,7 +35,7 @@ def fake(tmp_path_factory):
     d = tmp_path_factory.mktemp("smem")
     (d / "shim.cpp").write_text(SHIM)
     inc = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
-    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, "-I", inc, str(d / "shim.cpp"), "-o",
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I", CSRC, "-I", inc, str(d / "shim.cpp"), "-o",
                     str(d / "shim.so")], check=True)
     lib = C.CDLL(str(d / "shim.so"))
     lib.ask.argtypes = lib.launch.argtypes = lib.reset.argtypes = [C.c_size_t]

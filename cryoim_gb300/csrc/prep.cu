@@ -115,8 +115,9 @@ __global__ void k_prep_images(const float* __restrict__ imgs, int nx,
     float R2 = mask + 3.0f;
     if (R2 > (float)hh) R2 = (float)hh;
     const float x0 = ox[p] + (float)hh, y0 = oy[p] + (float)hh;
-    // squares that are certainly at or inside R1 and certainly beyond R2 (the root rounds by 2^-24)
-    const float in2 = R1 * R1 * 0.999999f, out2 = R2 * R2 * 1.000001f;
+    // squares that are certainly at or inside both radii (R1 is the larger one where the mask is wider
+    // than the box) and certainly beyond R2 (the root rounds by 2^-24)
+    const float R0 = fminf(R1, fmaxf(R2, 0.0f)), in2 = R0 * R0 * 0.999999f, out2 = R2 * R2 * 1.000001f;
     double summ = 0;
     if (use_mask) {
         float h = 0.f, l = 0.f;
@@ -150,7 +151,7 @@ __global__ void k_prep_images(const float* __restrict__ imgs, int nx,
             if (use_mask) {
                 const float xx = (-x0 + (float)ix) * (-x0 + (float)ix);
                 const float r2 = yy + xx;
-                const float ra = r2 <= in2 ? R1 : r2 > out2 ? R2 + 1.0f : sqrtf(r2);
+                const float ra = r2 <= in2 ? R0 : r2 > out2 ? R2 + 1.0f : sqrtf(r2);
                 if (ra > R1 && ra <= R2) {
                     float edge = (1.0f + cosf(pi * (ra - R1) / 6.0f)) / 2.0f;
                     v = (float)((double)(v * edge) + (double)(1.0f - edge) * summ);

@@ -1129,7 +1129,7 @@ int ensure_coarse(Ctx* c, float omax, float ostep, OriginDev* ob) {
         build_view_grid(2.0f * c->p.searchstep, &c->cgrid);
         const ViewGrid& g = c->cgrid;
         if (g.nom < 1 || g.V < 1) return fail(CRYOIM_ERR_SIZE, "coarse grid is empty");
-        const int R = c->p.max_r, r0 = c->p.min_r, Rc = std::max(r0 + 1, R / 2);
+        const int R = c->p.max_r, r0 = c->p.min_r, Rc = coarse_radius(r0, R);
         std::vector<int2> s;
         for (int ky = -Rc; ky <= Rc; ++ky)
             for (int hx = 0; hx <= Rc; ++hx) {
@@ -1161,7 +1161,7 @@ int ensure_coarse(Ctx* c, float omax, float ostep, OriginDev* ob) {
         c->n_orient_c = n;
         c->bmat_c_ready = true;
     }
-    return ensure_origin_plan(c, std::max(c->p.min_r + 1, c->p.max_r / 2), omax, 2.0f * ostep, false, ob);
+    return ensure_origin_plan(c, coarse_radius(c->p.min_r, c->p.max_r), omax, 2.0f * ostep, false, ob);
 }
 
 // A particle's proposed orientations: fine-grid indices, each once, in the order first

@@ -28,6 +28,12 @@ inline Band make_band(int nx, int min_r, int max_r) {
     b.AW = 2 * max_r + 3;
     return b;
 }
+// outer radius of the coarse level's band: half of the band's, at least two radii where the band has
+// them, and within it (the window, the ramps' table and the map's cube end there)
+inline int coarse_radius(int min_r, int max_r) {
+    const int rc = max_r / 2 > min_r ? max_r / 2 : min_r + 1;
+    return rc < max_r ? rc : max_r;
+}
 // accumulator index of frequency (hx, ky, lz)
 __host__ __device__ inline long acc_cell(const Band& b, int hx, int ky, int lz) {
     return ((long)lz * b.AW + (ky + b.max_r + 1)) * b.AW + (hx + b.max_r + 1);

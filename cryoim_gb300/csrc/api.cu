@@ -423,10 +423,14 @@ struct Ctx {
     int lanes = 6;
     std::vector<Ctx*> xlanes;
 
+    void drop_plans() {
+        for (auto& kv : plans) cufftDestroy(kv.second);
+        plans.clear();
+    }
     ~Ctx() {
         for (Ctx* x : xlanes) delete x;
         cudaSetDevice(device);
-        for (auto& kv : plans) cufftDestroy(kv.second);
+        drop_plans();
         ops.release(); tband.release(); tfcut0.release(); tort.release(); d_views.release();
         alpha.release(); imgs.release(); par.release(); fcut0.release(); ctf.release();
         tfcut.release(); state.release(); cand.release(); rpr.release(); rot.release();
@@ -2784,8 +2788,8 @@ int cryoim_set_params(void* ctx, const cryoim_params* p) {
     c->have_params = true;
     if (geom_changed) {
         c->rings = RingTable{};
-        for (auto& kv : c->plans) cufftDestroy(kv.second);
-        c->plans.clear();
+        c->drop_plans();
+        for (Ctx* h : c->xlanes) h->drop_plans();  // (theirs are of the images' size too)
         c->T = 0;  // templates depend on the band geometry
         c->grid_ready = false;
         c->rec_active = false;

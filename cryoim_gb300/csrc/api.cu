@@ -1511,7 +1511,7 @@ template <class RNG> void random_euler(RNG& rng, float* e) {
 int learn_render(Ctx* c, cudaTextureObject_t tex, const float* deul, const float* dpar, int B, float snr,
                  unsigned long long seed, bool ctf, float* img, float2* ft, float* var) {
     const int nx = c->p.fftsize;
-    launch_lp_render(tex, 2 * c->p.max_r + 3, c->p.max_r + 1, 2, nx, deul, dpar, B, c->p.apix,
+    launch_lp_render(tex, render_cube_radius(c->p.max_r), c->p.max_r + 1, 2, nx, deul, dpar, B, c->p.apix,
                      ctf ? c->p.vol : -1.0f, c->p.cs, c->p.ampwg, host_angles().deg2rad, ft, c->stream);
     cufftHandle h;
     int r;
@@ -1534,7 +1534,7 @@ struct CubeTexture {
 // 2 (maxR + 1) + 1 of the padded grid (maxR + 1 of the map's, twice oversampled), as a
 // texture.
 int render_cube(Ctx* c, const float* map3d, CubeTexture* ct) {
-    const int n = c->p.fftsize, m = 2 * n, Rc = 2 * c->p.max_r + 3;
+    const int n = c->p.fftsize, m = 2 * n, Rc = render_cube_radius(c->p.max_r);
     const long m3 = (long)m * m * m, c3 = (long)(2 * Rc + 3) * (2 * Rc + 3) * (2 * Rc + 3);
     DBuf<float> dmap;
     DBuf<float2> work, cube;

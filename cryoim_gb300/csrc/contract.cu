@@ -71,13 +71,13 @@ __global__ void k_map_checker(const float* __restrict__ map, int nx, float2* __r
 // Band cube of the transform: frequencies -(R+1) .. R+1 per axis, phase referenced to
 // the map centre ((-1)^(kx+ky+kz)), standard complex convention, scaled by 1/nx^3.
 __global__ void k_map_band(const float2* __restrict__ ft, int nx, int R, float2* __restrict__ cube) {
-    const int C = 2 * R + 3, h = nx / 2;
+    const int C = 2 * R + 3;
     const long total = (long)C * C * C;
     const float s = 1.0f / ((float)nx * (float)nx * (float)nx);
     for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (long)gridDim.x * blockDim.x) {
         int x = (int)(q % C), y = (int)((q / C) % C), z = (int)(q / ((long)C * C));
         int kx = x - (R + 1), ky = y - (R + 1), kz = z - (R + 1);
-        float2 v = ft[((long)(kz + h) * nx + (ky + h)) * nx + (kx + h)];
+        float2 v = ft[((long)freq_index(kz, nx) * nx + freq_index(ky, nx)) * nx + freq_index(kx, nx)];
         float sg = ((kx + ky + kz) & 1) ? -s : s;
         cube[q] = make_float2(v.x * sg, v.y * sg);
     }

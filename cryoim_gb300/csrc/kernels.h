@@ -28,6 +28,12 @@ inline Band make_band(int nx, int min_r, int max_r) {
     b.AW = 2 * max_r + 3;
     return b;
 }
+// index along an axis of frequency k of a centred nx-point transform; +nx/2 is -nx/2 (a cube of
+// frequencies with a margin of cells can reach it)
+__host__ __device__ inline int freq_index(int k, int nx) { return k < nx / 2 ? k + nx / 2 : k - nx / 2; }
+// radius of the band cube of the renderer, cut from the transform of the map padded to twice its side:
+// maxR + 1 of the map's frequencies; the cube has one cell more on each side (k_map_band)
+inline int render_cube_radius(int max_r) { return 2 * max_r + 3; }
 // outer radius of the coarse level's band: half of the band's, at least two radii where the band has
 // them, and within it (the window, the ramps' table and the map's cube end there)
 inline int coarse_radius(int min_r, int max_r) {

@@ -10,9 +10,13 @@
 //               of the centred 3D Fourier map, project2d_FT3dTo2d.f90:30-83)
 // Stacking (Re, Im) along K turns it into one real contraction
 //     C[(p,s), R] = sum_k A[(p,s), k] B[R, k],   K = 2 x samples,
-// which gemm_tc.cu runs on the tensor cores in BF16 with FP32 accumulation.  The
-// normalisation sums are FP64; the best candidates are rescored in FP64 here and with
-// the reference's phase residual (k_pr_single) by the driver.
+// which gemm_tc.cu runs on the tensor cores in BF16 or e4m3 with FP32 accumulation.  The local form
+// contracts it so, a row of A per origin.  The global forms' rows of A are the particle under a
+// basis of its origin grid (origin_basis.h), whose products the k_up_* kernels here expand to all
+// origins in FP32, and where the grid's omegas pair up half a turn apart B holds the first of each
+// pair: the two halves of K are contracted apart and summed or subtracted.  The normalisation sums
+// are FP64; the best candidates are rescored in FP64 here and with the reference's phase residual
+// by the driver.
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
